@@ -134,18 +134,46 @@ constexpr int64_t kScanTile = (int64_t)kScanThreads * kScanPer;
 
 inline size_t scan_tmp_bytes(size_t n) { return ((n + kScanTile - 1) / kScanTile + 1) * 8; }
 
-__global__ void k_scan_reduce(const int64_t* __restrict__ x, int64_t n, int64_t* __restrict__ part) {
-  const int64_t base = (int64_t)blockIdx.x * kScanTile;
-  uint64_t s = 0;
-  for (int j = 0; j < kScanPer; ++j) {
-    const int64_t i = base + (int64_t)j * kScanThreads + threadIdx.x;
-    if (i < n) s += (uint64_t)x[i];
+// T: int64_t or uint32_t (sums wrap).  A warp takes 256 consecutive elements in rounds
+// of one 16-byte vector per lane, so every access is coalesced (eight consecutive
+// elements per thread touched each sector in eight separate loads).  x is 16-byte aligned.
+template <typename T>
+struct ScanItems {
+  static constexpr int V = 16 / sizeof(T), R = kScanPer / V;
+  alignas(16) T v[R][V];
+  __device__ __forceinline__ static int64_t at(int r) {
+    return (int64_t)blockIdx.x * kScanTile + (int64_t)(threadIdx.x >> 5) * (32 * kScanPer) +
+           (int64_t)r * (32 * V) + (int64_t)(threadIdx.x & 31) * V;
   }
+  __device__ __forceinline__ void load(const T* __restrict__ x, int64_t n) {
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const int64_t i = at(r);
+      if (i + V <= n) {
+        *reinterpret_cast<uint4*>(v[r]) = *reinterpret_cast<const uint4*>(x + i);
+      } else {
+#pragma unroll
+        for (int j = 0; j < V; ++j) v[r][j] = i + j < n ? x[i + j] : (T)0;
+      }
+    }
+  }
+};
+template <typename T>
+__global__ void __launch_bounds__(kScanThreads) k_scan_reduce(const T* __restrict__ x, int64_t n,
+                                                              T* __restrict__ part) {
+  ScanItems<T> it;
+  it.load(x, n);
+  uint64_t s = 0;
+#pragma unroll
+  for (int r = 0; r < it.R; ++r)
+#pragma unroll
+    for (int j = 0; j < it.V; ++j) s += (uint64_t)it.v[r][j];
   uint64_t total = 0;
   block_exclusive_scan<uint64_t>(s, &total);
-  if (threadIdx.x == 0) part[blockIdx.x] = (int64_t)total;
+  if (threadIdx.x == 0) part[blockIdx.x] = (T)total;
 }
-__global__ void k_scan_parts(int64_t* part, int64_t np) {
+template <typename T>
+__global__ void k_scan_parts(T* part, int64_t np) {
   // single CTA: exclusive scan of the tile totals in place
   uint64_t carry = 0;
   for (int64_t c0 = 0; c0 < np; c0 += blockDim.x) {
@@ -153,38 +181,70 @@ __global__ void k_scan_parts(int64_t* part, int64_t np) {
     const uint64_t v = i < np ? (uint64_t)part[i] : 0;
     uint64_t total = 0;
     const uint64_t ex = block_exclusive_scan<uint64_t>(v, &total);
-    if (i < np) part[i] = (int64_t)(carry + ex);
+    if (i < np) part[i] = (T)(carry + ex);
     carry += total;
   }
 }
-__global__ void k_scan_apply(int64_t* __restrict__ x, int64_t n, const int64_t* __restrict__ part) {
-  const int64_t base = (int64_t)blockIdx.x * kScanTile + (int64_t)threadIdx.x * kScanPer;
-  uint64_t v[kScanPer];
-  uint64_t s = 0;
+template <typename T>
+__global__ void __launch_bounds__(kScanThreads) k_scan_apply(T* __restrict__ x, int64_t n,
+                                                             const T* __restrict__ part) {
+  __shared__ uint64_t s_warp[kScanThreads / 32];
+  using I = ScanItems<T>;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  I it;
+  it.load(x, n);
+  uint64_t before[I::R], run = 0;   // sum of the warp's elements before this lane's vector of round r
 #pragma unroll
-  for (int j = 0; j < kScanPer; ++j) {
-    const int64_t i = base + j;
-    v[j] = i < n ? (uint64_t)x[i] : 0;
-    s += v[j];
+  for (int r = 0; r < I::R; ++r) {
+    uint64_t s = 0;
+#pragma unroll
+    for (int j = 0; j < I::V; ++j) s += (uint64_t)it.v[r][j];
+    uint64_t incl = s;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint64_t y = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += y;
+    }
+    before[r] = run + incl - s;
+    run += __shfl_sync(0xffffffffu, incl, 31);
   }
-  uint64_t run = block_exclusive_scan<uint64_t>(s) + (uint64_t)part[blockIdx.x];
+  if (lane == 0) s_warp[warp] = run;
+  __syncthreads();
+  uint64_t base = (uint64_t)part[blockIdx.x];
+  for (int w = 0; w < warp; ++w) base += s_warp[w];
 #pragma unroll
-  for (int j = 0; j < kScanPer; ++j) {
-    const int64_t i = base + j;
-    run += v[j];
-    if (i < n) x[i] = (int64_t)run;
+  for (int r = 0; r < I::R; ++r) {
+    uint64_t acc = base + before[r];
+#pragma unroll
+    for (int j = 0; j < I::V; ++j) {
+      acc += (uint64_t)it.v[r][j];
+      it.v[r][j] = (T)acc;
+    }
+    const int64_t i = I::at(r);
+    if (i + I::V <= n) {
+      *reinterpret_cast<uint4*>(x + i) = *reinterpret_cast<const uint4*>(it.v[r]);
+    } else {
+#pragma unroll
+      for (int j = 0; j < I::V; ++j)
+        if (i + j < n) x[i + j] = it.v[r][j];
+    }
   }
 }
 
-// Inclusive scan of x[0..n) in place (three launches, counted into `kernels`).
-inline int device_inclusive_scan_i64(int64_t* x, int64_t n, int64_t* tmp, cudaStream_t st, int& kernels) {
+// Inclusive scan of x[0..n) in place (three launches, counted into `kernels`); tmp
+// holds scan_tmp_bytes(n).
+template <typename T>
+inline int device_inclusive_scan(T* x, int64_t n, void* tmp, cudaStream_t st, int& kernels) {
   if (n <= 0) return 0;
   const int64_t np = (n + kScanTile - 1) / kScanTile;
-  k_scan_reduce<<<(unsigned)np, kScanThreads, 0, st>>>(x, n, tmp);
-  k_scan_parts<<<1, 1024, 0, st>>>(tmp, np);
-  k_scan_apply<<<(unsigned)np, kScanThreads, 0, st>>>(x, n, tmp);
+  k_scan_reduce<T><<<(unsigned)np, kScanThreads, 0, st>>>(x, n, static_cast<T*>(tmp));
+  k_scan_parts<T><<<1, 1024, 0, st>>>(static_cast<T*>(tmp), np);
+  k_scan_apply<T><<<(unsigned)np, kScanThreads, 0, st>>>(x, n, static_cast<const T*>(tmp));
   kernels += 3;
   return (int)cudaGetLastError();
+}
+inline int device_inclusive_scan_i64(int64_t* x, int64_t n, int64_t* tmp, cudaStream_t st, int& kernels) {
+  return device_inclusive_scan<int64_t>(x, n, tmp, st, kernels);
 }
 
 }  // namespace

@@ -1,0 +1,42 @@
+// bw_keyblock.cuh -- one-tree replay over large key domains (bw_keyblock.cu).
+#pragma once
+#include <cuda_runtime.h>
+#include <cstdint>
+
+#include "bw_gpu.h"
+#include "bw_pipeline.cuh"
+
+namespace bw {
+
+constexpr int kKbMaxBlocks = 4096;            // key blocks (partition digits held in shared memory)
+constexpr int kKbSlotStep = 512;              // slots per block: a multiple of 16 warps x 32 lanes ...
+constexpr int kKbMaxSlots = 20 * kKbSlotStep; // ... and at most 10,240 (80 KB of int64, two CTAs per SM)
+constexpr int kKbPtTile = 4096;               // points per partition tile
+constexpr int kKbPrTile = 4096;               // queries per partition tile (two probes each)
+constexpr uint32_t kKbMinKeys = 1u << kWinBits;   // smaller domains stay with the state-block pipeline
+
+enum {
+  KB_SOFF, KB_TEOFF, KB_TQOFF, KB_TC, KB_TBOFF, KB_TBITS, KB_TCARRY, KB_TGSUM, KB_LASTQ, KB_MISC, KB_EOFF, KB_QOFF,
+  KB_FORK, KB_NEXT, KB_CNT, KB_EHEAD, KB_XHEAD, KB_RANK, KB_SCAN, KB_STEP, KB_W, KB_EP, KB_TIME, KB_COLSTATE,
+  KB_COLTIME, KB_COLSTEP, KB_POS, KB_PTHIST, KB_PTS, KB_SEG, KB_ROWS, KB_PRHIST, KB_PRS, KB_ACC, KB_COUNT
+};
+
+struct KbSpec {
+  int32_t S = 0;
+  uint32_t C = 0;
+  int64_t E = 0, Q = 0;
+  int32_t m = 0;           // event slots per key block
+  int32_t B = 0;           // key blocks
+  int32_t segs = 0;        // tour segments of the row pass
+  int64_t pt_tiles = 0, pr_tiles = 0;
+  size_t off[KB_COUNT];
+  size_t total = 0;
+};
+
+// Whether a replay that would take the general pipeline (spec `s`, workspace
+// `general_bytes`) is replayed by key blocks instead; fills `k` when it is.
+bool kb_select(const BwReplayArgs* a, const PipeSpec& s, size_t general_bytes, KbSpec& k);
+int kb_enqueue(const KbSpec& k, const PipeSpec& s, const BwReplayArgs* a, EventSet* timing, int* kernels);
+const int32_t* kb_status_word(const KbSpec& k, const void* workspace);
+
+}  // namespace bw

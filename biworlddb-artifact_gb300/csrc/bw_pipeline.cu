@@ -2305,6 +2305,54 @@ int pipe_bind(const PipeSpec& s, void* workspace, cudaStream_t st) {
   return report(cudaStreamSynchronize(st), "table upload sync");
 }
 
+// Stages 0 to 2 up to the ranked segments (shared with the key-block replay).
+int pipe_tour(const PipeSpec& s, bool forest, const TourArrays& w, const int32_t* parent, const BwEvent* events,
+              const BwQuery* queries, cudaStream_t st, EventSet* timing, int& kernels) {
+  const int32_t S = s.S, T = s.T;
+  const int grid = s.sms * 8;
+  int rc = 0;
+  int32_t* status = w.misc + M_STATUS;
+  auto chk = [&](const char* what) { ++kernels; return report(cudaGetLastError(), what); };
+  auto mark = [&](int i) { return timing ? report(cudaEventRecord(timing->ev[i], st), "event record") : 0; };
+  // ---- 0/1. init + ingest
+  k_init<<<(std::max(T, 16) + 255) / 256, 256, 0, st>>>(w.misc, w.tt, T, forest ? 0 : 1, S, s.E, s.Q, s.Cmax, s.nb1);
+  if ((rc = chk("k_init"))) return rc;
+  if (s.E > 0) {
+    k_offsets<true><<<grid, 256, 0, st>>>(events, s.E, w.tt, T, S, w.eoff, status);
+    if ((rc = chk("k_offsets(events)"))) return rc;
+  } else {
+    k_fill_i64<<<grid, 256, 0, st>>>(w.eoff, (int64_t)S + 1, 0);
+    if ((rc = chk("k_fill(eoff)"))) return rc;
+  }
+  if (s.Q > 0) {
+    k_offsets<false><<<grid, 256, 0, st>>>(queries, s.Q, w.tt, T, S, w.qoff, status);
+    if ((rc = chk("k_offsets(queries)"))) return rc;
+  } else {
+    k_fill_i64<<<grid, 256, 0, st>>>(w.qoff, (int64_t)S + 1, 0);
+    if ((rc = chk("k_fill(qoff)"))) return rc;
+  }
+
+  if ((rc = mark(1))) return rc;
+  // ---- 2. linearise
+  if ((rc = report(cudaMemsetAsync(w.fork_head, 0xFF, (size_t)S * 4, st), "memset"))) return rc;
+  k_lin_children<<<grid, 256, 0, st>>>(parent, S, w.tt, T, w.gpar, w.fork_head, w.next_sib, s.chain_hint ? 1 : 0, status);
+  if ((rc = chk("k_lin_children"))) return rc;
+  const int32_t* gp = w.gpar ? w.gpar : parent;   // one tree: global = local ids
+  k_lin_flags<<<grid, 256, 0, st>>>(gp, w.fork_head, S, w.cnt, status);
+  if ((rc = chk("k_lin_flags"))) return rc;
+  if ((rc = device_inclusive_scan_i64(w.cnt, S, w.scan_tmp, st, kernels))) return report((cudaError_t)rc, "scan");
+  k_lin_heads<<<grid, 256, 0, st>>>(w.cnt, S, w.ehead, w.xhead, status);
+  if ((rc = chk("k_lin_heads"))) return rc;
+  k_lin_rank_init<<<grid, 256, 0, st>>>(w.cnt, w.ehead, w.xhead, gp, w.fork_head, w.next_sib, S, w.rank, status);
+  if ((rc = chk("k_lin_rank_init"))) return rc;
+  int32_t round = 0;
+  for (int64_t span = 1; span < 2 * (int64_t)s.Smax; span <<= 1, ++round) {
+    k_lin_round<<<grid, 256, 0, st>>>(w.rank, w.cnt, S, w.misc + M_ROUNDS, round, status);
+    if ((rc = chk("k_lin_round"))) return rc;
+  }
+  return 0;
+}
+
 int pipe_enqueue(const PipeSpec& s, void* workspace, const int32_t* parent, const BwEvent* events,
                  const BwQuery* queries, int64_t* answers, cudaStream_t st, EventSet* timing, int* kernels_out) {
   // both sweeps stage events with 16-byte copies (cp.async, cp.async.bulk)
@@ -2348,42 +2396,10 @@ int pipe_enqueue(const PipeSpec& s, void* workspace, const int32_t* parent, cons
   if (timing) timing->chain = 0;
   if ((rc = mark(0))) return rc;
 
-  // ---- 0/1. init + ingest
-  k_init<<<(std::max(T, 16) + 255) / 256, 256, 0, st>>>(misc, tt, T, forest ? 0 : 1, S, s.E, s.Q, s.Cmax, s.nb1);
-  if ((rc = chk("k_init"))) return rc;
-  if (s.E > 0) {
-    k_offsets<true><<<grid, 256, 0, st>>>(events, s.E, tt, T, S, eoff, status);
-    if ((rc = chk("k_offsets(events)"))) return rc;
-  } else {
-    k_fill_i64<<<grid, 256, 0, st>>>(eoff, (int64_t)S + 1, 0);
-    if ((rc = chk("k_fill(eoff)"))) return rc;
-  }
-  if (s.Q > 0) {
-    k_offsets<false><<<grid, 256, 0, st>>>(queries, s.Q, tt, T, S, qoff, status);
-    if ((rc = chk("k_offsets(queries)"))) return rc;
-  } else {
-    k_fill_i64<<<grid, 256, 0, st>>>(qoff, (int64_t)S + 1, 0);
-    if ((rc = chk("k_fill(qoff)"))) return rc;
-  }
-
-  if ((rc = mark(1))) return rc;
-  // ---- 2. linearise
-  if ((rc = report(cudaMemsetAsync(fork_head, 0xFF, (size_t)S * 4, st), "memset"))) return rc;
-  k_lin_children<<<grid, 256, 0, st>>>(parent, S, tt, T, gpar, fork_head, next_sib, s.chain_hint ? 1 : 0, status);
-  if ((rc = chk("k_lin_children"))) return rc;
-  const int32_t* gp = gpar ? gpar : parent;   // one tree: global = local ids
-  k_lin_flags<<<grid, 256, 0, st>>>(gp, fork_head, S, cnt, status);
-  if ((rc = chk("k_lin_flags"))) return rc;
-  if ((rc = device_inclusive_scan_i64(cnt, S, scan_tmp, st, kernels))) return report((cudaError_t)rc, "scan");
-  k_lin_heads<<<grid, 256, 0, st>>>(cnt, S, ehead, xhead, status);
-  if ((rc = chk("k_lin_heads"))) return rc;
-  k_lin_rank_init<<<grid, 256, 0, st>>>(cnt, ehead, xhead, gp, fork_head, next_sib, S, rank_a, status);
-  if ((rc = chk("k_lin_rank_init"))) return rc;
-  int32_t round = 0;
-  for (int64_t span = 1; span < 2 * (int64_t)s.Smax; span <<= 1, ++round) {
-    k_lin_round<<<grid, 256, 0, st>>>(rank_a, cnt, S, misc + M_ROUNDS, round, status);
-    if ((rc = chk("k_lin_round"))) return rc;
-  }
+  TourArrays ta;
+  ta.tt = tt; ta.misc = misc; ta.eoff = eoff; ta.qoff = qoff; ta.gpar = gpar; ta.fork_head = fork_head;
+  ta.next_sib = next_sib; ta.cnt = cnt; ta.ehead = ehead; ta.xhead = xhead; ta.rank = rank_a; ta.scan_tmp = scan_tmp;
+  if ((rc = pipe_tour(s, forest, ta, parent, events, queries, st, timing, kernels))) return rc;
   const uint64_t* src = rank_a;
   k_lin_steps<<<grid, 256, 0, st>>>(src, cnt, ehead, xhead, S, tt, T, eoff, qoff, partner, desc, work, status);
   if ((rc = chk("k_lin_steps"))) return rc;

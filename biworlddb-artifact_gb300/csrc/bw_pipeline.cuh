@@ -251,6 +251,22 @@ int pipe_bind(const PipeSpec& spec, void* workspace, cudaStream_t st);
 // Enqueue the whole pipeline (kernels and memsets only: capturable in a CUDA graph).
 int pipe_enqueue(const PipeSpec& spec, void* workspace, const int32_t* parent, const BwEvent* events,
                  const BwQuery* queries, int64_t* answers, cudaStream_t st, EventSet* timing, int* kernels);
+// Arrays of the ingest and linearise stages; `rank` holds (next, distance to the end of
+// the tour) per segment once pipe_tour's kernels have run.
+struct TourArrays {
+  TreeTabs tt;
+  int32_t* misc;
+  int64_t *eoff, *qoff;      // S + 1 each
+  int32_t* gpar;             // forests: global parents (one tree: NULL)
+  int32_t *fork_head, *next_sib;
+  int64_t* cnt;
+  int32_t *ehead, *xhead;
+  uint64_t* rank;            // 2 S
+  int64_t* scan_tmp;
+};
+int pipe_tour(const PipeSpec& spec, bool forest, const TourArrays& w, const int32_t* parent, const BwEvent* events,
+              const BwQuery* queries, cudaStream_t st, EventSet* timing, int& kernels);
+
 // Euler-tile sweep (bw_esweep.cu): the inputs of k_sweep, the rank capacities the
 // prepare pass cut the slices with, events as 16-byte records (16-byte aligned).
 struct EsParams {

@@ -14,6 +14,7 @@
 #include "bw_common.cuh"
 #include "bw_pipeline.cuh"
 #include "bw_chain.cuh"
+#include "bw_keyblock.cuh"
 
 namespace bw {
 namespace {
@@ -56,6 +57,29 @@ int chain_spec_of(const BwReplayArgs* a, ChainSpec& s) {
   return chain_spec(a, sms, s);
 }
 
+// The path a replay takes, with its plan and workspace.
+struct Route {
+  bool chain = false, kb = false;
+  ChainSpec cs;
+  PipeSpec s;
+  KbSpec k;
+  size_t need = 0;
+};
+int route_of(const BwReplayArgs* a, Route& r) {
+  r.chain = chain_selected(a);
+  int rc = r.chain ? chain_spec_of(a, r.cs) : spec_of(a, r.s);
+  if (rc) return rc;
+  if (r.chain) {
+    r.need = r.cs.total;
+    return 0;
+  }
+  Layout L;
+  pipe_layout(r.s, L);
+  r.kb = kb_select(a, r.s, L.total, r.k);
+  r.need = r.kb ? r.k.total : L.total;
+  return 0;
+}
+
 }  // namespace
 }  // namespace bw
 
@@ -63,20 +87,10 @@ using namespace bw;
 
 extern "C" int bw_replay_workspace_size(const BwReplayArgs* a, size_t* bytes) {
   if (validate_args(a) || !bytes) return BW_EINVAL;
-  if (chain_selected(a)) {
-    ChainSpec cs;
-    int rc = chain_spec_of(a, cs);
-    if (rc) return rc;
-    *bytes = cs.total;
-    return 0;
-  }
-  PipeSpec s;
-  int rc = spec_of(a, s);
-  if (rc) return rc;
-  Layout L;
-  pipe_layout(s, L);
-  *bytes = L.total;
-  return 0;
+  Route r;
+  const int rc = route_of(a, r);
+  if (!rc) *bytes = r.need;
+  return rc;
 }
 
 extern "C" int bw_replay_launch(const BwReplayArgs* a) {
@@ -84,19 +98,11 @@ extern "C" int bw_replay_launch(const BwReplayArgs* a) {
       (a->n_queries && (!a->queries || !a->answers)))
     return BW_EINVAL;
   if ((reinterpret_cast<uintptr_t>(a->workspace) & 255) != 0) return BW_EINVAL;
-  const bool chain = chain_selected(a);
-  PipeSpec s;
-  ChainSpec cs;
-  int rc = chain ? chain_spec_of(a, cs) : spec_of(a, s);
+  Route r;
+  int rc = route_of(a, r);
   if (rc) return rc;
-  size_t need = cs.total;
-  if (!chain) {
-    Layout L;
-    pipe_layout(s, L);
-    need = L.total;
-  }
-  if (a->workspace_bytes < need) {
-    std::fprintf(stderr, "bw_replay: workspace %zu < required %zu bytes\n", a->workspace_bytes, need);
+  if (a->workspace_bytes < r.need) {
+    std::fprintf(stderr, "bw_replay: workspace %zu < required %zu bytes\n", a->workspace_bytes, r.need);
     return BW_EINVAL;
   }
   EventSet* evs = nullptr;
@@ -110,14 +116,15 @@ extern "C" int bw_replay_launch(const BwReplayArgs* a) {
     evs = &g_sets[g_sets_used++];
   }
   int kernels = 0;
-  rc = chain ? chain_enqueue(cs, a, evs, &kernels)
-             : pipe_enqueue(s, a->workspace, a->parent, a->events, a->queries, a->answers,
-                            static_cast<cudaStream_t>(a->stream), evs, &kernels);
+  rc = r.chain ? chain_enqueue(r.cs, a, evs, &kernels)
+       : r.kb  ? kb_enqueue(r.k, r.s, a, evs, &kernels)
+               : pipe_enqueue(r.s, a->workspace, a->parent, a->events, a->queries, a->answers,
+                              static_cast<cudaStream_t>(a->stream), evs, &kernels);
   if (rc) return rc;
   std::lock_guard<std::mutex> g(g_info_mu);
   g_last.kernels = kernels;
-  g_last.blocks = chain ? cs.B : s.B;
-  g_last.chain = chain ? 1 : 0;
+  g_last.blocks = r.chain ? r.cs.B : r.kb ? r.k.B : r.s.B;
+  g_last.chain = r.chain ? 1 : 0;
   return 0;
 }
 
@@ -153,13 +160,12 @@ extern "C" int bw_replay_stage_times(float* ms, int32_t* launches) {
 
 extern "C" int bw_replay_status(const BwReplayArgs* a, int32_t* status) {
   if (validate_args(a) || !a->workspace || !status) return BW_EINVAL;
-  const int32_t* word = chain_status_word(a->workspace);
-  if (!chain_selected(a)) {
-    PipeSpec s;
-    int rc = spec_of(a, s);
-    if (rc) return rc;
-    word = pipe_status_word(s, a->workspace);
-  }
+  Route r;
+  const int rc = route_of(a, r);
+  if (rc) return rc;
+  const int32_t* word = r.chain ? chain_status_word(a->workspace)
+                        : r.kb  ? kb_status_word(r.k, a->workspace)
+                                : pipe_status_word(r.s, a->workspace);
   cudaStream_t st = static_cast<cudaStream_t>(a->stream);
   int32_t v = 0;
   cudaError_t e = cudaMemcpyAsync(&v, word, 4, cudaMemcpyDeviceToHost, st);
