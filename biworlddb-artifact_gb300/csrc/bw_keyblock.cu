@@ -28,8 +28,9 @@
 //   sweep     k_kb_sweep   one CTA per key block: L of every probe (below).
 //   answers   k_kb_answers  acc, kept in tour order, to the queries' own places.
 //
-// Measured on 20M events over 10M keys, 100k states, 100M range queries (the
-// versioned sparse-key workload): see k_kb_sweep and kb_select.
+// Measured on 20M events over 10M keys, 100k states and 100M range queries: 16.5 ms
+// (sweep 6.9, probe scatter 4.2, rows 1.2, probe count 1.1, points 1.3) against 624 ms
+// on the state-block pipeline.
 #include <cuda_runtime.h>
 #include <algorithm>
 #include <cstdint>
@@ -63,17 +64,18 @@ struct KbParams {
   uint32_t* coltime;    //   the queries before it (and after the last column: all),
   int32_t* colstep;     //   and its enter step
   uint32_t* pos;        // C + 1
-  uint32_t* pthist;
-  uint4* pts;           // {time, slot, delta}
+  uint4* tour;          // 2E: the points in tour order, {time, pos, delta}
+  uint32_t *pthist, *ptoff;   // tiles x B digit counts (then starts), B + 1 block starts
+  uint4* pts;           // the swept points by key block, {time, slot, delta}
   uint64_t* seg;        // segs x B
-  int64_t* rows;        // columns x B
-  uint32_t* prhist;
+  int64_t* rows;        // columns x Bs
+  uint32_t *prhist, *proff;
   uint2* prs;           // {query in tour order, slot | lower bound << 31}
   unsigned long long* acc;   // per query in tour order
   const int32_t* status;
   int32_t* ticket;
   int64_t E, Q, pt_tiles, pr_tiles;
-  int32_t S, B, segs;
+  int32_t S, B, Bs, segs;   // Bs: B rounded up to whole 32-byte sectors of a row
   uint32_t C, m;
 };
 
@@ -159,18 +161,6 @@ __device__ __forceinline__ int32_t kb_find_col(const uint32_t* coltime, int32_t 
   return lo;
 }
 
-// Point j of the tour: event of step t, negated on an exit.
-struct KbPoint {
-  uint32_t time, key;
-  uint64_t delta;
-};
-__device__ __forceinline__ KbPoint kb_point(const KbParams& p, int32_t t, int64_t j) {
-  const int32_t v = p.step[t], s = v < 0 ? ~v : v;
-  const uint4 e = __ldg(reinterpret_cast<const uint4*>(p.ev) + (p.eoff[s + 1] - (p.ep[t] - j)));
-  const uint64_t d = ((uint64_t)e.w << 32) | e.z;
-  return KbPoint{p.time[t], e.y, v < 0 ? (uint64_t)0 - d : d};
-}
-
 // Step range [s_t[0], s_t[1]] holding the points [j0, j1), j0 < j1 (whole CTA).
 __device__ __forceinline__ void kb_step_range(const KbParams& p, int64_t j0, int64_t j1, int32_t* s_t) {
   if (threadIdx.x < 2) s_t[threadIdx.x] = kb_find_step(p.ep, 0, 2 * p.S - 1, threadIdx.x ? j1 - 1 : j0);
@@ -182,52 +172,79 @@ __device__ __forceinline__ void kb_col_range(const KbParams& p, int64_t j0, int6
   __syncthreads();
 }
 
+// ------------------------------------------------------------------ digit starts
+// hist[tile][d] = items of digit d in the tile -> output position of the first of them
+// (all items of smaller digits, then those of earlier tiles), off[d] = start of the
+// digit, off[B] = all items.  Column sums and column prefixes over chunks of tiles, so
+// that every access runs along the digits (a digit-major matrix cost a sector per count).
+constexpr int kStartChunks = 64;
+__device__ __forceinline__ void kb_chunk(int64_t tiles, int64_t& t0, int64_t& t1) {
+  t0 = tiles * blockIdx.y / kStartChunks;
+  t1 = tiles * (blockIdx.y + 1) / kStartChunks;
+}
+__global__ void __launch_bounds__(128) k_kb_start_sum(const uint32_t* __restrict__ hist, int32_t B, int64_t tiles,
+                                                      uint32_t* __restrict__ part, const int32_t* status) {
+  const int32_t d = blockIdx.x * 128 + threadIdx.x;
+  if (*status || d >= B) return;
+  int64_t t0, t1;
+  kb_chunk(tiles, t0, t1);
+  uint32_t s = 0;
+#pragma unroll 8
+  for (int64_t t = t0; t < t1; ++t) s += hist[t * B + d];
+  part[(int64_t)blockIdx.y * B + d] = s;
+}
+__global__ void __launch_bounds__(1024) k_kb_start_scan(uint32_t* part, int32_t B, uint32_t* off,
+                                                        const int32_t* status) {
+  if (*status) return;
+  uint32_t carry = 0;
+  for (int32_t d0 = 0; d0 < B; d0 += 1024) {
+    const int32_t d = d0 + threadIdx.x;
+    uint32_t n = 0, total = 0;
+    if (d < B) {
+#pragma unroll 8
+      for (int c = 0; c < kStartChunks; ++c) n += part[(int64_t)c * B + d];
+    }
+    uint32_t run = carry + block_exclusive_scan<uint32_t>(n, &total);
+    if (d < B) {
+      off[d] = run;
+#pragma unroll 8
+      for (int c = 0; c < kStartChunks; ++c) {
+        const uint32_t x = part[(int64_t)c * B + d];
+        part[(int64_t)c * B + d] = run;
+        run += x;
+      }
+    }
+    carry += total;
+  }
+  if (threadIdx.x == 0) off[B] = carry;
+}
+__global__ void __launch_bounds__(128) k_kb_start_apply(uint32_t* __restrict__ hist, int32_t B, int64_t tiles,
+                                                        const uint32_t* __restrict__ part, const int32_t* status) {
+  const int32_t d = blockIdx.x * 128 + threadIdx.x;
+  if (*status || d >= B) return;
+  int64_t t0, t1;
+  kb_chunk(tiles, t0, t1);
+  uint32_t run = part[(int64_t)blockIdx.y * B + d];
+  for (int64_t t = t0; t < t1; t += 16) {   // in place: a batch is loaded before it is written
+    uint32_t x[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) x[i] = t + i < t1 ? hist[(t + i) * B + d] : 0u;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      if (t + i < t1) hist[(t + i) * B + d] = run;
+      run += x[i];
+    }
+  }
+}
+
+// ------------------------------------------------------------------ points
 // An event of the last key of its key block lies below no probe of the block: it
 // counts in the rows only (which also keeps a hot key out of the sweep).
 __device__ __forceinline__ bool kb_swept(const KbParams& p, uint32_t key, uint32_t b) { return p.pos[key + 1] / p.m == b; }
+constexpr uint32_t kRowsOnly = 0x80000000u;   // in a tour point's pos (positions stay below 2^31)
 
-// Stable rank of a warp's ITEMS x 32 digits (kNone: no item) within the warp; wc: the
-// warp's counters, zeroed.  r[j] = earlier items of the warp with the same digit.
-template <int ITEMS>
-__device__ __forceinline__ void kb_rank(uint16_t* wc, const uint32_t (&d)[ITEMS], uint16_t (&r)[ITEMS]) {
-  const unsigned lt = (1u << (threadIdx.x & 31)) - 1u;
-#pragma unroll
-  for (int j = 0; j < ITEMS; ++j) {
-    const unsigned peers = __match_any_sync(kAll, d[j]);
-    const uint32_t old = d[j] != kNone ? wc[d[j]] : 0u;
-    __syncwarp();
-    r[j] = (uint16_t)(old + __popc(peers & lt));
-    if (d[j] != kNone && (peers & lt) == 0) wc[d[j]] = (uint16_t)(old + __popc(peers));
-    __syncwarp();
-  }
-}
-// Counters of the CTA's NW warps -> output position of each warp's first item per digit.
-template <int NW>
-__device__ __forceinline__ void kb_bases(uint16_t* wc, uint32_t* base, int32_t B, int32_t Bp, const uint32_t* hist,
-                                         int64_t ntiles) {
-  __syncthreads();
-  for (int32_t d = threadIdx.x; d < B; d += NW * 32) {
-    uint32_t run = 0;
-#pragma unroll
-    for (int w = 0; w < NW; ++w) {
-      const uint32_t c = wc[w * Bp + d];
-      wc[w * Bp + d] = (uint16_t)run;
-      run += c;
-    }
-    base[d] = hist[(int64_t)d * ntiles + blockIdx.x] - run;   // inclusive counts
-  }
-  __syncthreads();
-}
-__device__ __forceinline__ void kb_write_hist(const uint32_t* h, int32_t B, uint32_t* hist, int64_t ntiles) {
-  __syncthreads();
-  for (int32_t d = threadIdx.x; d < B; d += blockDim.x) hist[(int64_t)d * ntiles + blockIdx.x] = h[d];
-}
-
-constexpr int kPtWarps = 16, kPtItems = kKbPtTile / (kPtWarps * 32);
-constexpr int kPrWarps = 16, kPrItems = 2 * kKbPrTile / (kPrWarps * 32);
-inline size_t kb_scatter_smem(int32_t B, int warps) { return (size_t)B * 4 + (size_t)warps * ((B + 7) & ~7) * 2 + 16; }
-
-__global__ void __launch_bounds__(kPtWarps * 32) k_kb_point_count(KbParams p) {
+// The points of a tile, written out in tour order, and the swept ones counted by block.
+__global__ void __launch_bounds__(256) k_kb_points(KbParams p) {
   if (*p.status) return;
   extern __shared__ __align__(16) uint32_t h[];
   __shared__ int32_t s_t[2];
@@ -236,58 +253,98 @@ __global__ void __launch_bounds__(kPtWarps * 32) k_kb_point_count(KbParams p) {
   const int64_t j0 = (int64_t)blockIdx.x * kKbPtTile, j1 = imin64(j0 + kKbPtTile, kb_points(p));
   if (j0 < j1) {
     kb_step_range(p, j0, j1, s_t);
-    for (int64_t j = j0 + threadIdx.x; j < j1; j += blockDim.x) {
-      const int32_t t = kb_find_step(p.ep, s_t[0], s_t[1], j);
-      const KbPoint x = kb_point(p, t, j);
-      const uint32_t b = p.pos[x.key] / p.m;
-      if (kb_swept(p, x.key, b)) atomicAdd(h + b, 1u);
+    const int32_t ta = s_t[0], tz = s_t[1];
+#pragma unroll 4
+    for (int64_t j = j0 + threadIdx.x; j < j1; j += 256) {
+      const int32_t t = kb_find_step(p.ep, ta, tz, j);
+      const int32_t v = p.step[t], s = v < 0 ? ~v : v;
+      const uint4 e = __ldg(reinterpret_cast<const uint4*>(p.ev) + (p.eoff[s + 1] - (p.ep[t] - j)));
+      const uint64_t d = ((uint64_t)e.w << 32) | e.z, sd = v < 0 ? (uint64_t)0 - d : d;
+      const uint32_t ps = p.pos[e.y], b = ps / p.m;
+      const bool swept = kb_swept(p, e.y, b);
+      if (swept) atomicAdd(h + b, 1u);
+      p.tour[j] = make_uint4(p.time[t], ps | (swept ? 0u : kRowsOnly), (uint32_t)sd, (uint32_t)(sd >> 32));
     }
   }
-  kb_write_hist(h, p.B, p.pthist, p.pt_tiles);
+  __syncthreads();
+  for (int32_t d = threadIdx.x; d < p.B; d += blockDim.x) p.pthist[(int64_t)blockIdx.x * p.B + d] = h[d];
 }
 
-__global__ void __launch_bounds__(kPtWarps * 32, 2) k_kb_point_scatter(KbParams p) {
+// Stable scatter by key block: four warps, 1,024 consecutive points each, ranked by
+// ballots over the digit's bits (__match_any_sync took some 400 cycles with 32 distinct
+// digits) in per-warp counters.
+constexpr int kPtWarps = 4, kPtRounds = kKbPtTile / (kPtWarps * 32);
+inline size_t kb_scatter_smem(int32_t B) { return (size_t)((B + 3) & ~3) * 4 + (size_t)kPtWarps * ((B + 7) & ~7) * 2; }
+__global__ void __launch_bounds__(kPtWarps * 32, 10) k_kb_point_scatter(KbParams p, int bits) {
   if (*p.status) return;
   extern __shared__ __align__(16) uint32_t base[];
-  __shared__ int32_t s_t[2];
   const int32_t Bp = (p.B + 7) & ~7;
-  uint16_t* wc = reinterpret_cast<uint16_t*>(base + ((p.B + 3) & ~3));
+  uint16_t* wall = reinterpret_cast<uint16_t*>(base + ((p.B + 3) & ~3));
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  uint16_t* wc = wall + warp * Bp;
+  const unsigned lt = (1u << lane) - 1u;
   const int64_t j0 = (int64_t)blockIdx.x * kKbPtTile, j1 = imin64(j0 + kKbPtTile, kb_points(p));
   if (j0 >= j1) return;
-  for (int32_t i = threadIdx.x; i < kPtWarps * Bp / 2; i += blockDim.x) reinterpret_cast<uint32_t*>(wc)[i] = 0;
-  kb_step_range(p, j0, j1, s_t);
-  uint32_t d[kPtItems], slot[kPtItems], time[kPtItems];
-  uint64_t delta[kPtItems];
-  uint16_t r[kPtItems];
+  for (int32_t i = threadIdx.x; i < kPtWarps * Bp / 8; i += blockDim.x) reinterpret_cast<uint4*>(wall)[i] = make_uint4(0, 0, 0, 0);
+  for (int32_t i = threadIdx.x; i < p.B; i += blockDim.x) base[i] = p.pthist[(int64_t)blockIdx.x * p.B + i];
+  __syncthreads();
+  const int64_t w0 = j0 + warp * (kPtRounds * 32) + lane;
+  uint32_t r[kPtRounds / 2];   // rank inside the warp, two rounds a word
+  uint32_t batch[8];           // positions of the next rounds, read ahead of the ranking
 #pragma unroll
-  for (int i = 0; i < kPtItems; ++i) {
-    const int64_t j = j0 + (warp * kPtItems + i) * 32 + lane;
-    d[i] = kNone;
-    if (j < j1) {
-      const KbPoint x = kb_point(p, kb_find_step(p.ep, s_t[0], s_t[1], j), j);
-      const uint32_t ps = p.pos[x.key], b = ps / p.m;
-      if (kb_swept(p, x.key, b)) d[i] = b;
-      slot[i] = ps - b * p.m;
-      time[i] = x.time;
-      delta[i] = x.delta;
+  for (int i = 0; i < kPtRounds; ++i) {
+    if (i % 8 == 0) {
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        const int64_t j = w0 + (i + k) * 32;
+        batch[k] = j < j1 ? __ldg(&p.tour[j].y) : kRowsOnly;
+      }
+    }
+    const uint32_t ps = batch[i % 8];
+    const bool in = !(ps & kRowsOnly);
+    const uint32_t d = ps / p.m;
+    unsigned peers = __ballot_sync(kAll, in);
+    for (int k = 0; k < bits; ++k) {
+      const bool one = (d >> k) & 1u;
+      const unsigned m = __ballot_sync(kAll, one);
+      peers &= one ? m : ~m;
+    }
+    const uint32_t old = in ? wc[d] : 0u;
+    __syncwarp();
+    const uint32_t rk = old + __popc(peers & lt);
+    if (i & 1) r[i / 2] |= rk << 16; else r[i / 2] = rk;
+    if (in && (peers & lt) == 0) wc[d] = (uint16_t)(old + __popc(peers));
+    __syncwarp();
+  }
+  __syncthreads();
+  for (int32_t d = threadIdx.x; d < p.B; d += blockDim.x) {
+    uint32_t run = 0;
+#pragma unroll
+    for (int w = 0; w < kPtWarps; ++w) {
+      const uint32_t c = wall[w * Bp + d];
+      wall[w * Bp + d] = (uint16_t)run;
+      run += c;
     }
   }
-  kb_rank<kPtItems>(wc + warp * Bp, d, r);
-  kb_bases<kPtWarps>(wc, base, p.B, Bp, p.pthist, p.pt_tiles);
+  __syncthreads();
 #pragma unroll
-  for (int i = 0; i < kPtItems; ++i)
-    if (d[i] != kNone)
-      p.pts[(size_t)base[d[i]] + wc[warp * Bp + d[i]] + r[i]] =
-          make_uint4(time[i], slot[i], (uint32_t)delta[i], (uint32_t)(delta[i] >> 32));
+  for (int i = 0; i < kPtRounds; ++i) {
+    const int64_t j = w0 + i * 32;
+    if (j >= j1) continue;
+    uint4 x = __ldg(p.tour + j);
+    if (x.y & kRowsOnly) continue;
+    const uint32_t d = x.y / p.m;
+    x.y -= d * p.m;
+    p.pts[(size_t)base[d] + wc[d] + ((r[i / 2] >> (16 * (i & 1))) & 0xffffu)] = x;
+  }
 }
 
 // ------------------------------------------------------------------ rows
-__device__ __forceinline__ void kb_add_points(const KbParams& p, unsigned long long* vec, int64_t j0, int64_t j1,
-                                              int32_t t0, int32_t t1) {
+__device__ __forceinline__ void kb_add_points(const KbParams& p, unsigned long long* vec, int64_t j0, int64_t j1) {
+#pragma unroll 4
   for (int64_t j = j0 + threadIdx.x; j < j1; j += blockDim.x) {
-    const KbPoint x = kb_point(p, kb_find_step(p.ep, t0, t1, j), j);
-    shared_add_u64(vec + p.pos[x.key] / p.m, x.delta);
+    const uint4 x = __ldg(p.tour + j);
+    shared_add_u64(vec + (x.y & ~kRowsOnly) / p.m, ((uint64_t)x.w << 32) | x.z);
   }
 }
 __device__ __forceinline__ int64_t kb_seg_start(const KbParams& p, int32_t g) {
@@ -295,17 +352,12 @@ __device__ __forceinline__ int64_t kb_seg_start(const KbParams& p, int32_t g) {
 }
 
 // Net delta of every tour segment in every key block.
-__global__ void __launch_bounds__(256) k_kb_seg(KbParams p) {
+__global__ void __launch_bounds__(512) k_kb_seg(KbParams p) {
   if (*p.status) return;
   extern __shared__ __align__(16) unsigned long long vec[];
-  __shared__ int32_t s_t[2];
   for (int32_t i = threadIdx.x; i < p.B; i += blockDim.x) vec[i] = 0;
   __syncthreads();
-  const int64_t j0 = kb_seg_start(p, blockIdx.x), j1 = kb_seg_start(p, blockIdx.x + 1);
-  if (j0 < j1) {
-    kb_step_range(p, j0, j1, s_t);
-    kb_add_points(p, vec, j0, j1, s_t[0], s_t[1]);
-  }
+  kb_add_points(p, vec, kb_seg_start(p, blockIdx.x), kb_seg_start(p, blockIdx.x + 1));
   __syncthreads();
   for (int32_t i = threadIdx.x; i < p.B; i += blockDim.x) p.seg[(size_t)blockIdx.x * p.B + i] = vec[i];
 }
@@ -343,12 +395,16 @@ __device__ __forceinline__ int32_t kb_col_after(const KbParams& p, int32_t nc, i
 }
 
 // A segment's columns: the running vector over the key blocks (shared memory) takes
-// the points up to the column and is written out scanned.  Bound by the row writes.
-__global__ void __launch_bounds__(256) k_kb_rows(KbParams p) {
+// the points up to the column and is written out scanned, four entries a thread and
+// pass.  Two barriers a column: the vector is complete; the warps' sums are written
+// (and the vector read, so that the next column's points may follow).
+constexpr int kRowThreads = 512;
+__global__ void __launch_bounds__(kRowThreads, 3) k_kb_rows(KbParams p) {
   if (*p.status) return;
-  extern __shared__ __align__(16) unsigned long long vec[];
-  unsigned long long* out = vec + p.B;
+  extern __shared__ __align__(16) unsigned long long vec[];   // Bs
   __shared__ int32_t s_c[2];
+  __shared__ uint64_t s_sum[2][2][kRowThreads / 32];          // by column parity and pass
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t j0 = kb_seg_start(p, blockIdx.x), j1 = kb_seg_start(p, blockIdx.x + 1);
   if (threadIdx.x < 2) {
     const bool last = blockIdx.x + 1 == (unsigned)p.segs;
@@ -356,31 +412,55 @@ __global__ void __launch_bounds__(256) k_kb_rows(KbParams p) {
     // columns of the segment: point counts in (j0, j1], and those without points in the first one
     s_c[threadIdx.x] = threadIdx.x ? (last ? nc : kb_col_after(p, nc, j1)) : (blockIdx.x ? kb_col_after(p, nc, j0) : 0);
   }
-  for (int32_t i = threadIdx.x; i < p.B; i += blockDim.x) vec[i] = p.seg[(size_t)blockIdx.x * p.B + i];
+  for (int32_t i = threadIdx.x; i < p.Bs; i += kRowThreads) vec[i] = i < p.B ? p.seg[(size_t)blockIdx.x * p.B + i] : 0;
   __syncthreads();
-  const int32_t per = ((p.B + 255) / 256) | 1;   // odd: a thread's entries start in different banks
-  const int32_t i0 = min(p.B, (int32_t)threadIdx.x * per), i1 = min(p.B, i0 + per);
   int64_t j = j0;
-  int32_t t = 0;
-  if (s_c[0] < s_c[1]) t = kb_find_step(p.ep, 0, 2 * p.S - 1, j0);
-  for (int32_t c = s_c[0]; c < s_c[1]; ++c) {
-    const int32_t tc = p.colstep[c];
-    const int64_t je = p.ep[tc];
-    kb_add_points(p, vec, j, je, t, tc);
+  const int32_t c0 = s_c[0], c1 = s_c[1];
+  for (int32_t c = c0; c < c1; ++c) {
+    const int64_t je = p.ep[p.colstep[c]];
+    kb_add_points(p, vec, j, je);
     j = je;
-    t = tc;
     __syncthreads();
-    uint64_t s = 0;
-    for (int32_t i = i0; i < i1; ++i) s += vec[i];
-    uint64_t run = block_exclusive_scan<uint64_t>(s);
-    for (int32_t i = i0; i < i1; ++i) {
-      out[i] = run;
-      run += vec[i];
+    uint64_t v[2][4], ex[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {   // entries 4 tid .. 4 tid + 3, and 2,048 further on
+      const int32_t i = h * 4 * kRowThreads + 4 * threadIdx.x;
+      ex[h] = 0;
+      if (h * 4 * kRowThreads >= p.Bs) continue;
+#pragma unroll
+      for (int k = 0; k < 4; ++k) v[h][k] = i < p.Bs ? vec[i + k] : 0;
+      const uint64_t s = v[h][0] + v[h][1] + v[h][2] + v[h][3];
+      uint64_t incl = s;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint64_t y = __shfl_up_sync(kAll, incl, o);
+        if (lane >= o) incl += y;
+      }
+      ex[h] = incl - s;
+      if (lane == 31) s_sum[c & 1][h][warp] = incl;
     }
     __syncthreads();
-    int64_t* row = p.rows + (size_t)c * p.B;
-    for (int32_t i = threadIdx.x; i < p.B; i += blockDim.x) row[i] = (int64_t)out[i];
-    __syncthreads();
+    uint64_t run0 = 0;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int32_t i = h * 4 * kRowThreads + 4 * threadIdx.x;
+      if (h * 4 * kRowThreads >= p.Bs) continue;
+      uint64_t w = lane < kRowThreads / 32 ? s_sum[c & 1][h][lane] : 0;
+#pragma unroll
+      for (int o = 1; o < kRowThreads / 32; o <<= 1) {
+        const uint64_t y = __shfl_up_sync(kAll, w, o);
+        if (lane >= o) w += y;
+      }
+      const uint64_t below = __shfl_sync(kAll, w, warp ? warp - 1 : 0);
+      uint64_t a = run0 + (warp ? below : 0) + ex[h];
+      run0 += __shfl_sync(kAll, w, kRowThreads / 32 - 1);
+      if (i < p.Bs) {
+        int64_t* row = p.rows + (size_t)c * p.Bs + i;
+        const uint64_t b1 = a + v[h][0], b2 = b1 + v[h][1], b3 = b2 + v[h][2];
+        reinterpret_cast<longlong2*>(row)[0] = make_longlong2((int64_t)a, (int64_t)b1);
+        reinterpret_cast<longlong2*>(row)[1] = make_longlong2((int64_t)b2, (int64_t)b3);
+      }
+    }
   }
 }
 
@@ -394,8 +474,10 @@ __global__ void __launch_bounds__(512) k_kb_probe_count(KbParams p) {
   for (int32_t i = threadIdx.x; i < p.B; i += blockDim.x) h[i] = 0;
   const int64_t j0 = (int64_t)blockIdx.x * kKbPrTile, j1 = imin64(j0 + kKbPrTile, p.Q);
   kb_col_range(p, j0, j1, s_c);
-  for (int64_t j = j0 + threadIdx.x; j < j1; j += blockDim.x) {
-    const int32_t c = kb_find_col(p.coltime, s_c[0], s_c[1], (uint32_t)j);
+  const int32_t ca = s_c[0], cz = s_c[1];
+#pragma unroll 4
+  for (int64_t j = j0 + threadIdx.x; j < j1; j += 512) {
+    const int32_t c = kb_find_col(p.coltime, ca, cz, (uint32_t)j);
     const int64_t q = p.qoff[p.colstate[c]] + (j - p.coltime[c]);
     const uint32_t lo = p.qs[q].lo, hi = p.qs[q].hi;
     uint32_t a = 0, z = 0;
@@ -410,223 +492,193 @@ __global__ void __launch_bounds__(512) k_kb_probe_count(KbParams p) {
       if (z != bz * p.m) atomicAdd(h + bz, 1u);
     }
   }
-  kb_write_hist(h, p.B, p.prhist, p.pr_tiles);
+  __syncthreads();
+  for (int32_t d = threadIdx.x; d < p.B; d += blockDim.x) p.prhist[(int64_t)blockIdx.x * p.B + d] = h[d];
 }
 
-// Lanes 2i and 2i + 1 hold the lower and upper bound of a query, so that a warp's
-// probes are in tour order.
-__global__ void __launch_bounds__(kPrWarps * 32, 2) k_kb_probe_scatter(KbParams p) {
+// Scatter by key block in rounds of 256 queries (at most 512 probes of a block): rounds
+// are in tour order, the probes of one round in any -- the sweep looks one page of 512
+// ahead.  acc becomes the part of the answer in whole key blocks.  Bound by the random
+// sectors of its stores and row reads (4.2 ms for 200M probes; 5.2 ms with stable ranks
+// from __match_any_sync).
+constexpr int kPrThreads = 256;
+__global__ void __launch_bounds__(kPrThreads) k_kb_probe_scatter(KbParams p) {
   if (*p.status) return;
-  extern __shared__ __align__(16) uint32_t base[];
+  extern __shared__ __align__(16) uint32_t next[];
   __shared__ int32_t s_c[2];
-  const int32_t Bp = (p.B + 7) & ~7;
-  uint16_t* wc = reinterpret_cast<uint16_t*>(base + ((p.B + 3) & ~3));
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int64_t j0 = (int64_t)blockIdx.x * kKbPrTile, j1 = imin64(j0 + kKbPrTile, p.Q);
-  for (int32_t i = threadIdx.x; i < kPrWarps * Bp / 2; i += blockDim.x) reinterpret_cast<uint32_t*>(wc)[i] = 0;
+  for (int32_t i = threadIdx.x; i < p.B; i += kPrThreads) next[i] = p.prhist[(int64_t)blockIdx.x * p.B + i];
   kb_col_range(p, j0, j1, s_c);
-  uint32_t d[kPrItems], slot[kPrItems];
-  uint16_t r[kPrItems];
-#pragma unroll
-  for (int i = 0; i < kPrItems; ++i) {
-    const int64_t j = j0 + (warp * kPrItems + i) * 16 + (lane >> 1);
-    d[i] = kNone;
-    slot[i] = 0;
-    if (j < j1) {
-      const unsigned long long az = p.acc[j];
-      const uint32_t a = (uint32_t)az, z = (uint32_t)(az >> 32);
-      const uint32_t x = (lane & 1) ? z : a, b = x / p.m;
-      slot[i] = x - b * p.m;
-      if (a != z && slot[i]) d[i] = b;
+  const int32_t ca = s_c[0], cz = s_c[1];
+  auto load = [&](int64_t j) -> unsigned long long { return j < j1 ? p.acc[j] : 0; };
+  // the row entries of a query's bounds, requested a round before they are subtracted
+  auto rows = [&](int64_t j, unsigned long long az, int64_t& ra, int64_t& rz) {
+    const uint32_t ba = (uint32_t)az / p.m, bz = (uint32_t)(az >> 32) / p.m;
+    ra = rz = 0;
+    if (ba != bz) {
+      const int64_t* row = p.rows + (size_t)kb_find_col(p.coltime, ca, cz, (uint32_t)j) * p.Bs;
+      ra = __ldg(row + ba);
+      rz = __ldg(row + bz);
     }
-  }
-  kb_rank<kPrItems>(wc + warp * Bp, d, r);
-  kb_bases<kPrWarps>(wc, base, p.B, Bp, p.prhist, p.pr_tiles);
-#pragma unroll
-  for (int i = 0; i < kPrItems; ++i) {
-    const int64_t j = j0 + (warp * kPrItems + i) * 16 + (lane >> 1);
-    if (d[i] != kNone)
-      p.prs[(size_t)base[d[i]] + wc[warp * Bp + d[i]] + r[i]] =
-          make_uint2((uint32_t)j, slot[i] | ((lane & 1) ? 0u : 0x80000000u));
-    if (j < j1 && !(lane & 1)) {
-      const unsigned long long az = p.acc[j];
-      const uint32_t ba = (uint32_t)az / p.m, bz = (uint32_t)(az >> 32) / p.m;
-      uint64_t v = 0;
-      if (ba != bz) {
-        const int64_t* row = p.rows + (size_t)kb_find_col(p.coltime, s_c[0], s_c[1], (uint32_t)j) * p.B;
-        v = (uint64_t)row[bz] - (uint64_t)row[ba];
-      }
-      p.acc[j] = v;   // read by this lane pair only, both reads above
+  };
+  int64_t j = j0 + threadIdx.x, ra, rz;
+  unsigned long long az = load(j), n1 = load(j + kPrThreads);
+  rows(j, az, ra, rz);
+  for (int64_t r0 = j0; r0 < j1; r0 += kPrThreads, j += kPrThreads) {
+    const unsigned long long n2 = load(j + 2 * kPrThreads);
+    int64_t na, nz;
+    rows(j + kPrThreads, n1, na, nz);   // (past the tile: an empty query)
+    const uint32_t a = (uint32_t)az, z = (uint32_t)(az >> 32);
+    if (a != z) {
+      const uint32_t ba = a / p.m, bz = z / p.m, sa = a - ba * p.m, sz = z - bz * p.m;
+      if (sa) p.prs[atomicAdd(next + ba, 1u)] = make_uint2((uint32_t)j, sa | 0x80000000u);
+      if (sz) p.prs[atomicAdd(next + bz, 1u)] = make_uint2((uint32_t)j, sz);
     }
-    __syncwarp();
+    if (j < j1) p.acc[j] = (uint64_t)rz - (uint64_t)ra;
+    az = n1; n1 = n2; ra = na; rz = nz;
+    __syncthreads();
   }
 }
 
 // ------------------------------------------------------------------ sweep
 // One key block at a time per CTA: its points (signed deltas at slots) and probes
 // (prefixes over the slots), both in tour order.  The points before the current tile
-// of 32 are held as a prefix structure of radix 32 over the slots: T0[s] = sum of the
-// slots below s in s's group of 32, T1 = sum of the groups below in the warp's range,
-// W = the warps' totals.  A probe is one read of each plus its correction inside the
-// tile, tab[points before it in time][points below it by slot], for which a seventeenth
-// warp sorts the next tile's slots and sums its table while the tile is probed.  Sixteen
-// warps own m / 16 slots each and apply the tile's points in their range without atomics:
-// the 32 lanes add to the tail of the point's group, T1 stays in registers.
-constexpr int kSwWarps = 16, kSwThreads = kSwWarps * 32 + 32, kSwPage = kSwWarps * 32;
+// of 32 are held as a prefix structure over the slots: T0[s] = sum of the slots below s
+// in s's group of 32, T1 = sum of the groups below.  A probe reads one of each and adds
+// the tile's own points before it in time and below it by slot (32 broadcast reads,
+// four in flight).  After the tile's probes the sixteen warps apply its points without
+// atomics: the 32 lanes of the warp that owns the group add to T0's tail of it (an entry
+// is always the same lane's), T1 stays in registers, a lane per group, and takes the
+// points of lower ranges as one warp sum.
+//
+// Bound by instruction issue (58 % of the slots) and the two barriers a tile.  On 20M
+// events over 10M keys with 100M range queries (1.25M tiles, 200M probes) the sweep takes
+// 6.9 ms; with a table of each tile's corrections, built by one or two warps of their own
+// while the tile before it was probed, it took 12 to 14.4 ms (the builders' dependent
+// chains ran 2,400 cycles and more a tile), with one 32-step loop a probe and a
+// seventeenth warp 8.4 ms (17 warps leave 32 registers a thread at three CTAs an SM).
+constexpr int kSwWarps = 16, kSwThreads = kSwWarps * 32;
+constexpr int kSwRing = 8;                   // tiles of points in shared memory
 struct KbSweepSmem {
+  uint4 pt[kSwRing][32];                     // by tile mod kSwRing: {time, slot, delta}
   unsigned long long T1[kKbMaxSlots / 32];
-  unsigned long long W[kSwWarps];
-  unsigned long long tab[2][32 * 32];       // [x - 1][y - 1]
-  uint4 pt[2][32];                           // {time, slot, delta}
-  uint32_t tm[2][32], sorted[2][32];
-  uint32_t next_time[2];                     // time of the tile after (kNone: none)
   int32_t block;
 };
-
-// Values of v[0..32) (ascending) that are < x (kLess) or <= x.
-template <bool kLess>
-__device__ __forceinline__ int kb_below(const uint32_t* v, uint32_t x) {
-  int n = 0;
-#pragma unroll
-  for (int s = 16; s; s >>= 1) {
-    const uint32_t y = v[n + s - 1];
-    if (kLess ? y < x : y <= x) n += s;
-  }
-  const uint32_t y = v[n];
-  return n + ((kLess ? y < x : y <= x) ? 1 : 0);
+__device__ __forceinline__ void kb_copy16(void* dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
+               : "memory");
+}
+// Sum over the warp, modulo 2^64, in three 32-bit reductions (32 values of 24 bits fit).
+__device__ __forceinline__ uint64_t kb_warp_sum(uint64_t v) {
+  const uint32_t a = __reduce_add_sync(kAll, (uint32_t)v & 0xffffffu);
+  const uint32_t b = __reduce_add_sync(kAll, (uint32_t)(v >> 24) & 0xffffffu);
+  const uint32_t c = __reduce_add_sync(kAll, (uint32_t)(v >> 48));
+  return (uint64_t)a + ((uint64_t)b << 24) + ((uint64_t)c << 48);
 }
 
-__global__ void __launch_bounds__(kSwThreads, 2) k_kb_sweep(KbParams p) {
+// v += the point's delta when it lies at or before time tm and below slot r (two
+// predicated adds; a select of the 64-bit delta and an add took twice as many).
+__device__ __forceinline__ void kb_add_if(uint64_t& v, const uint4& x, uint32_t tm, uint32_t r) {
+  uint32_t lo = (uint32_t)v, hi = (uint32_t)(v >> 32);
+  asm("{\n\t.reg .pred q;\n\tsetp.le.u32 q, %2, %3;\n\tsetp.lt.and.u32 q, %4, %5, q;\n\t"
+      "@q add.cc.u32 %0, %0, %6;\n\t@q addc.u32 %1, %1, %7;\n\t}"
+      : "+r"(lo), "+r"(hi)
+      : "r"(x.x), "r"(tm), "r"(x.y), "r"(r), "r"(x.z), "r"(x.w));
+  v = ((uint64_t)hi << 32) | lo;
+}
+
+__global__ void __launch_bounds__(kSwThreads, kSwCtas) k_kb_sweep(KbParams p) {
   if (*p.status) return;
   extern __shared__ __align__(16) unsigned long long T0[];   // m slots
   __shared__ KbSweepSmem sm;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const bool builder = warp == kSwWarps;
-  const uint32_t g = p.m / kKbSlotStep, span = g * 32;       // groups and slots of a warp
-  const uint32_t inv = 65536u / g + 1u;                      // x / g = x * inv >> 16 for x < 320
+  const bool copier = warp == kSwWarps - 1;
+  const uint32_t g = p.m / kKbSlotStep, span = g * 32, first = warp * span;   // groups, slots, first slot of a warp
   for (;;) {
     __syncthreads();
     if (tid == 0) sm.block = atomicAdd(p.ticket, 1);
     __syncthreads();
     const int32_t b = sm.block;
     if (b >= p.B) break;
-    const uint32_t p0 = b ? p.pthist[(int64_t)b * p.pt_tiles - 1] : 0u, p1 = p.pthist[(int64_t)(b + 1) * p.pt_tiles - 1];
-    const uint32_t q0 = b ? p.prhist[(int64_t)b * p.pr_tiles - 1] : 0u, q1 = p.prhist[(int64_t)(b + 1) * p.pr_tiles - 1];
-    if (p0 == p1 || q0 == q1) continue;
+    const uint32_t p0 = p.ptoff[b], p1 = p.ptoff[b + 1], q1 = p.proff[b + 1];
+    uint32_t page = p.proff[b];
+    if (p0 == p1 || page == q1) continue;
     const uint32_t nt = (p1 - p0 + 31) / 32;
     for (uint32_t i = tid; i < p.m / 2; i += kSwThreads) reinterpret_cast<uint4*>(T0)[i] = make_uint4(0, 0, 0, 0);
     for (uint32_t i = tid; i < p.m / 32; i += kSwThreads) sm.T1[i] = 0;
-    if (tid < kSwWarps) sm.W[tid] = 0;
-    // the builder's points of a tile; past the end: at a time after every query
-    auto load_point = [&](uint32_t k) -> uint4 {
+    // a tile's points (a missing one: at a time after every query, above every slot)
+    auto copy_points = [&](uint32_t k) {
       const uint32_t i = p0 + 32 * k + lane;
-      return k < nt && i < p1 ? __ldg(p.pts + i) : make_uint4(kNone, kNone, 0u, 0u);
+      uint4* at = &sm.pt[k % kSwRing][lane];
+      if (k < nt && i < p1) kb_copy16(at, p.pts + i);
+      else *at = make_uint4(kNone, kNone, 0u, 0u);
+      asm volatile("cp.async.commit_group;" ::: "memory");
     };
-    auto build = [&](uint32_t k, uint4 x, uint32_t next_first) {
-      const int f = k & 1;
-      int below = 0, at = 0;   // points with a smaller slot; its place among the sorted
-#pragma unroll 8
-      for (int i = 0; i < 32; ++i) {
-        const uint32_t y = __shfl_sync(kAll, x.y, i);
-        below += y < x.y;
-        at += y < x.y || (y == x.y && i < lane);
-      }
-      sm.pt[f][lane] = x;
-      sm.tm[f][lane] = x.x;
-      sm.sorted[f][at] = x.y;
-      if (lane == 0) sm.next_time[f] = next_first;
-      uint64_t acc = 0;        // column lane + 1: points taken so far among the lane + 1 lowest slots
-#pragma unroll 8
-      for (int i = 0; i < 32; ++i) {
-        const int r = __shfl_sync(kAll, below, i);
-        const uint64_t d = ((uint64_t)__shfl_sync(kAll, x.w, i) << 32) | __shfl_sync(kAll, x.z, i);
-        acc += r <= lane ? d : 0;
-        sm.tab[f][i * 32 + lane] = acc;
-      }
-    };
-    uint4 nx = make_uint4(0, 0, 0, 0), nx2 = nx;   // builder: tiles k + 1 and k + 2
-    if (builder) {
-      const uint4 x = load_point(0);
-      nx = load_point(1);
-      nx2 = load_point(2);
-      build(0, x, __shfl_sync(kAll, nx.x, 0));
+    if (copier) {
+      for (uint32_t k = 0; k < kSwRing - 1; ++k) copy_points(k);
+      asm volatile("cp.async.wait_group %0;" ::"n"(kSwRing - 3) : "memory");   // tiles 0 and 1 have landed
     }
-    auto load_probe = [&](uint32_t i) -> uint2 {
-      return !builder && i < q1 ? __ldg(p.prs + i) : make_uint2(0u, kNone);
-    };
-    uint32_t page = q0;
-    uint2 pr = load_probe(page + tid), pn = load_probe(page + kSwPage + tid);
-    bool done = pr.y == kNone;                       // (slots stay below 2^31 - 1)
-    uint64_t t1 = 0, wtot = 0;                       // lane's group sum below, warp total
+    auto load_probe = [&](uint32_t i) -> uint2 { return i < q1 ? __ldg(p.prs + i) : make_uint2(0u, kNone); };
+    // this thread's probe of the page, of the next one and of the one after
+    uint2 pr = load_probe(page + tid), pn = load_probe(page + kSwThreads + tid),
+          pl = load_probe(page + 2 * kSwThreads + tid);
+    bool done = pr.y == kNone, donen = pn.y == kNone;   // (slots stay below 2^31 - 1)
+    uint64_t t1 = 0;                                    // T1 of the warp's group `lane`
     __syncthreads();
     for (uint32_t k = 0; k < nt; ++k) {
-      const int f = k & 1;
-      const uint32_t limit = sm.next_time[f];
-      uint64_t wpre = 0;                             // totals of the warps below `lane`
-      if (!builder) {
-        const uint64_t own = lane < kSwWarps ? sm.W[lane] : 0;
-        wpre = own;
-#pragma unroll
-        for (int o = 1; o < kSwWarps; o <<= 1) {
-          const uint64_t y = __shfl_up_sync(kAll, wpre, o);
-          if (lane >= o) wpre += y;
-        }
-        wpre -= own;
-      }
+      const uint4* pt = sm.pt[k % kSwRing];
+      const uint32_t limit = sm.pt[(k + 1) % kSwRing][0].x;
       bool more = true;
-      for (bool first = true; more; first = false) {
-        if (builder) {
-          if (first && k + 1 < nt) {
-            const uint4 x = nx;
-            nx = nx2;
-            nx2 = load_point(k + 3);
-            build(k + 1, x, __shfl_sync(kAll, nx.x, 0));
+      while (more) {
+        // the page's and the next page's probes of the tile (the order is loose within a page)
+        auto answer = [&](const uint2& q, bool& fin) {
+          const bool in = !fin && q.x < limit;
+          if (!__any_sync(kAll, in)) return;
+          const uint32_t r = in ? q.y & 0x7fffffffu : 0u, tm = in ? q.x : 0u;
+          const uint32_t last = __reduce_max_sync(kAll, tm);
+          uint64_t v = sm.T1[r >> 5] + T0[r];
+#pragma unroll 1
+          for (int i = 0; i < 32; i += 4) {   // four reads in flight, up to the warp's last probe in time
+            uint4 x[4];
+#pragma unroll
+            for (int h = 0; h < 4; ++h) x[h] = pt[i + h];
+#pragma unroll
+            for (int h = 0; h < 4; ++h) kb_add_if(v, x[h], tm, r);
+            if (x[3].x > last) break;
           }
-        } else {
-          const bool in = !done && pr.x < limit;
-          if (__any_sync(kAll, in)) {
-            const uint32_t r = pr.y & 0x7fffffffu, rs = in ? r : 0u;
-            const uint64_t w = __shfl_sync(kAll, wpre, (int)(((rs >> 5) * inv) >> 16));
-            if (in) {
-              uint64_t v = w + sm.T1[r >> 5] + T0[r];
-              const int x = kb_below<false>(sm.tm[f], pr.x), y = kb_below<true>(sm.sorted[f], r);
-              if (x && y) v += sm.tab[f][(x - 1) * 32 + y - 1];
-              if (v) atomicAdd(p.acc + pr.x, (unsigned long long)((pr.y >> 31) ? (uint64_t)0 - v : v));
-              done = true;
-            }
-          }
-        }
-        more = __syncthreads_and(builder || done);   // the whole page is answered
+          if (in && v) atomicAdd(p.acc + q.x, (unsigned long long)((q.y >> 31) ? (uint64_t)0 - v : v));
+          fin |= in;
+        };
+        answer(pr, done);
+        answer(pn, donen);
+        more = __syncthreads_and(done);              // the whole page is answered
         if (more) {
-          page += kSwPage;
+          page += kSwThreads;
           if (page >= q1) break;
           pr = pn;
-          pn = load_probe(page + kSwPage + tid);
-          done = pr.y == kNone;
+          done = donen;
+          pn = pl;
+          donen = pn.y == kNone;
+          pl = load_probe(page + 2 * kSwThreads + tid);
         }
       }
       if (more) break;                               // no probes are left
-      if (!builder) {                                // the tile's points into the prefixes
-        const uint32_t s = sm.pt[f][lane].y;
-        uint32_t hit = __ballot_sync(kAll, s - warp * span < span);
-        if (hit) {
-          do {
-            const int i = __ffs(hit) - 1;
-            hit &= hit - 1;
-            const uint4 x = sm.pt[f][i];
-            const uint64_t d = ((uint64_t)x.w << 32) | x.z;
-            const uint32_t q = x.y & 31u;
-            if (lane > (int)q) T0[(x.y & ~31u) + lane] += d;
-            if (lane > (int)((x.y >> 5) - warp * g)) t1 += d;
-            wtot += d;
-            __syncwarp();
-          } while (hit);
-          if (lane < (int)g) sm.T1[warp * g + lane] = t1;
-          if (lane == 0) sm.W[warp] = wtot;
-        }
+      if (copier) copy_points(k + kSwRing - 1);      // into the place of tile k - 1
+      const uint4 mine = pt[lane];
+      uint32_t hit = __ballot_sync(kAll, mine.y - first < span);
+      t1 += kb_warp_sum(mine.y < first ? ((uint64_t)mine.w << 32) | mine.z : 0);
+      while (hit) {
+        const uint4 x = pt[__ffs(hit) - 1];
+        hit &= hit - 1;
+        const uint64_t d = ((uint64_t)x.w << 32) | x.z;
+        if (lane > (int)(x.y & 31u)) T0[(x.y & ~31u) + lane] += d;
+        if (lane > (int)((x.y - first) >> 5)) t1 += d;
       }
+      if (lane < (int)g) sm.T1[warp * g + lane] = t1;
+      if (copier) asm volatile("cp.async.wait_group %0;" ::"n"(kSwRing - 3) : "memory");   // tiles k + 1 and k + 2
       __syncthreads();
     }
+    if (copier) asm volatile("cp.async.wait_all;" ::: "memory");   // before the ring is used again
   }
 }
 
@@ -646,12 +698,12 @@ inline size_t al256(size_t x) { return (x + 255) & ~size_t(255); }
 // Workspace of the replay with blocks of k.m slots.
 void kb_layout(const PipeSpec& s, KbSpec& k) {
   k.B = (int32_t)(s.E / k.m + 1);   // a bound past every event has slot E: its block is E / m
-  k.segs = 8 * s.sms;
+  k.segs = 3 * s.sms;   // one wave of the row pass (three CTAs an SM)
   k.pt_tiles = (2 * s.E + kKbPtTile - 1) / kKbPtTile;
   k.pr_tiles = (s.Q + kKbPrTile - 1) / kKbPrTile;
   const size_t S = (size_t)s.S, S2 = 2 * S, B = (size_t)k.B;
   const size_t cols = (size_t)std::min<int64_t>(s.S, s.Q);
-  const size_t scan_n = std::max({S2, (size_t)s.Cmax + 1, B * (size_t)k.pt_tiles, B * (size_t)k.pr_tiles});
+  const size_t scan_n = std::max(S2, (size_t)s.Cmax + 1);
   size_t o = 0;
   auto take = [&](int i, size_t bytes) { k.off[i] = o; o = al256(o + bytes); };
   take(KB_SOFF, 8); take(KB_TEOFF, 16); take(KB_TQOFF, 16); take(KB_TC, 4); take(KB_TBOFF, 8); take(KB_TBITS, 8);
@@ -664,11 +716,15 @@ void kb_layout(const PipeSpec& s, KbSpec& k) {
   take(KB_STEP, S2 * 4); take(KB_W, S2 * 8); take(KB_EP, S2 * 8); take(KB_TIME, S2 * 4);
   take(KB_COLSTATE, cols * 4); take(KB_COLTIME, (cols + 1) * 4); take(KB_COLSTEP, cols * 4);
   take(KB_POS, ((size_t)s.Cmax + 2) * 4);
+  take(KB_TOUR, 2 * (size_t)s.E * 16);
   take(KB_PTHIST, B * (size_t)k.pt_tiles * 4);
+  take(KB_PTOFF, (B + 1) * 4);
   take(KB_PTS, 2 * (size_t)s.E * 16);
   take(KB_SEG, (size_t)k.segs * B * 8);
-  take(KB_ROWS, cols * B * 8);
+  take(KB_ROWS, cols * ((B + 3) & ~(size_t)3) * 8);
   take(KB_PRHIST, B * (size_t)k.pr_tiles * 4);
+  take(KB_PROFF, (B + 1) * 4);
+  take(KB_PART, kStartChunks * B * 4);
   take(KB_PRS, 2 * (size_t)s.Q * 8);
   take(KB_ACC, (size_t)s.Q * 8);
   k.total = o;
@@ -684,9 +740,7 @@ int kb_attrs() {
   std::lock_guard<std::mutex> g(mu);
   if (dev >= 0 && dev < 64 && done[dev]) return 0;
   const struct { const void* f; size_t bytes; } need[] = {
-      {(const void*)k_kb_point_scatter, kb_scatter_smem(kKbMaxBlocks, kPtWarps)},
-      {(const void*)k_kb_probe_scatter, kb_scatter_smem(kKbMaxBlocks, kPrWarps)},
-      {(const void*)k_kb_rows, (size_t)kKbMaxBlocks * 16},
+      {(const void*)k_kb_point_scatter, kb_scatter_smem(kKbMaxBlocks)},
       {(const void*)k_kb_sweep, (size_t)kKbMaxSlots * 8}};
   for (const auto& n : need)
     if ((rc = report(cudaFuncSetAttribute(n.f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)n.bytes), "smem attr")))
@@ -702,12 +756,12 @@ bool kb_select(const BwReplayArgs* a, const PipeSpec& s, size_t general_bytes, K
   if (s.E < 1 || s.Q < 1 || s.Q >= ((int64_t)1 << 30)) return false;
   k = KbSpec();
   k.S = s.S; k.C = s.Cmax; k.E = s.E; k.Q = s.Q;
-  // about four blocks per sweep CTA (two CTAs an SM), larger ones where the rows would
+  // about four blocks per sweep CTA, larger ones where the rows would
   // not fit.  Never more scratch than twice the state-block pipeline's or 32 MiB, and nothing
   // that fits the allocation-free entry's 32 MiB there may outgrow them here.
   const size_t small = (size_t)32 << 20;
   const size_t limit = general_bytes > small ? 2 * general_bytes : small;
-  int64_t steps = std::min<int64_t>(s.E / (8 * (int64_t)s.sms * kKbSlotStep) + 1, kKbMaxSlots / kKbSlotStep);
+  int64_t steps = std::min<int64_t>(s.E / (4 * kSwCtas * (int64_t)s.sms * kKbSlotStep) + 1, kKbMaxSlots / kKbSlotStep);
   for (; steps * kKbSlotStep <= kKbMaxSlots; ++steps) {
     k.m = (int32_t)steps * kKbSlotStep;
     if (s.E / k.m + 1 > kKbMaxBlocks) continue;
@@ -743,14 +797,13 @@ int kb_enqueue(const KbSpec& k, const PipeSpec& s, const BwReplayArgs* a, EventS
   p.step = (int32_t*)at(KB_STEP); p.w = (int64_t*)at(KB_W); p.ep = (int64_t*)at(KB_EP); p.time = (uint32_t*)at(KB_TIME);
   p.colstate = (int32_t*)at(KB_COLSTATE); p.coltime = (uint32_t*)at(KB_COLTIME); p.colstep = (int32_t*)at(KB_COLSTEP);
   p.pos = (uint32_t*)at(KB_POS); p.pthist = (uint32_t*)at(KB_PTHIST); p.pts = (uint4*)at(KB_PTS);
+  p.tour = (uint4*)at(KB_TOUR); p.ptoff = (uint32_t*)at(KB_PTOFF); p.proff = (uint32_t*)at(KB_PROFF);
   p.seg = (uint64_t*)at(KB_SEG); p.rows = (int64_t*)at(KB_ROWS); p.prhist = (uint32_t*)at(KB_PRHIST);
   p.prs = (uint2*)at(KB_PRS); p.acc = (unsigned long long*)at(KB_ACC);
   p.status = ta.misc + M_STATUS; p.ticket = ta.misc + M_SWEEP_TICKET;
   p.E = k.E; p.Q = k.Q; p.pt_tiles = k.pt_tiles; p.pr_tiles = k.pr_tiles;
-  p.S = k.S; p.B = k.B; p.segs = k.segs; p.C = k.C; p.m = (uint32_t)k.m;
+  p.S = k.S; p.B = k.B; p.Bs = (k.B + 3) & ~3; p.segs = k.segs; p.C = k.C; p.m = (uint32_t)k.m;
 
-  const size_t pt_smem = kb_scatter_smem(k.B, kPtWarps), pr_smem = kb_scatter_smem(k.B, kPrWarps);
-  const size_t row_smem = (size_t)k.B * 16, sweep_smem = (size_t)k.m * 8;
   int rc = kb_attrs();
   if (rc) return rc;
   int kernels = 0;
@@ -773,27 +826,37 @@ int kb_enqueue(const KbSpec& k, const PipeSpec& s, const BwReplayArgs* a, EventS
   if ((rc = device_inclusive_scan<uint32_t>(p.pos, (int64_t)k.C + 1, ta.scan_tmp, st, kernels)))
     return report((cudaError_t)rc, "scan");
   if ((rc = mark(3))) return rc;
-  k_kb_point_count<<<(unsigned)k.pt_tiles, kPtWarps * 32, (size_t)k.B * 4, st>>>(p);
-  if ((rc = chk("k_kb_point_count"))) return rc;
-  if ((rc = device_inclusive_scan<uint32_t>(p.pthist, (int64_t)k.B * k.pt_tiles, ta.scan_tmp, st, kernels)))
-    return report((cudaError_t)rc, "scan");
-  k_kb_point_scatter<<<(unsigned)k.pt_tiles, kPtWarps * 32, pt_smem, st>>>(p);
+  uint32_t* part = (uint32_t*)at(KB_PART);
+  auto starts = [&](uint32_t* hist, int64_t tiles, uint32_t* off) -> int {
+    const dim3 g((unsigned)((k.B + 127) / 128), kStartChunks);
+    k_kb_start_sum<<<g, 128, 0, st>>>(hist, k.B, tiles, part, p.status);
+    if ((rc = chk("k_kb_start_sum"))) return rc;
+    k_kb_start_scan<<<1, 1024, 0, st>>>(part, k.B, off, p.status);
+    if ((rc = chk("k_kb_start_scan"))) return rc;
+    k_kb_start_apply<<<g, 128, 0, st>>>(hist, k.B, tiles, part, p.status);
+    return chk("k_kb_start_apply");
+  };
+  int bits = 1;
+  while ((1 << bits) < k.B) ++bits;
+  k_kb_points<<<(unsigned)k.pt_tiles, 256, (size_t)k.B * 4, st>>>(p);
+  if ((rc = chk("k_kb_points"))) return rc;
+  if ((rc = starts(p.pthist, k.pt_tiles, p.ptoff))) return rc;
+  k_kb_point_scatter<<<(unsigned)k.pt_tiles, kPtWarps * 32, kb_scatter_smem(k.B), st>>>(p, bits);
   if ((rc = chk("k_kb_point_scatter"))) return rc;
   if ((rc = mark(4))) return rc;
-  k_kb_seg<<<k.segs, 256, (size_t)k.B * 8, st>>>(p);
+  k_kb_seg<<<k.segs, 512, (size_t)k.B * 8, st>>>(p);
   if ((rc = chk("k_kb_seg"))) return rc;
   k_kb_segscan<<<(k.B + 31) / 32, 1024, 0, st>>>(p);
   if ((rc = chk("k_kb_segscan"))) return rc;
-  k_kb_rows<<<k.segs, 256, row_smem, st>>>(p);
+  k_kb_rows<<<k.segs, kRowThreads, (size_t)p.Bs * 8, st>>>(p);
   if ((rc = chk("k_kb_rows"))) return rc;
   if ((rc = mark(5))) return rc;
   k_kb_probe_count<<<(unsigned)k.pr_tiles, 512, (size_t)k.B * 4, st>>>(p);
   if ((rc = chk("k_kb_probe_count"))) return rc;
-  if ((rc = device_inclusive_scan<uint32_t>(p.prhist, (int64_t)k.B * k.pr_tiles, ta.scan_tmp, st, kernels)))
-    return report((cudaError_t)rc, "scan");
-  k_kb_probe_scatter<<<(unsigned)k.pr_tiles, kPrWarps * 32, pr_smem, st>>>(p);
+  if ((rc = starts(p.prhist, k.pr_tiles, p.proff))) return rc;
+  k_kb_probe_scatter<<<(unsigned)k.pr_tiles, kPrThreads, (size_t)k.B * 4, st>>>(p);
   if ((rc = chk("k_kb_probe_scatter"))) return rc;
-  k_kb_sweep<<<std::min(k.B, 2 * s.sms), kSwThreads, sweep_smem, st>>>(p);
+  k_kb_sweep<<<std::min(k.B, kSwCtas * s.sms), kSwThreads, (size_t)k.m * 8, st>>>(p);
   if ((rc = chk("k_kb_sweep"))) return rc;
   k_kb_answers<<<(unsigned)k.pr_tiles, 256, 0, st>>>(p);
   if ((rc = chk("k_kb_answers"))) return rc;

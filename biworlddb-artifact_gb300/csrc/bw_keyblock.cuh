@@ -10,7 +10,8 @@ namespace bw {
 
 constexpr int kKbMaxBlocks = 4096;            // key blocks (partition digits held in shared memory)
 constexpr int kKbSlotStep = 512;              // slots per block: a multiple of 16 warps x 32 lanes ...
-constexpr int kKbMaxSlots = 20 * kKbSlotStep; // ... and at most 10,240 (80 KB of int64, two CTAs per SM)
+constexpr int kKbMaxSlots = 16 * kKbSlotStep; // ... and at most 8,192 (64 KB of int64: three CTAs per SM)
+constexpr int kSwCtas = 3;                    // sweep CTAs per SM
 constexpr int kKbPtTile = 4096;               // points per partition tile
 constexpr int kKbPrTile = 4096;               // queries per partition tile (two probes each)
 constexpr uint32_t kKbMinKeys = 1u << kWinBits;   // smaller domains stay with the state-block pipeline
@@ -18,7 +19,8 @@ constexpr uint32_t kKbMinKeys = 1u << kWinBits;   // smaller domains stay with t
 enum {
   KB_SOFF, KB_TEOFF, KB_TQOFF, KB_TC, KB_TBOFF, KB_TBITS, KB_TCARRY, KB_TGSUM, KB_LASTQ, KB_MISC, KB_EOFF, KB_QOFF,
   KB_FORK, KB_NEXT, KB_CNT, KB_EHEAD, KB_XHEAD, KB_RANK, KB_SCAN, KB_STEP, KB_W, KB_EP, KB_TIME, KB_COLSTATE,
-  KB_COLTIME, KB_COLSTEP, KB_POS, KB_PTHIST, KB_PTS, KB_SEG, KB_ROWS, KB_PRHIST, KB_PRS, KB_ACC, KB_COUNT
+  KB_COLTIME, KB_COLSTEP, KB_POS, KB_TOUR, KB_PTHIST, KB_PTOFF, KB_PTS, KB_SEG, KB_ROWS, KB_PRHIST,
+  KB_PROFF, KB_PART, KB_PRS, KB_ACC, KB_COUNT
 };
 
 struct KbSpec {

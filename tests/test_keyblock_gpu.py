@@ -23,7 +23,7 @@ CASES = [
     ("fork", 2000, 300_000, 30000, 4097, "uniform", "one_state"),
     ("fork", 2000, 300_000, 30000, 1, "uniform", "any"),
     ("fork", 40000, 300_000, 1, 2000, "uniform", "any"),
-    ("fork", 30000, 500_000, 900_000, 300_000, "uniform", "any"),    # two steps of slots a block
+    ("fork", 30000, 500_000, 1_000_000, 300_000, "uniform", "any"),  # two steps of slots a block
 ]
 
 
@@ -56,7 +56,7 @@ def test_matches_oracle_and_state_blocks(bw, torch_cuda, oracle_mod, case):
         plan.launch(p, e, q, got)
         assert plan.status() == 0
         np.testing.assert_array_equal(got.cpu().numpy(), want)
-    m = 512 * (len(ev) // (8 * bw.device_info()[0] * 512) + 1)
+    m = 512 * (len(ev) // (12 * bw.device_info()[0] * 512) + 1)
     assert plan.info()[1] == len(ev) // m + 1, "not the key-block path"
     np.testing.assert_array_equal(bw.replay(p, C, e, q, path="general").cpu().numpy(), want)
 
