@@ -6,10 +6,9 @@
 // Over a sparse 2^40-key universe a bitmap is not affordable, so here the same rank
 // (number of index keys below k) and the same range sum (pre[rank(hi)-1] -
 // pre[rank(lo)-1]) come from:
-//   build    LSD radix sort of the (key, amount) pairs, 8 bits per pass, stable
-//            tile scatter (per-warp digit counts, __match_any_sync ranks);
-//            run-length merge of equal keys with the amounts summed; inclusive scan
-//            of the amounts (the cumulative prefix `pre`); a bucket LUT
+//   build    LSD radix sort of the (key, amount) pairs, 8 bits per pass
+//            (bw_sort.cuh); run-length merge of equal keys with the cumulative
+//            amounts (the prefix `pre`) in two passes over the pairs; a bucket LUT
 //            lut[b] = #keys below b << shift sized to the caller's byte budget,
 //            filled by warps that each cover the bucket gaps of 32 keys with
 //            coalesced stores; the low `shift` bits of every key as u16 when
@@ -22,118 +21,155 @@
 
 #include "bw_gpu.h"
 #include "bw_common.cuh"
+#include "bw_sort.cuh"
 
 namespace bw {
 namespace {
 
-constexpr int kSortThreads = 256;
-constexpr int kSortItems = 16;                          // per thread
-constexpr int kSortTile = kSortThreads * kSortItems;    // 4096 pairs per CTA
-constexpr int kSortWarps = kSortThreads / 32;
-constexpr int kDigits = 256;
-
 inline size_t al256(size_t x) { return (x + 255) & ~size_t(255); }
 
-// Per-tile digit counts, digit-major: hist[d * ntiles + tile].
-// The first pass (check_bits > 0) also flags keys outside [0, 2^check_bits).
-__global__ void __launch_bounds__(kSortThreads) k_sort_hist(const uint64_t* __restrict__ keys, int64_t n,
-                                                            int shift, int64_t ntiles, int64_t* __restrict__ hist,
-                                                            int check_bits, int32_t* __restrict__ status) {
-  __shared__ unsigned cnt[kDigits];
-  cnt[threadIdx.x] = 0;
-  __syncthreads();
-  const int64_t base = (int64_t)blockIdx.x * kSortTile;
-  bool bad = false;
-#pragma unroll 4
-  for (int j = 0; j < kSortItems; ++j) {
-    const int64_t i = base + (int64_t)j * kSortThreads + threadIdx.x;
-    if (i < n) {
-      const uint64_t k = keys[i];
-      atomicAdd(&cnt[(unsigned)(k >> shift) & 255u], 1u);
-      if (check_bits > 0 && (k >> check_bits) != 0) bad = true;
-    }
+// Sort pass over (key, amount) pairs kept in two arrays.
+struct CsrIO {
+  const uint64_t* k;
+  const int64_t* v;
+  uint64_t* ko;
+  int64_t* vo;
+  int bits;
+  static constexpr int kBadStatus = 1;
+  __device__ __forceinline__ uint4 load(int64_t i) const {
+    const uint64_t a = k[i], b = (uint64_t)v[i];
+    return make_uint4((uint32_t)a, (uint32_t)(a >> 32), (uint32_t)b, (uint32_t)(b >> 32));
   }
-  if (bad) atomicExch(status, 1);
-  __syncthreads();
-  hist[(int64_t)threadIdx.x * ntiles + blockIdx.x] = cnt[threadIdx.x];
-}
+  __device__ __forceinline__ uint32_t key(int64_t i, int shift) const { return (uint32_t)(k[i] >> shift); }
+  __device__ __forceinline__ bool bad(int64_t i) const { return (k[i] >> bits) != 0; }
+  static __device__ __forceinline__ uint32_t digits(const uint4& x, int shift) {
+    return (uint32_t)((((uint64_t)x.y << 32) | x.x) >> shift);
+  }
+  __device__ __forceinline__ void store(int64_t at, const uint4& x) const {
+    ko[at] = ((uint64_t)x.y << 32) | x.x;
+    vo[at] = (int64_t)(((uint64_t)x.w << 32) | x.z);
+  }
+};
 
-// Stable scatter of one tile by digit.  Warp w owns items [w*32*kSortItems, ...) of
-// the tile in groups of 32; ranks inside a group come from __match_any_sync, and
-// groups, warps and tiles are taken in input order, so equal digits keep their order.
-__global__ void __launch_bounds__(kSortThreads) k_sort_scatter(
-    const uint64_t* __restrict__ kin, const int64_t* __restrict__ vin, uint64_t* __restrict__ kout,
-    int64_t* __restrict__ vout, int64_t n, int shift, int64_t ntiles, const int64_t* __restrict__ hist_incl) {
-  __shared__ unsigned wcnt[kSortWarps][kDigits];
-  __shared__ int64_t dbase[kDigits];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  for (int w = 0; w < kSortWarps; ++w) wcnt[w][threadIdx.x] = 0;
-  __syncthreads();
-  const int64_t base = (int64_t)blockIdx.x * kSortTile + (int64_t)warp * (32 * kSortItems);
-  uint64_t k[kSortItems];
-  int64_t v[kSortItems];
-#pragma unroll
-  for (int j = 0; j < kSortItems; ++j) {
-    const int64_t i = base + j * 32 + lane;
-    k[j] = i < n ? kin[i] : 0;
-    v[j] = i < n ? vin[i] : 0;
+// Run-length merge of the sorted pairs in two passes over them: run ends and amounts
+// per tile, then (with the tiles' prefixes) every run's key, cumulative amount and low
+// bits at its place.  A warp takes 256 consecutive pairs, two per lane and round.
+// (Separate flag, scan and compaction kernels moved 2 GB for 20M pairs and took 290 us; now 66 + 11 + 134.)
+constexpr int kRunThreads = 512, kRunRounds = 4;
+constexpr int64_t kRunTile = (int64_t)kRunThreads * 2 * kRunRounds;
+struct RunPair {
+  uint64_t k0, k1, v0, v1;
+  bool f0, f1;               // the pair's items end a run
+  // items i and i + 1 (i even) of n; every lane of the warp calls it, lanes consecutive
+  __device__ __forceinline__ RunPair(const uint64_t* __restrict__ k, const int64_t* __restrict__ v, int64_t i, int64_t n) {
+    k0 = k1 = v0 = v1 = 0;
+    if (i + 1 < n) {
+      const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(k + i);
+      const longlong2 b = *reinterpret_cast<const longlong2*>(v + i);
+      k0 = a.x; k1 = a.y; v0 = (uint64_t)b.x; v1 = (uint64_t)b.y;
+    } else if (i < n) {
+      k0 = k[i]; v0 = (uint64_t)v[i];
+    }
+    uint64_t next = __shfl_down_sync(0xffffffffu, k0, 1);
+    if ((threadIdx.x & 31) == 31 && i + 2 < n) next = k[i + 2];
+    f0 = i < n && (i + 1 == n || k1 != k0);
+    f1 = i + 1 < n && (i + 2 == n || next != k1);
   }
+};
+__device__ __forceinline__ int64_t run_at(int r) {
+  return (int64_t)blockIdx.x * kRunTile + (int64_t)(threadIdx.x >> 5) * (64 * kRunRounds) + r * 64 +
+         2 * (int64_t)(threadIdx.x & 31);
+}
+__global__ void __launch_bounds__(kRunThreads) k_run_sums(const uint64_t* __restrict__ k, const int64_t* __restrict__ v,
+                                                          int64_t n, uint64_t* __restrict__ part) {
+  uint64_t ends = 0, sum = 0;
+#pragma unroll
+  for (int r = 0; r < kRunRounds; ++r) {
+    const RunPair x(k, v, run_at(r), n);
+    ends += (x.f0 ? 1 : 0) + (x.f1 ? 1 : 0);
+    sum += x.v0 + x.v1;
+  }
+  uint64_t te = 0, ts = 0;
+  block_exclusive_scan<uint64_t>(ends, &te);
+  block_exclusive_scan<uint64_t>(sum, &ts);
+  if (threadIdx.x == 0) {
+    part[2 * (int64_t)blockIdx.x] = te;
+    part[2 * (int64_t)blockIdx.x + 1] = ts;
+  }
+}
+__global__ void __launch_bounds__(1024) k_run_parts(uint64_t* part, int64_t tiles) {
+  uint64_t ce = 0, cs = 0;
+  for (int64_t t0 = 0; t0 < tiles; t0 += 1024) {
+    const int64_t t = t0 + threadIdx.x;
+    const uint64_t e = t < tiles ? part[2 * t] : 0, s = t < tiles ? part[2 * t + 1] : 0;
+    uint64_t te = 0, ts = 0;
+    const uint64_t xe = block_exclusive_scan<uint64_t>(e, &te), xs = block_exclusive_scan<uint64_t>(s, &ts);
+    if (t < tiles) {
+      part[2 * t] = ce + xe;
+      part[2 * t + 1] = cs + xs;
+    }
+    ce += te;
+    cs += ts;
+  }
+}
+__global__ void __launch_bounds__(kRunThreads) k_run_write(const uint64_t* __restrict__ k, const int64_t* __restrict__ v,
+                                                           int64_t n, int shift, const uint64_t* __restrict__ part,
+                                                           uint64_t* __restrict__ ukeys, int64_t* __restrict__ pre,
+                                                           uint16_t* __restrict__ low, int64_t* __restrict__ count) {
+  __shared__ uint64_t s_e[kRunThreads / 32], s_s[kRunThreads / 32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const unsigned lt = (1u << lane) - 1u;
-#pragma unroll
-  for (int j = 0; j < kSortItems; ++j) {
-    const bool valid = base + j * 32 + lane < n;
-    const unsigned d = valid ? ((unsigned)(k[j] >> shift) & 255u) : 256u;
-    const unsigned peers = __match_any_sync(0xffffffffu, d);
-    if (valid && (peers & lt) == 0) wcnt[warp][d] += __popc(peers);
-    __syncwarp();
-  }
-  __syncthreads();
-  {
-    const int d = threadIdx.x;
-    unsigned run = 0;
-    for (int w = 0; w < kSortWarps; ++w) {
-      const unsigned c = wcnt[w][d];
-      wcnt[w][d] = run;
-      run += c;
-    }
-    dbase[d] = hist_incl[(int64_t)d * ntiles + blockIdx.x] - (int64_t)run;
-  }
-  __syncthreads();
-#pragma unroll
-  for (int j = 0; j < kSortItems; ++j) {
-    const bool valid = base + j * 32 + lane < n;
-    const unsigned d = valid ? ((unsigned)(k[j] >> shift) & 255u) : 256u;
-    const unsigned peers = __match_any_sync(0xffffffffu, d);
-    if (valid) {
-      const int64_t pos = dbase[d] + wcnt[warp][d] + __popc(peers & lt);
-      kout[pos] = k[j];
-      vout[pos] = v[j];
-    }
-    __syncwarp();
-    if (valid && (peers & lt) == 0) wcnt[warp][d] += __popc(peers);
-    __syncwarp();
-  }
-}
-
-// flag[i] = 1 where i is the last item of a run of equal keys.
-__global__ void k_run_flags(const uint64_t* __restrict__ k, int64_t n, int64_t* __restrict__ flag) {
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    flag[i] = (i + 1 == n || k[i + 1] != k[i]) ? 1 : 0;
-}
-
-// The last item of every run writes its key, the cumulative amount and the low bits
-// at its run index (pos[i] - 1); the last item overall writes the count.
-__global__ void k_run_compact(const uint64_t* __restrict__ k, const int64_t* __restrict__ vscan,
-                              const int64_t* __restrict__ pos, int64_t n, int shift, uint64_t* __restrict__ ukeys,
-                              int64_t* __restrict__ pre, uint16_t* __restrict__ low, int64_t* __restrict__ count) {
   const uint64_t mask = shift >= 64 ? ~0ull : ((1ull << shift) - 1ull);
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    if (i + 1 == n || k[i + 1] != k[i]) {
-      const int64_t u = pos[i] - 1;
-      ukeys[u] = k[i];
-      pre[u] = vscan[i];
-      if (low) low[u] = (uint16_t)(k[i] & mask);
-      if (i + 1 == n) *count = pos[i];
+  uint64_t k0[kRunRounds], k1[kRunRounds], c0[kRunRounds], c1[kRunRounds];   // keys, cumulative amounts in the warp
+  uint32_t at[kRunRounds], f[kRunRounds];
+  uint32_t ends = 0;
+  uint64_t run = 0;
+#pragma unroll
+  for (int r = 0; r < kRunRounds; ++r) {
+    const RunPair x(k, v, run_at(r), n);
+    const unsigned m0 = __ballot_sync(0xffffffffu, x.f0), m1 = __ballot_sync(0xffffffffu, x.f1);
+    at[r] = ends + __popc(m0 & lt) + __popc(m1 & lt);
+    ends += __popc(m0) + __popc(m1);
+    f[r] = (x.f0 ? 1u : 0u) | (x.f1 ? 2u : 0u);
+    const uint64_t s = x.v0 + x.v1;
+    uint64_t incl = s;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint64_t y = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += y;
+    }
+    k0[r] = x.k0;
+    k1[r] = x.k1;
+    c0[r] = run + incl - x.v1;
+    c1[r] = run + incl;
+    run += __shfl_sync(0xffffffffu, incl, 31);
+  }
+  if (lane == 0) {
+    s_e[warp] = ends;
+    s_s[warp] = run;
+  }
+  __syncthreads();
+  uint64_t be = part[2 * (int64_t)blockIdx.x], bs = part[2 * (int64_t)blockIdx.x + 1];
+  for (int w = 0; w < warp; ++w) {
+    be += s_e[w];
+    bs += s_s[w];
+  }
+#pragma unroll
+  for (int r = 0; r < kRunRounds; ++r) {
+    int64_t u = (int64_t)(be + at[r]);
+    const int64_t i = run_at(r);
+    if (f[r] & 1u) {
+      ukeys[u] = k0[r];
+      pre[u] = (int64_t)(bs + c0[r]);
+      if (low) low[u] = (uint16_t)(k0[r] & mask);
+      ++u;
+      if (i + 1 == n) *count = u;
+    }
+    if (f[r] & 2u) {
+      ukeys[u] = k1[r];
+      pre[u] = (int64_t)(bs + c1[r]);
+      if (low) low[u] = (uint16_t)(k1[r] & mask);
+      if (i + 2 == n) *count = u + 1;
     }
   }
 }
@@ -181,14 +217,29 @@ __global__ void k_lut_tail(const uint64_t* __restrict__ ukeys, const int64_t* __
     lut[b] = (uint32_t)m;
 }
 
-// rank(k) = number of index keys below k; *present when k is one of them.
+// rank(k) = number of index keys below k; *present when k is one of them.  V4: the
+// LUT is read as aligned groups of four entries, which hold both ends of a bucket three
+// times in four (the lookups are bound by the sectors the L1 and L2 serve; 100M point
+// lookups: 1.11 -> 1.04 ms).
+template <bool V4>
 __device__ __forceinline__ int64_t csr_rank(const BwCsr& x, int64_t m, uint64_t k, bool& present) {
   present = false;
   if (x.key_bits < 64 && (k >> x.key_bits) != 0) return m;
   const int64_t b = (int64_t)(k >> x.shift);
+  int64_t lo, hi;
+  if constexpr (V4) {
+    const uint4 q = __ldg(reinterpret_cast<const uint4*>(x.lut) + (b >> 2));
+    const int c = (int)(b & 3);
+    lo = c == 0 ? q.x : c == 1 ? q.y : c == 2 ? q.z : q.w;
+    hi = c == 0 ? q.y : c == 1 ? q.z : q.w;
+    if (c == 3) hi = b + 1 < x.n_buckets ? (int64_t)__ldg(x.lut + b + 1) : m;
+  } else {
+    lo = __ldg(x.lut + b);
+    hi = b + 1 < x.n_buckets ? (int64_t)__ldg(x.lut + b + 1) : m;
+  }
   // clamped to [0, m]: an index built from flagged input stays memory-safe
-  int64_t lo = imin64(__ldg(x.lut + b), m);
-  int64_t hi = b + 1 < x.n_buckets ? imin64(__ldg(x.lut + b + 1), m) : m;
+  lo = imin64(lo, m);
+  hi = imin64(hi, m);
   const int64_t end = hi;   // the bucket's keys are [lo, end)
   if (x.low) {
     // keys of one bucket share their high bits: compare the low `shift` bits
@@ -208,41 +259,60 @@ __device__ __forceinline__ int64_t csr_rank(const BwCsr& x, int64_t m, uint64_t 
   return lo;
 }
 
+// Lookup inputs and outputs are streamed (evict first): they are read or written once,
+// and the L2 is left to the index.
+__device__ __forceinline__ ulonglong2 stream_ld(const ulonglong2* p) { return __ldcs(p); }
+
+template <bool V4>
 __global__ void k_csr_point(BwCsr x, const uint64_t* __restrict__ keys, int64_t n, int64_t* __restrict__ out) {
   const int64_t m = *x.count;
   const int64_t npairs = n >> 1;
   const ulonglong2* kv = reinterpret_cast<const ulonglong2*>(keys);
   longlong2* ov = reinterpret_cast<longlong2*>(out);
   for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < npairs; p += (int64_t)gridDim.x * blockDim.x) {
-    const ulonglong2 k = kv[p];
+    const ulonglong2 k = stream_ld(kv + p);
     bool pa, pb;
-    const int64_t ra = csr_rank(x, m, k.x, pa);
-    const int64_t rb = csr_rank(x, m, k.y, pb);
-    ov[p] = make_longlong2(pa ? ra : -ra - 1, pb ? rb : -rb - 1);
+    const int64_t ra = csr_rank<V4>(x, m, k.x, pa);
+    const int64_t rb = csr_rank<V4>(x, m, k.y, pb);
+    __stcs(ov + p, make_longlong2(pa ? ra : -ra - 1, pb ? rb : -rb - 1));
   }
   if ((n & 1) && blockIdx.x == 0 && threadIdx.x == 0) {
     bool pr;
-    const int64_t r = csr_rank(x, m, keys[n - 1], pr);
+    const int64_t r = csr_rank<V4>(x, m, keys[n - 1], pr);
     out[n - 1] = pr ? r : -r - 1;
   }
 }
 
-__global__ void k_csr_range(BwCsr x, const uint64_t* __restrict__ bounds, int64_t n, int64_t* __restrict__ out) {
+// Range lookups in two kernels: the ranks of both bounds into `out`, then their
+// difference and the amounts between them.  LUT, low bits and prefix sums together
+// (164 MB for 10M keys and a 64 MiB LUT) do not stay in the L2; either kernel's share
+// does, and the 3.2 GB of ranks written and read back for 100M ranges cost less than
+// the misses (one kernel: 5.87 ms; two: 1.83 + 1.23 ms).
+template <bool V4>
+__global__ void k_csr_range_ranks(BwCsr x, const uint64_t* __restrict__ bounds, int64_t n, int64_t* __restrict__ out) {
   const int64_t m = *x.count;
   const ulonglong2* bv = reinterpret_cast<const ulonglong2*>(bounds);
   longlong2* ov = reinterpret_cast<longlong2*>(out);
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    const ulonglong2 q = bv[i];
+    const ulonglong2 q = stream_ld(bv + i);
     bool pr;
-    const int64_t a = csr_rank(x, m, q.x, pr);
-    const int64_t b = csr_rank(x, m, q.y, pr);
+    const int64_t a = csr_rank<V4>(x, m, q.x, pr);
+    const int64_t b = csr_rank<V4>(x, m, q.y, pr);
+    __stcs(ov + i, make_longlong2(a, b));
+  }
+}
+__global__ void k_csr_range_sums(BwCsr x, int64_t n, int64_t* out) {
+  longlong2* ov = reinterpret_cast<longlong2*>(out);
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    const longlong2 r = __ldcs(ov + i);
+    const int64_t a = r.x, b = r.y;
     uint64_t sum = 0;
     if (a != b) {
       const uint64_t shi = b ? (uint64_t)__ldg(x.pre + b - 1) : 0;
       const uint64_t slo = a ? (uint64_t)__ldg(x.pre + a - 1) : 0;
       sum = shi - slo;
     }
-    ov[i] = make_longlong2(b - a, (int64_t)sum);
+    __stcs(ov + i, make_longlong2(b - a, (int64_t)sum));
   }
 }
 
@@ -251,44 +321,49 @@ __global__ void k_csr_range(BwCsr x, const uint64_t* __restrict__ bounds, int64_
 // the replay reports as out of range), and query records over rank intervals -- a
 // point lookup of a present key is [rank, rank + 1), of an absent one empty; a range
 // lookup [lo, hi) over keys is [rank(lo), rank(hi)) over ranks.
+template <bool V4>
 __global__ void k_csr_events(BwCsr x, const uint32_t* __restrict__ states, const uint64_t* __restrict__ keys,
                              const int64_t* __restrict__ deltas, int64_t n, BwEvent* __restrict__ out) {
   const int64_t m = *x.count;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     bool pr;
-    const int64_t r = csr_rank(x, m, keys[i], pr);
+    const int64_t r = csr_rank<V4>(x, m, __ldcs(keys + i), pr);
     BwEvent e;
-    e.state = states[i];
+    e.state = __ldcs(states + i);
     e.key = (uint32_t)(pr ? r : m);
-    e.delta = deltas[i];
+    e.delta = __ldcs(deltas + i);
     out[i] = e;
   }
 }
+template <bool V4>
 __global__ void k_csr_queries(BwCsr x, const uint32_t* __restrict__ states, const uint64_t* __restrict__ lo,
                               const uint64_t* __restrict__ hi, int64_t n, BwQuery* __restrict__ out) {
   const int64_t m = *x.count;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     bool pr;
-    const int64_t a = csr_rank(x, m, lo[i], pr);
+    const int64_t a = csr_rank<V4>(x, m, __ldcs(lo + i), pr);
     BwQuery q;
-    q.state = states[i];
+    q.state = __ldcs(states + i);
     if (!hi) {
       q.lo = pr ? (uint32_t)a : 0u;
       q.hi = pr ? (uint32_t)a + 1u : 0u;
     } else {
       bool pb;
       q.lo = (uint32_t)a;
-      q.hi = (uint32_t)csr_rank(x, m, hi[i], pb);
+      q.hi = (uint32_t)csr_rank<V4>(x, m, __ldcs(hi + i), pb);
     }
-    out[i] = q;
+    __stcs(&out[i].state, q.state);
+    __stcs(&out[i].lo, q.lo);
+    __stcs(&out[i].hi, q.hi);
   }
 }
 
 struct CsrLayout {
   int32_t shift = 0, passes = 0;
-  int64_t nb = 0, ntiles = 0;
+  int64_t nb = 0;
+  RsLayout rs;
   size_t off_count, off_status, off_keys, off_pre, off_low, off_lut;     // persistent index
-  size_t off_ka, off_va, off_kb, off_vb, off_hist, off_tmp;  // build scratch
+  size_t off_ka, off_va, off_kb, off_vb, off_hist, off_part, off_base, off_runs;  // build scratch
   size_t total;
 };
 
@@ -299,7 +374,7 @@ int csr_layout(int64_t n, int32_t key_bits, size_t budget, CsrLayout& L) {
   L.nb = (int64_t)1 << lb;
   L.shift = key_bits - lb;
   L.passes = (key_bits + 7) / 8;
-  L.ntiles = (n + kSortTile - 1) / kSortTile;
+  L.rs = rs_layout(n, L.passes);
   const size_t un = (size_t)(n > 0 ? n : 1);
   size_t o = 0;
   auto take = [&](size_t bytes) { const size_t at = o; o = al256(o + bytes); return at; };
@@ -313,10 +388,10 @@ int csr_layout(int64_t n, int32_t key_bits, size_t budget, CsrLayout& L) {
   L.off_va = take(un * 8);
   L.off_kb = take(un * 8);
   L.off_vb = take(un * 8);
-  const size_t nh = (size_t)kDigits * (size_t)(L.ntiles > 0 ? L.ntiles : 1);
-  L.off_hist = take(nh * 8);
-  const size_t scan_n = nh > un ? nh : un;
-  L.off_tmp = take(scan_tmp_bytes(scan_n));
+  L.off_hist = take(L.rs.hist);
+  L.off_part = take(L.rs.part);
+  L.off_base = take(L.rs.base);
+  L.off_runs = take(((un + kRunTile - 1) / kRunTile) * 16);
   L.total = o;
   return 0;
 }
@@ -371,46 +446,37 @@ extern "C" int bw_csr_build(const uint64_t* keys, const int64_t* amounts, int64_
   int64_t* va = reinterpret_cast<int64_t*>(ws + L.off_va);
   uint64_t* kb = reinterpret_cast<uint64_t*>(ws + L.off_kb);
   int64_t* vb = reinterpret_cast<int64_t*>(ws + L.off_vb);
-  int64_t* hist = reinterpret_cast<int64_t*>(ws + L.off_hist);
-  int64_t* tmp = reinterpret_cast<int64_t*>(ws + L.off_tmp);
+  uint32_t* hist = reinterpret_cast<uint32_t*>(ws + L.off_hist);
+  uint32_t* part = reinterpret_cast<uint32_t*>(ws + L.off_part);
+  uint64_t* base = reinterpret_cast<uint64_t*>(ws + L.off_base);
+  uint64_t* runs = reinterpret_cast<uint64_t*>(ws + L.off_runs);
   int rc;
-  int kernels = 0;
   if ((rc = report(cudaMemsetAsync(count, 0, 8, st), "memset"))) return rc;
   if ((rc = report(cudaMemsetAsync(status, 0, 4, st), "memset"))) return rc;
   const int64_t n = n_items;
-  uint64_t* ksorted = ka;
-  int64_t* vsorted = va;
   if (n > 0) {
-    // ---- LSD radix sort, 8 bits per pass; pass p reads (src) and writes (dst)
-    const uint64_t* ksrc = keys;
-    const int64_t* vsrc = amounts;
-    uint64_t* kdst = ka;
-    int64_t* vdst = va;
+    // ---- LSD radix sort, 8 bits per pass; pass p reads (k, v) and writes (ko, vo)
+    if ((rc = report(cudaMemsetAsync(part, 0, L.rs.part, st), "memset"))) return rc;
+    CsrIO io{keys, amounts, ka, va, key_bits};
     for (int p = 0; p < L.passes; ++p) {
-      const int shift = 8 * p;
-      k_sort_hist<<<(unsigned)L.ntiles, kSortThreads, 0, st>>>(ksrc, n, shift, L.ntiles, hist,
-                                                                p == 0 ? key_bits : 0, status);
-      if ((rc = report(cudaGetLastError(), "k_sort_hist"))) return rc;
-      if ((rc = device_inclusive_scan_i64(hist, (int64_t)kDigits * L.ntiles, tmp, st, kernels))) return rc;
-      k_sort_scatter<<<(unsigned)L.ntiles, kSortThreads, 0, st>>>(ksrc, vsrc, kdst, vdst, n, shift, L.ntiles, hist);
-      if ((rc = report(cudaGetLastError(), "k_sort_scatter"))) return rc;
-      ksorted = kdst;
-      vsorted = vdst;
-      ksrc = kdst;
-      vsrc = vdst;
-      kdst = (kdst == ka) ? kb : ka;
-      vdst = (vdst == va) ? vb : va;
+      if ((rc = report((cudaError_t)rs_pass(io, n, 8 * p, L.rs, hist, part + (size_t)p * L.rs.chunks * kRsDigits, base,
+                                            p == 0, status, st), "sort pass")))
+        return rc;
+      io.k = io.ko;
+      io.v = io.vo;
+      io.ko = io.k == ka ? kb : ka;
+      io.vo = io.v == va ? vb : va;
     }
-    // ---- run-length merge: cumulative amounts (inclusive scan of the sorted
-    // amounts, read at the last item of each run) and run indices
-    int64_t* pos = reinterpret_cast<int64_t*>(ksorted == ka ? kb : ka);   // free buffer
-    const int g = grid_for(n, 256);
-    k_run_flags<<<g, 256, 0, st>>>(ksorted, n, pos);
-    if ((rc = report(cudaGetLastError(), "k_run_flags"))) return rc;
-    if ((rc = device_inclusive_scan_i64(pos, n, tmp, st, kernels))) return rc;
-    if ((rc = device_inclusive_scan_i64(vsorted, n, tmp, st, kernels))) return rc;
-    k_run_compact<<<g, 256, 0, st>>>(ksorted, vsorted, pos, n, L.shift, ukeys, pre, low, count);
-    if ((rc = report(cudaGetLastError(), "k_run_compact"))) return rc;
+    const uint64_t* ksorted = io.k;
+    const int64_t* vsorted = io.v;
+    // ---- run-length merge
+    const int64_t tiles = (n + kRunTile - 1) / kRunTile;
+    k_run_sums<<<(unsigned)tiles, kRunThreads, 0, st>>>(ksorted, vsorted, n, runs);
+    if ((rc = report(cudaGetLastError(), "k_run_sums"))) return rc;
+    k_run_parts<<<1, 1024, 0, st>>>(runs, tiles);
+    if ((rc = report(cudaGetLastError(), "k_run_parts"))) return rc;
+    k_run_write<<<(unsigned)tiles, kRunThreads, 0, st>>>(ksorted, vsorted, n, L.shift, runs, ukeys, pre, low, count);
+    if ((rc = report(cudaGetLastError(), "k_run_write"))) return rc;
     k_lut_fill<<<grid_for(n, 256), 256, 0, st>>>(ukeys, count, L.shift, L.nb, lut);
     if ((rc = report(cudaGetLastError(), "k_lut_fill"))) return rc;
   }
@@ -428,6 +494,9 @@ extern "C" int bw_csr_build(const uint64_t* keys, const int64_t* amounts, int64_
   return 0;
 }
 
+// Whether the LUT can be read as groups of four entries.
+static bool lut4(const BwCsr* x) { return (reinterpret_cast<uintptr_t>(x->lut) & 15) == 0 && x->n_buckets >= 4; }
+
 static int check_index(const BwCsr* x) {
   if (!x || !x->count || !x->status || !x->lut || !x->keys || !x->pre || x->key_bits < 1 || x->key_bits > 63 || x->shift < 0 ||
       x->shift > x->key_bits || x->n_buckets != ((int64_t)1 << (x->key_bits - x->shift)) || (x->low && x->shift > 16))
@@ -439,7 +508,8 @@ extern "C" int bw_csr_point(const BwCsr* idx, const uint64_t* keys, int64_t n, i
   if (check_index(idx) || n < 0 || (n > 0 && (!keys || !out))) return BW_EINVAL;
   if (n == 0) return 0;
   if ((reinterpret_cast<uintptr_t>(keys) & 15) || (reinterpret_cast<uintptr_t>(out) & 15)) return BW_EINVAL;
-  k_csr_point<<<grid_for((n + 1) / 2, 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(*idx, keys, n, out);
+  (lut4(idx) ? k_csr_point<true> : k_csr_point<false>)<<<grid_for((n + 1) / 2, 256), 256, 0,
+                                                         static_cast<cudaStream_t>(stream)>>>(*idx, keys, n, out);
   return report(cudaGetLastError(), "k_csr_point");
 }
 
@@ -447,8 +517,12 @@ extern "C" int bw_csr_range(const BwCsr* idx, const uint64_t* bounds, int64_t n,
   if (check_index(idx) || n < 0 || (n > 0 && (!bounds || !out))) return BW_EINVAL;
   if (n == 0) return 0;
   if ((reinterpret_cast<uintptr_t>(bounds) & 15) || (reinterpret_cast<uintptr_t>(out) & 15)) return BW_EINVAL;
-  k_csr_range<<<grid_for(n, 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(*idx, bounds, n, out);
-  return report(cudaGetLastError(), "k_csr_range");
+  const cudaStream_t st = static_cast<cudaStream_t>(stream);
+  (lut4(idx) ? k_csr_range_ranks<true> : k_csr_range_ranks<false>)<<<grid_for(n, 256), 256, 0, st>>>(*idx, bounds, n, out);
+  const int rc = report(cudaGetLastError(), "k_csr_range_ranks");
+  if (rc) return rc;
+  k_csr_range_sums<<<grid_for(n, 256), 256, 0, st>>>(*idx, n, out);
+  return report(cudaGetLastError(), "k_csr_range_sums");
 }
 
 extern "C" int bw_csr_status(const BwCsr* idx, int32_t* status) {
@@ -462,7 +536,9 @@ extern "C" int bw_csr_events(const BwCsr* idx, const uint32_t* states, const uin
                              int64_t n, BwEvent* out, void* stream) {
   if (check_index(idx) || n < 0 || (n > 0 && (!states || !keys || !deltas || !out))) return BW_EINVAL;
   if (n == 0) return 0;
-  k_csr_events<<<grid_for(n, 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(*idx, states, keys, deltas, n, out);
+  (lut4(idx) ? k_csr_events<true> : k_csr_events<false>)<<<grid_for(n, 256), 256, 0,
+                                                           static_cast<cudaStream_t>(stream)>>>(*idx, states, keys,
+                                                                                                deltas, n, out);
   return report(cudaGetLastError(), "k_csr_events");
 }
 
@@ -470,6 +546,8 @@ extern "C" int bw_csr_queries(const BwCsr* idx, const uint32_t* states, const ui
                               int64_t n, BwQuery* out, void* stream) {
   if (check_index(idx) || n < 0 || (n > 0 && (!states || !lo || !out))) return BW_EINVAL;
   if (n == 0) return 0;
-  k_csr_queries<<<grid_for(n, 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(*idx, states, lo, hi, n, out);
+  (lut4(idx) ? k_csr_queries<true> : k_csr_queries<false>)<<<grid_for(n, 256), 256, 0,
+                                                             static_cast<cudaStream_t>(stream)>>>(*idx, states, lo, hi,
+                                                                                                  n, out);
   return report(cudaGetLastError(), "k_csr_queries");
 }
