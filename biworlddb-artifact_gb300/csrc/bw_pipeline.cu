@@ -423,6 +423,7 @@ struct PrepParams {
 // so steps with few events still fill the warp.  Loop bounds are warp-uniform and f
 // is called by all 32 lanes (valid marks real events), so f may use warp-collective
 // operations.
+constexpr int kPrepBatch = 4;
 template <typename F>
 __device__ __forceinline__ void for_block_events(const PrepParams& p, int32_t t0, int32_t t1, int mode, F&& f) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
@@ -460,30 +461,34 @@ __device__ __forceinline__ void for_block_events(const PrepParams& p, int32_t t0
       if (lane >= o) incl += y;
     }
     const int32_t total = __shfl_sync(0xffffffffu, incl, 31);
-    for (int32_t g0 = 0; g0 < total; g0 += 32) {
-      const int32_t g = g0 + lane;
-      int32_t lo = 0, hi = 31;   // first lane whose inclusive count exceeds g
+    // kPrepBatch flattened events a lane at a time: their reads are in flight together
+    // (one at a time left a memory latency per 32 events of a warp)
+    for (int32_t g0 = 0; g0 < total; g0 += 32 * kPrepBatch) {
+      uint4 e[kPrepBatch];
+      uint32_t fl[kPrepBatch];   // 1: an event, 2: negated, 4: twice
 #pragma unroll
-      for (int it = 0; it < 5; ++it) {
-        const int32_t mid = (lo + hi) >> 1;
-        const int32_t v = __shfl_sync(0xffffffffu, incl, mid);
-        if (v > g) hi = mid; else lo = mid + 1;
+      for (int u = 0; u < kPrepBatch; ++u) {
+        const int32_t g = g0 + 32 * u + lane;
+        int32_t lo = 0, hi = 31;   // first lane whose inclusive count exceeds g
+#pragma unroll
+        for (int it = 0; it < 5; ++it) {
+          const int32_t mid = (lo + hi) >> 1;
+          const int32_t v = __shfl_sync(0xffffffffu, incl, mid);
+          if (v > g) hi = mid; else lo = mid + 1;
+        }
+        const int32_t off = __shfl_sync(0xffffffffu, incl - cnt, lo);
+        const uint32_t s_e0 = __shfl_sync(0xffffffffu, e0, lo);
+        fl[u] = __shfl_sync(0xffffffffu, 1u | (neg ? 2u : 0u) | (twice ? 4u : 0u), lo);
+        e[u] = make_uint4(0, 0, 0, 0);
+        if (g < total) e[u] = __ldg(reinterpret_cast<const uint4*>(p.ev) + ((int64_t)s_e0 + (g - off)));
+        else fl[u] = 0;
       }
-      const int32_t src = lo;
-      const int32_t s_incl = __shfl_sync(0xffffffffu, incl, src);
-      const int32_t s_cnt = __shfl_sync(0xffffffffu, cnt, src);
-      const uint32_t s_e0 = __shfl_sync(0xffffffffu, e0, src);
-      const bool s_neg = __shfl_sync(0xffffffffu, neg ? 1 : 0, src) != 0;
-      const bool s_twice = __shfl_sync(0xffffffffu, twice ? 1 : 0, src) != 0;
-      const bool valid = g < total;
-      uint32_t k = 0;
-      uint64_t v = 0;
-      if (valid) {
-        const BwEvent e = p.ev[(int64_t)s_e0 + (g - (s_incl - s_cnt))];
-        k = e.key;
-        v = s_neg ? (uint64_t)0 - (uint64_t)e.delta : (uint64_t)e.delta;
+#pragma unroll
+      for (int u = 0; u < kPrepBatch; ++u) {
+        if (g0 + 32 * u >= total) break;   // warp-uniform
+        const uint64_t d = ((uint64_t)e[u].w << 32) | e[u].z;
+        f(e[u].y, (fl[u] & 2u) ? (uint64_t)0 - d : d, (fl[u] & 1u) != 0, (fl[u] & 4u) != 0);
       }
-      f(k, v, valid, s_twice);
     }
   }
 }
@@ -667,7 +672,7 @@ __device__ void prepare_block_b(const PrepParams& p, int32_t b, unsigned char* s
 // only the bitmap window (several CTAs per SM); pass B also holds the slice
 // histogram, so it runs as its own kernel over the blocks that hand a carry on.
 template <int Pass>
-__global__ void __launch_bounds__(kPrepThreads, Pass == 0 ? 3 : 2) k_prepare(PrepParams p) {
+__global__ void __launch_bounds__(kPrepThreads, 2) k_prepare(PrepParams p) {
   if (*p.status) return;  // bounds/descriptors are not trustworthy after an input error
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ int32_t s_ticket;
@@ -2042,8 +2047,10 @@ static size_t sweep_budget(int ctas_per_sm) { return (size_t)(kSmemPerSM / ctas_
 // uneven trees), else by the query/event ratio.
 static void finish_spec(PipeSpec& s, const Tuning& tune, bool forest) {
   s.tile = tune.tile >= kTileNarrowId && tune.tile <= kTileMaxId ? tune.tile
-           : forest ? kTileEulerId : (s.Q * 8 >= s.E ? kTileNarrowId : kTileWideId);
-  if (s.tile >= kTileNarrow512Id) s.ctas_per_sm = 1;   // a 512-thread CTA takes the SM's registers
+           : forest ? kTileEulerId
+           : s.Q >= kQueryDense * (int64_t)s.S ? kTileQueryId : (s.Q * 8 >= s.E ? kTileNarrowId : kTileEulerId);
+  if (s.tile == kTileQueryId) s.ctas_per_sm = 2;
+  else if (s.tile >= kTileNarrow512Id) s.ctas_per_sm = 1;   // a 512-thread CTA takes the SM's registers
   const int32_t nw = words_of(s.Cmax);
   const size_t bud = sweep_budget(s.ctas_per_sm);
   switch (s.tile) {
@@ -2054,6 +2061,12 @@ static void finish_spec(PipeSpec& s, const Tuning& tune, bool forest) {
       s.SL = sweep_layout<TileNarrow512>(nw, bud);
       s.SL.cap32 = std::min<uint32_t>(s.SL.cap32, kEsCap32);
       s.SL.cap64 = std::min<uint32_t>(s.SL.cap64, kEsCap64);
+      break;
+    case kTileQueryId:
+      s.QL = qsweep_layout(nw);
+      s.SL = sweep_layout<TileNarrow>(nw, bud);   // (its rank-table window; the capacities are the sweep's)
+      s.SL.cap32 = s.QL.cap32;
+      s.SL.cap64 = s.QL.cap64;
       break;
     case kTileNarrow512Id: s.SL = sweep_layout<TileNarrow512>(nw, bud); break;
     case kTileWide512Id: s.SL = sweep_layout<TileWide512>(nw, bud); break;
@@ -2068,7 +2081,7 @@ static void finish_spec(PipeSpec& s, const Tuning& tune, bool forest) {
 }
 
 int pipe_spec_one(int32_t S, uint32_t C, int64_t E, int64_t Q, int32_t blocks, bool chain, const Tuning& tune,
-                  int sms, PipeSpec& s) {
+                  int sms, PipeSpec& s, int64_t min_work) {
   if (S < 1 || S >= (1 << 30) || C < 1 || E < 0 || Q < 0 || E >= ((int64_t)1 << 32) ||
       Q >= ((int64_t)1 << 32))
     return BW_EINVAL;
@@ -2081,7 +2094,6 @@ int pipe_spec_one(int32_t S, uint32_t C, int64_t E, int64_t Q, int32_t blocks, b
   } else {
     B = 2 * (int64_t)sms;                            // two sweep CTAs per SM hide each other's latency
     if (tune.block_work > 0) B = (work + tune.block_work - 1) / tune.block_work;
-    const int64_t min_work = 65536;                  // below this a block is launch-dominated
     if (work / min_work < B) B = work / min_work;
     const double carry_budget = 4.0e9;               // bytes of dense carry rows
     const int64_t by_mem = (int64_t)(carry_budget / (8.0 * ((double)C + 1.0)));
@@ -2125,7 +2137,7 @@ int pipe_spec_forest(int32_t T, const int64_t* soff, const int64_t* eoff, const 
   s.ctas_per_sm = tune.ctas_per_sm > 0 ? tune.ctas_per_sm : 2;
   finish_spec(s, tune, true);   // the sweep layout depends only on the domains and the tuning
   int64_t target = tune.block_work > 0 ? tune.block_work
-                                       : std::max<int64_t>(65536, Wtot / (4 * (int64_t)s.ctas_per_sm * sms));
+                                       : std::max<int64_t>(kMinWorkCoarse, Wtot / (4 * (int64_t)s.ctas_per_sm * sms));
   std::vector<int32_t> nb(T);
   for (;;) {                       // the block work doubles until the carry rows fit
     int64_t carry = 0, blocks = 0;
@@ -2277,6 +2289,7 @@ static int ensure_attrs() {
                                         kSmemLimit - 1024), "smem attr")))
     return rc;
   if ((rc = report((cudaError_t)esweep_attrs(), "smem attr"))) return rc;
+  if ((rc = report((cudaError_t)qsweep_attrs(), "smem attr"))) return rc;
   if (dev >= 0 && dev < 64) done[dev] = true;
   return 0;
 }
@@ -2457,13 +2470,15 @@ int pipe_enqueue(const PipeSpec& s, void* workspace, const int32_t* parent, cons
     sp.bits = pp.bits; sp.rlut = pp.rlut; sp.slices = pp.slices; sp.nslices = pp.nslices; sp.carry = pp.carry;
     sp.answers = answers; sp.status = status; sp.bmode = bmode; sp.ticket = misc + M_SWEEP_TICKET;
     const int sgrid = std::min(B, s.ctas_per_sm * s.sms);
-    if (s.tile == kTileEulerId) {
+    if (s.tile == kTileEulerId || s.tile == kTileQueryId) {
       EsParams ep;
       ep.ev = reinterpret_cast<const uint4*>(events); ep.qs = queries; ep.desc = desc; ep.blocks = blocks;
       ep.order = order; ep.B = B; ep.cap32 = SL.cap32; ep.cap64 = SL.cap64;
       ep.bits = pp.bits; ep.rlut = pp.rlut; ep.slices = pp.slices; ep.nslices = pp.nslices; ep.carry = pp.carry;
       ep.answers = answers; ep.status = status; ep.bmode = bmode; ep.ticket = misc + M_SWEEP_TICKET;
-      if ((rc = report((cudaError_t)esweep_launch(ep, std::min(B, s.sms), st), "k_esweep"))) return rc;
+      if (s.tile == kTileEulerId) rc = report((cudaError_t)esweep_launch(ep, std::min(B, s.sms), st), "k_esweep");
+      else rc = report((cudaError_t)qsweep_launch(ep, s.QL, std::min(B, 2 * s.sms), st), "k_qsweep");
+      if (rc) return rc;
       ++kernels;
       if ((rc = mark(6))) return rc;
       if (kernels_out) *kernels_out = kernels;

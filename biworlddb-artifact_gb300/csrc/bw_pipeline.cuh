@@ -29,6 +29,15 @@ constexpr int kCarryChunk = 256;              // columns per carry unit
 constexpr int64_t kStepCost = 4;              // fixed cost of an Euler step, in event units
 constexpr int64_t kQueryStepCost = 64;        // extra cost of a step with queries (two CTA barriers)
 constexpr int64_t kQueryCost = 2;             // a query is two prefix probes
+// Smallest block of a tree that does not fill the GPU (two blocks an SM), in est_work
+// units.  At 65,536 a tree of 12,000 states and 200,000 events had 25 blocks and its sweep
+// took MW_OLD us, at 16,384 MW_NEW us.  The larger value stays for callers whose scratch the
+// smaller blocks would outgrow.
+constexpr int64_t kMinWork = 16384, kMinWorkCoarse = 65536;
+// Queries per state from which a tree is swept a step at a time by bw_qsweep.cu: measured
+// against k_sweep's narrow tile, 15 a state 1.02 and 1.18 ms, 18 a state 0.60 and 0.63 ms,
+// 167 a state 0.33 and 0.49 ms (4M events) and 2.3 and 4.6 ms (40M), 2 a state 0.94 and 0.44 ms.
+constexpr int64_t kQueryDense = 24;
 
 // Estimated sweep work of a tree (or a whole forest) from its sizes: every event is
 // applied on enter and on exit, every state is entered and left, and at most
@@ -79,11 +88,13 @@ using TileWide = TileCfg<4, 1, 64, 256, 256, true, true>;          // event-heav
 using TileNarrow512 = TileCfg<2, 1, 128, 512, 512, false, true>;   // 16 warps (one CTA per SM), own staging, flat
 using TileWide512 = TileCfg<2, 1, 64, 256, 512, true, true>;
 using TileSpec512 = TileCfg<1, 1, 64, 512, 512, false, true, true>;   // 15 replay warps + 1 staging warp
+// kTileQueryId: the query-step sweep of bw_qsweep.cu (a step at a time, a thread per
+// event and per query bound; two CTAs per SM).
 // kTileEulerId: the Euler-tile sweep of bw_esweep.cu (bulk-copied signed event tiles,
 // flat window, a producer warp; one CTA per SM) instead of k_sweep.
 enum { kTileAuto = 0, kTileNarrowId = 1, kTileWideId = 2, kTileNarrow512Id = 3, kTileWide512Id = 4, kTileSpec512Id = 5,
-       kTileEulerId = 6 };
-constexpr int kTileMaxId = 6;
+       kTileEulerId = 6, kTileQueryId = 7 };
+constexpr int kTileMaxId = 7;
 // Window capacity of the Euler-tile sweep: int32 entries, or int64 ones in the same
 // bytes (the prepare pass cuts its rank slices with the k_sweep window's capacities,
 // 27,904 and 13,824 entries, which both fit).
@@ -178,6 +189,15 @@ __host__ __device__ inline SweepLayout sweep_layout(int32_t nwords, size_t budge
   return L;
 }
 
+// Window of the query-step sweep (bw_qsweep.cu): runs of 512 ranks that fit beside a
+// rank table of `ww` words, and the rank capacities the prepare pass cuts slices with.
+struct QsLayout {
+  int32_t ww = 0;
+  uint32_t supers = 0, cap32 = 0, cap64 = 0;
+  size_t bytes = 0;
+};
+QsLayout qsweep_layout(int32_t nwords);
+
 // ------------------------------------------------------------------ host plan
 // Tunable knobs of a pipeline (picked by the caller or the forest autotuner).
 struct Tuning {
@@ -205,6 +225,7 @@ struct PipeSpec {
   int32_t tile = kTileNarrowId;
   int32_t sms = 0;
   SweepLayout SL{};
+  QsLayout QL{};                // tile 7
   bool chain_hint = false;
   // one-tree scalars (T == 1): tables are written by a kernel at each launch
   int32_t nb1 = 1;
@@ -244,7 +265,7 @@ int pipe_spec_forest(int32_t T, const int64_t* soff, const int64_t* eoff, const 
                      const uint32_t* C, const Tuning& tune, int sms, PipeSpec& spec);
 // Spec of one tree (the plain replay).
 int pipe_spec_one(int32_t S, uint32_t C, int64_t E, int64_t Q, int32_t blocks, bool chain, const Tuning& tune,
-                  int sms, PipeSpec& spec);
+                  int sms, PipeSpec& spec, int64_t min_work = kMinWork);
 void pipe_layout(const PipeSpec& spec, Layout& L);
 // Upload the forest tables into the workspace (no-op for one tree).  Synchronous.
 int pipe_bind(const PipeSpec& spec, void* workspace, cudaStream_t st);
@@ -289,6 +310,8 @@ struct EsParams {
 };
 int esweep_attrs();   // one-time shared-memory opt-in (cudaError_t as int)
 int esweep_launch(const EsParams& p, int grid, cudaStream_t st);
+int qsweep_attrs();
+int qsweep_launch(const EsParams& p, const QsLayout& q, int grid, cudaStream_t st);
 
 // Device address of the status word inside a workspace laid out for `spec`.
 const int32_t* pipe_status_word(const PipeSpec& spec, const void* workspace);

@@ -1,0 +1,362 @@
+// bw_qsweep.cu -- query-step sweep of the general (tree) pipeline, for trees whose
+// states are asked many queries each (tile 7).
+//
+// A block's Euler steps are replayed one at a time by all 512 threads: thread i applies
+// event i of the step; at a step with queries threads 2i and 2i + 1 take the lower and
+// upper bound of query i.  The window over the block's key ranks (shared memory) holds
+// plain values, totals of 16 ranks (both by no-return atomics) and, rebuilt by sixteen
+// warp scans before a query step that follows updates, the prefixes of the totals inside
+// every 512 ranks; a warp scans the totals of the 512s itself.  A probe is one prefix,
+// one shuffle and at most four 128-bit reads of values -- per thread, so a step's queries
+// cost a few hundred cycles together, however many they are up to 256.
+//
+// The carried part of every answer is written beforehand by k_qcarry, a block's queries
+// side by side over its carry row (random reads of one 512 KB row at a time stay in the
+// L2; inside the sweep 304 rows were read at once); the sweep adds the window's part with
+// a no-return atomic.  A thread's event and bound of a step are copied into shared-memory
+// slots of its own three steps ahead (cp.async: register loads four steps ahead shared
+// their scoreboards with the step's own shared-memory reads and cost a memory latency a
+// step), the step descriptors through a ring.
+//
+// Bound by the latency of the three barriers of a query step, two CTAs an SM to overlap
+// them.  QS_MEASURED
+#include <cuda_runtime.h>
+#include <cstdint>
+
+#include "bw_gpu.h"
+#include "bw_common.cuh"
+#include "bw_pipeline.cuh"
+
+namespace bw {
+namespace {
+
+constexpr int kQsThreads = 512, kQsWarps = kQsThreads / 32;
+constexpr uint32_t kQsGroup = 16, kQsRunGroups = 128, kQsSuper = kQsGroup * kQsRunGroups;   // ranks of a total, of a run
+constexpr uint32_t kQsMaxRuns = 16;                  // one warp each
+constexpr int kQsRing = 128;                         // step descriptors
+constexpr int kQsSlots = 9;                          // slot arrays of a word per thread
+constexpr uint32_t kFull = 0xffffffffu;
+static_assert(kQsRunGroups == 4 * 32, "a warp scans the totals of one run, four a lane");
+
+struct QsSmem {
+  size_t rl, leaf, gsum, gpre, stot, ring, slots, bytes;
+};
+__host__ __device__ inline size_t qs_al(size_t x) { return (x + 15) & ~size_t(15); }
+// `supers` runs of 2,048 int32 ranks (half as many int64 ones in the same bytes).
+__host__ __device__ inline QsSmem qs_smem(int32_t ww, uint32_t supers) {
+  QsSmem L;
+  size_t o = qs_al((size_t)ww * 8);
+  L.rl = o;    o = qs_al(o + ((size_t)ww + 2) * 2);
+  L.leaf = o;  o = qs_al(o + (size_t)supers * kQsSuper * 4);
+  L.gsum = o;  o = qs_al(o + (size_t)supers * kQsRunGroups * 4);
+  L.gpre = o;  o = qs_al(o + (size_t)supers * kQsRunGroups * 4);
+  L.stot = o;  o = qs_al(o + (size_t)supers * 4);
+  L.ring = o;  o = qs_al(o + (size_t)kQsRing * 16);
+  L.slots = o; o = qs_al(o + (size_t)kQsSlots * kQsThreads * 4);
+  L.bytes = o;
+  return L;
+}
+
+__device__ __forceinline__ void qs_copy16(void* dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
+               : "memory");
+}
+
+__device__ __forceinline__ void qs_copy4(void* dst, const void* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
+               : "memory");
+}
+
+template <typename Node>
+__device__ __forceinline__ Node qs_scan(Node v, int lane) {   // inclusive, over the warp
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const Node y = __shfl_up_sync(kFull, v, o);
+    if (lane >= o) v += y;
+  }
+  return v;
+}
+
+// Prefix of i < 16 ranks inside a group: Fenwick nodes 1 .. 15 of the group at g (node n
+// at g[n - 1]; the sixteenth word is unused), four independent reads.
+template <typename Node>
+__device__ __forceinline__ Node qs_partial(const Node* g, uint32_t i) {
+  Node s = 0;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    if (i) s += g[i - 1];
+    i &= i - 1;
+  }
+  return s;
+}
+// Four consecutive totals of a lane: loaded, scanned over the warp's 128, exclusive
+// prefixes stored; returns the run's total in lane 31.
+__device__ __forceinline__ uint32_t qs_run(const uint32_t* in, uint32_t* out, int lane) {
+  const uint4 v = reinterpret_cast<const uint4*>(in)[lane];
+  const uint32_t s1 = v.x + v.y, s2 = s1 + v.z, s3 = s2 + v.w, incl = qs_scan(s3, lane), ex = incl - s3;
+  reinterpret_cast<uint4*>(out)[lane] = make_uint4(ex, ex + v.x, ex + s1, ex + s2);
+  return incl;
+}
+__device__ __forceinline__ unsigned long long qs_run(const unsigned long long* in, unsigned long long* out, int lane) {
+  const ulonglong2 a = reinterpret_cast<const ulonglong2*>(in)[2 * lane], b = reinterpret_cast<const ulonglong2*>(in)[2 * lane + 1];
+  const unsigned long long s1 = a.x + a.y, s2 = s1 + b.x, s3 = s2 + b.y, incl = qs_scan(s3, lane), ex = incl - s3;
+  reinterpret_cast<ulonglong2*>(out)[2 * lane] = make_ulonglong2(ex, ex + a.x);
+  reinterpret_cast<ulonglong2*>(out)[2 * lane + 1] = make_ulonglong2(ex + s1, ex + s2);
+  return incl;
+}
+
+template <typename Node>
+__device__ __forceinline__ void qs_block(const EsParams& p, int32_t ww, uint32_t supers, unsigned char* sm, int32_t b) {
+  const BlockTab bt = p.blocks[b];
+  const int32_t t0 = bt.t0, t1 = bt.t1;
+  if (t0 >= t1) return;
+  const QsSmem L = qs_smem(ww, supers);
+  uint64_t* bits = reinterpret_cast<uint64_t*>(sm);
+  uint16_t* rl = reinterpret_cast<uint16_t*>(sm + L.rl);
+  Node* leaf = reinterpret_cast<Node*>(sm + L.leaf);
+  Node* gsum = reinterpret_cast<Node*>(sm + L.gsum);
+  Node* gpre = reinterpret_cast<Node*>(sm + L.gpre);
+  Node* stot = reinterpret_cast<Node*>(sm + L.stot);
+  uint4* ring = reinterpret_cast<uint4*>(sm + L.ring);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  uint32_t* slots = reinterpret_cast<uint32_t*>(sm + L.slots) + threadIdx.x;   // word w of this thread: slots[w * 512]
+  constexpr int kDepth = sizeof(Node) == 4 ? 3 : 2;   // steps copied ahead
+  constexpr int kWords = sizeof(Node) == 4 ? 2 : 3;   // key and delta words; the bounds follow
+  const int32_t nsl = p.nslices[b];
+  const Slice* bsl = p.slices + (size_t)b * kMaxSlices;
+  for (int32_t si = 0; si < nsl; ++si) {
+    const Slice s = bsl[si];
+    if (s.n == 0) continue;   // no keys: no part of any answer
+    const uint32_t klo = (uint32_t)s.word_lo << 6;
+    const uint32_t khi = (uint32_t)min((uint64_t)s.word_hi << 6, (uint64_t)bt.C);
+    const uint32_t nsup = s.n / kQsSuper + 1;   // rank s.n lies in the last run
+    {
+      const uint64_t* gbits = p.bits + bt.bits_off + s.word_lo;
+      const uint32_t* grl = p.rlut + bt.bits_off + b + s.word_lo;
+      const int32_t nwd = s.word_hi - s.word_lo;
+      for (int32_t i = tid; i < nwd; i += kQsThreads) {
+        bits[i] = gbits[i];
+        rl[i] = (uint16_t)(grl[i] - s.rank_lo);
+      }
+      uint4* z = reinterpret_cast<uint4*>(leaf);
+      for (uint32_t i = tid; i < nsup * kQsSuper * sizeof(Node) / 16; i += kQsThreads) z[i] = make_uint4(0, 0, 0, 0);
+      for (uint32_t i = tid; i < nsup * kQsRunGroups; i += kQsThreads) gsum[i] = gpre[i] = 0;
+      for (uint32_t i = tid; i < nsup; i += kQsThreads) stot[i] = 0;
+    }
+    // descriptors: step t at ring[t % kQsRing]; half a ring is requested at the start of
+    // the other half and has landed by its middle
+    const uint4 none = make_uint4(0, 0, 0, 0);
+    auto request = [&](int32_t from) {
+      if (tid < kQsRing / 2) {
+        const int32_t t = from + tid;
+        if (t < t1) qs_copy16(ring + (t & (kQsRing - 1)), p.desc + t);
+        else ring[t & (kQsRing - 1)] = none;
+      }
+    };
+    const int32_t a0 = t0 & ~(kQsRing / 2 - 1);   // halves are aligned
+    request(a0);
+    request(a0 + kQsRing / 2);
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();
+    auto key_rank = [&](uint32_t k) -> uint32_t {   // slice rank of a bound
+      if (k <= klo) return 0u;
+      if (k >= khi) return s.n;
+      const uint32_t x = k - klo, w = x >> 6;
+      return (uint32_t)rl[w] + (uint32_t)__popcll(bits[w] & ((1ull << (x & 63)) - 1ull));
+    };
+    auto apply = [&](const uint4& e, bool neg) {
+      const uint32_t x = e.y - klo;
+      if (x >= khi - klo) return;
+      const uint32_t w = x >> 6, r = (uint32_t)rl[w] + (uint32_t)__popcll(bits[w] & ((1ull << (x & 63)) - 1ull));
+      Node* g = leaf + (r & ~(kQsGroup - 1));
+      uint32_t n = (r & (kQsGroup - 1)) + 1;
+      uint64_t d = ((uint64_t)e.w << 32) | e.z;
+      if (neg) d = (uint64_t)0 - d;
+      auto add = [&](Node* at) {
+        if constexpr (sizeof(Node) == 4) atomicAdd(at, (uint32_t)d);
+        else shared_add_u64(at, d);
+      };
+      add(gsum + r / kQsGroup);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        if (n < kQsGroup) add(g + n - 1);
+        n += n & (0u - n);
+      }
+    };
+    auto bound_at = [&](uint32_t q) -> uint32_t {   // this thread's bound of query q
+      const uint32_t* x = reinterpret_cast<const uint32_t*>(p.qs + q);
+      return __ldg(x + 1 + (tid & 1));
+    };
+    // step t's event and bound of this thread into stage t % kDepth
+    auto copy = [&](int32_t t, int stage) {
+      if (t < t1) {
+        const uint4 d = ring[t & (kQsRing - 1)];
+        if (tid < (int32_t)d.z) {
+          const uint32_t* e = reinterpret_cast<const uint32_t*>(p.ev + d.x + tid) + 1;
+#pragma unroll
+          for (int w = 0; w < kWords; ++w) qs_copy4(slots + (stage * kWords + w) * kQsThreads, e + w);
+        }
+        if ((tid >> 1) < (int32_t)d.w)
+          qs_copy4(slots + (kDepth * kWords + stage) * kQsThreads,
+                   reinterpret_cast<const uint32_t*>(p.qs + (d.y + (tid >> 1))) + 1 + (tid & 1));
+      }
+      asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    // the window's part of the pair's query: prefix at hi - prefix at lo
+    auto answer = [&](bool in, uint32_t q, uint32_t x, uint32_t r, Node spre) {
+      Node v = gpre[r / kQsGroup] + qs_partial(leaf + (r & ~(kQsGroup - 1)), r & (kQsGroup - 1));
+      v += __shfl_sync(kFull, spre, (int)(r / kQsSuper));
+      v = __shfl_down_sync(kFull, v, 1) - v;
+      const uint32_t xh = __shfl_down_sync(kFull, x, 1);
+      if (in && !(tid & 1) && xh > x) {
+        const uint64_t a = sizeof(Node) == 4 ? (uint64_t)(int64_t)(int32_t)v : (uint64_t)v;
+        if (a) atomicAdd(reinterpret_cast<unsigned long long*>(p.answers + q), (unsigned long long)a);
+      }
+    };
+    bool dirty = false;   // (the same in every thread) updates since the prefixes were built
+    int stage = 0;        // t % kDepth, from t0
+#pragma unroll
+    for (int k = 0; k < kDepth; ++k) copy(t0 + k, k);
+    for (int32_t t = t0; t < t1; ++t) {
+      const int32_t half = t & (kQsRing / 2 - 1);
+      if (half == 0 && t > t0) {
+        __syncthreads();                       // every thread is past the half before
+        request(t + kQsRing / 2);
+      } else if (half == kQsRing / 4) {
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        __syncthreads();
+      }
+      asm volatile("cp.async.wait_group %0;" ::"n"(kDepth - 1) : "memory");   // this thread's copies of step t
+      const uint4 d = ring[t & (kQsRing - 1)];
+      const int32_t ne = (int32_t)d.z, nq = (int32_t)d.w;
+      if (tid < ne) {
+        uint4 e;
+        e.y = slots[stage * kWords * kQsThreads];
+        e.z = slots[(stage * kWords + 1) * kQsThreads];
+        e.w = kWords == 3 ? slots[(stage * kWords + 2) * kQsThreads] : 0u;
+        apply(e, nq < 0);
+        for (int32_t i = kQsThreads + tid; i < ne; i += kQsThreads) apply(__ldg(p.ev + (size_t)d.x + i), nq < 0);
+      }
+      dirty |= ne > 0;
+      if (nq > 0) {
+        const bool mine = (tid >> 1) < nq, active = warp * 16 < nq;
+        const uint32_t x0 = mine ? slots[(kDepth * kWords + stage) * kQsThreads] : 0u, r0 = mine ? key_rank(x0) : 0u;
+        if (dirty) {
+          __syncthreads();                     // the updates of every step so far
+          if (warp < (int)nsup) {
+            const Node total = qs_run(gsum + warp * kQsRunGroups, gpre + warp * kQsRunGroups, lane);
+            if (lane == 31) stot[warp] = total;
+          }
+          __syncthreads();
+        }
+        if (active) {
+          const Node own = lane < (int)nsup ? stot[lane] : (Node)0;
+          Node spre = own;                     // totals of the runs below run `lane`
+#pragma unroll
+          for (int o = 1; o < (int)kQsMaxRuns; o <<= 1) {
+            const Node y = __shfl_up_sync(kFull, spre, o);
+            if (lane >= o) spre += y;
+          }
+          spre -= own;
+          answer(mine, d.y + (tid >> 1), x0, r0, spre);
+          for (int32_t q0 = kQsThreads / 2; q0 + warp * 16 < nq; q0 += kQsThreads / 2) {   // more than 256 queries
+            const int32_t q = q0 + (tid >> 1);
+            const uint32_t x = q < nq ? bound_at(d.y + q) : 0u;
+            answer(q < nq, d.y + q, x, q < nq ? key_rank(x) : 0u, spre);
+          }
+        }
+        __syncthreads();                       // probes done before the next updates
+        dirty = false;
+      }
+      copy(t + kDepth, stage);
+      stage = stage + 1 == kDepth ? 0 : stage + 1;
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();
+  }
+}
+
+// The carried part of every query's answer (0 where the block starts its tree).  CTA
+// (part, block): a warp takes eight consecutive steps at a time and their queries,
+// flattened.  The parts of a block run side by side, so that some eighty carry rows are
+// read at a time and stay in the L2.
+constexpr int kQcParts = 16, kQcSteps = 8;
+__global__ void __launch_bounds__(256) k_qcarry(EsParams p) {
+  if (*p.status) return;
+  const BlockTab bt = p.blocks[blockIdx.y];
+  const int64_t* crow = bt.carry_in >= 0 ? p.carry + bt.carry_in : nullptr;
+  const int lane = threadIdx.x & 31, warp = blockIdx.x * 8 + (threadIdx.x >> 5);
+  for (int32_t c = bt.t0 + kQcSteps * warp; c < bt.t1; c += kQcSteps * 8 * kQcParts) {
+    const uint4 d = lane < kQcSteps && c + lane < bt.t1 ? __ldg(reinterpret_cast<const uint4*>(p.desc) + c + lane)
+                                                        : make_uint4(0, 0, 0, 0);
+    const uint32_t n = (int32_t)d.w > 0 ? d.w : 0u;
+    uint32_t incl = n;
+#pragma unroll
+    for (int o = 1; o < kQcSteps; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(kFull, incl, o);
+      if (lane >= o) incl += y;
+    }
+    const uint32_t total = __shfl_sync(kFull, incl, kQcSteps - 1);
+#pragma unroll 2
+    for (uint32_t g0 = 0; g0 < total; g0 += 32) {
+      const uint32_t g = g0 + lane;
+      int lo = 0, hi = kQcSteps - 1;   // first step whose inclusive count exceeds g
+#pragma unroll
+      for (int it = 0; it < 3; ++it) {
+        const int mid = (lo + hi) >> 1;
+        if (__shfl_sync(kFull, incl, mid) > g) hi = mid; else lo = mid + 1;
+      }
+      const uint32_t before = __shfl_sync(kFull, incl - n, lo), q0 = __shfl_sync(kFull, d.y, lo);
+      if (g < total) {
+        const uint32_t q = q0 + (g - before);
+        const uint32_t a = __ldg(&p.qs[q].lo), z = __ldg(&p.qs[q].hi);
+        p.answers[q] = crow && a < z ? (int64_t)((uint64_t)__ldg(crow + z) - (uint64_t)__ldg(crow + a)) : 0;
+      }
+    }
+  }
+}
+
+__global__ void __launch_bounds__(kQsThreads, 2) k_qsweep(EsParams p, int32_t ww, uint32_t supers) {
+  extern __shared__ __align__(16) unsigned char sm[];
+  __shared__ int32_t s_ticket;
+  if (*p.status) return;   // never index with descriptors of rejected input
+  for (;;) {
+    __syncthreads();
+    if (threadIdx.x == 0) s_ticket = atomicAdd(p.ticket, 1);
+    __syncthreads();
+    const int32_t i = s_ticket;
+    if (i >= p.B) break;
+    const int32_t b = p.order ? p.order[i] : i;
+    if (p.bmode[b]) qs_block<uint32_t>(p, ww, supers, sm, b);
+    else qs_block<unsigned long long>(p, ww, supers, sm, b);
+  }
+}
+
+}  // namespace
+
+// Rank capacities for domains of `nwords` bitmap words (two CTAs an SM): as many runs of
+// 2,048 as fit, the last rank kept for bounds past the last key.
+QsLayout qsweep_layout(int32_t nwords) {
+  QsLayout q;
+  q.ww = nwords < kWinWords ? nwords : kWinWords;
+  const size_t budget = (size_t)kSmemPerSM / 2 - 1024 - 256;
+  uint32_t n = 2;
+  while (n < kQsMaxRuns && qs_smem(q.ww, n + 1).bytes <= budget) ++n;
+  q.supers = n;
+  q.cap32 = n * kQsSuper - 1;
+  q.cap64 = (n / 2) * kQsSuper - 1;
+  q.bytes = qs_smem(q.ww, n).bytes;
+  return q;
+}
+
+int qsweep_attrs() {
+  return (int)cudaFuncSetAttribute(k_qsweep, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemPerSM / 2 - 1024);
+}
+
+int qsweep_launch(const EsParams& p, const QsLayout& q, int grid, cudaStream_t st) {
+  k_qcarry<<<dim3(kQcParts, (unsigned)p.B), 256, 0, st>>>(p);
+  k_qsweep<<<grid, kQsThreads, q.bytes, st>>>(p, q.ww, q.supers);
+  return (int)cudaGetLastError();
+}
+
+}  // namespace bw

@@ -42,12 +42,28 @@ int device_sms(int* sms) {
   return report(e, "device query");
 }
 
-int spec_of(const BwReplayArgs* a, PipeSpec& s) {
+// The general pipeline's plan and layout.  Where coarse blocks fit the allocation-free
+// entry's 32 MiB, the finest ones that still do: what fitted before the blocks were made
+// finer fits now.
+int spec_of(const BwReplayArgs* a, PipeSpec& s, Layout& L) {
   int sms = 0;
   int rc = device_sms(&sms);
   if (rc) return rc;
-  return pipe_spec_one(a->n_states, a->n_keys, a->n_events, a->n_queries, a->blocks,
-                       (a->flags & BW_REPLAY_CHAIN_HINT) != 0, Tuning(), sms, s);
+  const size_t small = (size_t)32 << 20;
+  auto plan = [&](int64_t min_work) {
+    const int r = pipe_spec_one(a->n_states, a->n_keys, a->n_events, a->n_queries, a->blocks,
+                                (a->flags & BW_REPLAY_CHAIN_HINT) != 0, Tuning(), sms, s, min_work);
+    if (!r) pipe_layout(s, L);
+    return r;
+  };
+  if ((rc = plan(kMinWork)) || L.total <= small || a->blocks > 0) return rc;
+  if ((rc = plan(kMinWorkCoarse))) return rc;
+  const bool fits = L.total <= small;
+  for (int64_t w = kMinWork; w < kMinWorkCoarse; w += w / 4) {
+    if ((rc = plan(w))) return rc;
+    if (!fits || L.total <= small) return 0;
+  }
+  return plan(kMinWorkCoarse);
 }
 
 int chain_spec_of(const BwReplayArgs* a, ChainSpec& s) {
@@ -67,14 +83,13 @@ struct Route {
 };
 int route_of(const BwReplayArgs* a, Route& r) {
   r.chain = chain_selected(a);
-  int rc = r.chain ? chain_spec_of(a, r.cs) : spec_of(a, r.s);
+  Layout L;
+  int rc = r.chain ? chain_spec_of(a, r.cs) : spec_of(a, r.s, L);
   if (rc) return rc;
   if (r.chain) {
     r.need = r.cs.total;
     return 0;
   }
-  Layout L;
-  pipe_layout(r.s, L);
   r.kb = kb_select(a, r.s, L.total, r.k);
   r.need = r.kb ? r.k.total : L.total;
   return 0;
