@@ -160,7 +160,9 @@ struct ScanItems {
 };
 template <typename T>
 __global__ void __launch_bounds__(kScanThreads) k_scan_reduce(const T* __restrict__ x, int64_t n,
-                                                              T* __restrict__ part) {
+                                                              T* __restrict__ part, const int32_t* n_dev) {
+  if (n_dev) n = imin64(n, *n_dev);
+  if ((int64_t)blockIdx.x * kScanTile >= n) return;
   ScanItems<T> it;
   it.load(x, n);
   uint64_t s = 0;
@@ -173,8 +175,10 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_reduce(const T* __restric
   if (threadIdx.x == 0) part[blockIdx.x] = (T)total;
 }
 template <typename T>
-__global__ void k_scan_parts(T* part, int64_t np) {
+__global__ void k_scan_parts(T* part, int64_t n, const int32_t* n_dev) {
   // single CTA: exclusive scan of the tile totals in place
+  if (n_dev) n = imin64(n, *n_dev);
+  const int64_t np = (n + kScanTile - 1) / kScanTile;
   uint64_t carry = 0;
   for (int64_t c0 = 0; c0 < np; c0 += blockDim.x) {
     const int64_t i = c0 + threadIdx.x;
@@ -187,7 +191,9 @@ __global__ void k_scan_parts(T* part, int64_t np) {
 }
 template <typename T>
 __global__ void __launch_bounds__(kScanThreads) k_scan_apply(T* __restrict__ x, int64_t n,
-                                                             const T* __restrict__ part) {
+                                                             const T* __restrict__ part, const int32_t* n_dev) {
+  if (n_dev) n = imin64(n, *n_dev);
+  if ((int64_t)blockIdx.x * kScanTile >= n) return;
   __shared__ uint64_t s_warp[kScanThreads / 32];
   using I = ScanItems<T>;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -232,14 +238,15 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_apply(T* __restrict__ x, 
 }
 
 // Inclusive scan of x[0..n) in place (three launches, counted into `kernels`); tmp
-// holds scan_tmp_bytes(n).
+// holds scan_tmp_bytes(n).  n_dev: the count on the device, n its upper bound.
 template <typename T>
-inline int device_inclusive_scan(T* x, int64_t n, void* tmp, cudaStream_t st, int& kernels) {
+inline int device_inclusive_scan(T* x, int64_t n, void* tmp, cudaStream_t st, int& kernels,
+                                 const int32_t* n_dev = nullptr) {
   if (n <= 0) return 0;
   const int64_t np = (n + kScanTile - 1) / kScanTile;
-  k_scan_reduce<T><<<(unsigned)np, kScanThreads, 0, st>>>(x, n, static_cast<T*>(tmp));
-  k_scan_parts<T><<<1, 1024, 0, st>>>(static_cast<T*>(tmp), np);
-  k_scan_apply<T><<<(unsigned)np, kScanThreads, 0, st>>>(x, n, static_cast<const T*>(tmp));
+  k_scan_reduce<T><<<(unsigned)np, kScanThreads, 0, st>>>(x, n, static_cast<T*>(tmp), n_dev);
+  k_scan_parts<T><<<1, 1024, 0, st>>>(static_cast<T*>(tmp), n, n_dev);
+  k_scan_apply<T><<<(unsigned)np, kScanThreads, 0, st>>>(x, n, static_cast<const T*>(tmp), n_dev);
   kernels += 3;
   return (int)cudaGetLastError();
 }

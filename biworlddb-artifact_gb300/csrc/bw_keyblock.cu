@@ -707,7 +707,7 @@ void kb_layout(const PipeSpec& s, KbSpec& k) {
   size_t o = 0;
   auto take = [&](int i, size_t bytes) { k.off[i] = o; o = al256(o + bytes); };
   take(KB_SOFF, 8); take(KB_TEOFF, 16); take(KB_TQOFF, 16); take(KB_TC, 4); take(KB_TBOFF, 8); take(KB_TBITS, 8);
-  take(KB_TCARRY, 8); take(KB_TGSUM, 8); take(KB_LASTQ, 4);
+  take(KB_TCARRY, 8); take(KB_TGSUM, 8); take(KB_LASTQ, 4); take(KB_TTOFF, 8);
   take(KB_MISC, 256);
   take(KB_EOFF, (S + 1) * 8); take(KB_QOFF, (S + 1) * 8);
   take(KB_FORK, S * 4); take(KB_NEXT, S * 4); take(KB_CNT, S * 8); take(KB_EHEAD, S * 4); take(KB_XHEAD, S * 4);
@@ -775,7 +775,9 @@ const int32_t* kb_status_word(const KbSpec& k, const void* workspace) {
   return reinterpret_cast<const int32_t*>(static_cast<const char*>(workspace) + k.off[KB_MISC]) + M_STATUS;
 }
 
-int kb_enqueue(const KbSpec& k, const PipeSpec& s, const BwReplayArgs* a, EventSet* timing, int* kernels_out) {
+int kb_enqueue(const KbSpec& k, const PipeSpec& spec, const BwReplayArgs* a, EventSet* timing, int* kernels_out) {
+  PipeSpec s = spec;
+  s.contract = false;   // columns and points are taken from the states themselves
   if ((reinterpret_cast<uintptr_t>(a->events) & 15u) != 0) {
     std::fprintf(stderr, "bw replay: events must be 16-byte aligned (got %p)\n", static_cast<const void*>(a->events));
     return BW_EINVAL;
@@ -787,6 +789,7 @@ int kb_enqueue(const KbSpec& k, const PipeSpec& s, const BwReplayArgs* a, EventS
   ta.tt.soff = (int32_t*)at(KB_SOFF); ta.tt.eoff = (int64_t*)at(KB_TEOFF); ta.tt.qoff = (int64_t*)at(KB_TQOFF);
   ta.tt.C = (uint32_t*)at(KB_TC); ta.tt.boff = (int32_t*)at(KB_TBOFF); ta.tt.bits = (int64_t*)at(KB_TBITS);
   ta.tt.carry = (int64_t*)at(KB_TCARRY); ta.tt.gsum = (int64_t*)at(KB_TGSUM); ta.tt.last_q = (int32_t*)at(KB_LASTQ);
+  ta.tt.noff = ta.tt.soff; ta.tt.toff = (int32_t*)at(KB_TTOFF);
   ta.misc = (int32_t*)at(KB_MISC); ta.eoff = (int64_t*)at(KB_EOFF); ta.qoff = (int64_t*)at(KB_QOFF);
   ta.gpar = nullptr; ta.fork_head = (int32_t*)at(KB_FORK); ta.next_sib = (int32_t*)at(KB_NEXT);
   ta.cnt = (int64_t*)at(KB_CNT); ta.ehead = (int32_t*)at(KB_EHEAD); ta.xhead = (int32_t*)at(KB_XHEAD);

@@ -71,9 +71,12 @@ __host__ __device__ __forceinline__ int32_t words_of(uint32_t C) { return (int32
 __global__ void k_init(int32_t* misc, TreeTabs tt, int32_t T, int one_tree, int32_t S, int64_t E, int64_t Q,
                        uint32_t C, int32_t nb) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < 64) misc[i] = 0;
+  if (i < 64) misc[i] = i == M_NODES ? S : i == M_STEPS ? 2 * S : 0;
   for (int t = i; t < T; t += gridDim.x * blockDim.x) tt.last_q[t] = 0;
+  if (!one_tree)
+    for (int t = i; t <= T; t += gridDim.x * blockDim.x) tt.toff[t] = 2 * tt.soff[t];
   if (one_tree && i == 0) {
+    tt.toff[0] = 0; tt.toff[1] = 2 * S;
     tt.soff[0] = 0; tt.soff[1] = S;
     tt.eoff[0] = 0; tt.eoff[1] = E;
     tt.qoff[0] = 0; tt.qoff[1] = Q;
@@ -211,14 +214,92 @@ __global__ void k_lin_children(const int32_t* parent, int32_t S, TreeTabs tt, in
   }
 }
 
+// Contracted tours.  Where few states are asked, a run of chained states that no fork and
+// no query separates is one node of the tour: its events are adjacent in memory and come
+// and go together, and its queries are those of its last state.  The contracted tree keeps
+// the order of ids (a node's parent is a smaller node, its continuation the next one), so
+// everything below runs on nodes as it does on states.  On the batched uneven trees (20
+// states a run, 1,000 queries a tree) 19 % as many nodes as states.
+// k_ct_mark: parents checked (as k_lin_children does) and forked states marked.
+__global__ void k_ct_mark(const int32_t* parent, int32_t S, TreeTabs tt, int32_t T, int32_t* gpar, uint8_t* forked,
+                          int chain_only, int32_t* status) {
+  int64_t lo, hi;
+  warp_range(S, lo, hi);
+  int32_t t = T > 1 && lo < hi ? find_tree(tt.soff, T, imin64(lo + (threadIdx.x & 31), S - 1)) : 0;
+  for (int32_t v = (int32_t)lo + (threadIdx.x & 31); v < hi; v += 32) {
+    if (T > 1) t = tree_forward(tt.soff, T, t, v);
+    const int32_t s0 = tt.soff[t], l = v - s0;
+    const int32_t p = parent[v];
+    int32_t gp = -1;
+    if (l == 0) {
+      if (p != -1) set_status(status, BW_STATUS_BAD_PARENT);
+    } else if (p < 0 || p >= l) {
+      set_status(status, BW_STATUS_BAD_PARENT);
+    } else {
+      gp = s0 + p;
+    }
+    if (gpar) gpar[v] = gp;
+    if (l > 0 && gp >= 0 && gp != v - 1) {
+      if (chain_only) set_status(status, BW_STATUS_BAD_PARENT);
+      forked[gp] = 1;
+    }
+  }
+}
+// ends[v] = 1 where v is the last state of its node (then scanned).
+__global__ void k_ct_ends(const int32_t* gpar, const uint8_t* forked, const int64_t* qoff, int32_t S, uint32_t* ends,
+                          const int32_t* status) {
+  if (*status) return;
+  for (int32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < S; v += gridDim.x * blockDim.x)
+    ends[v] = qoff[v + 1] > qoff[v] || forked[v] || !(v + 1 < S && gpar[v + 1] == v) ? 1u : 0u;
+}
+__global__ void k_ct_nodes(const int32_t* gpar, const uint32_t* ends, const int64_t* eoff, const int64_t* qoff,
+                           int32_t S, TreeTabs tt, int32_t T, int64_t* neoff, int64_t* nqoff, int32_t* npar,
+                           int32_t* fork_head, int32_t* misc) {
+  if (misc[M_STATUS]) return;
+  const int32_t i0 = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
+  for (int32_t t = i0; t <= T; t += stride) {
+    const int32_t s0 = tt.soff[t];
+    tt.noff[t] = s0 ? (int32_t)ends[s0 - 1] : 0;
+  }
+  for (int32_t v = i0; v < S; v += stride) {
+    const uint32_t e = ends[v], ep = v ? ends[v - 1] : 0u, epp = v > 1 ? ends[v - 2] : 0u;
+    const bool last = e != ep;
+    const int32_t i = (int32_t)e - (last ? 1 : 0);
+    if (last) {
+      neoff[i + 1] = eoff[v + 1];
+      nqoff[i + 1] = qoff[v + 1];
+      fork_head[i] = -1;
+    }
+    if (v == 0 || ep != epp) {   // the first state of its node: its parent ends a node
+      const int32_t p = gpar[v];
+      npar[i] = p < 0 ? -1 : (int32_t)ends[p] - 1;
+    }
+    if (v == 0) neoff[0] = nqoff[0] = 0;
+    if (v == S - 1) {
+      misc[M_NODES] = (int32_t)e;
+      misc[M_STEPS] = 2 * (int32_t)e;
+    }
+  }
+}
+__global__ void k_ct_children(const int32_t* npar, const int32_t* nodes, int32_t* fork_head, int32_t* next_sib,
+                              const int32_t* status) {
+  if (*status) return;
+  const int32_t n = *nodes;
+  for (int32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const int32_t p = npar[i];
+    next_sib[i] = p >= 0 && p != i - 1 ? atomicExch(&fork_head[p], i) : -1;
+  }
+}
+
 // Segment heads.  enter(v) follows enter(v-1) exactly when v continues v-1; exit(v)
 // follows exit(v+1) exactly when v+1 continues v and v has no forks.  An arc that
 // follows another way heads a segment: a maximal run of consecutive arcs (enter
 // segments go up the state ids, exit segments down).  cnt[v] packs the two head
 // flags (enter | exit << 32) for an inclusive scan.
-__global__ void k_lin_flags(const int32_t* gpar, const int32_t* fork_head, int32_t S, int64_t* cnt,
+__global__ void k_lin_flags(const int32_t* gpar, const int32_t* fork_head, const int32_t* nodes, int64_t* cnt,
                             const int32_t* status) {
   if (*status) return;
+  const int32_t S = *nodes;
   for (int32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < S; v += gridDim.x * blockDim.x) {
     const bool cont = v + 1 < S && gpar[v + 1] == v;
     const bool eh = !(v > 0 && gpar[v] == v - 1);
@@ -227,8 +308,9 @@ __global__ void k_lin_flags(const int32_t* gpar, const int32_t* fork_head, int32
   }
 }
 
-__global__ void k_lin_heads(const int64_t* cnt, int32_t S, int32_t* ehead, int32_t* xhead, const int32_t* status) {
+__global__ void k_lin_heads(const int64_t* cnt, const int32_t* nodes, int32_t* ehead, int32_t* xhead, const int32_t* status) {
   if (*status) return;
+  const int32_t S = *nodes;
   for (int32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < S; v += gridDim.x * blockDim.x) {
     const uint64_t c = (uint64_t)cnt[v], cp = v ? (uint64_t)cnt[v - 1] : 0ull;
     const uint32_t e = (uint32_t)c, x = (uint32_t)(c >> 32);
@@ -247,9 +329,10 @@ __device__ __forceinline__ uint64_t pack_rank(int32_t next, uint32_t dist) {
 // follows its tail arc in the Euler tour; every tree's list ends at the exit of its
 // root.  r = (successor, length) for weighted list ranking.
 __global__ void k_lin_rank_init(const int64_t* cnt, const int32_t* ehead, const int32_t* xhead, const int32_t* gpar,
-                                const int32_t* fork_head, const int32_t* next_sib, int32_t S, uint64_t* r,
+                                const int32_t* fork_head, const int32_t* next_sib, const int32_t* nodes, uint64_t* r,
                                 const int32_t* status) {
   if (*status) return;
+  const int32_t S = *nodes;
   const uint64_t tot = (uint64_t)cnt[S - 1];
   const int64_t He = (uint32_t)tot, H = He + (int64_t)(tot >> 32);
   auto eid = [&](int32_t w) { return (int32_t)((uint32_t)cnt[w]) - 1; };
@@ -287,9 +370,10 @@ __global__ void k_lin_rank_init(const int64_t* cnt, const int32_t* ehead, const 
 // consistent pair even while its owner updates it (jumping further ahead keeps
 // dist(x) = the lengths from x up to next(x)).  Round r records whether any pointer
 // is still live; a round after one that found none returns at once.
-__global__ void k_lin_round(uint64_t* __restrict__ r, const int64_t* cnt, int32_t S, int32_t* live, int32_t round,
+__global__ void k_lin_round(uint64_t* __restrict__ r, const int64_t* cnt, const int32_t* nodes, int32_t* live, int32_t round,
                             const int32_t* status) {
   if (*status) return;
+  const int32_t S = *nodes;
   if (round > 0 && live[round - 1] == 0) return;
   const uint64_t tot = (uint64_t)cnt[S - 1];
   const int64_t H = (int64_t)(uint32_t)tot + (int64_t)(tot >> 32);
@@ -305,22 +389,82 @@ __global__ void k_lin_round(uint64_t* __restrict__ r, const int64_t* cnt, int32_
   if (__syncthreads_or(any) && threadIdx.x == 0) live[round] = 1;
 }
 
-// Step sequence (each step's enter/exit partner), per-step descriptors and work, and each tree's last
-// step that answers a query.  Tree t's tour occupies steps [2 s0, 2 s0 + 2 ns): the
-// head arc of a segment sits at 2 s0 + 2 ns - dist, the other arcs follow it.
-__global__ void k_lin_steps(const uint64_t* r, const int64_t* cnt, const int32_t* ehead, const int32_t* xhead,
-                            int32_t S, TreeTabs tt, int32_t T, const int64_t* eoff, const int64_t* qoff,
-                            int32_t* partner, StepDesc* desc, int64_t* work, const int32_t* status) {
+// Tour steps of node v's enter and exit.  Tree t's tour occupies steps [2 n0, 2 n0 + 2 nn)
+// of its nodes [n0, n0 + nn): the head arc of a segment sits at 2 n0 + 2 nn - dist, the
+// other arcs follow it.
+struct ArcPos {
+  int64_t pe, px;
+};
+__device__ __forceinline__ ArcPos arc_pos(const uint64_t* r, uint64_t c, uint64_t cp, int64_t He, const int32_t* ehead,
+                                          const int32_t* xhead, int64_t end, int32_t v) {
+  const int64_t eid = (int64_t)(uint32_t)c - 1, xid = (int64_t)(cp >> 32);   // exit heads below v
+  return ArcPos{end - (int64_t)(uint32_t)r[eid] + (v - ehead[eid]),
+                end - (int64_t)(uint32_t)r[He + xid] + (xhead[xid] - v)};
+}
+
+// Contracted tours drop the nodes no query needs: those with no query between their
+// enter and their exit.  k_lin_pos: every node's steps, and the queries of every step
+// (scanned); k_lin_keep: whether a step stays (scanned: its new place).  On the batched
+// uneven trees 57 % of the states are needed.
+__global__ void k_lin_pos(const uint64_t* r, const int64_t* cnt, const int32_t* ehead, const int32_t* xhead,
+                          const int32_t* nodes, TreeTabs tt, int32_t T, const int64_t* qoff, int32_t* tin, int32_t* tout,
+                          uint32_t* nq, const int32_t* status) {
   if (*status) return;
+  const int32_t S = *nodes;
   const int64_t He = (uint32_t)(uint64_t)cnt[S - 1];
   int64_t lo, hi;
   warp_range(S, lo, hi);
-  int32_t t = T > 1 && lo < hi ? find_tree(tt.soff, T, imin64(lo + (threadIdx.x & 31), S - 1)) : 0;
-  // the state's counters and ranges, loaded one iteration ahead
+  int32_t t = T > 1 && lo < hi ? find_tree(tt.noff, T, imin64(lo + (threadIdx.x & 31), S - 1)) : 0;
+  for (int32_t v = (int32_t)lo + (threadIdx.x & 31); v < hi; v += 32) {
+    if (T > 1) t = tree_forward(tt.noff, T, t, v);
+    const ArcPos a = arc_pos(r, (uint64_t)cnt[v], v ? (uint64_t)cnt[v - 1] : 0ull, He, ehead, xhead,
+                             2 * (int64_t)tt.noff[t + 1], v);
+    tin[v] = (int32_t)a.pe;
+    tout[v] = (int32_t)a.px;
+    nq[a.pe] = (uint32_t)(qoff[v + 1] - qoff[v]);
+    nq[a.px] = 0;
+  }
+}
+__global__ void k_lin_keep(const int32_t* nodes, const int32_t* tin, const int32_t* tout, const int64_t* qoff,
+                           const uint32_t* nq, uint32_t* keep, const int32_t* status) {
+  if (*status) return;
+  const int32_t S = *nodes;
+  for (int32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < S; v += gridDim.x * blockDim.x) {
+    const int32_t pe = tin[v], px = tout[v];
+    const uint32_t k = nq[px] != nq[pe] - (uint32_t)(qoff[v + 1] - qoff[v]) ? 1u : 0u;
+    keep[pe] = k;
+    keep[px] = k;
+  }
+}
+__global__ void k_lin_trees(const uint32_t* keep, TreeTabs tt, int32_t T, int32_t* misc) {
+  if (misc[M_STATUS]) return;
+  for (int32_t t = blockIdx.x * blockDim.x + threadIdx.x; t <= T; t += gridDim.x * blockDim.x) {
+    const int32_t n0 = tt.noff[t];
+    const int32_t at = n0 ? (int32_t)keep[2 * (int64_t)n0 - 1] : 0;
+    tt.toff[t] = at;
+    if (t == T) misc[M_STEPS] = at;
+  }
+}
+
+// Step sequence (each step's enter/exit partner), per-step descriptors and work, and each
+// tree's last step that answers a query.  kKept: the steps kept, at their new places.
+template <bool kKept>
+__global__ void k_lin_steps(const uint64_t* r, const int64_t* cnt, const int32_t* ehead, const int32_t* xhead,
+                            const int32_t* tin, const int32_t* tout, const uint32_t* keep, const int32_t* nodes,
+                            TreeTabs tt, int32_t T, const int64_t* eoff, const int64_t* qoff, int32_t* partner,
+                            StepDesc* desc, int64_t* work, const int32_t* status) {
+  if (*status) return;
+  const int32_t S = *nodes;
+  const int64_t He = kKept ? 0 : (int64_t)(uint32_t)(uint64_t)cnt[S - 1];
+  int64_t lo, hi;
+  warp_range(S, lo, hi);
+  int32_t t = T > 1 && lo < hi ? find_tree(tt.noff, T, imin64(lo + (threadIdx.x & 31), S - 1)) : 0;
+  // the node's counters and ranges, loaded one iteration ahead
   struct Pre { uint64_t c, cp; int64_t e0, e1, q0, q1; };
   auto load = [&](int32_t v) -> Pre {
     Pre x;
-    x.c = (uint64_t)cnt[v]; x.cp = v ? (uint64_t)cnt[v - 1] : 0ull;
+    if (kKept) { x.c = (uint64_t)(uint32_t)tin[v]; x.cp = (uint64_t)(uint32_t)tout[v]; }
+    else { x.c = (uint64_t)cnt[v]; x.cp = v ? (uint64_t)cnt[v - 1] : 0ull; }
     x.e0 = eoff[v]; x.e1 = eoff[v + 1]; x.q0 = qoff[v]; x.q1 = qoff[v + 1];
     return x;
   };
@@ -329,15 +473,18 @@ __global__ void k_lin_steps(const uint64_t* r, const int64_t* cnt, const int32_t
   for (int32_t v = (int32_t)lo + (threadIdx.x & 31); v < hi; v += 32) {
     const Pre pr = nx;
     if (v + 32 < hi) nx = load(v + 32);
-    if (T > 1) t = tree_forward(tt.soff, T, t, v);
-    const int32_t s0 = tt.soff[t], ns = tt.soff[t + 1] - s0;
-    const int64_t base = 2 * (int64_t)s0 + 2 * (int64_t)ns;
-    const uint64_t c = pr.c, cp = pr.cp;
-    const int64_t eid = (int64_t)(uint32_t)c - 1;
-    const int64_t xh = (int64_t)(c >> 32) - (int64_t)(cp >> 32);
-    const int64_t xid = (int64_t)(c >> 32) - xh;       // exit heads below v
-    const int64_t pe = base - (int64_t)(uint32_t)r[eid] + (v - ehead[eid]);
-    const int64_t px = base - (int64_t)(uint32_t)r[He + xid] + (xhead[xid] - v);
+    if (T > 1) t = tree_forward(tt.noff, T, t, v);
+    int64_t pe, px;
+    if (kKept) {
+      const uint32_t k = keep[pr.c];
+      if (k == (pr.c ? keep[pr.c - 1] : 0u)) continue;   // dropped
+      pe = (int64_t)k - 1;
+      px = (int64_t)keep[pr.cp] - 1;
+    } else {
+      const ArcPos a = arc_pos(r, pr.c, pr.cp, He, ehead, xhead, 2 * (int64_t)tt.noff[t + 1], v);
+      pe = a.pe;
+      px = a.px;
+    }
     const int64_t e0 = pr.e0, q0 = pr.q0;
     const int32_t ne = (int32_t)(pr.e1 - e0), nq = (int32_t)(pr.q1 - q0);
     partner[pe] = (int32_t)px;
@@ -371,8 +518,7 @@ __global__ void k_blocks(const int64_t* work, TreeTabs tt, int32_t T, int32_t B,
   x.carry_out = idx < nb - 1 ? tt.carry[t] + (int64_t)idx * ((int64_t)C + 1) : -1;
   x.t0 = x.t1 = 0;
   if (!*status) {
-    const int64_t s0 = tt.soff[t], ns = tt.soff[t + 1] - s0;
-    const int64_t a = 2 * s0, zf = a + 2 * ns;
+    const int64_t a = tt.toff[t], zf = tt.toff[t + 1];
     const int32_t lq = tt.last_q[t];
     const int64_t z = lq > 0 ? (lq < zf ? lq : zf) : a;
     const int64_t base = a > 0 ? work[a - 1] : 0;
@@ -2049,6 +2195,8 @@ static void finish_spec(PipeSpec& s, const Tuning& tune, bool forest) {
   s.tile = tune.tile >= kTileNarrowId && tune.tile <= kTileMaxId ? tune.tile
            : forest ? kTileEulerId
            : s.Q >= kQueryDense * (int64_t)s.S ? kTileQueryId : (s.Q * 8 >= s.E ? kTileNarrowId : kTileEulerId);
+  s.contract = s.E < ((int64_t)1 << 31) &&   // (a node's events are counted in 32 bits)
+               (tune.contract >= 0 ? tune.contract != 0 : s.Q * kContract <= (int64_t)s.S);
   if (s.tile == kTileQueryId) s.ctas_per_sm = 2;
   else if (s.tile >= kTileNarrow512Id) s.ctas_per_sm = 1;   // a 512-thread CTA takes the SM's registers
   const int32_t nw = words_of(s.Cmax);
@@ -2223,8 +2371,8 @@ void pipe_layout(const PipeSpec& s, Layout& L) {
   take(W_RANKB, 0);               // (list ranking runs in place)
   take(W_STEPS, S2 * 4);
   take(W_DESC, S2 * sizeof(StepDesc));
-  take(W_TIN, 0);                 // (enter/exit partners replace tin/tout)
-  take(W_TOUT, 0);
+  take(W_TIN, s.contract ? S * 4 : 0);
+  take(W_TOUT, s.contract ? S * 4 : 0);
   take(W_WORK, S2 * 8);
   take(W_SCAN, scan_tmp_bytes(S2));
   take(W_BLOCKS, B * sizeof(BlockTab));
@@ -2235,10 +2383,15 @@ void pipe_layout(const PipeSpec& s, Layout& L) {
   take(W_NSLICES, B * 4);
   take(W_CARRY, (size_t)s.carry_words * 8);
   take(W_GSUM, (size_t)s.gsum_words * 8);
+  take(W_TNOFF, s.contract ? (T + 1) * 4 : 0);
+  take(W_TTOFF, (T + 1) * 4);
+  take(W_NEOFF, s.contract ? (S + 1) * 8 : 0);
+  take(W_NQOFF, s.contract ? (S + 1) * 8 : 0);
+  take(W_NPAR, s.contract ? S * 4 : 0);
   L.total = o;
 }
 
-static TreeTabs tree_tabs(const Layout& L, char* ws) {
+static TreeTabs tree_tabs(const PipeSpec& s, const Layout& L, char* ws) {
   TreeTabs tt;
   tt.soff = reinterpret_cast<int32_t*>(ws + L.off[W_TSOFF]);
   tt.eoff = reinterpret_cast<int64_t*>(ws + L.off[W_TEOFF]);
@@ -2249,6 +2402,8 @@ static TreeTabs tree_tabs(const Layout& L, char* ws) {
   tt.carry = reinterpret_cast<int64_t*>(ws + L.off[W_TCARRY]);
   tt.gsum = reinterpret_cast<int64_t*>(ws + L.off[W_TGSUM]);
   tt.last_q = reinterpret_cast<int32_t*>(ws + L.off[W_LASTQ]);
+  tt.noff = reinterpret_cast<int32_t*>(ws + L.off[s.contract ? W_TNOFF : W_TSOFF]);
+  tt.toff = reinterpret_cast<int32_t*>(ws + L.off[W_TTOFF]);
   return tt;
 }
 
@@ -2347,20 +2502,37 @@ int pipe_tour(const PipeSpec& s, bool forest, const TourArrays& w, const int32_t
 
   if ((rc = mark(1))) return rc;
   // ---- 2. linearise
-  if ((rc = report(cudaMemsetAsync(w.fork_head, 0xFF, (size_t)S * 4, st), "memset"))) return rc;
-  k_lin_children<<<grid, 256, 0, st>>>(parent, S, w.tt, T, w.gpar, w.fork_head, w.next_sib, s.chain_hint ? 1 : 0, status);
-  if ((rc = chk("k_lin_children"))) return rc;
   const int32_t* gp = w.gpar ? w.gpar : parent;   // one tree: global = local ids
-  k_lin_flags<<<grid, 256, 0, st>>>(gp, w.fork_head, S, w.cnt, status);
+  const int32_t* nodes = w.misc + M_NODES;
+  if (s.contract) {
+    if ((rc = report(cudaMemsetAsync(w.forked, 0, (size_t)S, st), "memset"))) return rc;
+    k_ct_mark<<<grid, 256, 0, st>>>(parent, S, w.tt, T, w.gpar, w.forked, s.chain_hint ? 1 : 0, status);
+    if ((rc = chk("k_ct_mark"))) return rc;
+    k_ct_ends<<<grid, 256, 0, st>>>(gp, w.forked, w.qoff, S, w.ends, status);
+    if ((rc = chk("k_ct_ends"))) return rc;
+    if ((rc = device_inclusive_scan<uint32_t>(w.ends, S, w.scan_tmp, st, kernels))) return report((cudaError_t)rc, "scan");
+    k_ct_nodes<<<grid, 256, 0, st>>>(gp, w.ends, w.eoff, w.qoff, S, w.tt, T, w.neoff, w.nqoff, w.npar, w.fork_head,
+                                     w.misc);
+    if ((rc = chk("k_ct_nodes"))) return rc;
+    gp = w.npar;
+    k_ct_children<<<grid, 256, 0, st>>>(gp, nodes, w.fork_head, w.next_sib, status);
+    if ((rc = chk("k_ct_children"))) return rc;
+  } else {
+    if ((rc = report(cudaMemsetAsync(w.fork_head, 0xFF, (size_t)S * 4, st), "memset"))) return rc;
+    k_lin_children<<<grid, 256, 0, st>>>(parent, S, w.tt, T, w.gpar, w.fork_head, w.next_sib, s.chain_hint ? 1 : 0,
+                                         status);
+    if ((rc = chk("k_lin_children"))) return rc;
+  }
+  k_lin_flags<<<grid, 256, 0, st>>>(gp, w.fork_head, nodes, w.cnt, status);
   if ((rc = chk("k_lin_flags"))) return rc;
-  if ((rc = device_inclusive_scan_i64(w.cnt, S, w.scan_tmp, st, kernels))) return report((cudaError_t)rc, "scan");
-  k_lin_heads<<<grid, 256, 0, st>>>(w.cnt, S, w.ehead, w.xhead, status);
+  if ((rc = device_inclusive_scan<int64_t>(w.cnt, S, w.scan_tmp, st, kernels, nodes))) return report((cudaError_t)rc, "scan");
+  k_lin_heads<<<grid, 256, 0, st>>>(w.cnt, nodes, w.ehead, w.xhead, status);
   if ((rc = chk("k_lin_heads"))) return rc;
-  k_lin_rank_init<<<grid, 256, 0, st>>>(w.cnt, w.ehead, w.xhead, gp, w.fork_head, w.next_sib, S, w.rank, status);
+  k_lin_rank_init<<<grid, 256, 0, st>>>(w.cnt, w.ehead, w.xhead, gp, w.fork_head, w.next_sib, nodes, w.rank, status);
   if ((rc = chk("k_lin_rank_init"))) return rc;
   int32_t round = 0;
   for (int64_t span = 1; span < 2 * (int64_t)s.Smax; span <<= 1, ++round) {
-    k_lin_round<<<grid, 256, 0, st>>>(w.rank, w.cnt, S, w.misc + M_ROUNDS, round, status);
+    k_lin_round<<<grid, 256, 0, st>>>(w.rank, w.cnt, nodes, w.misc + M_ROUNDS, round, status);
     if ((rc = chk("k_lin_round"))) return rc;
   }
   return 0;
@@ -2379,7 +2551,7 @@ int pipe_enqueue(const PipeSpec& s, void* workspace, const int32_t* parent, cons
   pipe_layout(s, L);
   char* ws = static_cast<char*>(workspace);
   auto at = [&](int slot) { return ws + L.off[slot]; };
-  const TreeTabs tt = tree_tabs(L, ws);
+  const TreeTabs tt = tree_tabs(s, L, ws);
   int32_t* misc = reinterpret_cast<int32_t*>(at(W_MISC));
   int32_t* status = misc + M_STATUS;
   int64_t* eoff = reinterpret_cast<int64_t*>(at(W_EOFF));
@@ -2412,14 +2584,38 @@ int pipe_enqueue(const PipeSpec& s, void* workspace, const int32_t* parent, cons
   TourArrays ta;
   ta.tt = tt; ta.misc = misc; ta.eoff = eoff; ta.qoff = qoff; ta.gpar = gpar; ta.fork_head = fork_head;
   ta.next_sib = next_sib; ta.cnt = cnt; ta.ehead = ehead; ta.xhead = xhead; ta.rank = rank_a; ta.scan_tmp = scan_tmp;
+  ta.neoff = reinterpret_cast<int64_t*>(at(W_NEOFF)); ta.nqoff = reinterpret_cast<int64_t*>(at(W_NQOFF));
+  ta.npar = reinterpret_cast<int32_t*>(at(W_NPAR));
+  // node numbers and fork marks live in the step descriptors, which are written last
+  ta.ends = reinterpret_cast<uint32_t*>(at(W_DESC)); ta.forked = reinterpret_cast<uint8_t*>(at(W_DESC)) + (size_t)s.S * 4;
   if ((rc = pipe_tour(s, forest, ta, parent, events, queries, st, timing, kernels))) return rc;
-  const uint64_t* src = rank_a;
-  k_lin_steps<<<grid, 256, 0, st>>>(src, cnt, ehead, xhead, S, tt, T, eoff, qoff, partner, desc, work, status);
+  const int32_t *nodes = misc + M_NODES, *steps = misc + M_STEPS;
+  if (s.contract) {
+    // scratch that is free here: the work array (queries per step), the rank array (steps
+    // kept, once the positions are out of it)
+    int32_t *tin = reinterpret_cast<int32_t*>(at(W_TIN)), *tout = reinterpret_cast<int32_t*>(at(W_TOUT));
+    uint32_t *nq = reinterpret_cast<uint32_t*>(work), *keep = reinterpret_cast<uint32_t*>(rank_a);
+    k_lin_pos<<<grid, 256, 0, st>>>(rank_a, cnt, ehead, xhead, nodes, tt, T, ta.nqoff, tin, tout, nq, status);
+    if ((rc = chk("k_lin_pos"))) return rc;
+    if ((rc = device_inclusive_scan<uint32_t>(nq, 2 * (int64_t)S, scan_tmp, st, kernels, steps)))
+      return report((cudaError_t)rc, "scan");
+    k_lin_keep<<<grid, 256, 0, st>>>(nodes, tin, tout, ta.nqoff, nq, keep, status);
+    if ((rc = chk("k_lin_keep"))) return rc;
+    if ((rc = device_inclusive_scan<uint32_t>(keep, 2 * (int64_t)S, scan_tmp, st, kernels, steps)))
+      return report((cudaError_t)rc, "scan");
+    k_lin_trees<<<(T + 256) / 256, 256, 0, st>>>(keep, tt, T, misc);
+    if ((rc = chk("k_lin_trees"))) return rc;
+    k_lin_steps<true><<<grid, 256, 0, st>>>(nullptr, nullptr, nullptr, nullptr, tin, tout, keep, nodes, tt, T, ta.neoff,
+                                            ta.nqoff, partner, desc, work, status);
+  } else {
+    k_lin_steps<false><<<grid, 256, 0, st>>>(rank_a, cnt, ehead, xhead, nullptr, nullptr, nullptr, nodes, tt, T, eoff,
+                                             qoff, partner, desc, work, status);
+  }
   if ((rc = chk("k_lin_steps"))) return rc;
 
   if ((rc = mark(2))) return rc;
   // ---- 3. blocks
-  if ((rc = device_inclusive_scan_i64(work, 2 * (int64_t)S, scan_tmp, st, kernels)))
+  if ((rc = device_inclusive_scan<int64_t>(work, 2 * (int64_t)S, scan_tmp, st, kernels, steps)))
     return report((cudaError_t)rc, "scan");
   k_blocks<<<(B + 127) / 128, 128, 0, st>>>(work, tt, T, B, blocks, status);
   if ((rc = chk("k_blocks"))) return rc;

@@ -34,6 +34,8 @@ constexpr int64_t kQueryCost = 2;             // a query is two prefix probes
 // took MW_OLD us, at 16,384 MW_NEW us.  The larger value stays for callers whose scratch the
 // smaller blocks would outgrow.
 constexpr int64_t kMinWork = 16384, kMinWorkCoarse = 65536;
+// A tour is contracted when at most one state in kContract has a query (see k_ct_nodes).
+constexpr int64_t kContract = 2;
 // Queries per state from which a tree is swept a step at a time by bw_qsweep.cu: measured
 // against k_sweep's narrow tile, 15 a state 1.02 and 1.18 ms, 18 a state 0.60 and 0.63 ms,
 // 167 a state 0.33 and 0.49 ms (4M events) and 2.3 and 4.6 ms (40M), 2 a state 0.94 and 0.44 ms.
@@ -140,6 +142,8 @@ struct TreeTabs {
   int64_t* carry;        // T   first carry word of the tree's rows
   int64_t* gsum;         // T   first group-sum word
   int32_t* last_q;       // T   last step answering a query + 1 (0: none)
+  int32_t* noff;         // T+1 first tour node (states: soff; contracted: written per launch)
+  int32_t* toff;         // T+1 first tour step
 };
 
 // Shared-memory layout of the sweep for a rank-table window of `ww` words.
@@ -204,6 +208,7 @@ struct Tuning {
   int64_t block_work = 0;   // target work per state block (est_work units); 0 = auto
   int32_t ctas_per_sm = 0;  // persistent sweep CTAs per SM (1 or 2); 0 = auto
   int32_t slice_ranks = 0;  // cap on the ranks of one LUT slice (0 = all that fit shared memory)
+  int32_t contract = -1;    // 1 / 0: contracted tour or not (-1: by the queries per state)
   int32_t tile = 0;         // sweep tile geometry: kTileNarrowId, kTileWideId, 0 = by query/event ratio
 };
 
@@ -227,6 +232,7 @@ struct PipeSpec {
   SweepLayout SL{};
   QsLayout QL{};                // tile 7
   bool chain_hint = false;
+  bool contract = false;        // the tour runs over contracted nodes, without those no query needs
   // one-tree scalars (T == 1): tables are written by a kernel at each launch
   int32_t nb1 = 1;
   // forest host tables, uploaded once by bind (empty for the plain one-tree spec)
@@ -238,7 +244,7 @@ struct PipeSpec {
 };
 
 struct Layout {
-  size_t off[40];
+  size_t off[48];
   size_t total;
 };
 
@@ -246,11 +252,12 @@ enum {
   W_TSOFF, W_TEOFF, W_TQOFF, W_TC, W_TBOFF, W_TBITS, W_TCARRY, W_TGSUM, W_LASTQ, W_UNITS, W_ORDER,
   W_MISC, W_EOFF, W_QOFF, W_GPAR, W_FORK, W_NEXT, W_CNT, W_EHEAD, W_XHEAD, W_RANKA, W_RANKB,
   W_STEPS, W_DESC, W_TIN, W_TOUT, W_WORK, W_SCAN, W_BLOCKS, W_BMODE, W_BITS, W_RLUT, W_SLICES,
-  W_NSLICES, W_CARRY, W_GSUM, W_COUNT
+  W_NSLICES, W_CARRY, W_GSUM, W_TNOFF, W_TTOFF, W_NEOFF, W_NQOFF, W_NPAR, W_COUNT
 };
 
 // misc words
-enum { M_STATUS = 0, M_PREP_TICKET = 1, M_SWEEP_TICKET = 2, M_CHAIN = 3, M_PREPB_TICKET = 4, M_ROUNDS = 32 };  // 64 words
+enum { M_STATUS = 0, M_PREP_TICKET = 1, M_SWEEP_TICKET = 2, M_CHAIN = 3, M_PREPB_TICKET = 4, M_NODES = 5, M_STEPS = 6,
+       M_ROUNDS = 32 };  // 64 words
 
 // Stage timing events of one launch: stage i runs from ev[i] to ev[i + 1]; a chain
 // launch (chain = 1) records the sweep from ev[BW_STAGE_SWEEP] to ev[BW_STAGE_SWEEP+1]
@@ -284,6 +291,12 @@ struct TourArrays {
   int32_t *ehead, *xhead;
   uint64_t* rank;            // 2 S
   int64_t* scan_tmp;
+  // contracted tours: event and query offsets and parents of the nodes; S words of scratch
+  // for the node numbers and S bytes for the fork marks
+  int64_t *neoff, *nqoff;
+  int32_t* npar;
+  uint32_t* ends;
+  uint8_t* forked;
 };
 int pipe_tour(const PipeSpec& spec, bool forest, const TourArrays& w, const int32_t* parent, const BwEvent* events,
               const BwQuery* queries, cudaStream_t st, EventSet* timing, int& kernels);

@@ -50,19 +50,28 @@ int spec_of(const BwReplayArgs* a, PipeSpec& s, Layout& L) {
   int rc = device_sms(&sms);
   if (rc) return rc;
   const size_t small = (size_t)32 << 20;
+  Tuning tune;
   auto plan = [&](int64_t min_work) {
     const int r = pipe_spec_one(a->n_states, a->n_keys, a->n_events, a->n_queries, a->blocks,
-                                (a->flags & BW_REPLAY_CHAIN_HINT) != 0, Tuning(), sms, s, min_work);
+                                (a->flags & BW_REPLAY_CHAIN_HINT) != 0, tune, sms, s, min_work);
     if (!r) pipe_layout(s, L);
     return r;
   };
-  if ((rc = plan(kMinWork)) || L.total <= small || a->blocks > 0) return rc;
+  if ((rc = plan(kMinWork)) || L.total <= small) return rc;
+  // does the plainest plan fit?
+  tune.contract = 0;
   if ((rc = plan(kMinWorkCoarse))) return rc;
   const bool fits = L.total <= small;
-  for (int64_t w = kMinWork; w < kMinWorkCoarse; w += w / 4) {
-    if ((rc = plan(w))) return rc;
-    if (!fits || L.total <= small) return 0;
+  tune.contract = -1;
+  if (!fits || a->blocks > 0) {
+    if ((rc = plan(kMinWork)) || !fits || L.total <= small) return rc;
+    tune.contract = 0;
+    return plan(kMinWork);
   }
+  for (int64_t w = kMinWork; w < kMinWorkCoarse; w += w / 4) {
+    if ((rc = plan(w)) || L.total <= small) return rc;
+  }
+  tune.contract = 0;
   return plan(kMinWorkCoarse);
 }
 
