@@ -19,8 +19,8 @@
 //     order and exit events from the back, so an event's sign is its side of the
 //     stage; a query records how many enter and exit events of the tile precede it,
 //     and its bounds arrive by cp.async tracked by the same barrier;
-//   * sixteen consumer warps take a tile: each thread loads its two events (and, for
-//     int32 windows, repacks them as signed (key, delta) pairs), each warp its
+//   * thirty consumer warps take a tile: each thread loads its event (and, for
+//     int32 windows, repacks it as a signed (key, delta) pair), each warp its
 //     queries, and the stage is released on its "empty" mbarrier (int64 windows: after
 //     the scans, which then read the stage itself).  One warp per
 //     query: before a consumer barrier the probe of the window over [lo, hi) as it
@@ -31,7 +31,7 @@
 //     the tree's key domain fits it, else over the block's key ranks one rank slice at
 //     a time (popcount rank table of the prepare pass); int32 entries when the block's
 //     applied |delta| sum is below 2^31 (every partial sum is then exact), int64 ones
-//     otherwise; 32-entry chunk totals for windows above 4,096 entries.
+//     otherwise; totals of 32 and of 1,024 entries for windows above 256 and 4,096.
 //
 // Per tile the consumers meet at most twice: before the probes (the previous tiles'
 // updates are complete; the barrier also agrees on lost waits) and after them.  Every
@@ -48,15 +48,25 @@
 namespace bw {
 namespace {
 
-constexpr int kEsNC = 512;                 // consumer threads
+// Consumers: an event each and tiles of as many, so that a tile's queries (17 of the batched
+// trees') mostly find a warp each.  512 threads with two events took 4.35 ms on the batched
+// trees, 960 take 3.73 (two events each and a window of 20,480 entries: 3.57, but a third
+// fewer int64 entries).
+constexpr int kEsNC = 960;                 // consumer threads
 constexpr int kEsNWC = kEsNC / 32;         // consumer warps
 constexpr int kEsThreads = kEsNC + 64;     // plus the producer warps (planner, issuer)
-constexpr int kEsEPT = 2;                  // events per consumer thread per tile
+constexpr int kEsEPT = 1;                  // events per consumer thread per tile
 constexpr int kEsTile = kEsNC * kEsEPT;    // events per tile
 constexpr int kEsStages = 3;
-constexpr int kEsQB = 64;                  // queries per tile
+constexpr int kEsQB = 60;                  // queries per tile
 constexpr int kEsQW = kEsQB / kEsNWC;      // queries per consumer warp per tile
-constexpr uint32_t kEsFlat = 4096;         // windows up to this size keep no chunk totals
+// Windows above kEsFlat entries keep totals of 32-entry chunks, those above kEsDeep also
+// totals of 1,024 entries, so that a probe reads at most five words a lane.  The chunk
+// totals of small windows and the second level cost an atomic per event each and save a
+// probe up to 32 reads: at one query per 60 events of the batched trees the sweep took
+// 4.66 ms with one level above 4,096 entries, 4.35 ms so.
+constexpr uint32_t kEsFlat = 256;
+constexpr uint32_t kEsDeep = 4096;
 constexpr int kEsRing = 256;               // planner's descriptor ring (steps)
 constexpr uint32_t kEsWaitLimit = 1u << 22;
 constexpr uint32_t kFull = 0xffffffffu;
@@ -70,7 +80,7 @@ struct EsCtl {
 
 // Dynamic shared memory (all regions 16-byte aligned).
 struct EsSmem {
-  size_t H, T, bits, rl, stage, pack, q, meta, bar, ctl, ring, plan, pmeta, bytes;
+  size_t H, T, U, bits, rl, stage, pack, q, meta, bar, ctl, ring, plan, pmeta, bytes;
 };
 __host__ __device__ constexpr size_t es_al(size_t x) { return (x + 15) & ~size_t(15); }
 __host__ __device__ constexpr EsSmem es_smem() {
@@ -78,6 +88,7 @@ __host__ __device__ constexpr EsSmem es_smem() {
   size_t o = 0;
   L.H = o;     o = es_al(o + (size_t)kEsCap32 * 4);                 // int32 x cap32 == int64 x cap64
   L.T = o;     o = es_al(o + (size_t)(kEsCap32 / 32) * 4);
+  L.U = o;     o = es_al(o + (size_t)(kEsCap32 / 1024 + 1) * 4);
   L.bits = o;  o = es_al(o + (size_t)kWinWords * 8);
   L.rl = o;    o = es_al(o + ((size_t)kWinWords + 2) * 2);          // slice-local ranks, uint16
   L.stage = o; o = es_al(o + (size_t)kEsStages * kEsTile * 16);
@@ -168,6 +179,7 @@ struct EsPass {
   uint32_t klo, khi;      // keys of the slice
   uint32_t nr;            // window entries
   int32_t nch;            // chunk totals (0: flat probes)
+  int32_t nsup;           // totals of 1,024 entries (0: none)
   bool dense, first;
   const int64_t* crow;    // carried key-prefix row (nullptr: the block starts its tree)
 };
@@ -463,7 +475,8 @@ __device__ bool es_issue(const EsParams& p, unsigned char* sm, const uint4* plan
 // Lane share of the window sum over entries [ra, rb) (ra < rb <= nr): partial chunks
 // from H, whole chunks from T; or flat 128-bit reads (H padded to whole uint4s).
 template <typename HT>
-__device__ __forceinline__ HT es_probe(const HT* H, const HT* T, int32_t nch, uint32_t ra, uint32_t rb, int lane) {
+__device__ __forceinline__ HT es_probe(const HT* H, const HT* T, const HT* U, int32_t nch, int32_t nsup, uint32_t ra,
+                                       uint32_t rb, int lane) {
   HT s = 0;
   if (nch) {
     const uint32_t clo = (ra + 31) >> 5, chi = rb >> 5;
@@ -474,7 +487,15 @@ __device__ __forceinline__ HT es_probe(const HT* H, const HT* T, int32_t nch, ui
     const uint32_t x = ra + lane, y = (chi << 5) + lane;
     if (x < (clo << 5)) s += H[x];
     if (y < rb) s += H[y];
-    for (uint32_t c = clo + lane; c < chi; c += 32) s += T[c];
+    const uint32_t slo = (clo + 31) >> 5, shi = chi >> 5;
+    if (!nsup || slo >= shi) {
+      for (uint32_t c = clo + lane; c < chi; c += 32) s += T[c];
+      return s;
+    }
+    const uint32_t cx = clo + lane, cy = (shi << 5) + lane, u = slo + lane;
+    if (cx < (slo << 5)) s += T[cx];
+    if (cy < chi) s += T[cy];
+    if (u < shi) s += U[u];   // (at most 28)
     return s;
   }
   constexpr uint32_t per = 16 / sizeof(HT);
@@ -525,6 +546,7 @@ __device__ bool es_consume(const EsParams& p, const EsPass& ps, unsigned char* s
   constexpr EsSmem L = es_smem();
   HT* H = reinterpret_cast<HT*>(sm + L.H);
   HT* T = reinterpret_cast<HT*>(sm + L.T);
+  HT* U = reinterpret_cast<HT*>(sm + L.U);
   const uint64_t* bits = reinterpret_cast<const uint64_t*>(sm + L.bits);
   const uint16_t* rl = reinterpret_cast<const uint16_t*>(sm + L.rl);
   const uint4* stages = reinterpret_cast<const uint4*>(sm + L.stage);
@@ -597,7 +619,7 @@ __device__ bool es_consume(const EsParams& p, const EsPass& ps, unsigned char* s
           const uint32_t a = lo > klo ? lo : klo, z = hi < khi ? hi : khi;
           if (a < z) {
             const uint32_t ra = rank_of(a), rb = rank_of(z);
-            if (ra < rb) part[r] = es_probe<HT>(H, T, ps.nch, ra, rb, lane);
+            if (ra < rb) part[r] = es_probe<HT>(H, T, U, ps.nch, ps.nsup, ra, rb, lane);
           }
         }
       }
@@ -663,10 +685,12 @@ __device__ bool es_consume(const EsParams& p, const EsPass& ps, unsigned char* s
             const int32_t v = (int32_t)e.z, d = neg ? -v : v;
             atomicAdd(reinterpret_cast<int32_t*>(H) + r, d);
             if (ps.nch) atomicAdd(reinterpret_cast<int32_t*>(T) + (r >> 5), d);
+            if (ps.nsup) atomicAdd(reinterpret_cast<int32_t*>(U) + (r >> 10), d);
           } else {
             const uint64_t v = ((uint64_t)e.w << 32) | e.z, d = neg ? (uint64_t)0 - v : v;
             shared_add_u64(reinterpret_cast<unsigned long long*>(H) + r, d);
             if (ps.nch) shared_add_u64(reinterpret_cast<unsigned long long*>(T) + (r >> 5), d);
+            if (ps.nsup) shared_add_u64(reinterpret_cast<unsigned long long*>(U) + (r >> 10), d);
           }
         }
       }
@@ -684,6 +708,7 @@ __device__ void es_setup(const EsParams& p, const EsPass& ps, const BlockTab& bt
   constexpr EsSmem L = es_smem();
   HT* H = reinterpret_cast<HT*>(sm + L.H);
   HT* T = reinterpret_cast<HT*>(sm + L.T);
+  HT* U = reinterpret_cast<HT*>(sm + L.U);
   uint64_t* bits = reinterpret_cast<uint64_t*>(sm + L.bits);
   uint16_t* rl = reinterpret_cast<uint16_t*>(sm + L.rl);
   const int tid = threadIdx.x;
@@ -692,6 +717,7 @@ __device__ void es_setup(const EsParams& p, const EsPass& ps, const BlockTab& bt
   uint4* H4 = reinterpret_cast<uint4*>(H);
   for (uint32_t i = tid; i < n16; i += kEsNC) H4[i] = make_uint4(0, 0, 0, 0);
   for (int32_t i = tid; i < ps.nch; i += kEsNC) T[i] = 0;
+  for (int32_t i = tid; i < ps.nsup; i += kEsNC) U[i] = 0;
   if (!ps.dense) {
     const uint64_t* gbits = p.bits + bt.bits_off;
     const uint32_t* grl = p.rlut + bt.bits_off + b;
@@ -763,6 +789,7 @@ __global__ void __launch_bounds__(kEsThreads, 1) k_esweep(EsParams p) {
       ps.khi = ps.dense ? C : (uint32_t)min((uint64_t)s.word_hi << 6, (uint64_t)C);
       ps.nr = ps.dense ? C : s.n;
       ps.nch = ps.nr > kEsFlat ? (int32_t)((ps.nr + 31) >> 5) : 0;
+      ps.nsup = ps.nr > kEsDeep ? (int32_t)((ps.nr + 1023) >> 10) : 0;
       ps.first = si == first_si;
       if (warp == kEsNWC) {
         es_plan(p, ps, ring, plan, pmeta, ctl, lane);

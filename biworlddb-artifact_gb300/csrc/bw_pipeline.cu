@@ -113,72 +113,135 @@ __device__ __forceinline__ int32_t tree_forward(const Off* off, int32_t T, int32
   return t;
 }
 
+// off[x] = the item of the group's first lane whose state reaches x, for every state x in
+// (lane 0's gprev, lane 31's g]; all lanes' g are non-decreasing from gprev on.  Short
+// ranges are written by the lanes whose state steps, long ones (fewer items than states)
+// by the whole warp.
+__device__ __forceinline__ void offsets_group(int64_t* off, int64_t i, int32_t g, int32_t gprev, int lane) {
+  const int32_t first = __shfl_sync(0xffffffffu, gprev, 0), last = __shfl_sync(0xffffffffu, g, 31);
+  if (last - first <= 64) {
+    for (int32_t x = gprev + 1; x <= g; ++x) off[x] = i;
+    return;
+  }
+  for (int32_t x0 = first + 1; x0 <= last; x0 += 128) {
+    int at[4];   // first lane with g >= x, four searches side by side
+#pragma unroll
+    for (int u = 0; u < 4; ++u) at[u] = 0;
+#pragma unroll
+    for (int s = 16; s; s >>= 1) {
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (__shfl_sync(0xffffffffu, g, at[u] + s - 1) < x0 + 32 * u + lane) at[u] += s;
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int32_t x = x0 + 32 * u + lane;
+      if (x <= last) off[x] = i - lane + at[u];
+    }
+  }
+}
+
+// Items are taken 128 a warp at a time (four reads in flight) while they belong to one
+// tree, are in range and in order; a group of 32 that is not goes lane by lane.
+// Bound by the reads where every state has items (3.5 GB of events: 1.02 -> 0.79 ms
+// with the tree's tables in registers instead of three table reads an item), by the writes where
+// few have (4M queries over 27M states: 0.26 -> 0.10 ms with the cooperative fill).
 template <bool kEvents>
-__global__ void k_offsets(const void* items, int64_t n, TreeTabs tt, int32_t T, int32_t S, int64_t* off,
-                          int32_t* status) {
+__global__ void __launch_bounds__(256) k_offsets(const void* items, int64_t n, TreeTabs tt, int32_t T, int32_t S,
+                                                 int64_t* off, int32_t* status) {
   const int64_t* toff = kEvents ? tt.eoff : tt.qoff;
   const BwEvent* ev = static_cast<const BwEvent*>(items);
   const BwQuery* qs = static_cast<const BwQuery*>(items);
   const int lane = threadIdx.x & 31;
-  int64_t lo, hi;
-  warp_range(n, lo, hi);
-  if (lo >= hi) return;
-  // global state of a tree-local state s of tree t (-2: out of its tree, reported by its own lane)
-  auto gstate_of = [&](int32_t t, uint32_t s) -> int64_t {
-    const int32_t s0 = tt.soff[t], ns = tt.soff[t + 1] - s0;
-    return s < (uint32_t)ns ? (int64_t)s0 + s : -2;
-  };
-  auto gstate = [&](int32_t t, int64_t i) -> int64_t { return gstate_of(t, kEvents ? ev[i].state : qs[i].state); };
-  // an item's (state, key) or (state, lo, hi), loaded one iteration ahead so a
-  // warp keeps two record loads in flight
-  struct Rec { uint32_t s, a, b; };
+  // items a warp takes at a time: few, so that long runs of states without items do not
+  // meet in one warp, but enough for the tree search at their start
+  const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
+  const int64_t chunk = kEvents ? imin64(2048, (n / (4 * warps) + 128) & ~(int64_t)127) : 128;
+  struct Rec { uint32_t s, a; };   // state; key, or the larger bound
   auto load = [&](int64_t i) -> Rec {
     Rec r;
     if (kEvents) {
       const uint2 v = __ldg(reinterpret_cast<const uint2*>(ev + i));   // state, key
-      r.s = v.x; r.a = v.y; r.b = 0;
+      r.s = v.x; r.a = v.y;
     } else {
-      r.s = qs[i].state; r.a = qs[i].lo; r.b = qs[i].hi;
+      const uint32_t* q = reinterpret_cast<const uint32_t*>(qs + i);
+      r.s = __ldg(q); r.a = max(__ldg(q + 1), __ldg(q + 2));
     }
     return r;
   };
-  int64_t gcarry = -1;   // global state of the item before this lane 0's item
-  if (lo > 0) {
-    int64_t gp = 0;
-    if (lane == 0) gp = gstate(T > 1 ? find_tree(toff, T, lo - 1) : 0, lo - 1);
-    gcarry = __shfl_sync(0xffffffffu, gp, 0);
-  }
-  int32_t t = T > 1 ? find_tree(toff, T, imin64(lo + lane, n - 1)) : 0;
-  Rec nx = lo + lane < hi ? load(lo + lane) : Rec{0, 0, 0};
-  for (int64_t i0 = lo; i0 < hi; i0 += 32) {
-    const int64_t i = i0 + lane;
-    const bool valid = i < hi;
-    const Rec rc = nx;
-    if (i + 32 < hi) nx = load(i + 32);
-    int64_t g = -2;
-    if (valid) {
-      if (T > 1) t = tree_forward(toff, T, t, i);
-      const uint32_t C = tt.C[t];
-      if (kEvents) {
-        if (rc.a >= C) set_status(status, BW_STATUS_EVENT_KEY_RANGE);
-      } else {
-        if (rc.a > C || rc.b > C) set_status(status, BW_STATUS_QUERY_RANGE);
+  // the current tree (warp-uniform): its items end at tend
+  int32_t t = 0;
+  int64_t tend = 0;
+  int32_t s0 = 0, ns = 0;
+  uint32_t amax = 0;   // largest key, or bound
+  auto enter = [&](int64_t i) {
+    if (T > 1) t = tree_forward(toff, T, t, i);
+    tend = toff[t + 1];
+    s0 = tt.soff[t];
+    ns = tt.soff[t + 1] - s0;
+    amax = tt.C[t] - (kEvents ? 1u : 0u);
+  };
+  // global state of the item before (a state out of its tree: -2, reported by its own lane)
+  auto gstate = [&](int32_t tr, uint32_t st) -> int32_t {
+    const int32_t b = tt.soff[tr], k = tt.soff[tr + 1] - b;
+    return st < (uint32_t)k ? b + (int32_t)st : -2;
+  };
+  for (int64_t lo = ((int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * chunk; lo < n; lo += warps * chunk) {
+    const int64_t hi = imin64(n, lo + chunk);
+    t = T > 1 ? find_tree(toff, T, lo > 0 ? lo - 1 : 0) : 0;   // (the tree of the item before)
+    int32_t gcarry = -1;
+    if (lo > 0) gcarry = gstate(t, kEvents ? ev[lo - 1].state : qs[lo - 1].state);
+    enter(lo);
+    for (int64_t i0 = lo; i0 < hi;) {
+      if (i0 >= tend) enter(i0);
+      const int64_t end = imin64(hi, tend);
+      Rec r[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) r[j] = i0 + 32 * j + 32 <= end ? load(i0 + 32 * j + lane) : Rec{0, 0};
+      int64_t next = i0;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        if (i0 + 32 * j + 32 > end) break;   // warp-uniform
+        const int64_t i = i0 + 32 * j + lane;
+        const int32_t g = s0 + (int32_t)r[j].s;
+        int32_t gprev = __shfl_up_sync(0xffffffffu, g, 1);
+        if (lane == 0) gprev = gcarry;
+        const bool ok = r[j].s < (uint32_t)ns && r[j].a <= amax && gprev != -2 && gprev <= g;
+        if (!__all_sync(0xffffffffu, ok)) break;
+        offsets_group(off, i, g, gprev, lane);
+        gcarry = __shfl_sync(0xffffffffu, g, 31);
+        next += 32;
       }
-      g = gstate_of(t, rc.s);
-      if (g == -2) set_status(status, BW_STATUS_STATE_RANGE);
+      if (next == i0) {
+        // up to 32 items of any trees, checked and written lane by lane
+        const int64_t i = i0 + lane;
+        const bool valid = i < hi;
+        int32_t g = -2;
+        if (valid) {
+          const int32_t tr = T > 1 ? tree_forward(toff, T, t, i) : 0;
+          const Rec x = load(i);
+          if (x.a > tt.C[tr] - (kEvents ? 1u : 0u))
+            set_status(status, kEvents ? BW_STATUS_EVENT_KEY_RANGE : BW_STATUS_QUERY_RANGE);
+          g = gstate(tr, x.s);
+          if (g == -2) set_status(status, BW_STATUS_STATE_RANGE);
+        }
+        int32_t gprev = __shfl_up_sync(0xffffffffu, g, 1);
+        if (lane == 0) gprev = gcarry;
+        gcarry = __shfl_sync(0xffffffffu, g, 31);
+        if (valid && g != -2 && gprev != -2) {
+          if (gprev > g) {   // an earlier tree's states are below every state of this tree
+            set_status(status, kEvents ? BW_STATUS_EVENTS_UNSORTED : BW_STATUS_QUERIES_UNSORTED);
+          } else {
+            for (int32_t x = gprev + 1; x <= g; ++x) off[x] = i;
+          }
+        }
+        if (i0 + 32 >= hi) gcarry = __shfl_sync(0xffffffffu, g, (int)(hi - 1 - i0));
+        next = i0 + 32;
+      }
+      i0 = next;
     }
-    int64_t gprev = __shfl_up_sync(0xffffffffu, g, 1);
-    if (lane == 0) gprev = gcarry;
-    gcarry = __shfl_sync(0xffffffffu, g, 31);
-    if (!valid || g == -2 || gprev == -2) continue;
-    if (gprev > g) {   // an earlier tree's states are below every state of this tree
-      set_status(status, kEvents ? BW_STATUS_EVENTS_UNSORTED : BW_STATUS_QUERIES_UNSORTED);
-      continue;
-    }
-    // off[x] = i for every global state x in (gprev, g]
-    for (int64_t x = gprev + 1; x <= g; ++x) off[x] = i;
-    if (i == n - 1)
-      for (int64_t x = g + 1; x <= S; ++x) off[x] = n;
+    if (hi == n && gcarry != -2)   // the states after the last item
+      for (int32_t x = gcarry + 1 + lane; x <= S; x += 32) off[x] = n;
   }
 }
 
@@ -365,13 +428,17 @@ __global__ void k_lin_rank_init(const int64_t* cnt, const int32_t* ehead, const 
   }
 }
 
-// One Wyllie pointer-jumping round, in place: dist(x) += dist(next(x)),
-// next(x) = next(next(x)).  A (next, dist) pair is one 64-bit word, so a read sees a
+// Pointer jumping, in place: dist(x) += dist(next(x)), next(x) = next(next(x)), up to
+// kLinJumps times a launch.  A (next, dist) pair is one 64-bit word, so a read sees a
 // consistent pair even while its owner updates it (jumping further ahead keeps
-// dist(x) = the lengths from x up to next(x)).  Round r records whether any pointer
-// is still live; a round after one that found none returns at once.
-__global__ void k_lin_round(uint64_t* __restrict__ r, const int64_t* cnt, const int32_t* nodes, int32_t* live, int32_t round,
-                            const int32_t* status) {
+// dist(x) = the lengths from x up to next(x)).  A launch after pointers that all span d
+// segments leaves them spanning at least (kLinJumps + 1) d, so five launches rank what took
+// twenty one-jump rounds of 4 us each; more where the words read were already updated.
+// Launch r records whether any pointer is still live; one after a launch that found none
+// returns at once.
+constexpr int kLinJumps = 15;
+__global__ void k_lin_round(uint64_t* __restrict__ r, const int64_t* cnt, const int32_t* nodes, int32_t* live,
+                            int32_t round, const int32_t* status) {
   if (*status) return;
   const int32_t S = *nodes;
   if (round > 0 && live[round - 1] == 0) return;
@@ -379,12 +446,17 @@ __global__ void k_lin_round(uint64_t* __restrict__ r, const int64_t* cnt, const 
   const int64_t H = (int64_t)(uint32_t)tot + (int64_t)(tot >> 32);
   bool any = false;
   for (int64_t x = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; x < H; x += (int64_t)gridDim.x * blockDim.x) {
-    const uint64_t a = r[x];
-    const int32_t nx = (int32_t)(a >> 32);
+    uint64_t a = __ldcg(reinterpret_cast<unsigned long long*>(r) + x);
+    int32_t nx = (int32_t)(a >> 32);
     if (nx < 0) continue;
-    const uint64_t b = r[nx];
-    r[x] = (b & 0xFFFFFFFF00000000ull) | (uint32_t)((uint32_t)a + (uint32_t)b);
-    any |= (int32_t)(b >> 32) >= 0;
+#pragma unroll 1
+    for (int k = 0; k < kLinJumps && nx >= 0; ++k) {
+      const uint64_t b = __ldcg(reinterpret_cast<unsigned long long*>(r) + nx);   // (not from the L1: others write it)
+      a = (b & 0xFFFFFFFF00000000ull) | (uint32_t)((uint32_t)a + (uint32_t)b);
+      nx = (int32_t)(b >> 32);
+    }
+    __stcg(reinterpret_cast<unsigned long long*>(r) + x, (unsigned long long)a);
+    any |= nx >= 0;
   }
   if (__syncthreads_or(any) && threadIdx.x == 0) live[round] = 1;
 }
@@ -496,7 +568,16 @@ __global__ void k_lin_steps(const uint64_t* r, const int64_t* cnt, const int32_t
     desc[px] = d;
     work[pe] = kStepCost + ne + (nq > 0 ? kQueryStepCost + kQueryCost * nq : 0);
     work[px] = kStepCost + ne;
-    if (nq > 0) atomicMax(&tt.last_q[t], (int32_t)pe + 1);
+    // one atomic per tree and warp (all of a tree's states on its one word took 190 us
+    // for 300,000 states)
+    const int32_t lq = nq > 0 ? (int32_t)pe + 1 : 0;
+    const unsigned here = __activemask();
+    if (T == 1 || __match_any_sync(here, t) == here) {
+      const int32_t m = __reduce_max_sync(here, lq);
+      if (m > 0 && (threadIdx.x & 31) == __ffs(here) - 1) atomicMax(&tt.last_q[t], m);
+    } else if (lq > 0) {
+      atomicMax(&tt.last_q[t], lq);
+    }
   }
 }
 
@@ -504,8 +585,12 @@ __global__ void k_lin_steps(const uint64_t* r, const int64_t* cnt, const int32_t
 // Block b of tree t (index i of nb) covers the steps of the tree's trimmed range
 // [a, z) (z = one past its last query step: later steps cannot change an answer)
 // whose inclusive work prefix lies in (i W / nb, (i + 1) W / nb].
-__global__ void k_blocks(const int64_t* work, TreeTabs tt, int32_t T, int32_t B, BlockTab* bt, const int32_t* status) {
-  const int32_t b = blockIdx.x * blockDim.x + threadIdx.x;
+// A warp per block: 32 steps are probed at a time, so a cut takes four or five reads in
+// a row (one thread's bisections took twenty).
+__global__ void __launch_bounds__(128) k_blocks(const int64_t* work, TreeTabs tt, int32_t T, int32_t B, BlockTab* bt,
+                                                const int32_t* status) {
+  const int32_t b = blockIdx.x * 4 + (threadIdx.x >> 5);
+  const int lane = threadIdx.x & 31;
   if (b >= B) return;
   const int32_t t = T > 1 ? find_tree(tt.boff, T, b) : 0;
   const int32_t idx = b - tt.boff[t], nb = tt.boff[t + 1] - tt.boff[t];
@@ -529,15 +614,20 @@ __global__ void k_blocks(const int64_t* work, TreeTabs tt, int32_t T, int32_t B,
       const int64_t lim = base + (int64_t)(((__int128)W * i) / nb);
       int64_t lo = a, hi = z;  // first step with work > lim
       while (lo < hi) {
-        const int64_t mid = (lo + hi) >> 1;
-        if (work[mid] <= lim) lo = mid + 1; else hi = mid;
+        const int64_t step = (hi - lo + 31) / 32, pos = lo + lane * step;
+        const unsigned in = __ballot_sync(0xffffffffu, pos < hi && work[pos] <= lim);   // a prefix of the lanes
+        const int n = __popc(in);
+        if (!n) { hi = lo; break; }
+        const int64_t last = lo + (int64_t)(n - 1) * step;   // work[last] <= lim
+        hi = n < 32 && last + step < hi ? last + step : hi;
+        lo = last + 1;
       }
       return lo;
     };
     x.t0 = (int32_t)cut(idx);
     x.t1 = (int32_t)cut(idx + 1);
   }
-  bt[b] = x;
+  if (lane == 0) bt[b] = x;
 }
 
 // ------------------------------------------------------------------ 4. prepare
@@ -2531,7 +2621,7 @@ int pipe_tour(const PipeSpec& s, bool forest, const TourArrays& w, const int32_t
   k_lin_rank_init<<<grid, 256, 0, st>>>(w.cnt, w.ehead, w.xhead, gp, w.fork_head, w.next_sib, nodes, w.rank, status);
   if ((rc = chk("k_lin_rank_init"))) return rc;
   int32_t round = 0;
-  for (int64_t span = 1; span < 2 * (int64_t)s.Smax; span <<= 1, ++round) {
+  for (int64_t span = 1; span < 2 * (int64_t)s.Smax; span *= kLinJumps + 1, ++round) {
     k_lin_round<<<grid, 256, 0, st>>>(w.rank, w.cnt, nodes, w.misc + M_ROUNDS, round, status);
     if ((rc = chk("k_lin_round"))) return rc;
   }
@@ -2617,7 +2707,7 @@ int pipe_enqueue(const PipeSpec& s, void* workspace, const int32_t* parent, cons
   // ---- 3. blocks
   if ((rc = device_inclusive_scan<int64_t>(work, 2 * (int64_t)S, scan_tmp, st, kernels, steps)))
     return report((cudaError_t)rc, "scan");
-  k_blocks<<<(B + 127) / 128, 128, 0, st>>>(work, tt, T, B, blocks, status);
+  k_blocks<<<(B + 3) / 4, 128, 0, st>>>(work, tt, T, B, blocks, status);
   if ((rc = chk("k_blocks"))) return rc;
 
   if ((rc = mark(3))) return rc;
