@@ -22,8 +22,7 @@
 //     the others answer the current tile's: the query records come through a
 //     32-record window that cp.async fills one tile ahead, and land in a
 //     double-buffered shared query buffer.
-// Carry (k_chain_colsum, k_chain_colfix): exclusive column scan over the blocks'
-// final prefix rows in two passes (segment sums, then segment-local prefixes), in
+// Carry (k_chain_carry): exclusive column scan over the blocks' final prefix rows, in
 // place: row b becomes the key prefix of the events of blocks 0 .. b-1.
 // Fix-up (k_chain_fixup): every query of block b >= 1 adds row[hi] - row[lo].
 #include <cuda_runtime.h>
@@ -60,11 +59,10 @@ struct ChainParams {
   int32_t S;
   uint32_t C;
   int32_t B;
-  int32_t nch, nseg;
+  int32_t nch;
   int64_t* rows;          // B rows of C+1 int64: key prefixes (row[k] = sum below key k)
   int64_t* wide;          // B rows of C int64: key histogram of the block's wide tiles
   int64_t* btab;          // B x (first query, end query)
-  int64_t* seg;           // nseg rows of C+1 uint64
   int32_t* status;
 };
 
@@ -640,29 +638,43 @@ __global__ void __launch_bounds__(NT, MINB) k_chain_sweep(ChainParams p) {
   }
 }
 
-// Segment sums of the block prefix rows, column by column (column 0 is always 0).
-__global__ void k_chain_colsum(ChainParams p) {
-  const uint32_t k = blockIdx.y * 256 + threadIdx.x + 1;
-  if (k > p.C) return;
-  const int b0 = blockIdx.x * kChainSegRows, b1 = min(p.B, b0 + kChainSegRows);
-  uint64_t s = 0;
-  for (int b = b0; b < b1; ++b) s += (uint64_t)p.rows[(int64_t)b * (p.C + 1) + k];
-  p.seg[(int64_t)blockIdx.x * (p.C + 1) + k] = (int64_t)s;
-}
-
-// Rows become exclusive column prefixes: row b = the key prefix of the carry of
-// blocks 0 .. b-1.
-__global__ void k_chain_colfix(ChainParams p) {
-  const uint32_t k = blockIdx.y * 256 + threadIdx.x + 1;
+// Rows become exclusive column prefixes: row b = the key prefix of the carry of blocks
+// 0 .. b-1.  A CTA takes 32 columns, a warp of 32 columns one of 32 ranges of the rows:
+// range sums, their prefix through shared memory, then the rows again (from the L2).
+// Bound by memory latency at few rows: 152 rows of 4,097 took 23 us as two kernels that
+// walked 16 rows (and up to nine segment sums) one after the other, 12 us so (both with
+// the fix-up; 608 rows 50 -> 26 us, 456 rows of 1,700 40 -> 21 us).
+__global__ void __launch_bounds__(1024) k_chain_carry(ChainParams p) {
+  __shared__ uint64_t s_sum[32][33];
+  const int x = threadIdx.x & 31, y = threadIdx.x >> 5;
+  const uint32_t k = blockIdx.x * 32 + x + 1;   // column 0 is always 0
+  const int b0 = (int)((int64_t)p.B * y / 32), b1 = (int)((int64_t)p.B * (y + 1) / 32);
+  const int64_t w = (int64_t)p.C + 1;
+  int64_t* col = p.rows + k;
+  constexpr int kBatch = 8;
+  uint64_t sum = 0, v[kBatch];
+  if (k <= p.C)
+    for (int b = b0; b < b1; b += kBatch) {
+#pragma unroll
+      for (int i = 0; i < kBatch; ++i) v[i] = b + i < b1 ? (uint64_t)col[(b + i) * w] : 0;
+#pragma unroll
+      for (int i = 0; i < kBatch; ++i) sum += v[i];
+    }
+  s_sum[y][x] = sum;
+  __syncthreads();
   if (k > p.C) return;
   uint64_t run = 0;
-  for (int s = 0; s < (int)blockIdx.x; ++s) run += (uint64_t)p.seg[(int64_t)s * (p.C + 1) + k];
-  const int b0 = blockIdx.x * kChainSegRows, b1 = min(p.B, b0 + kChainSegRows);
-  for (int b = b0; b < b1; ++b) {
-    int64_t* x = p.rows + (int64_t)b * (p.C + 1) + k;
-    const uint64_t v = (uint64_t)*x;
-    *x = (int64_t)run;
-    run += v;
+  for (int i = 0; i < y; ++i) run += s_sum[i][x];
+  for (int b = b0; b < b1; b += kBatch) {
+    if (b1 - b0 > kBatch) {   // (else the batch is still at hand)
+#pragma unroll
+      for (int i = 0; i < kBatch; ++i) v[i] = b + i < b1 ? (uint64_t)col[(b + i) * w] : 0;
+    }
+#pragma unroll
+    for (int i = 0; i < kBatch; ++i) {
+      if (b + i < b1) col[(b + i) * w] = (int64_t)run;
+      run += v[i];
+    }
   }
 }
 
@@ -684,8 +696,8 @@ __global__ void __launch_bounds__(kChainThreads) k_chain_fixup(ChainParams p) {
 struct Geometry {
   int threads, ept, minb, stages;
 };
-constexpr Geometry kGeometries[] = {{128, 4, 5, 3}, {256, 4, 3, 3}, {512, 2, 2, 3}, {256, 4, 4, 2}, {256, 3, 4, 3}};
-constexpr int kNumGeometries = 5;
+constexpr Geometry kGeometries[] = {{128, 4, 5, 3}, {256, 4, 3, 3}, {512, 2, 2, 3}, {256, 4, 4, 2}, {256, 3, 4, 3}, {384, 2, 3, 3}};
+constexpr int kNumGeometries = 6;
 
 // BW_CHAIN_GEOMETRY=<index into kGeometries> pins the geometry (tuning runs).
 // Otherwise, when the events fill every CTA with full state blocks, 256 threads
@@ -694,9 +706,16 @@ constexpr int kNumGeometries = 5;
 // events and a two-tile ring at three or more, 4 events and a three-tile ring at two
 // or more; else (few, short state blocks) 512 threads x 2 events, whose wide CTAs
 // finish each block soonest, with one block per SM while every block keeps at least
-// 2,048 events.  Tiles always stay large: smaller
+// 512 events.  Tiles always stay large: smaller
 // tiles shorten the in-tile scans but cost more per tile than they save, even on
 // query-dense chains (measured).
+// 384 threads x 2 events take the place of 256 where those get three CTAs on an SM and the
+// window is int64 (16M events, 4,000 keys: sweep 103 -> 94 us with 4,000 queries, 236 -> 201
+// with 320,000) or queries are dense (5M events, 8,000 keys, 400,000 queries: 307 -> 223;
+// with fewer queries 256 threads win, at 6,200 keys 97 to 134).  Where only one CTA of 512
+// fits but two of these do, two of 384 x 2 take its place with the int64 window (16M events,
+// 8,000 keys: 168 -> 123 us and 325 -> 237), two of 256 x 4 else (16,000 keys: 205 -> 141
+// and 409 -> 319).
 int geometry_override() {
   static const int g = [] {
     const char* v = std::getenv("BW_CHAIN_GEOMETRY");
@@ -744,6 +763,10 @@ int chain_spec(const BwReplayArgs* a, int sms, ChainSpec& s) {
   if (pin < 0 && fit[4] >= (s.w64 ? 3 : 4) && s.E >= (int64_t)sms * fit[4] * kChainMinBlockEvents) pin = 4;
   if (pin < 0 && fit[3] >= 3 && s.E >= (int64_t)sms * fit[3] * kChainMinBlockEvents) pin = 3;
   if (pin < 0 && fit[1] >= 2 && s.E >= (int64_t)sms * fit[1] * kChainMinBlockEvents) pin = 1;
+  if ((pin == 4 || pin == 3) && geometry_override() < 0 && fit[pin] == 3 && fit[5] >= 3 && (s.w64 || dense)) pin = 5;
+  const int two = s.w64 ? 5 : 3;
+  const bool pair = pin < 0 && fit[two] >= 2 && s.E >= (int64_t)sms * fit[two] * kChainMinBlockEvents;
+  if (pair) pin = two;
   // too few events to fill the GPU with full blocks: the widest CTA (512 threads)
   // finishes each short block soonest (measured on the 1M-event plain chain)
   const bool few = pin < 0;
@@ -765,22 +788,31 @@ int chain_spec(const BwReplayArgs* a, int sms, ChainSpec& s) {
     }
   }
   if (best < 0) return BW_EINVAL;
-  int64_t B = a->blocks > 0 ? a->blocks : (s.E + kChainMinBlockEvents - 1) / kChainMinBlockEvents;
-  // few events: one block per SM when every block still gets 2,048 events or more
-  if (a->blocks <= 0 && few && B < sms) B = std::min<int64_t>(sms, std::max<int64_t>(B, s.E / 2048));
-  const int64_t cap = (int64_t)sms * s.ctas_per_sm;
-  if (a->blocks <= 0 && B > cap) B = cap;
+  int64_t B = (s.E + kChainMinBlockEvents - 1) / kChainMinBlockEvents;
+  int64_t floor = B;
+  // few events: one block per SM when every block still gets 512 events or more (25,000
+  // events: 12 blocks 25 us a replay, 48 blocks 21 us)
+  if (few && B < sms) {
+    floor = std::min<int64_t>(sms, std::max<int64_t>(B, s.E / 2048));
+    B = std::min<int64_t>(sms, std::max<int64_t>(B, s.E / 512));
+  } else if (pair) {
+    floor = std::min<int64_t>(B, sms);
+  }
+  B = std::min<int64_t>(B, (int64_t)sms * s.ctas_per_sm);
+  // (the blocks that these rules add to `floor` take no more than the 32 MiB that the replay
+  // without allocations has)
+  const int64_t row_bytes = (int64_t)s.C * 16 + 24, small = ((int64_t)32 << 20) - 1024;
+  if (floor * row_bytes <= small) B = std::min(B, std::max(floor, small / row_bytes));
+  if (a->blocks > 0) B = a->blocks;
   if (B > s.E) B = s.E;
   if (B < 1) B = 1;
   if (B > (1 << 20)) return BW_EINVAL;
   s.B = (int32_t)B;
-  s.nseg = (s.B + kChainSegRows - 1) / kChainSegRows;
   auto al = [](size_t x) { return (x + 255) & ~size_t(255); };
   size_t o = 256;   // status word
   s.off_btab = o;  o = al(o + (size_t)s.B * 16);
   s.off_rows = o;  o = al(o + (size_t)s.B * (s.C + 1) * 8);
   s.off_wide = o;  o = al(o + (size_t)s.B * s.C * 8);
-  s.off_seg = o;   o = al(o + (size_t)s.nseg * (s.C + 1) * 8);
   s.total = o;
   return 0;
 }
@@ -792,7 +824,8 @@ int chain_enqueue(const ChainSpec& s, const BwReplayArgs* a, EventSet* evs, int*
                          (const void*)k_chain_sweep<512, 2, 2, 3, false>, (const void*)k_chain_sweep<256, 4, 4, 2, false>,
                          (const void*)k_chain_sweep<256, 3, 4, 3, false>, (const void*)k_chain_sweep<128, 4, 5, 3, true>,
                          (const void*)k_chain_sweep<256, 4, 3, 3, true>, (const void*)k_chain_sweep<512, 2, 2, 3, true>,
-                         (const void*)k_chain_sweep<256, 4, 4, 2, true>, (const void*)k_chain_sweep<256, 3, 4, 3, true>};
+                         (const void*)k_chain_sweep<256, 4, 4, 2, true>, (const void*)k_chain_sweep<256, 3, 4, 3, true>,
+                         (const void*)k_chain_sweep<384, 2, 3, 3, false>, (const void*)k_chain_sweep<384, 2, 3, 3, true>};
     for (const void* f : fns)
       if (g_attr_err == cudaSuccess) g_attr_err = cudaFuncSetAttribute(f, A, kSmemLimit);
   });
@@ -810,11 +843,9 @@ int chain_enqueue(const ChainSpec& s, const BwReplayArgs* a, EventSet* evs, int*
   p.C = s.C;
   p.B = s.B;
   p.nch = s.nch;
-  p.nseg = s.nseg;
   p.rows = reinterpret_cast<int64_t*>(ws + s.off_rows);
   p.wide = reinterpret_cast<int64_t*>(ws + s.off_wide);
   p.btab = reinterpret_cast<int64_t*>(ws + s.off_btab);
-  p.seg = reinterpret_cast<int64_t*>(ws + s.off_seg);
   p.status = reinterpret_cast<int32_t*>(ws);
   int rc = report(cudaMemsetAsync(ws, 0, 4, st), "status reset");
   if (rc) return rc;
@@ -832,17 +863,17 @@ int chain_enqueue(const ChainSpec& s, const BwReplayArgs* a, EventSet* evs, int*
     case 6: k_chain_sweep<256, 4, 4, 2, false><<<s.B, 256, s.smem, st>>>(p); break;
     case 7: k_chain_sweep<256, 4, 4, 2, true><<<s.B, 256, s.smem, st>>>(p); break;
     case 8: k_chain_sweep<256, 3, 4, 3, false><<<s.B, 256, s.smem, st>>>(p); break;
-    default: k_chain_sweep<256, 3, 4, 3, true><<<s.B, 256, s.smem, st>>>(p); break;
+    case 9: k_chain_sweep<256, 3, 4, 3, true><<<s.B, 256, s.smem, st>>>(p); break;
+    case 10: k_chain_sweep<384, 2, 3, 3, false><<<s.B, 384, s.smem, st>>>(p); break;
+    default: k_chain_sweep<384, 2, 3, 3, true><<<s.B, 384, s.smem, st>>>(p); break;
   }
   int k = 1;
   if ((rc = report(cudaGetLastError(), "chain sweep launch"))) return rc;
   if (evs && (rc = report(cudaEventRecord(evs->ev[BW_STAGE_SWEEP + 1], st), "event record"))) return rc;
   if (s.B > 1) {
-    const dim3 g((unsigned)s.nseg, (s.C + 255) / 256);   // columns 1 .. C
-    k_chain_colsum<<<g, 256, 0, st>>>(p);
-    k_chain_colfix<<<g, 256, 0, st>>>(p);
+    k_chain_carry<<<(s.C + 31) / 32, 1024, 0, st>>>(p);   // columns 1 .. C
     k_chain_fixup<<<s.B - 1, kChainThreads, 0, st>>>(p);
-    k += 3;
+    k += 2;
     if ((rc = report(cudaGetLastError(), "chain carry launch"))) return rc;
   }
   if (evs) {

@@ -24,7 +24,6 @@ constexpr int kChainTile = 1024;                                // largest tile,
 constexpr int kChainQBuf = 64;                                  // query records staged per tile
 constexpr uint32_t kChainMaxKeys = 32768;                       // key domain held in shared memory
 constexpr uint32_t kChainMaxKeys64 = 16384;                     // ... with the int64 window
-constexpr int kChainSegRows = 16;                               // block rows per column-scan segment
 constexpr int64_t kChainMinBlockEvents = 8192;
 
 struct ChainSpec {
@@ -33,14 +32,13 @@ struct ChainSpec {
   int64_t E = 0, Q = 0;
   int32_t B = 1;          // state blocks (= sweep CTAs)
   int32_t nch = 1;        // 32-key chunks of the window's chunk totals
-  int32_t nseg = 1;       // column-scan segments
   int32_t ctas_per_sm = 1;
   bool w64 = false;       // int64 window (BW_REPLAY_WIDE)
   int32_t geometry = 2;   // sweep geometry: index, threads per CTA, events per thread
   int32_t threads = 512;
   int32_t ept = 2;
   size_t smem = 0;        // dynamic shared memory of the sweep
-  size_t off_btab = 0, off_rows = 0, off_wide = 0, off_seg = 0, total = 0;   // workspace layout
+  size_t off_btab = 0, off_rows = 0, off_wide = 0, total = 0;   // workspace layout
 };
 
 // Whether a replay takes the chain path: the caller asserts a chain
