@@ -16,6 +16,7 @@
 //   lookup   one thread per 2 point keys / per range, 128-bit loads and stores;
 //            a bucket's keys are searched by bisection over the low bits.
 #include <cuda_runtime.h>
+#include <algorithm>
 #include <cstdint>
 #include <cstdio>
 
@@ -283,36 +284,44 @@ __global__ void k_csr_point(BwCsr x, const uint64_t* __restrict__ keys, int64_t 
   }
 }
 
-// Range lookups in two kernels: the ranks of both bounds into `out`, then their
-// difference and the amounts between them.  LUT, low bits and prefix sums together
-// (164 MB for 10M keys and a 64 MiB LUT) do not stay in the L2; either kernel's share
-// does, and the 3.2 GB of ranks written and read back for 100M ranges cost less than
-// the misses (one kernel: 5.87 ms; two: 1.83 + 1.23 ms).
-template <bool V4>
-__global__ void k_csr_range_ranks(BwCsr x, const uint64_t* __restrict__ bounds, int64_t n, int64_t* __restrict__ out) {
+// Range lookups.  LUT, low bits and prefix sums together (164 MB for 10M keys and a
+// 64 MiB LUT) do not stay in the L2; the LUT with the low bits does, and so do the prefix
+// sums.  So for large indexes each thread first writes the ranks of all its ranges into
+// `out`, then turns them into differences and sums; the grid is resident as a whole, so
+// its CTAs do either at about the same time (100M ranges over 10M keys: 5.7 -> 3.1 ms).
+// Below kSplitKeys the 32 bytes a range that this writes and reads back cost more than the
+// misses (20M ranges, one pass / two, us: 60,000 keys 403 / 436, 1.5M 427 / 483, 3M 513 /
+// 494, 6M 803 / 524).  The LUT's entries are read one by one here: groups of four (above)
+// cost the large index 5% and gain 2% on the smallest.
+constexpr int kRangeCtas = 6;                       // CTAs of 256 threads an SM holds
+constexpr int64_t kSplitKeys = (int64_t)7 << 19;    // 28 MB of prefix sums
+__device__ __forceinline__ longlong2 range_answer(const BwCsr& x, int64_t a, int64_t b) {
+  uint64_t sum = 0;
+  if (a != b) {
+    const uint64_t shi = b ? (uint64_t)__ldg(x.pre + b - 1) : 0;
+    const uint64_t slo = a ? (uint64_t)__ldg(x.pre + a - 1) : 0;
+    sum = shi - slo;
+  }
+  return make_longlong2(b - a, (int64_t)sum);
+}
+__global__ void __launch_bounds__(256, kRangeCtas) k_csr_range(BwCsr x, const uint64_t* __restrict__ bounds, int64_t n,
+                                                              int64_t* out) {
   const int64_t m = *x.count;
+  const bool split = m >= kSplitKeys;
   const ulonglong2* bv = reinterpret_cast<const ulonglong2*>(bounds);
   longlong2* ov = reinterpret_cast<longlong2*>(out);
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+  const int64_t i0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, step = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t i = i0; i < n; i += step) {
     const ulonglong2 q = stream_ld(bv + i);
     bool pr;
-    const int64_t a = csr_rank<V4>(x, m, q.x, pr);
-    const int64_t b = csr_rank<V4>(x, m, q.y, pr);
-    __stcs(ov + i, make_longlong2(a, b));
+    const int64_t a = csr_rank<false>(x, m, q.x, pr);
+    const int64_t b = csr_rank<false>(x, m, q.y, pr);
+    __stcs(ov + i, split ? make_longlong2(a, b) : range_answer(x, a, b));
   }
-}
-__global__ void k_csr_range_sums(BwCsr x, int64_t n, int64_t* out) {
-  longlong2* ov = reinterpret_cast<longlong2*>(out);
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+  if (!split) return;
+  for (int64_t i = i0; i < n; i += step) {
     const longlong2 r = __ldcs(ov + i);
-    const int64_t a = r.x, b = r.y;
-    uint64_t sum = 0;
-    if (a != b) {
-      const uint64_t shi = b ? (uint64_t)__ldg(x.pre + b - 1) : 0;
-      const uint64_t slo = a ? (uint64_t)__ldg(x.pre + a - 1) : 0;
-      sum = shi - slo;
-    }
-    __stcs(ov + i, make_longlong2(b - a, (int64_t)sum));
+    __stcs(ov + i, range_answer(x, r.x, r.y));
   }
 }
 
@@ -401,12 +410,16 @@ int report(cudaError_t e, const char* what) {
   return (int)e;
 }
 
-int grid_for(int64_t items, int threads) {
+int sm_count() {
   int sms = 0, dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
     sms = 148;
+  return sms;
+}
+
+int grid_for(int64_t items, int threads) {
   const int64_t want = (items + threads - 1) / threads;
-  const int64_t cap = (int64_t)sms * 16;
+  const int64_t cap = (int64_t)sm_count() * 16;
   return (int)(want < 1 ? 1 : (want < cap ? want : cap));
 }
 
@@ -494,8 +507,11 @@ extern "C" int bw_csr_build(const uint64_t* keys, const int64_t* amounts, int64_
   return 0;
 }
 
-// Whether the LUT can be read as groups of four entries.
-static bool lut4(const BwCsr* x) { return (reinterpret_cast<uintptr_t>(x->lut) & 15) == 0 && x->n_buckets >= 4; }
+// Whether the LUT is read as groups of four entries: where it can be, and stays in the L2
+// (20M points, 60,000 keys, singly / in fours: 64 MiB LUT 150 / 145 us, 256 MiB 252 / 275).
+static bool lut4(const BwCsr* x) {
+  return (reinterpret_cast<uintptr_t>(x->lut) & 15) == 0 && x->n_buckets >= 4 && x->n_buckets <= ((int64_t)1 << 25);
+}
 
 static int check_index(const BwCsr* x) {
   if (!x || !x->count || !x->status || !x->lut || !x->keys || !x->pre || x->key_bits < 1 || x->key_bits > 63 || x->shift < 0 ||
@@ -518,11 +534,9 @@ extern "C" int bw_csr_range(const BwCsr* idx, const uint64_t* bounds, int64_t n,
   if (n == 0) return 0;
   if ((reinterpret_cast<uintptr_t>(bounds) & 15) || (reinterpret_cast<uintptr_t>(out) & 15)) return BW_EINVAL;
   const cudaStream_t st = static_cast<cudaStream_t>(stream);
-  (lut4(idx) ? k_csr_range_ranks<true> : k_csr_range_ranks<false>)<<<grid_for(n, 256), 256, 0, st>>>(*idx, bounds, n, out);
-  const int rc = report(cudaGetLastError(), "k_csr_range_ranks");
-  if (rc) return rc;
-  k_csr_range_sums<<<grid_for(n, 256), 256, 0, st>>>(*idx, n, out);
-  return report(cudaGetLastError(), "k_csr_range_sums");
+  // no more CTAs than are resident at once
+  k_csr_range<<<std::min(grid_for(n, 256), sm_count() * kRangeCtas), 256, 0, st>>>(*idx, bounds, n, out);
+  return report(cudaGetLastError(), "k_csr_range");
 }
 
 extern "C" int bw_csr_status(const BwCsr* idx, int32_t* status) {
