@@ -659,73 +659,116 @@ struct PrepParams {
 // so steps with few events still fill the warp.  Loop bounds are warp-uniform and f
 // is called by all 32 lanes (valid marks real events), so f may use warp-collective
 // operations.
+//
+// A group of steps with more than kHeavySteps events (states with many events, or
+// contracted steps) is left for the end, when all warps share its events: 300 steps of 150
+// events kept ten of the sixteen warps busy, 60 contracted steps of 1,300 two (both passes:
+// 13.4M events, 90,452 states 1,320 -> 196 us; 18.8M events, 16,744 states 1,530 -> 410).
 constexpr int kPrepBatch = 4;
+constexpr int kHeavySteps = 512;    // (four batches of a warp)
+constexpr int kHeavyList = 96;      // groups left for the end; further ones are done where they occur
 template <typename F>
 __device__ __forceinline__ void for_block_events(const PrepParams& p, int32_t t0, int32_t t1, int mode, F&& f) {
+  __shared__ int32_t s_heavy[kHeavyList], s_nheavy;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-  // this lane's step of the next group, loaded one group ahead
-  StepDesc nd;
+  // (the callers' barriers separate this from an earlier pass's last read)
+  if (threadIdx.x == 0) s_nheavy = 0;
+  __syncthreads();
+  StepDesc nd;       // this lane's step of the next group, loaded one group ahead
   int32_t npt = 0;
   nd.e0 = 0; nd.q0 = 0; nd.ne = 0; nd.nq = 0;
-  if (t0 + 32 * warp + lane < t1) {
-    nd = p.desc[t0 + 32 * warp + lane];
-    npt = p.partner[t0 + 32 * warp + lane];
-  }
-  for (int32_t c = t0 + 32 * warp; c < t1; c += 32 * nw) {
-    const int32_t t = c + lane;
-    const StepDesc d = nd;
-    const int32_t pt = npt;   // the node's other step (exit of an enter, enter of an exit)
-    if (t + 32 * nw < t1) {
-      nd = p.desc[t + 32 * nw];
-      npt = p.partner[t + 32 * nw];
-    }
-    int32_t cnt = 0;
-    uint32_t e0 = 0;
-    bool neg = false, twice = false;
+  auto fetch = [&](int32_t t) {
     if (t < t1) {
-      neg = d.nq < 0;
-      twice = !neg && pt < t1;
+      nd = p.desc[t];
+      npt = p.partner[t];
+    }
+  };
+  int32_t cnt, incl;     // events that this lane's step contributes, and their inclusive sum
+  uint32_t e0, flags;    // first event; 1: an event, 2: negated, 4: twice
+  auto decode = [&](int32_t t, const StepDesc& d, int32_t pt) -> int32_t {   // pt: the node's other step
+    cnt = 0;
+    e0 = 0;
+    flags = 1u;
+    if (t < t1) {
+      const bool neg = d.nq < 0, twice = !neg && pt < t1;
       bool keep = true;
       if (neg) keep = pt < t0;                   // entered in this block: keys known, deltas cancel
       else if (mode == 1 && twice) keep = false; // leaves within this block: net zero
       if (keep) { cnt = d.ne; e0 = d.e0; }
+      flags = 1u | (neg ? 2u : 0u) | (twice ? 4u : 0u);
     }
-    int32_t incl = cnt;
+    incl = cnt;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
       const int32_t y = __shfl_up_sync(0xffffffffu, incl, o);
       if (lane >= o) incl += y;
     }
-    const int32_t total = __shfl_sync(0xffffffffu, incl, 31);
-    // kPrepBatch flattened events a lane at a time: their reads are in flight together
-    // (one at a time left a memory latency per 32 events of a warp)
-    for (int32_t g0 = 0; g0 < total; g0 += 32 * kPrepBatch) {
+    return __shfl_sync(0xffffffffu, incl, 31);
+  };
+  // kPrepBatch flattened events a lane at a time: their reads are in flight together
+  // (one at a time left a memory latency per 32 events of a warp)
+  auto batches = [&](int32_t first, int32_t total, int32_t stride) {
+    for (uint32_t g0 = (uint32_t)first; g0 < (uint32_t)total; g0 += (uint32_t)stride) {
       uint4 e[kPrepBatch];
-      uint32_t fl[kPrepBatch];   // 1: an event, 2: negated, 4: twice
+      uint32_t fl[kPrepBatch];
 #pragma unroll
       for (int u = 0; u < kPrepBatch; ++u) {
-        const int32_t g = g0 + 32 * u + lane;
+        const uint32_t g = g0 + 32 * u + lane;
         int32_t lo = 0, hi = 31;   // first lane whose inclusive count exceeds g
 #pragma unroll
         for (int it = 0; it < 5; ++it) {
           const int32_t mid = (lo + hi) >> 1;
           const int32_t v = __shfl_sync(0xffffffffu, incl, mid);
-          if (v > g) hi = mid; else lo = mid + 1;
+          if ((uint32_t)v > g) hi = mid; else lo = mid + 1;
         }
-        const int32_t off = __shfl_sync(0xffffffffu, incl - cnt, lo);
+        const uint32_t off = (uint32_t)__shfl_sync(0xffffffffu, incl - cnt, lo);
         const uint32_t s_e0 = __shfl_sync(0xffffffffu, e0, lo);
-        fl[u] = __shfl_sync(0xffffffffu, 1u | (neg ? 2u : 0u) | (twice ? 4u : 0u), lo);
+        fl[u] = __shfl_sync(0xffffffffu, flags, lo);
         e[u] = make_uint4(0, 0, 0, 0);
-        if (g < total) e[u] = __ldg(reinterpret_cast<const uint4*>(p.ev) + ((int64_t)s_e0 + (g - off)));
+        if (g < (uint32_t)total) e[u] = __ldg(reinterpret_cast<const uint4*>(p.ev) + ((int64_t)s_e0 + (g - off)));
         else fl[u] = 0;
       }
 #pragma unroll
       for (int u = 0; u < kPrepBatch; ++u) {
-        if (g0 + 32 * u >= total) break;   // warp-uniform
+        if (g0 + 32 * u >= (uint32_t)total) break;   // warp-uniform
         const uint64_t d = ((uint64_t)e[u].w << 32) | e[u].z;
         f(e[u].y, (fl[u] & 2u) ? (uint64_t)0 - d : d, (fl[u] & 1u) != 0, (fl[u] & 4u) != 0);
       }
     }
+  };
+  // (with six groups a warp the warps finish together as it is: 14,000 trees 870 us of
+  // prepare at 1,024 events a group, 820 at 2,048)
+  const int32_t heavy = t1 - t0 >= 192 * nw ? 4 * kHeavySteps : kHeavySteps;
+  fetch(t0 + 32 * warp + lane);
+  for (int32_t c = t0 + 32 * warp; c < t1; c += 32 * nw) {
+    const StepDesc d = nd;
+    const int32_t pt = npt;
+    fetch(c + lane + 32 * nw);
+    const int32_t total = decode(c + lane, d, pt);
+    if (total > heavy) {
+      int32_t i = 0;
+      if (lane == 0) i = atomicAdd(&s_nheavy, 1);
+      i = __shfl_sync(0xffffffffu, i, 0);
+      if (i < kHeavyList) {
+        if (lane == 0) s_heavy[i] = c;
+        continue;
+      }
+    }
+    batches(0, total, 32 * kPrepBatch);
+  }
+  __syncthreads();
+  const int32_t nh = min(s_nheavy, kHeavyList);
+  if (nh) fetch(s_heavy[0] + lane);
+  int32_t turn = warp;   // the groups' batches go round the warps
+  for (int32_t h = 0; h < nh; ++h) {
+    const int32_t c = s_heavy[h];
+    const StepDesc d = nd;
+    const int32_t pt = npt;
+    if (h + 1 < nh) fetch(s_heavy[h + 1] + lane);
+    const int32_t total = decode(c + lane, d, pt);
+    batches(turn * 32 * kPrepBatch, total, nw * 32 * kPrepBatch);
+    const int32_t nb = (total + 32 * kPrepBatch - 1) / (32 * kPrepBatch);
+    turn = (turn + nw - nb % nw) % nw;
   }
 }
 
@@ -882,21 +925,49 @@ __device__ void prepare_block_b(const PrepParams& p, int32_t b, unsigned char* s
       if (w < warp) start += x;
       total += x;
     }
-    for (uint32_t k0 = ka; k0 < kb; k0 += 32) {
-      const uint32_t k = k0 + lane;
-      uint64_t val = 0;
-      if (k < kb) {
-        const uint32_t x = k - klo;
-        if ((sbits[x >> 6] >> (x & 63)) & 1ull) val = hval(local_rank(sbits, srl, x));
-      }
-      uint64_t incl = val;
+    // 128 keys an iteration, as four scans of 32 side by side (one scan after the other
+    // made a row of 262,144 keys take 120 us); int32 histograms are scanned in 32 bits
+    for (uint32_t k0 = ka; k0 < kb; k0 += 128) {
+      uint64_t val[4], incl[4];
 #pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const uint64_t y = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += y;
+      for (int u = 0; u < 4; ++u) {
+        const uint32_t k = k0 + 32 * u + lane;
+        val[u] = 0;
+        if (k < kb) {
+          const uint32_t x = k - klo;
+          const uint64_t w = sbits[x >> 6];
+          if ((w >> (x & 63)) & 1ull) val[u] = hval(srl[x >> 6] + (uint32_t)__popcll(w & ((1ull << (x & 63)) - 1ull)));
+        }
+        incl[u] = val[u];
       }
-      if (k < kb) row[k] = (int64_t)(start + incl - val);
-      start += __shfl_sync(0xffffffffu, incl, 31);
+      if (h32) {
+        int32_t v[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) v[u] = (int32_t)(uint32_t)val[u];
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1)
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            const int32_t y = __shfl_up_sync(0xffffffffu, v[u], o);
+            if (lane >= o) v[u] += y;
+          }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) incl[u] = (uint64_t)(int64_t)v[u];
+      } else {
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1)
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            const uint64_t y = __shfl_up_sync(0xffffffffu, incl[u], o);
+            if (lane >= o) incl[u] += y;
+          }
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const uint32_t k = k0 + 32 * u + lane;
+        if (k < kb) row[k] = (int64_t)(start + incl[u] - val[u]);
+        start += __shfl_sync(0xffffffffu, incl[u], 31);
+      }
     }
     base += total;
     __syncthreads();
@@ -2377,6 +2448,20 @@ int pipe_spec_forest(int32_t T, const int64_t* soff, const int64_t* eoff, const 
   int64_t target = tune.block_work > 0 ? tune.block_work
                                        : std::max<int64_t>(kMinWorkCoarse, Wtot / (4 * (int64_t)s.ctas_per_sm * sms));
   std::vector<int32_t> nb(T);
+  // Where the automatic cut fills the sweep's CTAs once and a second time by less than half,
+  // blocks up to half as large again that fill them once take its place (61 trees: 187
+  // blocks -> 152, sweep 98 -> 73 us)
+  if (tune.block_work <= 0) {
+    auto blocks_at = [&](int64_t w) {
+      int64_t n = 0;
+      for (int32_t t = 0; t < T; ++t) n += std::max<int64_t>(1, (W[t] + w - 1) / w);
+      return n;
+    };
+    const int64_t slots = (int64_t)s.ctas_per_sm * sms, n = blocks_at(target);
+    if (n > slots && n < slots + slots / 2)
+      for (int64_t w = target; w <= target + target / 2; w += target / 16)
+        if (blocks_at(w) <= slots) { target = w; break; }
+  }
   for (;;) {                       // the block work doubles until the carry rows fit
     int64_t carry = 0, blocks = 0;
     for (int32_t t = 0; t < T; ++t) {
