@@ -2,7 +2,8 @@
 //
 // Sweep (k_chain_sweep, one CTA per state block; 128-512 threads, tiles of 512-1024
 // events, a ring of 2-3 tiles, the geometry picked per workload by occupancy):
-//   * the block's events [e0, e1) stream through the ring, each tile one
+//   * the block's events (an equal share, or, where queries are many, such that events and
+//     queries together are an equal share) stream through the ring, each tile one
 //     cp.async.bulk copy from global memory into shared memory completed on the
 //     stage's mbarrier (bounded waits);
 //   * the running key histogram of the block is an exact int32 window H[key] in
@@ -46,6 +47,12 @@ constexpr int kMaxWarps = kChainThreads / 32;
 constexpr int kChunkShift = 5;                   // chunk totals cover 32 keys each
 constexpr uint32_t kFlatKeys = 4096;             // key domains up to this size keep no chunk totals
 constexpr uint32_t kWaitLimit = 1u << 22;        // mbarrier polls before a stage is declared lost
+// A query costs a sweep CTA about what 64 events do.  Where the queries outweigh the events
+// the blocks are cut by both: a reference-native chain (300,000 states, an edit of 1,700 keys
+// every 75th, two queries a state) had its queries in few of its equal event ranges (sweep
+// 499 -> 318 us; 32 events a query 336, 128 315, 256 331), 6,636 states 96 -> 29 us.  Chains
+// with both spread evenly pay the search of the cut, some 3 us; hence not below.
+constexpr int32_t kQueryWeight = 64;
 constexpr uint32_t kFoldAt = 1u << 28;           // window |delta| sum that triggers a fold
 // A tile is int32-safe when every delta lies in (-2^19, 2^19): with at most 1024
 // events its absolute sum is then below 2^29.
@@ -60,6 +67,7 @@ struct ChainParams {
   uint32_t C;
   int32_t B;
   int32_t nch;
+  int32_t qweight;        // events a query counts for in the cut of the blocks (0: events only)
   int64_t* rows;          // B rows of C+1 int64: key prefixes (row[k] = sum below key k)
   int64_t* wide;          // B rows of C int64: key histogram of the block's wide tiles
   int64_t* btab;          // B x (first query, end query)
@@ -233,6 +241,70 @@ __device__ int64_t first_query_at_or_after(const BwQuery* qs, int64_t Q, uint32_
   }
 }
 
+// Events [e[0], e[1]) of block b where a query counts for p.qweight events: the points where
+// the walk through events and queries in state order (an event before the queries of its
+// state) has done b and b + 1 shares of the work.  Found on those diagonals by the whole
+// CTA, one probe of each per thread and round; ascending in b for sorted input, inside
+// [0, E] for any (so every event is in some block even then).
+__device__ void weighted_cut(const ChainParams& p, int64_t b, int64_t (&e)[2]) {
+  const int64_t K = p.qweight, work = p.E + K * p.Q, nt = blockDim.x;
+  int64_t target[2], hi[2];
+  bool done[2];
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    target[i] = work / p.B * (b + i) + work % p.B * (b + i) / p.B;
+    e[i] = max((int64_t)0, target[i] - K * p.Q);
+    hi[i] = min(target[i], p.E);
+    done[i] = false;
+  }
+  while (!done[0] || !done[1]) {
+    bool before[2];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const int64_t pos = e[i] + (int64_t)threadIdx.x * ((hi[i] - e[i] + nt - 1) / nt);
+      before[i] = false;
+      if (pos < hi[i]) {
+        const int64_t q = (target[i] - pos) / K;
+        before[i] = q >= p.Q || p.ev[pos].x <= p.qs[q].state;
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const int cnt = __syncthreads_count(before[i]);
+      const int64_t step = (hi[i] - e[i] + nt - 1) / nt;
+      if (step == 1) {
+        e[i] += cnt;
+        hi[i] = e[i];
+      } else if (step > 1) {
+        const int64_t lo = cnt ? e[i] + (int64_t)(cnt - 1) * step + 1 : e[i];
+        hi[i] = min(hi[i], e[i] + (int64_t)cnt * step);
+        e[i] = lo;
+      }
+      done[i] = hi[i] <= e[i];
+    }
+  }
+}
+
+// First query index in [from, Q) whose state is >= x (Q when none), found by one warp:
+// doubling steps, then 32 probes a round.
+__device__ int64_t next_query_at_or_after(const BwQuery* qs, int64_t Q, int64_t from, uint32_t x, int lane) {
+  int64_t pos = from + ((int64_t)32 << lane);
+  uint32_t lt = __ballot_sync(0xffffffffu, pos < Q && qs[pos].state < x);
+  int k = lt == 0xffffffffu ? 32 : __ffs(~lt) - 1;
+  int64_t lo = k ? from + ((int64_t)32 << (k - 1)) + 1 : from;
+  int64_t hi = k < 32 ? min(Q, from + ((int64_t)32 << k)) : Q;
+  while (hi > lo) {
+    const int64_t step = (hi - lo + 31) / 32;
+    pos = lo + lane * step;
+    k = __popc(__ballot_sync(0xffffffffu, pos < hi && qs[pos].state < x));
+    if (step == 1) return lo + k;
+    const int64_t nlo = k ? lo + (k - 1) * step + 1 : lo;
+    hi = min(hi, lo + k * step);
+    lo = nlo;
+  }
+  return lo;
+}
+
 // The query warp's window of the next 32 query records, copied into shared memory
 // with cp.async one tile before it is read (so the copy's latency stays hidden).
 __device__ __forceinline__ void qpre_issue(uint32_t* qpre, const BwQuery* qs, int64_t Q, int64_t base, int lane) {
@@ -281,6 +353,10 @@ __device__ void find_tile_queries(const ChainParams& p, uint32_t* qpre, int64_t&
     __syncwarp();   // every lane has read the window before it is refilled
     qcur += k;
     if (k < 32) break;
+    if (qcur - tq0 >= QB) {   // no more records are staged: only the end is asked for
+      qcur = next_query_at_or_after(p.qs, p.Q, qcur, x, lane);
+      break;
+    }
   }
   if (lane == 0) {
     tq[0] = tq0;
@@ -407,9 +483,10 @@ __global__ void __launch_bounds__(NT, MINB) k_chain_sweep(ChainParams p) {
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int b = blockIdx.x;
-  const int64_t e0 = (int64_t)b * p.E / p.B, e1 = (int64_t)(b + 1) * p.E / p.B;
-  const int64_t ne = e1 - e0;
-  const int ntiles = (int)((ne + TL - 1) / TL);
+  int64_t cut[2] = {(int64_t)b * p.E / p.B, (int64_t)(b + 1) * p.E / p.B};
+  if (p.qweight) weighted_cut(p, b, cut);
+  const int64_t e0 = cut[0], ne = cut[1] - cut[0];   // (no tile below 1)
+  const int ntiles = ne > 0 ? (int)((ne + TL - 1) / TL) : 0;
   int64_t* P = p.rows + (int64_t)b * (C + 1);
   int64_t* wrow = p.wide + (int64_t)b * C;
   auto tile_n = [&](int t) { return (int)min((int64_t)TL, ne - (int64_t)t * TL); };
@@ -420,7 +497,7 @@ __global__ void __launch_bounds__(NT, MINB) k_chain_sweep(ChainParams p) {
   if (tid == 0) {
     for (int s = 0; s < NS; ++s) mbar_init(&bar[s], 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    m->prev_state[0] = b > 0 ? p.ev[e0 - 1].x : 0u;
+    m->prev_state[0] = e0 > 0 ? p.ev[e0 - 1].x : 0u;
   }
   __syncthreads();
   int issued = 0;   // tiles whose copy was issued (thread 0)
@@ -442,7 +519,7 @@ __global__ void __launch_bounds__(NT, MINB) k_chain_sweep(ChainParams p) {
     if (lo > C || hi > C) set_status(p.status, BW_STATUS_QUERY_RANGE);
   }
   // the block's first query: position >= e0, i.e. state >= state of event e0 - 1
-  const int64_t qstart = b > 0 ? first_query_at_or_after(p.qs, p.Q, m->prev_state[0]) : 0;
+  const int64_t qstart = e0 > 0 ? first_query_at_or_after(p.qs, p.Q, m->prev_state[0]) : 0;
 
   int64_t qcur = qstart, pbase = qstart;
   if (warp == QW) qpre_issue(qpre, p.qs, p.Q, qcur, lane);
@@ -763,7 +840,7 @@ int chain_spec(const BwReplayArgs* a, int sms, ChainSpec& s) {
   if (pin < 0 && fit[4] >= (s.w64 ? 3 : 4) && s.E >= (int64_t)sms * fit[4] * kChainMinBlockEvents) pin = 4;
   if (pin < 0 && fit[3] >= 3 && s.E >= (int64_t)sms * fit[3] * kChainMinBlockEvents) pin = 3;
   if (pin < 0 && fit[1] >= 2 && s.E >= (int64_t)sms * fit[1] * kChainMinBlockEvents) pin = 1;
-  if ((pin == 4 || pin == 3) && geometry_override() < 0 && fit[pin] == 3 && fit[5] >= 3 && (s.w64 || dense)) pin = 5;
+  if ((pin == 4 || pin == 3) && geometry_override() < 0 && fit[pin] == 3 && fit[5] >= 3 && (s.w64 || s.Q * 128 > s.E)) pin = 5;
   const int two = s.w64 ? 5 : 3;
   const bool pair = pin < 0 && fit[two] >= 2 && s.E >= (int64_t)sms * fit[two] * kChainMinBlockEvents;
   if (pair) pin = two;
@@ -843,6 +920,7 @@ int chain_enqueue(const ChainSpec& s, const BwReplayArgs* a, EventSet* evs, int*
   p.C = s.C;
   p.B = s.B;
   p.nch = s.nch;
+  p.qweight = s.Q * kQueryWeight > s.E ? kQueryWeight : 0;
   p.rows = reinterpret_cast<int64_t*>(ws + s.off_rows);
   p.wide = reinterpret_cast<int64_t*>(ws + s.off_wide);
   p.btab = reinterpret_cast<int64_t*>(ws + s.off_btab);

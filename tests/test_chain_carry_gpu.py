@@ -1,5 +1,8 @@
 """GPU parity of the chain path's carry (k_chain_carry) and of its block and geometry rules.
 
+Where queries are many, the blocks are cut by events and queries together: clumped events,
+all events or all queries on one state (blocks without events), queries before the first and
+after the last event, more queries on one state than a tile stages.
 The carry splits the blocks' prefix rows into 32 ranges and holds up to eight rows of a
 range in registers: the block counts lie around both limits, the key domains around the
 32 columns that a CTA takes.  The workloads of the second test get three 384-thread CTAs an
@@ -50,5 +53,29 @@ def test_geometry_rules(bw, torch_cuda, C, E, Q, wide):
     assert r.chain_path(e)
     if C == 8001:
         assert r.workspace.numel() <= 32 << 20
+    _, want = replay(bw, torch_cuda, p, C, e, q, chain=True, path="general")
+    np.testing.assert_array_equal(got, want)
+
+
+@pytest.mark.parametrize("wide", [False, True])
+@pytest.mark.parametrize("blocks", [0, 1, 7, 400])
+@pytest.mark.parametrize("shape", ["clumps", "events on one state", "queries on one state", "queries at the ends"])
+def test_blocks_cut_by_events_and_queries(bw, torch_cuda, shape, blocks, wide):
+    rng = np.random.default_rng(len(shape) + blocks)
+    S, C, E, Q = 5000, 3001, 40_001, 9000
+    parent = evgen.make_tree(S, "chain", rng)
+    ev, qs = evgen.make_events(S, C, E, rng, big=wide), evgen.make_queries(S, C, Q, rng)
+    if shape == "clumps":
+        ev["state"] = np.sort(np.where(rng.random(E) < 0.9, rng.integers(0, 30, E) * 160, rng.integers(0, S, E)))
+    elif shape == "events on one state":
+        ev["state"] = 2500
+    elif shape == "queries on one state":
+        qs["state"] = 2500
+    else:
+        ev["state"] = np.sort(rng.integers(1000, 1200, E))
+        qs["state"] = np.sort(np.where(rng.random(Q) < 0.5, rng.integers(0, 1000, Q), rng.integers(1200, S, Q)))
+    p, e, q = evgen.to_device(torch_cuda, parent, ev, qs)
+    r, got = replay(bw, torch_cuda, p, C, e, q, chain=True, path="chain", blocks=blocks, wide=wide)
+    assert r.chain_path(e)
     _, want = replay(bw, torch_cuda, p, C, e, q, chain=True, path="general")
     np.testing.assert_array_equal(got, want)
