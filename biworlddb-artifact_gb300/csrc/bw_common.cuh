@@ -174,6 +174,9 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_reduce(const T* __restric
   block_exclusive_scan<uint64_t>(s, &total);
   if (threadIdx.x == 0) part[blockIdx.x] = (T)total;
 }
+// Exclusive scan of the tile totals in place, where they are too many for every tile's CTA
+// to sum the totals before its own (kScanSelf).
+constexpr int64_t kScanSelf = 2048;
 template <typename T>
 __global__ void k_scan_parts(T* part, int64_t n, const int32_t* n_dev) {
   // single CTA: exclusive scan of the tile totals in place
@@ -191,14 +194,25 @@ __global__ void k_scan_parts(T* part, int64_t n, const int32_t* n_dev) {
 }
 template <typename T>
 __global__ void __launch_bounds__(kScanThreads) k_scan_apply(T* __restrict__ x, int64_t n,
-                                                             const T* __restrict__ part, const int32_t* n_dev) {
+                                                             const T* __restrict__ part, int self,
+                                                             const int32_t* n_dev) {
   if (n_dev) n = imin64(n, *n_dev);
   if ((int64_t)blockIdx.x * kScanTile >= n) return;
-  __shared__ uint64_t s_warp[kScanThreads / 32];
+  __shared__ uint64_t s_warp[kScanThreads / 32], s_part[kScanThreads / 32];
   using I = ScanItems<T>;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   I it;
   it.load(x, n);
+  uint64_t ahead = 0;   // (self) the totals of the tiles before this one
+  if (self) {
+#pragma unroll
+    for (int j = 0; j < kScanSelf / kScanThreads; ++j) {
+      const int t = j * kScanThreads + threadIdx.x;
+      ahead += t < (int)blockIdx.x ? (uint64_t)part[t] : 0;
+    }
+#pragma unroll
+    for (int o = 16; o; o >>= 1) ahead += __shfl_xor_sync(0xffffffffu, ahead, o);
+  }
   uint64_t before[I::R], run = 0;   // sum of the warp's elements before this lane's vector of round r
 #pragma unroll
   for (int r = 0; r < I::R; ++r) {
@@ -214,9 +228,14 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_apply(T* __restrict__ x, 
     before[r] = run + incl - s;
     run += __shfl_sync(0xffffffffu, incl, 31);
   }
-  if (lane == 0) s_warp[warp] = run;
+  if (lane == 0) {
+    s_warp[warp] = run;
+    s_part[warp] = ahead;
+  }
   __syncthreads();
-  uint64_t base = (uint64_t)part[blockIdx.x];
+  uint64_t base = self ? 0 : (uint64_t)part[blockIdx.x];
+  if (self)
+    for (int w = 0; w < kScanThreads / 32; ++w) base += s_part[w];
   for (int w = 0; w < warp; ++w) base += s_warp[w];
 #pragma unroll
   for (int r = 0; r < I::R; ++r) {
@@ -237,17 +256,18 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_apply(T* __restrict__ x, 
   }
 }
 
-// Inclusive scan of x[0..n) in place (three launches, counted into `kernels`); tmp
-// holds scan_tmp_bytes(n).  n_dev: the count on the device, n its upper bound.
+// Inclusive scan of x[0..n) in place (two launches, three above 8M elements, counted into
+// `kernels`); tmp holds scan_tmp_bytes(n).  n_dev: the count on the device, n its upper bound.
 template <typename T>
 inline int device_inclusive_scan(T* x, int64_t n, void* tmp, cudaStream_t st, int& kernels,
                                  const int32_t* n_dev = nullptr) {
   if (n <= 0) return 0;
   const int64_t np = (n + kScanTile - 1) / kScanTile;
+  const bool self = np <= kScanSelf;
   k_scan_reduce<T><<<(unsigned)np, kScanThreads, 0, st>>>(x, n, static_cast<T*>(tmp), n_dev);
-  k_scan_parts<T><<<1, 1024, 0, st>>>(static_cast<T*>(tmp), n, n_dev);
-  k_scan_apply<T><<<(unsigned)np, kScanThreads, 0, st>>>(x, n, static_cast<const T*>(tmp), n_dev);
-  kernels += 3;
+  if (!self) k_scan_parts<T><<<1, 1024, 0, st>>>(static_cast<T*>(tmp), n, n_dev);
+  k_scan_apply<T><<<(unsigned)np, kScanThreads, 0, st>>>(x, n, static_cast<const T*>(tmp), self ? 1 : 0, n_dev);
+  kernels += self ? 2 : 3;
   return (int)cudaGetLastError();
 }
 inline int device_inclusive_scan_i64(int64_t* x, int64_t n, int64_t* tmp, cudaStream_t st, int& kernels) {

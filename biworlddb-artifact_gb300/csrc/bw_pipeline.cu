@@ -856,6 +856,24 @@ __device__ void prepare_block_a(const PrepParams& p, int32_t b, unsigned char* s
   __syncthreads();
 }
 
+// a[0 .. n] (a[n] = 0) becomes its exclusive prefix; returns a[n], the total.  Each thread
+// takes a run of odd length, so that the warp's accesses fall into distinct banks.
+template <typename T>
+__device__ __forceinline__ T block_prefix_in_place(T* a, uint32_t n) {
+  const uint32_t per = (n / blockDim.x + 1) | 1u, lo = threadIdx.x * per, hi = min(n + 1, lo + per);
+  T sum = 0;
+#pragma unroll 4
+  for (uint32_t i = lo; i < hi; ++i) sum += a[i];
+  T total, run = block_exclusive_scan<T>(sum, &total);
+  for (uint32_t i = lo; i < hi; ++i) {
+    const T v = a[i];
+    a[i] = run;
+    run += v;
+  }
+  __syncthreads();
+  return total;
+}
+
 // Pass B of block b (only blocks that hand a carry on, i.e. all but the last
 // block of each tree): per slice of pass A, the block's net key deltas gathered
 // in a shared histogram over the slice's ranks, written out as the dense
@@ -868,7 +886,6 @@ __device__ void prepare_block_b(const PrepParams& p, int32_t b, unsigned char* s
   // histogram: int32 per rank when the block's nodes are int32 (exact, same
   // bound), int64 otherwise; both fit the same bytes (cap32 ~ 2 * cap64)
   unsigned char* hist_raw = reinterpret_cast<unsigned char*>(srl + p.ww + 2 + (p.ww & 1));  // 8-byte aligned
-  __shared__ uint64_t s_wsum[kPrepThreads / 32];
   const int32_t t0 = bt.t0, t1 = bt.t1;
   const uint64_t* gbits = p.bits + bt.bits_off;
   const uint32_t* grl = p.rlut + bt.bits_off + b;
@@ -878,7 +895,6 @@ __device__ void prepare_block_b(const PrepParams& p, int32_t b, unsigned char* s
   const bool h32 = p.bmode[b] != 0;
   unsigned* hist32 = reinterpret_cast<unsigned*>(hist_raw);
   unsigned long long* hist64 = reinterpret_cast<unsigned long long*>(hist_raw);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
   uint64_t base = 0;  // key prefix at the start of the slice (same in every thread)
   for (int32_t si = 0; si < nsl; ++si) {
     const Slice s = gsl[si];
@@ -903,71 +919,18 @@ __device__ void prepare_block_b(const PrepParams& p, int32_t b, unsigned char* s
       });
     }
     __syncthreads();
-    auto hval = [&](uint32_t r) -> uint64_t {
-      return h32 ? (uint64_t)(int64_t)(int32_t)hist32[r] : (uint64_t)hist64[r];
-    };
-    // each warp writes a contiguous key range; its start value is the sum of the
-    // histogram over the ranks before the range (block scan of warp sums)
+    // the histogram becomes its exclusive prefix over the ranks (int32 stays exact: its
+    // sums are bounded like the nodes), and every key's entry is the prefix at its rank.
+    // Scanning the keys themselves cost a shuffle chain per 32 keys of the domain, touched
+    // or not (61 trees of up to 262,144 keys: this pass 104 -> 50 us; 304 rows of 65,536
+    // keys 69 -> 42).
+    const uint64_t total = h32 ? (uint64_t)(int64_t)(int32_t)block_prefix_in_place(hist32, s.n)
+                               : block_prefix_in_place(hist64, s.n);
     const uint32_t nk = khi - klo;
-    const uint32_t span = ((nk + nw - 1) / nw + 31) & ~31u;
-    const uint32_t ka = klo + imin64((int64_t)warp * span, nk), kb = klo + imin64((int64_t)(warp + 1) * span, nk);
-    const uint32_t ra = ka < khi ? local_rank(sbits, srl, ka - klo) : s.n;
-    const uint32_t rb = kb < khi ? local_rank(sbits, srl, kb - klo) : s.n;
-    uint64_t part = 0;
-    for (uint32_t r = ra + lane; r < rb; r += 32) part += hval(r);
-#pragma unroll
-    for (int o = 16; o; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
-    if (lane == 0) s_wsum[warp] = part;
-    __syncthreads();
-    uint64_t start = base, total = 0;
-    for (int w = 0; w < nw; ++w) {
-      const uint64_t x = s_wsum[w];
-      if (w < warp) start += x;
-      total += x;
-    }
-    // 128 keys an iteration, as four scans of 32 side by side (one scan after the other
-    // made a row of 262,144 keys take 120 us); int32 histograms are scanned in 32 bits
-    for (uint32_t k0 = ka; k0 < kb; k0 += 128) {
-      uint64_t val[4], incl[4];
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const uint32_t k = k0 + 32 * u + lane;
-        val[u] = 0;
-        if (k < kb) {
-          const uint32_t x = k - klo;
-          const uint64_t w = sbits[x >> 6];
-          if ((w >> (x & 63)) & 1ull) val[u] = hval(srl[x >> 6] + (uint32_t)__popcll(w & ((1ull << (x & 63)) - 1ull)));
-        }
-        incl[u] = val[u];
-      }
-      if (h32) {
-        int32_t v[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) v[u] = (int32_t)(uint32_t)val[u];
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1)
-#pragma unroll
-          for (int u = 0; u < 4; ++u) {
-            const int32_t y = __shfl_up_sync(0xffffffffu, v[u], o);
-            if (lane >= o) v[u] += y;
-          }
-#pragma unroll
-        for (int u = 0; u < 4; ++u) incl[u] = (uint64_t)(int64_t)v[u];
-      } else {
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1)
-#pragma unroll
-          for (int u = 0; u < 4; ++u) {
-            const uint64_t y = __shfl_up_sync(0xffffffffu, incl[u], o);
-            if (lane >= o) incl[u] += y;
-          }
-      }
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const uint32_t k = k0 + 32 * u + lane;
-        if (k < kb) row[k] = (int64_t)(start + incl[u] - val[u]);
-        start += __shfl_sync(0xffffffffu, incl[u], 31);
-      }
+#pragma unroll 4
+    for (uint32_t x = threadIdx.x; x < nk; x += kPrepThreads) {
+      const uint32_t r = local_rank(sbits, srl, x);
+      row[klo + x] = (int64_t)(base + (h32 ? (uint64_t)(int64_t)(int32_t)hist32[r] : (uint64_t)hist64[r]));
     }
     base += total;
     __syncthreads();
@@ -2486,7 +2449,7 @@ int pipe_spec_forest(int32_t T, const int64_t* soff, const int64_t* eoff, const 
     const int64_t width = (int64_t)C[t] + 1, rows = nb[t] - 1;
     const int64_t groups = (rows + kCarryGroup - 1) / kCarryGroup;
     const int64_t chunks = (width + kCarryChunk - 1) / kCarryChunk;
-    for (int64_t g = 0; g < groups; ++g)
+    for (int64_t g = 0; rows > 1 && g < groups; ++g)   // (a single row is its own prefix)
       for (int64_t c = 0; c < chunks; ++c) s.h_units.push_back(CarryUnit{t, (int32_t)g, (int32_t)c, 0});
     if (groups > 1) { s.group_pass = true; gsum += groups * width; }
     boff += nb[t];
