@@ -124,6 +124,36 @@ __device__ __forceinline__ void block_exclusive_scan_u64(unsigned long long* a, 
   __syncthreads();
 }
 
+// ------------------------------------------------------------------ chained launches
+// A chain of short kernels, each launched while the one before still runs: a kernel that
+// is launched by launch_chained() calls chain_wait() first, which lets its successor's CTAs
+// come onto the GPU and then waits until everything before it is done and visible.  Only
+// what the kernels of a chain hand on matters here, so that must not be read through the
+// non-coherent path (__ldg, const __restrict__), whose loads may move ahead of the wait.
+// Saves 1.5 to 2 us a launch (building the tours of 46 trees, 24 kernels: 111 -> 67 us).
+// Long kernels (`early` false) are launched the ordinary way: successors that wait for them
+// take places on the SMs unevenly (14,000 trees, 27M states: 1.33 -> 1.46 ms).
+__device__ __forceinline__ void chain_wait() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+constexpr int64_t kChainedStates = (int64_t)1 << 24;   // tours of fewer states are chained (7M: 375 -> 326 us)
+template <typename... P, typename... A>
+inline cudaError_t launch_chained(bool early, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
+                                  A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at = {};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = early ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 // ------------------------------------------------------------------ device scan
 // Kernels below have internal linkage: every translation unit that includes this
 // header gets its own copy.
@@ -145,7 +175,7 @@ struct ScanItems {
     return (int64_t)blockIdx.x * kScanTile + (int64_t)(threadIdx.x >> 5) * (32 * kScanPer) +
            (int64_t)r * (32 * V) + (int64_t)(threadIdx.x & 31) * V;
   }
-  __device__ __forceinline__ void load(const T* __restrict__ x, int64_t n) {
+  __device__ __forceinline__ void load(const T* x, int64_t n) {
 #pragma unroll
     for (int r = 0; r < R; ++r) {
       const int64_t i = at(r);
@@ -159,8 +189,8 @@ struct ScanItems {
   }
 };
 template <typename T>
-__global__ void __launch_bounds__(kScanThreads) k_scan_reduce(const T* __restrict__ x, int64_t n,
-                                                              T* __restrict__ part, const int32_t* n_dev) {
+__global__ void __launch_bounds__(kScanThreads) k_scan_reduce(const T* x, int64_t n, T* part, const int32_t* n_dev) {
+  chain_wait();
   if (n_dev) n = imin64(n, *n_dev);
   if ((int64_t)blockIdx.x * kScanTile >= n) return;
   ScanItems<T> it;
@@ -179,6 +209,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_reduce(const T* __restric
 constexpr int64_t kScanSelf = 2048;
 template <typename T>
 __global__ void k_scan_parts(T* part, int64_t n, const int32_t* n_dev) {
+  chain_wait();
   // single CTA: exclusive scan of the tile totals in place
   if (n_dev) n = imin64(n, *n_dev);
   const int64_t np = (n + kScanTile - 1) / kScanTile;
@@ -193,9 +224,9 @@ __global__ void k_scan_parts(T* part, int64_t n, const int32_t* n_dev) {
   }
 }
 template <typename T>
-__global__ void __launch_bounds__(kScanThreads) k_scan_apply(T* __restrict__ x, int64_t n,
-                                                             const T* __restrict__ part, int self,
+__global__ void __launch_bounds__(kScanThreads) k_scan_apply(T* x, int64_t n, const T* part, int self,
                                                              const int32_t* n_dev) {
+  chain_wait();
   if (n_dev) n = imin64(n, *n_dev);
   if ((int64_t)blockIdx.x * kScanTile >= n) return;
   __shared__ uint64_t s_warp[kScanThreads / 32], s_part[kScanThreads / 32];
@@ -263,12 +294,14 @@ inline int device_inclusive_scan(T* x, int64_t n, void* tmp, cudaStream_t st, in
                                  const int32_t* n_dev = nullptr) {
   if (n <= 0) return 0;
   const int64_t np = (n + kScanTile - 1) / kScanTile;
-  const bool self = np <= kScanSelf;
-  k_scan_reduce<T><<<(unsigned)np, kScanThreads, 0, st>>>(x, n, static_cast<T*>(tmp), n_dev);
-  if (!self) k_scan_parts<T><<<1, 1024, 0, st>>>(static_cast<T*>(tmp), n, n_dev);
-  k_scan_apply<T><<<(unsigned)np, kScanThreads, 0, st>>>(x, n, static_cast<const T*>(tmp), self ? 1 : 0, n_dev);
+  const bool self = np <= kScanSelf, early = n < 2 * kChainedStates;
+  cudaError_t e = launch_chained(early, k_scan_reduce<T>, (unsigned)np, kScanThreads, 0, st, x, n, static_cast<T*>(tmp), n_dev);
+  if (e == cudaSuccess && !self) e = launch_chained(early, k_scan_parts<T>, 1, 1024, 0, st, static_cast<T*>(tmp), n, n_dev);
+  if (e == cudaSuccess)
+    e = launch_chained(early, k_scan_apply<T>, (unsigned)np, kScanThreads, 0, st, x, n, static_cast<const T*>(tmp),
+                       self ? 1 : 0, n_dev);
   kernels += self ? 2 : 3;
-  return (int)cudaGetLastError();
+  return (int)e;
 }
 inline int device_inclusive_scan_i64(int64_t* x, int64_t n, int64_t* tmp, cudaStream_t st, int& kernels) {
   return device_inclusive_scan<int64_t>(x, n, tmp, st, kernels);

@@ -70,6 +70,7 @@ __host__ __device__ __forceinline__ int32_t words_of(uint32_t C) { return (int32
 // table row (from scalars, so no host-to-device copy is needed per launch).
 __global__ void k_init(int32_t* misc, TreeTabs tt, int32_t T, int one_tree, int32_t S, int64_t E, int64_t Q,
                        uint32_t C, int32_t nb) {
+  chain_wait();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < 64) misc[i] = i == M_NODES ? S : i == M_STEPS ? 2 * S : 0;
   for (int t = i; t < T; t += gridDim.x * blockDim.x) tt.last_q[t] = 0;
@@ -87,6 +88,7 @@ __global__ void k_init(int32_t* misc, TreeTabs tt, int32_t T, int one_tree, int3
 }
 
 __global__ void k_fill_i64(int64_t* p, int64_t n, int64_t v) {
+  chain_wait();
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
     p[i] = v;
 }
@@ -149,6 +151,7 @@ __device__ __forceinline__ void offsets_group(int64_t* off, int64_t i, int32_t g
 template <bool kEvents>
 __global__ void __launch_bounds__(256) k_offsets(const void* items, int64_t n, TreeTabs tt, int32_t T, int32_t S,
                                                  int64_t* off, int32_t* status) {
+  chain_wait();
   const int64_t* toff = kEvents ? tt.eoff : tt.qoff;
   const BwEvent* ev = static_cast<const BwEvent*>(items);
   const BwQuery* qs = static_cast<const BwQuery*>(items);
@@ -252,6 +255,7 @@ __global__ void __launch_bounds__(256) k_offsets(const void* items, int64_t n, T
 // (a state's answer only depends on its root path), only the step order.
 __global__ void k_lin_children(const int32_t* parent, int32_t S, TreeTabs tt, int32_t T, int32_t* gpar,
                                int32_t* fork_head, int32_t* next_sib, int chain_only, int32_t* status) {
+  chain_wait();
   int64_t lo, hi;
   warp_range(S, lo, hi);
   int32_t t = T > 1 && lo < hi ? find_tree(tt.soff, T, imin64(lo + (threadIdx.x & 31), S - 1)) : 0;
@@ -286,6 +290,7 @@ __global__ void k_lin_children(const int32_t* parent, int32_t S, TreeTabs tt, in
 // k_ct_mark: parents checked (as k_lin_children does) and forked states marked.
 __global__ void k_ct_mark(const int32_t* parent, int32_t S, TreeTabs tt, int32_t T, int32_t* gpar, uint8_t* forked,
                           int chain_only, int32_t* status) {
+  chain_wait();
   int64_t lo, hi;
   warp_range(S, lo, hi);
   int32_t t = T > 1 && lo < hi ? find_tree(tt.soff, T, imin64(lo + (threadIdx.x & 31), S - 1)) : 0;
@@ -311,6 +316,7 @@ __global__ void k_ct_mark(const int32_t* parent, int32_t S, TreeTabs tt, int32_t
 // ends[v] = 1 where v is the last state of its node (then scanned).
 __global__ void k_ct_ends(const int32_t* gpar, const uint8_t* forked, const int64_t* qoff, int32_t S, uint32_t* ends,
                           const int32_t* status) {
+  chain_wait();
   if (*status) return;
   for (int32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < S; v += gridDim.x * blockDim.x)
     ends[v] = qoff[v + 1] > qoff[v] || forked[v] || !(v + 1 < S && gpar[v + 1] == v) ? 1u : 0u;
@@ -318,6 +324,7 @@ __global__ void k_ct_ends(const int32_t* gpar, const uint8_t* forked, const int6
 __global__ void k_ct_nodes(const int32_t* gpar, const uint32_t* ends, const int64_t* eoff, const int64_t* qoff,
                            int32_t S, TreeTabs tt, int32_t T, int64_t* neoff, int64_t* nqoff, int32_t* npar,
                            int32_t* fork_head, int32_t* misc) {
+  chain_wait();
   if (misc[M_STATUS]) return;
   const int32_t i0 = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
   for (int32_t t = i0; t <= T; t += stride) {
@@ -346,6 +353,7 @@ __global__ void k_ct_nodes(const int32_t* gpar, const uint32_t* ends, const int6
 }
 __global__ void k_ct_children(const int32_t* npar, const int32_t* nodes, int32_t* fork_head, int32_t* next_sib,
                               const int32_t* status) {
+  chain_wait();
   if (*status) return;
   const int32_t n = *nodes;
   for (int32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
@@ -361,6 +369,7 @@ __global__ void k_ct_children(const int32_t* npar, const int32_t* nodes, int32_t
 // flags (enter | exit << 32) for an inclusive scan.
 __global__ void k_lin_flags(const int32_t* gpar, const int32_t* fork_head, const int32_t* nodes, int64_t* cnt,
                             const int32_t* status) {
+  chain_wait();
   if (*status) return;
   const int32_t S = *nodes;
   for (int32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < S; v += gridDim.x * blockDim.x) {
@@ -372,6 +381,7 @@ __global__ void k_lin_flags(const int32_t* gpar, const int32_t* fork_head, const
 }
 
 __global__ void k_lin_heads(const int64_t* cnt, const int32_t* nodes, int32_t* ehead, int32_t* xhead, const int32_t* status) {
+  chain_wait();
   if (*status) return;
   const int32_t S = *nodes;
   for (int32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < S; v += gridDim.x * blockDim.x) {
@@ -394,6 +404,7 @@ __device__ __forceinline__ uint64_t pack_rank(int32_t next, uint32_t dist) {
 __global__ void k_lin_rank_init(const int64_t* cnt, const int32_t* ehead, const int32_t* xhead, const int32_t* gpar,
                                 const int32_t* fork_head, const int32_t* next_sib, const int32_t* nodes, uint64_t* r,
                                 const int32_t* status) {
+  chain_wait();
   if (*status) return;
   const int32_t S = *nodes;
   const uint64_t tot = (uint64_t)cnt[S - 1];
@@ -437,8 +448,9 @@ __global__ void k_lin_rank_init(const int64_t* cnt, const int32_t* ehead, const 
 // Launch r records whether any pointer is still live; one after a launch that found none
 // returns at once.
 constexpr int kLinJumps = 15;
-__global__ void k_lin_round(uint64_t* __restrict__ r, const int64_t* cnt, const int32_t* nodes, int32_t* live,
+__global__ void k_lin_round(uint64_t* r, const int64_t* cnt, const int32_t* nodes, int32_t* live,
                             int32_t round, const int32_t* status) {
+  chain_wait();
   if (*status) return;
   const int32_t S = *nodes;
   if (round > 0 && live[round - 1] == 0) return;
@@ -481,6 +493,7 @@ __device__ __forceinline__ ArcPos arc_pos(const uint64_t* r, uint64_t c, uint64_
 __global__ void k_lin_pos(const uint64_t* r, const int64_t* cnt, const int32_t* ehead, const int32_t* xhead,
                           const int32_t* nodes, TreeTabs tt, int32_t T, const int64_t* qoff, int32_t* tin, int32_t* tout,
                           uint32_t* nq, const int32_t* status) {
+  chain_wait();
   if (*status) return;
   const int32_t S = *nodes;
   const int64_t He = (uint32_t)(uint64_t)cnt[S - 1];
@@ -499,6 +512,7 @@ __global__ void k_lin_pos(const uint64_t* r, const int64_t* cnt, const int32_t* 
 }
 __global__ void k_lin_keep(const int32_t* nodes, const int32_t* tin, const int32_t* tout, const int64_t* qoff,
                            const uint32_t* nq, uint32_t* keep, const int32_t* status) {
+  chain_wait();
   if (*status) return;
   const int32_t S = *nodes;
   for (int32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < S; v += gridDim.x * blockDim.x) {
@@ -509,6 +523,7 @@ __global__ void k_lin_keep(const int32_t* nodes, const int32_t* tin, const int32
   }
 }
 __global__ void k_lin_trees(const uint32_t* keep, TreeTabs tt, int32_t T, int32_t* misc) {
+  chain_wait();
   if (misc[M_STATUS]) return;
   for (int32_t t = blockIdx.x * blockDim.x + threadIdx.x; t <= T; t += gridDim.x * blockDim.x) {
     const int32_t n0 = tt.noff[t];
@@ -525,6 +540,7 @@ __global__ void k_lin_steps(const uint64_t* r, const int64_t* cnt, const int32_t
                             const int32_t* tin, const int32_t* tout, const uint32_t* keep, const int32_t* nodes,
                             TreeTabs tt, int32_t T, const int64_t* eoff, const int64_t* qoff, int32_t* partner,
                             StepDesc* desc, int64_t* work, const int32_t* status) {
+  chain_wait();
   if (*status) return;
   const int32_t S = *nodes;
   const int64_t He = kKept ? 0 : (int64_t)(uint32_t)(uint64_t)cnt[S - 1];
@@ -589,6 +605,7 @@ __global__ void k_lin_steps(const uint64_t* r, const int64_t* cnt, const int32_t
 // a row (one thread's bisections took twenty).
 __global__ void __launch_bounds__(128) k_blocks(const int64_t* work, TreeTabs tt, int32_t T, int32_t B, BlockTab* bt,
                                                 const int32_t* status) {
+  chain_wait();
   const int32_t b = blockIdx.x * 4 + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (b >= B) return;
@@ -943,6 +960,7 @@ __device__ void prepare_block_b(const PrepParams& p, int32_t b, unsigned char* s
 // histogram, so it runs as its own kernel over the blocks that hand a carry on.
 template <int Pass>
 __global__ void __launch_bounds__(kPrepThreads, 2) k_prepare(PrepParams p) {
+  chain_wait();
   if (*p.status) return;  // bounds/descriptors are not trustworthy after an input error
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ int32_t s_ticket;
@@ -981,6 +999,7 @@ __device__ __forceinline__ CarryUnit carry_unit(const CarryParams& p, int32_t u)
 }
 
 __global__ void k_carry_groups(CarryParams p) {
+  chain_wait();
   if (*p.status) return;
   const CarryUnit cu = carry_unit(p, blockIdx.x);
   const int32_t t = cu.tree;
@@ -1001,6 +1020,7 @@ __global__ void k_carry_groups(CarryParams p) {
 }
 
 __global__ void k_carry_apply(CarryParams p) {
+  chain_wait();
   if (*p.status) return;
   const CarryUnit cu = carry_unit(p, blockIdx.x);
   const int32_t t = cu.tree;
@@ -2618,23 +2638,29 @@ int pipe_tour(const PipeSpec& s, bool forest, const TourArrays& w, const int32_t
   const int grid = s.sms * 8;
   int rc = 0;
   int32_t* status = w.misc + M_STATUS;
-  auto chk = [&](const char* what) { ++kernels; return report(cudaGetLastError(), what); };
+  const bool early = S < kChainedStates;
+  cudaError_t e = cudaSuccess;   // of the last launch_chained()
+  auto chk = [&](const char* what) {
+    ++kernels;
+    if (e == cudaSuccess) e = cudaGetLastError();
+    return report(e, what);
+  };
   auto mark = [&](int i) { return timing ? report(cudaEventRecord(timing->ev[i], st), "event record") : 0; };
   // ---- 0/1. init + ingest
   k_init<<<(std::max(T, 16) + 255) / 256, 256, 0, st>>>(w.misc, w.tt, T, forest ? 0 : 1, S, s.E, s.Q, s.Cmax, s.nb1);
   if ((rc = chk("k_init"))) return rc;
   if (s.E > 0) {
-    k_offsets<true><<<grid, 256, 0, st>>>(events, s.E, w.tt, T, S, w.eoff, status);
+    e = launch_chained(early, k_offsets<true>, grid, 256, 0, st, events, s.E, w.tt, T, S, w.eoff, status);
     if ((rc = chk("k_offsets(events)"))) return rc;
   } else {
-    k_fill_i64<<<grid, 256, 0, st>>>(w.eoff, (int64_t)S + 1, 0);
+    e = launch_chained(early, k_fill_i64, grid, 256, 0, st, w.eoff, (int64_t)S + 1, 0);
     if ((rc = chk("k_fill(eoff)"))) return rc;
   }
   if (s.Q > 0) {
-    k_offsets<false><<<grid, 256, 0, st>>>(queries, s.Q, w.tt, T, S, w.qoff, status);
+    e = launch_chained(early, k_offsets<false>, grid, 256, 0, st, queries, s.Q, w.tt, T, S, w.qoff, status);
     if ((rc = chk("k_offsets(queries)"))) return rc;
   } else {
-    k_fill_i64<<<grid, 256, 0, st>>>(w.qoff, (int64_t)S + 1, 0);
+    e = launch_chained(early, k_fill_i64, grid, 256, 0, st, w.qoff, (int64_t)S + 1, 0);
     if ((rc = chk("k_fill(qoff)"))) return rc;
   }
 
@@ -2644,33 +2670,35 @@ int pipe_tour(const PipeSpec& s, bool forest, const TourArrays& w, const int32_t
   const int32_t* nodes = w.misc + M_NODES;
   if (s.contract) {
     if ((rc = report(cudaMemsetAsync(w.forked, 0, (size_t)S, st), "memset"))) return rc;
-    k_ct_mark<<<grid, 256, 0, st>>>(parent, S, w.tt, T, w.gpar, w.forked, s.chain_hint ? 1 : 0, status);
+    e = launch_chained(early, k_ct_mark, grid, 256, 0, st, parent, S, w.tt, T, w.gpar, w.forked, s.chain_hint ? 1 : 0,
+                       status);
     if ((rc = chk("k_ct_mark"))) return rc;
-    k_ct_ends<<<grid, 256, 0, st>>>(gp, w.forked, w.qoff, S, w.ends, status);
+    e = launch_chained(early, k_ct_ends, grid, 256, 0, st, gp, w.forked, w.qoff, S, w.ends, status);
     if ((rc = chk("k_ct_ends"))) return rc;
     if ((rc = device_inclusive_scan<uint32_t>(w.ends, S, w.scan_tmp, st, kernels))) return report((cudaError_t)rc, "scan");
-    k_ct_nodes<<<grid, 256, 0, st>>>(gp, w.ends, w.eoff, w.qoff, S, w.tt, T, w.neoff, w.nqoff, w.npar, w.fork_head,
-                                     w.misc);
+    e = launch_chained(early, k_ct_nodes, grid, 256, 0, st, gp, w.ends, w.eoff, w.qoff, S, w.tt, T, w.neoff, w.nqoff,
+                       w.npar, w.fork_head, w.misc);
     if ((rc = chk("k_ct_nodes"))) return rc;
     gp = w.npar;
-    k_ct_children<<<grid, 256, 0, st>>>(gp, nodes, w.fork_head, w.next_sib, status);
+    e = launch_chained(early, k_ct_children, grid, 256, 0, st, gp, nodes, w.fork_head, w.next_sib, status);
     if ((rc = chk("k_ct_children"))) return rc;
   } else {
     if ((rc = report(cudaMemsetAsync(w.fork_head, 0xFF, (size_t)S * 4, st), "memset"))) return rc;
-    k_lin_children<<<grid, 256, 0, st>>>(parent, S, w.tt, T, w.gpar, w.fork_head, w.next_sib, s.chain_hint ? 1 : 0,
-                                         status);
+    e = launch_chained(early, k_lin_children, grid, 256, 0, st, parent, S, w.tt, T, w.gpar, w.fork_head, w.next_sib,
+                       s.chain_hint ? 1 : 0, status);
     if ((rc = chk("k_lin_children"))) return rc;
   }
-  k_lin_flags<<<grid, 256, 0, st>>>(gp, w.fork_head, nodes, w.cnt, status);
+  e = launch_chained(early, k_lin_flags, grid, 256, 0, st, gp, w.fork_head, nodes, w.cnt, status);
   if ((rc = chk("k_lin_flags"))) return rc;
   if ((rc = device_inclusive_scan<int64_t>(w.cnt, S, w.scan_tmp, st, kernels, nodes))) return report((cudaError_t)rc, "scan");
-  k_lin_heads<<<grid, 256, 0, st>>>(w.cnt, nodes, w.ehead, w.xhead, status);
+  e = launch_chained(early, k_lin_heads, grid, 256, 0, st, w.cnt, nodes, w.ehead, w.xhead, status);
   if ((rc = chk("k_lin_heads"))) return rc;
-  k_lin_rank_init<<<grid, 256, 0, st>>>(w.cnt, w.ehead, w.xhead, gp, w.fork_head, w.next_sib, nodes, w.rank, status);
+  e = launch_chained(early, k_lin_rank_init, grid, 256, 0, st, w.cnt, w.ehead, w.xhead, gp, w.fork_head, w.next_sib,
+                     nodes, w.rank, status);
   if ((rc = chk("k_lin_rank_init"))) return rc;
   int32_t round = 0;
   for (int64_t span = 1; span < 2 * (int64_t)s.Smax; span *= kLinJumps + 1, ++round) {
-    k_lin_round<<<grid, 256, 0, st>>>(w.rank, w.cnt, nodes, w.misc + M_ROUNDS, round, status);
+    e = launch_chained(early, k_lin_round, grid, 256, 0, st, w.rank, w.cnt, nodes, w.misc + M_ROUNDS, round, status);
     if ((rc = chk("k_lin_round"))) return rc;
   }
   return 0;
@@ -2714,7 +2742,13 @@ int pipe_enqueue(const PipeSpec& s, void* workspace, const int32_t* parent, cons
   const int32_t S = s.S, T = s.T, B = s.B;
   const int grid = s.sms * 8;
   int kernels = 0;
-  auto chk = [&](const char* what) { ++kernels; return report(cudaGetLastError(), what); };
+  const bool early = S < kChainedStates;
+  cudaError_t e = cudaSuccess;   // of the last launch_chained()
+  auto chk = [&](const char* what) {
+    ++kernels;
+    if (e == cudaSuccess) e = cudaGetLastError();
+    return report(e, what);
+  };
   auto mark = [&](int i) { return timing ? report(cudaEventRecord(timing->ev[i], st), "event record") : 0; };
   if (timing) timing->chain = 0;
   if ((rc = mark(0))) return rc;
@@ -2733,21 +2767,22 @@ int pipe_enqueue(const PipeSpec& s, void* workspace, const int32_t* parent, cons
     // kept, once the positions are out of it)
     int32_t *tin = reinterpret_cast<int32_t*>(at(W_TIN)), *tout = reinterpret_cast<int32_t*>(at(W_TOUT));
     uint32_t *nq = reinterpret_cast<uint32_t*>(work), *keep = reinterpret_cast<uint32_t*>(rank_a);
-    k_lin_pos<<<grid, 256, 0, st>>>(rank_a, cnt, ehead, xhead, nodes, tt, T, ta.nqoff, tin, tout, nq, status);
+    e = launch_chained(early, k_lin_pos, grid, 256, 0, st, rank_a, cnt, ehead, xhead, nodes, tt, T, ta.nqoff, tin, tout,
+                       nq, status);
     if ((rc = chk("k_lin_pos"))) return rc;
     if ((rc = device_inclusive_scan<uint32_t>(nq, 2 * (int64_t)S, scan_tmp, st, kernels, steps)))
       return report((cudaError_t)rc, "scan");
-    k_lin_keep<<<grid, 256, 0, st>>>(nodes, tin, tout, ta.nqoff, nq, keep, status);
+    e = launch_chained(early, k_lin_keep, grid, 256, 0, st, nodes, tin, tout, ta.nqoff, nq, keep, status);
     if ((rc = chk("k_lin_keep"))) return rc;
     if ((rc = device_inclusive_scan<uint32_t>(keep, 2 * (int64_t)S, scan_tmp, st, kernels, steps)))
       return report((cudaError_t)rc, "scan");
-    k_lin_trees<<<(T + 256) / 256, 256, 0, st>>>(keep, tt, T, misc);
+    e = launch_chained(early, k_lin_trees, (T + 256) / 256, 256, 0, st, keep, tt, T, misc);
     if ((rc = chk("k_lin_trees"))) return rc;
-    k_lin_steps<true><<<grid, 256, 0, st>>>(nullptr, nullptr, nullptr, nullptr, tin, tout, keep, nodes, tt, T, ta.neoff,
-                                            ta.nqoff, partner, desc, work, status);
+    e = launch_chained(early, k_lin_steps<true>, grid, 256, 0, st, nullptr, nullptr, nullptr, nullptr, tin, tout, keep,
+                       nodes, tt, T, ta.neoff, ta.nqoff, partner, desc, work, status);
   } else {
-    k_lin_steps<false><<<grid, 256, 0, st>>>(rank_a, cnt, ehead, xhead, nullptr, nullptr, nullptr, nodes, tt, T, eoff,
-                                             qoff, partner, desc, work, status);
+    e = launch_chained(early, k_lin_steps<false>, grid, 256, 0, st, rank_a, cnt, ehead, xhead, nullptr, nullptr, nullptr,
+                       nodes, tt, T, eoff, qoff, partner, desc, work, status);
   }
   if ((rc = chk("k_lin_steps"))) return rc;
 
@@ -2755,7 +2790,7 @@ int pipe_enqueue(const PipeSpec& s, void* workspace, const int32_t* parent, cons
   // ---- 3. blocks
   if ((rc = device_inclusive_scan<int64_t>(work, 2 * (int64_t)S, scan_tmp, st, kernels, steps)))
     return report((cudaError_t)rc, "scan");
-  k_blocks<<<(B + 3) / 4, 128, 0, st>>>(work, tt, T, B, blocks, status);
+  e = launch_chained(early, k_blocks, (B + 3) / 4, 128, 0, st, work, tt, T, B, blocks, status);
   if ((rc = chk("k_blocks"))) return rc;
 
   if ((rc = mark(3))) return rc;
@@ -2774,11 +2809,11 @@ int pipe_enqueue(const PipeSpec& s, void* workspace, const int32_t* parent, cons
   if ((rc = report(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_a, k_prepare<0>, kPrepThreads, asmem),
                    "occupancy")))
     return rc;
-  k_prepare<0><<<std::min(B, std::max(occ_a, 1) * s.sms), kPrepThreads, asmem, st>>>(pp);
+  e = launch_chained(early, k_prepare<0>, std::min(B, std::max(occ_a, 1) * s.sms), kPrepThreads, asmem, st, pp);
   if ((rc = chk("k_prepare<0>"))) return rc;
   if (s.carry_words > 0) {   // some block hands a carry on
     pp.ticket = misc + M_PREPB_TICKET;
-    k_prepare<1><<<std::min(B, 2 * s.sms), kPrepThreads, psmem, st>>>(pp);
+    e = launch_chained(early, k_prepare<1>, std::min(B, 2 * s.sms), kPrepThreads, psmem, st, pp);
     if ((rc = chk("k_prepare<1>"))) return rc;
   }
 
@@ -2789,10 +2824,10 @@ int pipe_enqueue(const PipeSpec& s, void* workspace, const int32_t* parent, cons
     cp.carry = pp.carry; cp.gsum = reinterpret_cast<int64_t*>(at(W_GSUM)); cp.units = units;
     cp.chunks1 = (int32_t)(((int64_t)s.Cmax + 1 + kCarryChunk - 1) / kCarryChunk); cp.tt = tt; cp.status = status;
     if (s.group_pass) {
-      k_carry_groups<<<s.n_units, kCarryChunk, 0, st>>>(cp);
+      e = launch_chained(early, k_carry_groups, s.n_units, kCarryChunk, 0, st, cp);
       if ((rc = chk("k_carry_groups"))) return rc;
     }
-    k_carry_apply<<<s.n_units, kCarryChunk, 0, st>>>(cp);
+    e = launch_chained(early, k_carry_apply, s.n_units, kCarryChunk, 0, st, cp);
     if ((rc = chk("k_carry_apply"))) return rc;
   }
 

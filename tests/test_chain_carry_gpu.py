@@ -7,7 +7,8 @@ The carry splits the blocks' prefix rows into 32 ranges and holds up to eight ro
 range in registers: the block counts lie around both limits, the key domains around the
 32 columns that a CTA takes.  The workloads of the second test get three 384-thread CTAs an
 SM (dense queries; int64 window), two with fewer blocks, so that the rows stay within 32 MiB,
-and two of 256 threads.
+and two of 256 threads; the last is the first size whose carry
+is launched the ordinary way.
 Whole numbers: every answer is compared exactly, with the general path."""
 from __future__ import annotations
 
@@ -42,7 +43,8 @@ def test_carry_over_block_counts(bw, torch_cuda, blocks, C):
 
 
 @pytest.mark.parametrize("C,E,Q,wide", [(8000, 3_800_001, 90_001, False), (3001, 3_800_001, 400_000, True),
-                                        (8001, 2_600_003, 20_000, True), (16_384, 2_600_003, 20_000, False)])
+                                        (8001, 2_600_003, 20_000, True), (16_384, 2_600_003, 20_000, False),
+                                        (900, 4_194_304, 20_000, False)])
 def test_geometry_rules(bw, torch_cuda, C, E, Q, wide):
     rng = np.random.default_rng(C)
     S = 50_000

@@ -1,8 +1,8 @@
 """GPU parity of the tour building at the sizes where its kernels change.
 
 The inclusive scans sum the totals of earlier tiles in the kernel that applies them up to
-2,048 tiles of 4,096 elements (twice the states), above in a kernel of their own.  Whole
-numbers, compared exactly with the chain path or the oracle."""
+2,048 tiles of 4,096 elements (twice the states), above in a kernel of their own; tours
+below 2^24 states are built by chained launches.  Whole numbers, compared exactly with the chain path or the oracle."""
 from __future__ import annotations
 
 import numpy as np
@@ -21,7 +21,7 @@ def run(bw, torch, p, C, e, q, **kw):
     return out.cpu().numpy()
 
 
-@pytest.mark.parametrize("S", [4 << 20, (4 << 20) + 1])
+@pytest.mark.parametrize("S", [4 << 20, (4 << 20) + 1, (1 << 24) - 1, 1 << 24])
 def test_scan_of_many_tiles(bw, torch_cuda, S):
     rng = np.random.default_rng(S)
     C, E, Q = 300, 50_000, 5000
