@@ -1,7 +1,7 @@
 // bw_chain.cu -- single-pass replay of a linear version chain (see bw_chain.cuh).
 //
 // Sweep (k_chain_sweep, one CTA per state block; 128-512 threads, tiles of 512-1024
-// events, a ring of 2-3 tiles, the geometry picked per workload by occupancy):
+// events, three tiles or two in shared memory, the geometry picked per workload by occupancy):
 //   * the block's events (an equal share, or, where queries are many, such that events and
 //     queries together are an equal share) stream through the ring, each tile one
 //     cp.async.bulk copy from global memory into shared memory completed on the
@@ -80,21 +80,23 @@ struct ChainParams {
 struct Misc {
   uint32_t wsum[2][kMaxWarps];   // per-warp |delta| sum of a tile's window updates
   int64_t tq[2][2];              // queries [tq0, tq1) of a tile
-  uint32_t prev_state[2];        // state of the event before a tile
   int64_t tail_q0;
   unsigned long long scan[kMaxWarps];   // warp totals of the fold's key scan
 };
 
 // Dynamic shared memory of the sweep, every region 16-byte aligned.
 struct SweepSmem {
-  size_t ring, H, T, qbuf, qpre, bar, misc, bytes;
+  size_t ring, kd, st, H, T, qbuf, qpre, bar, misc, bytes;
 };
 __host__ __device__ inline size_t al16(size_t x) { return (x + 15) & ~size_t(15); }
-// hw: bytes of a window entry (4: int32 window, 8: int64 window)
+// hw: bytes of a window entry (4: int32 window, 8: int64 window).  With the int32 window the
+// current tile lies in its compact form, and the ring holds the ns - 1 tiles after it.
 __host__ __device__ inline SweepSmem sweep_smem(uint32_t C, int nch, int te, int ns, int hw) {
   SweepSmem L;
   size_t o = 0;
-  L.ring = o;  o = al16(o + (size_t)ns * te * 16);
+  L.ring = o;  o = al16(o + (size_t)(hw == 4 ? ns - 1 : ns) * te * 16);
+  L.kd = o;    o = al16(o + (hw == 4 ? (size_t)te * 8 : 0));
+  L.st = o;    o = al16(o + (hw == 4 ? (size_t)te * 4 : 0));
   L.H = o;     o = al16(o + (size_t)C * hw);
   L.T = o;     o = al16(o + (size_t)nch * hw);
   L.qbuf = o;  o = al16(o + 2 * (size_t)QB * 16);   // two tiles' query records
@@ -213,11 +215,14 @@ __device__ __forceinline__ uint64_t probe_flat64(const unsigned long long* H, ui
 
 // Position of a query in its tile: the number of the tile's events at or before
 // its state (upper bound over the tile's sorted states).
-__device__ __forceinline__ uint32_t tile_pos(const uint4* tile, int n, uint32_t qst) {
+__device__ __forceinline__ uint32_t state_of(const uint4& e) { return e.x; }
+__device__ __forceinline__ uint32_t state_of(uint32_t s) { return s; }
+template <typename R>
+__device__ __forceinline__ uint32_t tile_pos(const R* tile, int n, uint32_t qst) {
   uint32_t lo = 0, hi = (uint32_t)n;
   while (lo < hi) {
     const uint32_t mid = (lo + hi) >> 1;
-    if (tile[mid].x <= qst) lo = mid + 1; else hi = mid;
+    if (state_of(tile[mid]) <= qst) lo = mid + 1; else hi = mid;
   }
   return lo;
 }
@@ -384,10 +389,11 @@ __device__ __forceinline__ int64_t answer_one64(const ChainParams& p, const unsi
 }
 
 // Answer of one query by one warp, valid in lane 0: the folded key prefix row
-// (P[hi] - P[lo], when it holds data), the window probe, and the tile's first
-// `pos` events inside [lo, hi) (tile == nullptr: none).
+// (P[hi] - P[lo], when it holds data), the window probe, and the tile's first `pos` events
+// inside [lo, hi): from the compact tile, two (key, delta) pairs a lane and read; those of
+// a wide tile, whose deltas do not fit it, from global memory.
 __device__ __forceinline__ int64_t answer_one(const ChainParams& p, const int32_t* H, const int32_t* T,
-                                              const int64_t* P, bool rows_live, bool wide_tile, const uint4* tile,
+                                              const int64_t* P, bool rows_live, const uint2* kd, const uint4* wide_tile,
                                               uint32_t pos, uint32_t lo, uint32_t hi, int lane) {
   lo = min(lo, p.C);
   hi = min(hi, p.C);
@@ -397,18 +403,17 @@ __device__ __forceinline__ int64_t answer_one(const ChainParams& p, const int32_
   if (rows_live && lane < 2) pv = (uint64_t)__ldcg(P + (lane ? hi : lo));   // both ends in flight at once
   int32_t part = p.nch ? probe32(H, T, lo, hi, lane) : probe_flat(H, lo, hi, lane);
   uint64_t wide = 0;
-  if (tile) {
-    if (wide_tile) {
-      for (uint32_t j = lane; j < pos; j += 32) {
-        const uint4 e = tile[j];
-        if (e.y - lo < w) wide += ((uint64_t)e.w << 32) | e.z;
-      }
-    } else {
+  if (wide_tile) {
+    for (uint32_t j = lane; j < pos; j += 32) {
+      const uint4 e = wide_tile[j];
+      if (e.y - lo < w) wide += ((uint64_t)e.w << 32) | e.z;
+    }
+  } else {
 #pragma unroll 4
-      for (uint32_t j = lane; j < pos; j += 32) {
-        const uint4 e = tile[j];
-        if (e.y - lo < w) part += (int32_t)e.z;
-      }
+    for (uint32_t j = 2 * lane; j < pos; j += 64) {
+      const uint4 e = *reinterpret_cast<const uint4*>(kd + j);   // (key, delta) of events j and j + 1
+      if (e.x - lo < w) part += (int32_t)e.y;
+      if (j + 1 < pos && e.z - lo < w) part += (int32_t)e.w;
     }
   }
   uint64_t total = (uint64_t)(int64_t)(int32_t)__reduce_add_sync(0xffffffffu, (uint32_t)part);
@@ -467,6 +472,12 @@ __device__ void fold(const ChainParams& p, HT* H, HT* T, int64_t* P, int64_t* wi
 template <int NT, int EPT, int MINB, int NS, bool W64>
 __global__ void __launch_bounds__(NT, MINB) k_chain_sweep(ChainParams p) {
   constexpr int NW = NT / 32, QW = NW - 1, TL = NT * EPT;
+  // int32 window: every tile is copied into its compact form when its events are loaded,
+  // which frees its place in the ring a tile earlier and halves what a query's scan reads (the
+  // shared-memory pipe and issue bound the sweep: 100M events, 1M queries 893 -> 859 us; 20M
+  // events, 2M queries 922 -> 789)
+  constexpr bool kCompact = !W64;
+  constexpr int RS = kCompact ? NS - 1 : NS;
   chain_wait();
   static_assert(TL <= TE && NW <= kMaxWarps && NW >= 2, "tile geometry");
   extern __shared__ __align__(128) unsigned char sm[];
@@ -474,6 +485,8 @@ __global__ void __launch_bounds__(NT, MINB) k_chain_sweep(ChainParams p) {
   using HT = typename std::conditional<W64, unsigned long long, int32_t>::type;
   const SweepSmem SL = sweep_smem(C, p.nch, TL, NS, (int)sizeof(HT));
   uint4* ring = reinterpret_cast<uint4*>(sm + SL.ring);
+  uint2* kd = reinterpret_cast<uint2*>(sm + SL.kd);          // the tile's (key, delta)
+  uint32_t* kst = reinterpret_cast<uint32_t*>(sm + SL.st);   // ... and states
   HT* H = reinterpret_cast<HT*>(sm + SL.H);
   HT* T = reinterpret_cast<HT*>(sm + SL.T);
   uint32_t* qbuf = reinterpret_cast<uint32_t*>(sm + SL.qbuf);   // [2][QB] uint4, by tile parity
@@ -496,16 +509,15 @@ __global__ void __launch_bounds__(NT, MINB) k_chain_sweep(ChainParams p) {
   for (int i = tid; i < p.nch; i += NT) T[i] = 0;
   if (tid < 2 * kMaxWarps) m->wsum[tid / kMaxWarps][tid % kMaxWarps] = 0;
   if (tid == 0) {
-    for (int s = 0; s < NS; ++s) mbar_init(&bar[s], 1);
+    for (int s = 0; s < RS; ++s) mbar_init(&bar[s], 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    m->prev_state[0] = e0 > 0 ? p.ev[e0 - 1].x : 0u;
   }
   __syncthreads();
   int issued = 0;   // tiles whose copy was issued (thread 0)
   if (tid == 0) {
-    for (; issued < NS && issued < ntiles; ++issued)
-      bulk_load(ring + (issued % NS) * TL, p.ev + e0 + (int64_t)issued * TL, (uint32_t)tile_n(issued) * 16u,
-                &bar[issued % NS]);
+    for (; issued < RS && issued < ntiles; ++issued)
+      bulk_load(ring + (issued % RS) * TL, p.ev + e0 + (int64_t)issued * TL, (uint32_t)tile_n(issued) * 16u,
+                &bar[issued % RS]);
   }
   // input checks spread over every sweep thread: parent[v] = v - 1, and every query
   // (sorted by state, state and bounds in range) -- queries behind an out-of-order
@@ -520,7 +532,8 @@ __global__ void __launch_bounds__(NT, MINB) k_chain_sweep(ChainParams p) {
     if (lo > C || hi > C) set_status(p.status, BW_STATUS_QUERY_RANGE);
   }
   // the block's first query: position >= e0, i.e. state >= state of event e0 - 1
-  const int64_t qstart = e0 > 0 ? first_query_at_or_after(p.qs, p.Q, m->prev_state[0]) : 0;
+  uint32_t last = e0 > 0 ? p.ev[e0 - 1].x : 0u;   // state of the event before the tile to be loaded
+  const int64_t qstart = e0 > 0 ? first_query_at_or_after(p.qs, p.Q, last) : 0;
 
   int64_t qcur = qstart, pbase = qstart;
   if (warp == QW) qpre_issue(qpre, p.qs, p.Q, qcur, lane);
@@ -532,18 +545,36 @@ __global__ void __launch_bounds__(NT, MINB) k_chain_sweep(ChainParams p) {
   uint32_t win = 0;         // |delta| sum in the int32 window (the same in every thread)
   int bigp = 0, lost = 0;
   uint32_t bad = 0;         // event defects seen by this thread (reported at the end)
+  // this thread's events of the tile in ring place `rt`: into registers and the compact
+  // tile, with their order checked (the state before each comes from the previous lane;
+  // lane 0 reads it from the tile, for the first event it is the last tile's)
+  auto load_tile = [&](const uint4* rt, int n) -> int {
+    int wide = 0;
+#pragma unroll
+    for (int k = 0; k < EPT; ++k) {
+      const int idx = tid + k * NT;
+      cur[k] = idx < n ? rt[idx] : make_uint4(0, 0, 0, 0);
+      const uint32_t up = __shfl_up_sync(0xffffffffu, cur[k].x, 1);
+      if (idx < n) {
+        const uint32_t prev = lane ? up : (idx ? rt[idx - 1].x : last);
+        bad |= (cur[k].x < prev ? 1u : 0u) | (cur[k].x >= (uint32_t)p.S ? 2u : 0u);
+        if (kCompact) {
+          kd[idx] = make_uint2(cur[k].y, cur[k].z);
+          kst[idx] = cur[k].x;
+        }
+      }
+      if (!W64) wide |= !small_delta(cur[k]);
+    }
+    last = rt[n - 1].x;
+    return wide;
+  };
   if (ntiles > 0) {
     if (!mbar_wait(&bar[0], 0)) {
       set_status(p.status, BW_STATUS_TIMEOUT);
       lost = 1;
     } else {
       const int n = tile_n(0);
-#pragma unroll
-      for (int k = 0; k < EPT; ++k) {
-        const int idx = tid + k * NT;
-        cur[k] = idx < n ? ring[idx] : make_uint4(0, 0, 0, 0);
-        if (!W64) bigp |= !small_delta(cur[k]);
-      }
+      bigp = load_tile(ring, n);
       if (warp == QW) find_tile_queries(p, qpre, pbase, qcur, ring, n, qbuf_of(0), m->tq[0], lane);
     }
   }
@@ -564,12 +595,12 @@ __global__ void __launch_bounds__(NT, MINB) k_chain_sweep(ChainParams p) {
   int t = 0;
   for (; t < ntiles && !aborted; ++t) {
     const int n = tile_n(t);
-    const uint4* tile = ring + (t % NS) * TL;
-    if (tid == 0 && t >= 1 && issued < ntiles) {
-      // stage (t-1) % NS was released by the barrier that ended tile t-1
+    const uint4* tile = ring + (t % RS) * TL;   // (int64 window)
+    if (tid == 0 && (kCompact || t >= 1) && issued < ntiles) {
+      // the place of tile t (compact) or t - 1 was released by the barrier that ended tile t-1
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-      bulk_load(ring + (issued % NS) * TL, p.ev + e0 + (int64_t)issued * TL, (uint32_t)tile_n(issued) * 16u,
-                &bar[issued % NS]);
+      bulk_load(ring + (issued % RS) * TL, p.ev + e0 + (int64_t)issued * TL, (uint32_t)tile_n(issued) * 16u,
+                &bar[issued % RS]);
       ++issued;
     }
     const int64_t tq0 = m->tq[t & 1][0], tq1 = m->tq[t & 1][1];
@@ -597,8 +628,8 @@ __global__ void __launch_bounds__(NT, MINB) k_chain_sweep(ChainParams p) {
     if (has_q) {
       if (warp == QW) {
         if (t + 1 < ntiles) {
-          const uint4* nt = ring + ((t + 1) % NS) * TL;
-          if (!mbar_wait(&bar[(t + 1) % NS], (uint32_t)(((t + 1) / NS) & 1))) {
+          const uint4* nt = ring + ((t + 1) % RS) * TL;
+          if (!mbar_wait(&bar[(t + 1) % RS], (uint32_t)(((t + 1) / RS) & 1))) {
             set_status(p.status, BW_STATUS_TIMEOUT);
             lost = 1;
           } else {
@@ -619,26 +650,22 @@ __global__ void __launch_bounds__(NT, MINB) k_chain_sweep(ChainParams p) {
           const uint32_t* r = reinterpret_cast<const uint32_t*>(p.qs + i);
           lo = r[1];
           hi = r[2];
-          pos = tile_pos(tile, n, r[0]);
+          pos = kCompact ? tile_pos(kst, n, r[0]) : tile_pos(tile, n, r[0]);
         }
         int64_t a;
         if constexpr (W64) a = answer_one64(p, H, T, tile, pos, lo, hi, lane);
-        else a = answer_one(p, H, T, P, rows_live, big != 0, tile, pos, lo, hi, lane);
+        else a = answer_one(p, H, T, P, rows_live, kd, big ? p.ev + e0 + (int64_t)t * TL : nullptr, pos, lo, hi, lane);
         if (lane == 0) p.ans[i] = a;
       }
       __syncthreads();
     }
-    // apply the tile (the state before each event comes from the previous lane; lane
-    // 0 reads it from the tile, or from the previous tile for the first event)
+    // apply the tile
     uint32_t wsum = 0;
 #pragma unroll
     for (int k = 0; k < EPT; ++k) {
       const int idx = tid + k * NT;
-      const uint32_t up = __shfl_up_sync(0xffffffffu, cur[k].x, 1);
       if (idx < n) {
         const uint4 e = cur[k];
-        const uint32_t prev = lane ? up : (idx ? tile[idx - 1].x : m->prev_state[t & 1]);
-        bad |= (e.x < prev ? 1u : 0u) | (e.x >= (uint32_t)p.S ? 2u : 0u);
         if (e.y >= C) {
           bad |= 4u;
         } else if (W64) {
@@ -660,23 +687,17 @@ __global__ void __launch_bounds__(NT, MINB) k_chain_sweep(ChainParams p) {
       const uint32_t ws = __reduce_add_sync(0xffffffffu, wsum);
       if (lane == 0) m->wsum[t & 1][warp] = ws;
     }
-    if (tid == 0) m->prev_state[(t + 1) & 1] = tile[n - 1].x;
     // next tile: wait for its copy, load this thread's events (and, when no query
     // phase ran, let the query warp find the next tile's queries)
     bigp = 0;
     if (t + 1 < ntiles) {
       const int nn = tile_n(t + 1);
-      const uint4* nt = ring + ((t + 1) % NS) * TL;
-      if (!mbar_wait(&bar[(t + 1) % NS], (uint32_t)(((t + 1) / NS) & 1))) {
+      const uint4* nt = ring + ((t + 1) % RS) * TL;
+      if (!mbar_wait(&bar[(t + 1) % RS], (uint32_t)(((t + 1) / RS) & 1))) {
         set_status(p.status, BW_STATUS_TIMEOUT);
         lost = 1;
       } else {
-#pragma unroll
-        for (int k = 0; k < EPT; ++k) {
-          const int idx = tid + k * NT;
-          cur[k] = idx < nn ? nt[idx] : make_uint4(0, 0, 0, 0);
-          if (!W64) bigp |= !small_delta(cur[k]);
-        }
+        bigp = load_tile(nt, nn);
         if (warp == QW && !next_found)
           find_tile_queries(p, qpre, pbase, qcur, nt, nn, qbuf_of(t + 1), m->tq[(t + 1) & 1], lane);
       }
@@ -693,7 +714,7 @@ __global__ void __launch_bounds__(NT, MINB) k_chain_sweep(ChainParams p) {
     // wait (bounded) for the copies still in flight before the CTA exits: tiles
     // from the one whose wait gave up to the last one issued
     if (tid == 0)
-      for (int u = t; u < issued; ++u) mbar_wait(&bar[u % NS], (uint32_t)((u / NS) & 1));
+      for (int u = t; u < issued; ++u) mbar_wait(&bar[u % RS], (uint32_t)((u / RS) & 1));
     __syncthreads();
     return;
   }
@@ -780,23 +801,28 @@ constexpr Geometry kGeometries[] = {{128, 4, 5, 3}, {256, 4, 3, 3}, {512, 2, 2, 
                                     {256, 4, 4, 2}, {256, 3, 4, 3}, {384, 2, 3, 3}};
 constexpr int kNumGeometries = 6;
 
+// (`stages` counts the tile in work, which the int32 window keeps in its compact form.)
 // BW_CHAIN_GEOMETRY=<index into kGeometries> pins the geometry (tuning runs).
-// Otherwise, when the events fill every CTA with full state blocks, 256 threads
-// with (in this order of preference, measured on byte-dominated chains) 3 events
-// each and a three-tile ring at four CTAs per SM (three with the int64 window), 4
-// events and a two-tile ring at three or more, 4 events and a three-tile ring at two
-// or more; else (few, short state blocks) 512 threads x 2 events, whose wide CTAs
-// finish each block soonest, with one block per SM while every block keeps at least
-// 512 events.  Tiles always stay large: smaller
-// tiles shorten the in-tile scans but cost more per tile than they save, even on
-// query-dense chains (measured).
-// 384 threads x 2 events take the place of 256 where those get three CTAs on an SM and the
-// window is int64 (16M events, 4,000 keys: sweep 103 -> 94 us with 4,000 queries, 236 -> 201
-// with 320,000) or queries are dense (5M events, 8,000 keys, 400,000 queries: 307 -> 223;
-// with fewer queries 256 threads win, at 6,200 keys 97 to 134).  Where only one CTA of 512
-// fits but two of these do, two of 384 x 2 take its place with the int64 window (16M events,
-// 8,000 keys: 168 -> 123 us and 325 -> 237), two of 256 x 4 else (16,000 keys: 205 -> 141
-// and 409 -> 319).
+// Otherwise, when the events fill every CTA with full state blocks, the first that fits of
+//   384 x 2 (threads x events), two CTAs an SM or more: int32 window, dense queries, chunk
+//     totals (8,000 keys, 12 events a query: 554 us against 625 to 800; 16,000 keys 623
+//     against 751 to 851; with 1,000 and 4,096 keys, where 256 x 3 gets four CTAs, it is no
+//     faster: 533 / 509, 540 / 536);
+//   256 x 4, three: int32 window, few queries (4,096 keys, 1,000 events a query: 108 us
+//     against 114; 100 events a query 157 against 159 to 162);
+//   256 x 3, four CTAs (three with the int64 window); 256 x 4 and two stages, three (or 256 x
+//     3 where it gets as many: 131 against 133);
+//   256 x 4, two.
+// 384 x 2 takes the place of the last but one and of 256 x 3 where those get three CTAs
+// and it does too, with the int64 window (4,000 keys: 94 us against 102 to 109) or a query in
+// 256 events and more (8,000 keys, 100 events a query: 180 against 202; 400: 152 against
+// 131).  All 16M events, sweep alone.
+// Where only one CTA of 512 fits but two of these do, two of 384 x 2 take its place with the
+// int64 window (8,000 keys: 168 -> 123 us), two of 256 x 4 else.
+// Else (few, short state blocks) 512 threads x 2 events, whose wide CTAs finish each block
+// soonest, with one block per SM while every block keeps at least 512 events.  Tiles always
+// stay large: smaller tiles shorten the in-tile scans but cost more per tile than they
+// save, even on query-dense chains.
 int geometry_override() {
   static const int g = [] {
     const char* v = std::getenv("BW_CHAIN_GEOMETRY");
@@ -841,14 +867,17 @@ int chain_spec(const BwReplayArgs* a, int sms, ChainSpec& s) {
     if (fit[g] > G.minb) fit[g] = G.minb;
   }
   if (pin >= 0 && fit[pin] < 1) pin = -1;
-  if (pin < 0 && fit[4] >= (s.w64 ? 3 : 4) && s.E >= (int64_t)sms * fit[4] * kChainMinBlockEvents) pin = 4;
-  if (pin < 0 && fit[3] >= 3 && s.E >= (int64_t)sms * fit[3] * kChainMinBlockEvents) pin = 3;
-  if (pin < 0 && fit[1] >= 2 && s.E >= (int64_t)sms * fit[1] * kChainMinBlockEvents) pin = 1;
-  if ((pin == 4 || pin == 3) && geometry_override() < 0 && fit[pin] == 3 && fit[5] >= 3 &&
-      (s.w64 || s.Q * 128 > s.E))
-    pin = 5;
+  const bool pinned = pin >= 0;
+  auto full = [&](int g, int ctas) { return fit[g] >= ctas && s.E >= (int64_t)sms * fit[g] * kChainMinBlockEvents; };
+  if (pin < 0 && !s.w64 && dense && s.C > kFlatKeys && full(5, 2)) pin = 5;
+  if (pin < 0 && !s.w64 && !dense && full(1, 3)) pin = 1;
+  if (pin < 0 && full(4, s.w64 ? 3 : 4)) pin = 4;
+  if (pin < 0 && full(3, 3)) pin = 3;
+  if (pin < 0 && full(1, 2)) pin = 1;
+  if (!pinned && (pin == 4 || pin == 3) && fit[pin] == 3 && fit[5] >= 3 && (s.w64 || s.Q * 256 > s.E)) pin = 5;
+  if (!pinned && pin == 3 && fit[4] >= fit[3]) pin = 4;
   const int two = s.w64 ? 5 : 3;
-  const bool pair = pin < 0 && fit[two] >= 2 && s.E >= (int64_t)sms * fit[two] * kChainMinBlockEvents;
+  const bool pair = pin < 0 && full(two, 2);
   if (pair) pin = two;
   // too few events to fill the GPU with full blocks: the widest CTA (512 threads)
   // finishes each short block soonest (measured on the 1M-event plain chain)
