@@ -96,7 +96,7 @@ using TileSpec512 = TileCfg<1, 1, 64, 512, 512, false, true, true>;   // 15 repl
 // flat window, a producer warp; one CTA per SM) instead of k_sweep.
 enum { kTileAuto = 0, kTileNarrowId = 1, kTileWideId = 2, kTileNarrow512Id = 3, kTileWide512Id = 4, kTileSpec512Id = 5,
        kTileEulerId = 6, kTileQueryId = 7 };
-constexpr int kTileMaxId = 7;
+constexpr int kTileMaxId = kTileEulerId;   // largest that a forest's tuning may name; the next is chosen only
 // Window capacity of the Euler-tile sweep: int32 entries, or int64 ones in the same
 // bytes (the prepare pass cuts its rank slices with the k_sweep window's capacities,
 // 27,904 and 13,824 entries, which both fit).

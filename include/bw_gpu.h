@@ -404,7 +404,7 @@ typedef struct {
                            CTA per SM), 5 the 512-thread tile with one warp staging
                            tiles for the other fifteen, 6 the Euler-tile sweep (a
                            planner and an issuer warp bulk-copy signed event tiles for
-                           sixteen consumer warps over a flat shared-memory window; one
+                           thirty consumer warps over a flat shared-memory window; one
                            CTA per SM); 0 = 6 */
   int32_t reserved;
 } BwForestTuning;

@@ -32,7 +32,7 @@ def test_heavy_groups(bw, torch_cuda, oracle_mod, S, E, C, Q, blocks, hot):
         ev["state"] = np.sort(st)
     want = oracle_mod.ev_sweep(parent, C, ev, qs)
     p, e, q = evgen.to_device(torch_cuda, parent, ev, qs)
-    for tile in (1, 6, 7):
+    for tile in (1, 6):
         f = bw.Forest([0, S], [0, E], [0, Q], [C], tuning=dict(tile=tile, block_work=0 if not blocks else max(1, 2 * E // blocks)))
         out = torch_cuda.empty(Q, dtype=torch_cuda.int64, device=p.device)
         f.launch(p, e, q, out)
