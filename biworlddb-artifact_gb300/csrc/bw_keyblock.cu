@@ -28,8 +28,8 @@
 //   sweep     k_kb_sweep   one CTA per key block: L of every probe (below).
 //   answers   k_kb_answers  acc, kept in tour order, to the queries' own places.
 //
-// Measured on 20M events over 10M keys, 100k states and 100M range queries: 16.5 ms
-// (sweep 6.9, probe scatter 4.2, rows 1.2, probe count 1.1, points 1.3) against 624 ms
+// Measured on 20M events over 10M keys, 100k states and 100M range queries: 15.7 ms
+// (sweep 6.9, probe scatter 3.9, rows 1.2, probe count 1.1, points 1.3) against 624 ms
 // on the state-block pipeline.
 #include <cuda_runtime.h>
 #include <algorithm>
@@ -501,7 +501,12 @@ __global__ void __launch_bounds__(512) k_kb_probe_count(KbParams p) {
 // ahead.  acc becomes the part of the answer in whole key blocks.  Bound by the random
 // sectors of its stores and row reads (4.2 ms for 200M probes; 5.2 ms with stable ranks
 // from __match_any_sync).
+// Four CTAs an SM, by their shared memory: the tiles at work write to a sector in every key
+// block each, and those of eight CTAs an SM do not stay in the L2 until they are full
+// (2,442 key blocks: eight CTAs 12.60 ms for the probes and the sweep, five 12.34, four
+// 12.32, two 12.6).
 constexpr int kPrThreads = 256;
+constexpr size_t kPrSmem = (size_t)56 << 10;
 __global__ void __launch_bounds__(kPrThreads) k_kb_probe_scatter(KbParams p) {
   if (*p.status) return;
   extern __shared__ __align__(16) uint32_t next[];
@@ -741,6 +746,7 @@ int kb_attrs() {
   if (dev >= 0 && dev < 64 && done[dev]) return 0;
   const struct { const void* f; size_t bytes; } need[] = {
       {(const void*)k_kb_point_scatter, kb_scatter_smem(kKbMaxBlocks)},
+      {(const void*)k_kb_probe_scatter, kPrSmem},
       {(const void*)k_kb_sweep, (size_t)kKbMaxSlots * 8}};
   for (const auto& n : need)
     if ((rc = report(cudaFuncSetAttribute(n.f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)n.bytes), "smem attr")))
@@ -857,7 +863,8 @@ int kb_enqueue(const KbSpec& k, const PipeSpec& spec, const BwReplayArgs* a, Eve
   k_kb_probe_count<<<(unsigned)k.pr_tiles, 512, (size_t)k.B * 4, st>>>(p);
   if ((rc = chk("k_kb_probe_count"))) return rc;
   if ((rc = starts(p.prhist, k.pr_tiles, p.proff))) return rc;
-  k_kb_probe_scatter<<<(unsigned)k.pr_tiles, kPrThreads, (size_t)k.B * 4, st>>>(p);
+  static_assert((size_t)kKbMaxBlocks * 4 <= kPrSmem, "probe scatter shared memory");
+  k_kb_probe_scatter<<<(unsigned)k.pr_tiles, kPrThreads, kPrSmem, st>>>(p);
   if ((rc = chk("k_kb_probe_scatter"))) return rc;
   k_kb_sweep<<<std::min(k.B, kSwCtas * s.sms), kSwThreads, (size_t)k.m * 8, st>>>(p);
   if ((rc = chk("k_kb_sweep"))) return rc;
