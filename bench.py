@@ -34,8 +34,9 @@ record as the line (``--scale`` multiplies the sizes).
 * e2e: the same through the public API with pinned host buffers: every step
   copies parent/events/queries host->device and the answers device->host.
 * roofline: the dominant kernel -- the chain sweep (k_chain_sweep) on chains, the
-  Euler-tile tree sweep (k_esweep) on forests, the tree sweep (k_sweep) on single
-  trees -- with its algorithmic bytes (16 per event
+  Euler-tile tree sweep (k_esweep) on forests, the query-step sweep (k_qsweep) or the
+  tree sweep (k_sweep) on single trees, the key-block sweep (k_kb_sweep) on versioned
+  keys -- with its algorithmic bytes (16 per event
   record, 12 per query record, 8 per answer) over its mean launch time (CUDA
   events on the launch stream), against the measured HBM copy bandwidth.
 * cpu_baseline: the oracle's restatement of the reference's CPU path on the box's
@@ -427,7 +428,8 @@ def plain_record(args, bw, dev, name: str, scale: float, steps: int, warmup: int
         e2e = {"value": ws * Q / (ems / 1e3), "unit": "answers/s", "h2d_bytes_per_step": in_bytes,
                "d2h_bytes_per_step": 8 * Q, "ms_per_step": ems}
     peak, peak_kind = measured_peaks()
-    kernel = "k_chain_sweep" if chain_path else "k_sweep"
+    # single trees: the query-step sweep where a state is asked 24 queries and more
+    kernel = "k_chain_sweep" if chain_path else "k_qsweep" if Q >= 24 * S else "k_sweep"
     sweep_bytes = 16 * E + 20 * Q
     sweep_ms = stage_mean["sweep"]
     achieved = sweep_bytes / (sweep_ms / 1e3) / 1e9
@@ -575,11 +577,10 @@ def csr_versioned_record(args, bw, dev, steps: int, scale: float = 1.0) -> dict:
                        "point_lookups": L, "range_lookups": L, "topology": "tree (chain with forks, p=0.9)",
                        "key_universe_bits": w.key_bits, "l2": "inputs larger than L2 (no flush needed)"},
             "phases_ms": {"index_and_rank_mapping": idx_ms, "point_replay": pt_ms, "range_replay": rg_ms},
-            "roofline": {"bound": "hbm", "kernel": "k_sweep", "achieved": sweep_bytes / (pt_ms / 1e3) / 1e9,
+            "roofline": {"bound": "hbm", "kernel": "k_kb_sweep", "achieved": sweep_bytes / (pt_ms / 1e3) / 1e9,
                          "peak": peak, "unit": "GB/s", "frac": sweep_bytes / (pt_ms / 1e3) / 1e9 / peak,
                          "peak_kind": peak_kind, "traffic": None, "algorithmic_bytes_per_launch": sweep_bytes,
-                         "note": "whole point replay over the rank domain; a 10M-key domain takes several rank "
-                                 "slices per block, each sweeping the block's events again"},
+                         "note": "whole point replay over the rank domain, by key blocks"},
             "cpu_baseline": {"value": 200_000 / cpu_s, "unit": "lookups/s", "cores": 1, "kind": "port",
                              "sample": f"preorder replay of all {E} events answering 200,000 sampled lookups "
                                        f"({cpu_s:.1f} s)"},
