@@ -1,15 +1,18 @@
 // bw_sort.cuh -- stable radix partition of 16-byte items, 8 bits a pass, shared by the
 // sparse-key index build and the grouping by state.
 //
-// A pass is three kernels: k_rs_hist counts the digits of every 4,096-item tile
+// A pass is three kernels: k_rs_hist counts the digits of every 2,048-item tile
 // (tile-major, so every access runs along the digits) and adds them to its chunk of
 // tiles; k_rs_start turns the counts into starts (digit totals and earlier chunks are
 // summed by every chunk's CTA, then a prefix down its tiles); k_rs_scatter ranks a tile
 // and writes it digit by digit.  Ranks inside a warp come from eight ballots a round: with
 // 32 distinct digits __match_any_sync took some 400 cycles.  The tile is put in digit order
-// in shared memory first, so that a warp's store covers two or three runs of
-// consecutive addresses instead of 32.
-// Measured on 20M 16-byte pairs: scatter 455 -> 158 us a pass (4.1 TB/s), counts 46 -> 32.
+// in shared memory first, so that a warp's store covers four or five runs of
+// consecutive addresses instead of 32.  Tiles of 256 threads and eight items, four CTAs an
+// SM: longer runs cost more in occupancy than they save (index build of 20M pairs: 4,096 items
+// 1,392 us, 2,048 1,344 to 1,362, 1,536 1,415, 2,560 1,360, 8,192 1,540).
+// Measured on 20M 16-byte pairs, before and after with tiles of 4,096: scatter 455 -> 158 us a
+// pass (4.1 TB/s), counts 46 -> 32; with 2,048 scatter 142.
 #pragma once
 #include <cuda_runtime.h>
 #include <cstdint>
@@ -19,7 +22,7 @@
 namespace bw {
 namespace {
 
-constexpr int kRsThreads = 512, kRsWarps = kRsThreads / 32, kRsItems = 8;
+constexpr int kRsThreads = 256, kRsWarps = kRsThreads / 32, kRsItems = 8;
 constexpr int kRsTile = kRsThreads * kRsItems;
 constexpr int kRsDigits = 256;
 constexpr int kRsChunks = 128;            // chunks of tiles (at most; a multiple of 64)
@@ -89,7 +92,7 @@ __global__ void __launch_bounds__(kRsThreads) k_rs_hist(IO io, int64_t n, int sh
 // hist[tile][d] = those of the chunk's earlier tiles.  Every chunk's CTA sums all chunks,
 // four groups of threads a quarter each (one group took 27 us for 256 chunks), and the
 // groups take a quarter of the chunk's tiles each (one group took 21 us for 38 tiles a chunk,
-// four 9.5).
+// four 9.5, and 12.5 for 76).
 __global__ void __launch_bounds__(4 * kRsDigits) k_rs_start(uint32_t* hist, const uint32_t* part, int64_t tiles,
                                                             int32_t chunks, uint64_t* base) {
   chain_wait();
@@ -148,7 +151,7 @@ __global__ void __launch_bounds__(4 * kRsDigits) k_rs_start(uint32_t* hist, cons
 }
 
 template <typename IO>
-__global__ void __launch_bounds__(kRsThreads, 2) k_rs_scatter(IO io, int64_t n, int shift, int64_t tiles,
+__global__ void __launch_bounds__(kRsThreads, 4) k_rs_scatter(IO io, int64_t n, int shift, int64_t tiles,
                                                               int32_t chunks, const uint32_t* hist,
                                                               const uint64_t* base) {
   chain_wait();

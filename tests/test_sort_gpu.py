@@ -1,5 +1,5 @@
 """The radix partition behind the index build and the grouping, at the edges of its
-tiles (4,096 items), chunks and passes, against numpy."""
+tiles (2,048 items), chunks and passes, against numpy."""
 from __future__ import annotations
 
 import numpy as np
@@ -7,7 +7,7 @@ import pytest
 
 pytestmark = pytest.mark.gpu
 
-SIZES = [1, 31, 4095, 4096, 4097, 3 * 4096 + 1, 300 * 4096 + 77]
+SIZES = [1, 31, 2047, 2048, 2049, 4095, 4096, 4097, 3 * 4096 + 1, 300 * 4096 + 77]
 
 
 @pytest.mark.parametrize("n", SIZES)
