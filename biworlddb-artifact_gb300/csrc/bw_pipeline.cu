@@ -249,6 +249,7 @@ __global__ void __launch_bounds__(256) k_offsets(const void* items, int64_t n, T
 }
 
 // ------------------------------------------------------------------ 2. linearise
+constexpr int kStateBatch = 4;   // states a thread reads at a time
 // Global parents and fork lists.  The continuation child v+1 of v (parent v+1 = v)
 // is always visited first and is not listed; every other child c of p ("fork") is
 // pushed on p's list by atomic exchange.  Child order does not change any answer
@@ -288,38 +289,65 @@ __global__ void k_lin_children(const int32_t* parent, int32_t S, TreeTabs tt, in
 // everything below runs on nodes as it does on states.  On the batched uneven trees (20
 // states a run, 1,000 queries a tree) 19 % as many nodes as states.
 // k_ct_mark: parents checked (as k_lin_children does) and forked states marked.
+// (Four parents in flight a lane: 27.5M states 80 -> 61 us.)
 __global__ void k_ct_mark(const int32_t* parent, int32_t S, TreeTabs tt, int32_t T, int32_t* gpar, uint8_t* forked,
                           int chain_only, int32_t* status) {
   chain_wait();
   int64_t lo, hi;
   warp_range(S, lo, hi);
   int32_t t = T > 1 && lo < hi ? find_tree(tt.soff, T, imin64(lo + (threadIdx.x & 31), S - 1)) : 0;
-  for (int32_t v = (int32_t)lo + (threadIdx.x & 31); v < hi; v += 32) {
-    if (T > 1) t = tree_forward(tt.soff, T, t, v);
-    const int32_t s0 = tt.soff[t], l = v - s0;
-    const int32_t p = parent[v];
-    int32_t gp = -1;
-    if (l == 0) {
-      if (p != -1) set_status(status, BW_STATUS_BAD_PARENT);
-    } else if (p < 0 || p >= l) {
-      set_status(status, BW_STATUS_BAD_PARENT);
-    } else {
-      gp = s0 + p;
-    }
-    if (gpar) gpar[v] = gp;
-    if (l > 0 && gp >= 0 && gp != v - 1) {
-      if (chain_only) set_status(status, BW_STATUS_BAD_PARENT);
-      forked[gp] = 1;
+  for (int32_t v0 = (int32_t)lo + (threadIdx.x & 31); v0 < hi; v0 += 32 * kStateBatch) {
+    int32_t ps[kStateBatch];
+#pragma unroll
+    for (int u = 0; u < kStateBatch; ++u) ps[u] = v0 + 32 * u < hi ? parent[v0 + 32 * u] : 0;
+#pragma unroll
+    for (int u = 0; u < kStateBatch; ++u) {
+      const int32_t v = v0 + 32 * u;
+      if (v >= hi) break;
+      if (T > 1) t = tree_forward(tt.soff, T, t, v);
+      const int32_t s0 = tt.soff[t], l = v - s0;
+      const int32_t p = ps[u];
+      int32_t gp = -1;
+      if (l == 0) {
+        if (p != -1) set_status(status, BW_STATUS_BAD_PARENT);
+      } else if (p < 0 || p >= l) {
+        set_status(status, BW_STATUS_BAD_PARENT);
+      } else {
+        gp = s0 + p;
+      }
+      if (gpar) gpar[v] = gp;
+      if (l > 0 && gp >= 0 && gp != v - 1) {
+        if (chain_only) set_status(status, BW_STATUS_BAD_PARENT);
+        forked[gp] = 1;
+      }
     }
   }
 }
 // ends[v] = 1 where v is the last state of its node (then scanned).
+// Bound by memory latency: a thread has kStateBatch states in flight (a store between them
+// kept the next reads back: 27.5M states, k_ct_ends 140 -> 81 us, k_ct_nodes 200 -> 163).
 __global__ void k_ct_ends(const int32_t* gpar, const uint8_t* forked, const int64_t* qoff, int32_t S, uint32_t* ends,
                           const int32_t* status) {
   chain_wait();
   if (*status) return;
-  for (int32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < S; v += gridDim.x * blockDim.x)
-    ends[v] = qoff[v + 1] > qoff[v] || forked[v] || !(v + 1 < S && gpar[v + 1] == v) ? 1u : 0u;
+  const int32_t stride = gridDim.x * blockDim.x;
+  for (int64_t v0 = blockIdx.x * blockDim.x + threadIdx.x; v0 < S; v0 += (int64_t)kStateBatch * stride) {
+    uint32_t e[kStateBatch];
+#pragma unroll
+    for (int u = 0; u < kStateBatch; ++u) {
+      const int64_t v = v0 + (int64_t)u * stride;
+      e[u] = 0;
+      if (v < S) {
+        const int64_t q0 = qoff[v], q1 = qoff[v + 1];
+        const uint8_t f = forked[v];
+        const int32_t next = v + 1 < S ? gpar[v + 1] : -1;
+        e[u] = (q1 > q0) | (f != 0) | (next != (int32_t)v) ? 1u : 0u;
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < kStateBatch; ++u)
+      if (v0 + (int64_t)u * stride < S) ends[v0 + (int64_t)u * stride] = e[u];
+  }
 }
 __global__ void k_ct_nodes(const int32_t* gpar, const uint32_t* ends, const int64_t* eoff, const int64_t* qoff,
                            int32_t S, TreeTabs tt, int32_t T, int64_t* neoff, int64_t* nqoff, int32_t* npar,
@@ -331,23 +359,46 @@ __global__ void k_ct_nodes(const int32_t* gpar, const uint32_t* ends, const int6
     const int32_t s0 = tt.soff[t];
     tt.noff[t] = s0 ? (int32_t)ends[s0 - 1] : 0;
   }
-  for (int32_t v = i0; v < S; v += stride) {
-    const uint32_t e = ends[v], ep = v ? ends[v - 1] : 0u, epp = v > 1 ? ends[v - 2] : 0u;
-    const bool last = e != ep;
-    const int32_t i = (int32_t)e - (last ? 1 : 0);
-    if (last) {
-      neoff[i + 1] = eoff[v + 1];
-      nqoff[i + 1] = qoff[v + 1];
-      fork_head[i] = -1;
+  for (int64_t v0 = i0; v0 < S; v0 += (int64_t)kStateBatch * stride) {
+    uint32_t e[kStateBatch], ep[kStateBatch], epp[kStateBatch];
+#pragma unroll
+    for (int u = 0; u < kStateBatch; ++u) {
+      const int64_t v = v0 + (int64_t)u * stride;
+      const bool in = v < S;
+      e[u] = in ? ends[v] : 0u;
+      ep[u] = in && v ? ends[v - 1] : 0u;
+      epp[u] = in && v > 1 ? ends[v - 2] : 0u;
     }
-    if (v == 0 || ep != epp) {   // the first state of its node: its parent ends a node
-      const int32_t p = gpar[v];
-      npar[i] = p < 0 ? -1 : (int32_t)ends[p] - 1;
+    int64_t eo[kStateBatch], qo[kStateBatch];
+    int32_t par[kStateBatch];
+#pragma unroll
+    for (int u = 0; u < kStateBatch; ++u) {
+      const int64_t v = v0 + (int64_t)u * stride;
+      const bool last = e[u] != ep[u];
+      eo[u] = v < S && last ? eoff[v + 1] : 0;
+      qo[u] = v < S && last ? qoff[v + 1] : 0;
+      par[u] = v < S && (v == 0 || ep[u] != epp[u]) ? gpar[v] : -1;   // the first state of its node
     }
-    if (v == 0) neoff[0] = nqoff[0] = 0;
-    if (v == S - 1) {
-      misc[M_NODES] = (int32_t)e;
-      misc[M_STEPS] = 2 * (int32_t)e;
+    uint32_t pn[kStateBatch];
+#pragma unroll
+    for (int u = 0; u < kStateBatch; ++u) pn[u] = par[u] < 0 ? 0u : ends[par[u]];   // its parent ends a node
+#pragma unroll
+    for (int u = 0; u < kStateBatch; ++u) {
+      const int64_t v = v0 + (int64_t)u * stride;
+      if (v >= S) break;
+      const bool last = e[u] != ep[u];
+      const int32_t i = (int32_t)e[u] - (last ? 1 : 0);
+      if (last) {
+        neoff[i + 1] = eo[u];
+        nqoff[i + 1] = qo[u];
+        fork_head[i] = -1;
+      }
+      if (v == 0 || ep[u] != epp[u]) npar[i] = (int32_t)pn[u] - 1;
+      if (v == 0) neoff[0] = nqoff[0] = 0;
+      if (v == S - 1) {
+        misc[M_NODES] = (int32_t)e[u];
+        misc[M_STEPS] = 2 * (int32_t)e[u];
+      }
     }
   }
 }

@@ -30,3 +30,17 @@ def test_scan_of_many_tiles(bw, torch_cuda, S):
     p, e, q = evgen.to_device(torch_cuda, parent, ev, qs)
     want = run(bw, torch_cuda, p, C, e, q, chain=True, path="chain")
     np.testing.assert_array_equal(run(bw, torch_cuda, p, C, e, q), want)
+
+
+@pytest.mark.parametrize("kind", ["fork", "chain", "star", "bushy"])
+@pytest.mark.parametrize("S,C,E,Q", [(1, 1, 40, 24), (50, 1, 500, 1200), (300, 70_000, 9000, 8000), (200, 300, 0, 5000),
+                                     (64, 20_000, 50_000, 1537), (3000, 4097, 100_000, 72_001)])
+def test_query_step_sweep(bw, torch_cuda, oracle_mod, S, C, E, Q, kind):
+    """Single trees whose states are asked 24 queries and more take the query-step sweep."""
+    rng = np.random.default_rng(S + C)
+    parent = evgen.make_tree(S, kind, rng)
+    ev, qs = evgen.make_events(S, C, E, rng, zipf=1.2, big=S == 300), evgen.make_queries(S, C, Q, rng)
+    want = oracle_mod.ev_sweep(parent, C, ev, qs)
+    p, e, q = evgen.to_device(torch_cuda, parent, ev, qs)
+    for blocks in (0, 1, 7):
+        np.testing.assert_array_equal(run(bw, torch_cuda, p, C, e, q, blocks=blocks), want)
