@@ -718,7 +718,8 @@ struct PrepParams {
   int32_t* ticket;
 };
 
-// Visit the (key, signed delta) of the block's steps that matter: mode 0 (key
+// Visit the events of the block's steps that matter (f takes the event, whether there is
+// one, whether its delta is taken off and whether it is applied twice): mode 0 (key
 // set) skips exits of nodes entered in the block (their keys come with the
 // enter, flagged by `twice` since the sweep applies them twice); mode 1 (net
 // deltas) also skips enters of nodes that exit in the block, since the two cancel.
@@ -751,34 +752,40 @@ __device__ __forceinline__ void for_block_events(const PrepParams& p, int32_t t0
       npt = p.partner[t];
     }
   };
-  int32_t cnt, incl;     // events that this lane's step contributes, and their inclusive sum
-  uint32_t e0, flags;    // first event; 1: an event, 2: negated, 4: twice
+  int32_t incl;          // inclusive sum of the events that the lanes' steps contribute
+  uint32_t base;         // this lane's first event less the events before it (modulo 2^32)
+  unsigned negated, doubled;   // lanes whose events are taken off; are applied twice
   auto decode = [&](int32_t t, const StepDesc& d, int32_t pt) -> int32_t {   // pt: the node's other step
-    cnt = 0;
-    e0 = 0;
-    flags = 1u;
+    int32_t cnt = 0;
+    uint32_t e0 = 0;
+    bool neg = false, twice = false;
     if (t < t1) {
-      const bool neg = d.nq < 0, twice = !neg && pt < t1;
+      neg = d.nq < 0;
+      twice = !neg && pt < t1;
       bool keep = true;
       if (neg) keep = pt < t0;                   // entered in this block: keys known, deltas cancel
       else if (mode == 1 && twice) keep = false; // leaves within this block: net zero
       if (keep) { cnt = d.ne; e0 = d.e0; }
-      flags = 1u | (neg ? 2u : 0u) | (twice ? 4u : 0u);
     }
+    negated = __ballot_sync(0xffffffffu, neg);
+    doubled = __ballot_sync(0xffffffffu, twice);
     incl = cnt;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
       const int32_t y = __shfl_up_sync(0xffffffffu, incl, o);
       if (lane >= o) incl += y;
     }
+    base = e0 - (uint32_t)(incl - cnt);
     return __shfl_sync(0xffffffffu, incl, 31);
   };
   // kPrepBatch flattened events a lane at a time: their reads are in flight together
-  // (one at a time left a memory latency per 32 events of a warp)
+  // (one at a time left a memory latency per 32 events of a warp).  Bound by issue (61 %): one
+  // word a lane finds an event, the flags are warp masks, sums and signs are in 32 bits where
+  // they fit (14,000 trees: both passes 850 -> 776 us; 40M events, 300,000 states 286 -> 253)
   auto batches = [&](int32_t first, int32_t total, int32_t stride) {
     for (uint32_t g0 = (uint32_t)first; g0 < (uint32_t)total; g0 += (uint32_t)stride) {
       uint4 e[kPrepBatch];
-      uint32_t fl[kPrepBatch];
+      int32_t own[kPrepBatch];   // the lane that owns the event
 #pragma unroll
       for (int u = 0; u < kPrepBatch; ++u) {
         const uint32_t g = g0 + 32 * u + lane;
@@ -789,18 +796,15 @@ __device__ __forceinline__ void for_block_events(const PrepParams& p, int32_t t0
           const int32_t v = __shfl_sync(0xffffffffu, incl, mid);
           if ((uint32_t)v > g) hi = mid; else lo = mid + 1;
         }
-        const uint32_t off = (uint32_t)__shfl_sync(0xffffffffu, incl - cnt, lo);
-        const uint32_t s_e0 = __shfl_sync(0xffffffffu, e0, lo);
-        fl[u] = __shfl_sync(0xffffffffu, flags, lo);
+        own[u] = lo;
+        const uint32_t at = __shfl_sync(0xffffffffu, base, lo) + g;
         e[u] = make_uint4(0, 0, 0, 0);
-        if (g < (uint32_t)total) e[u] = __ldg(reinterpret_cast<const uint4*>(p.ev) + ((int64_t)s_e0 + (g - off)));
-        else fl[u] = 0;
+        if (g < (uint32_t)total) e[u] = __ldg(reinterpret_cast<const uint4*>(p.ev) + at);
       }
 #pragma unroll
       for (int u = 0; u < kPrepBatch; ++u) {
         if (g0 + 32 * u >= (uint32_t)total) break;   // warp-uniform
-        const uint64_t d = ((uint64_t)e[u].w << 32) | e[u].z;
-        f(e[u].y, (fl[u] & 2u) ? (uint64_t)0 - d : d, (fl[u] & 1u) != 0, (fl[u] & 4u) != 0);
+        f(e[u], g0 + 32 * u + lane < (uint32_t)total, ((negated >> own[u]) & 1u) != 0, ((doubled >> own[u]) & 1u) != 0);
       }
     }
   };
@@ -859,7 +863,7 @@ __device__ void prepare_block_a(const PrepParams& p, int32_t b, unsigned char* s
   Slice* gsl = p.slices + (size_t)b * kMaxSlices;
   if (threadIdx.x == 0) s_nsl = 0;
   uint32_t rank_base = 0;
-  uint64_t mass = 0;  // per-thread partial of the block's applied |delta| sum
+  uint32_t mass = 0, over = 0;  // per-thread partial of the block's applied |delta| sum
 
   // ---- pass A: per window, key bitmap -> rank table -> slices
   for (int32_t w0 = 0; w0 < nwords; w0 += p.ww) {
@@ -868,18 +872,21 @@ __device__ void prepare_block_a(const PrepParams& p, int32_t b, unsigned char* s
     __syncthreads();
     const uint32_t klo = (uint32_t)w0 << 6;
     const uint32_t khi = (uint32_t)imin64((int64_t)(w0 + ww) << 6, (int64_t)C);
-    for_block_events(p, t0, t1, 0, [&](uint32_t k, uint64_t v, bool valid, bool twice) {
-      if (valid && k >= klo && k < khi) shared_set_bit(sbits, k - klo);
-      if (valid && w0 == 0) {
-        // |delta| summed over every application the sweep makes (saturating)
-        const uint64_t a = (v >> 63) ? (uint64_t)0 - v : v;
-        const uint64_t m = (a > (1ull << 33) ? (1ull << 33) : a) << (twice ? 1 : 0);
-        mass = mass + m > (1ull << 40) ? (1ull << 40) : mass + m;   // 512 partials stay < 2^49
+    for_block_events(p, t0, t1, 0, [&](const uint4& e, bool valid, bool, bool twice) {
+      if (valid && e.y - klo < khi - klo) shared_set_bit(sbits, e.y - klo);
+      if (w0 == 0) {   // (a missing event's delta is 0)
+        // |delta| summed over every application the sweep makes, in 31 bits; bit 31 of
+        // `over` stays set once a delta or the sum needs more
+        const int32_t lo = (int32_t)e.z;
+        const uint32_t a = e.w == (uint32_t)(lo >> 31) ? (lo < 0 ? 0u - e.z : e.z) : 0x80000000u;
+        const uint32_t m = (a & 0x7fffffffu) << (twice ? 1 : 0), sum = mass + (m & 0x7fffffffu);
+        over |= a | m | sum;
+        mass = sum & 0x7fffffffu;
       }
     });
     if (w0 == 0) {
       uint64_t tot = 0;
-      block_exclusive_scan<uint64_t>(mass, &tot);   // block total
+      block_exclusive_scan<uint64_t>((over >> 31) ? 1ull << 31 : (uint64_t)mass, &tot);   // block total
       if (threadIdx.x == 0) s_mode = tot < (1ull << 31) ? 1 : 0;
     }
     __syncthreads();
@@ -978,11 +985,12 @@ __device__ void prepare_block_b(const PrepParams& p, int32_t b, unsigned char* s
     const uint32_t klo = (uint32_t)s.word_lo << 6;
     const uint32_t khi = (uint32_t)imin64((int64_t)s.word_hi << 6, (int64_t)C);
     if (s.n) {
-      for_block_events(p, t0, t1, 1, [&](uint32_t k, uint64_t d, bool valid, bool) {
-        if (valid && k >= klo && k < khi) {
-          const uint32_t r = local_rank(sbits, srl, k - klo);
-          if (h32) atomicAdd(hist32 + r, (unsigned)d);
-          else shared_add_u64(hist64 + r, d);
+      for_block_events(p, t0, t1, 1, [&](const uint4& e, bool valid, bool neg, bool) {
+        if (valid && e.y - klo < khi - klo) {
+          const uint32_t r = local_rank(sbits, srl, e.y - klo);
+          const uint64_t d = ((uint64_t)e.w << 32) | e.z;
+          if (h32) atomicAdd(hist32 + r, neg ? 0u - e.z : e.z);
+          else shared_add_u64(hist64 + r, neg ? (uint64_t)0 - d : d);
         }
       });
     }

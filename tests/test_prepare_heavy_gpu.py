@@ -42,3 +42,22 @@ def test_heavy_groups(bw, torch_cuda, oracle_mod, S, E, C, Q, blocks, hot):
     r.launch(p, e, q, out)
     assert r.status() == 0
     np.testing.assert_array_equal(out.cpu().numpy(), want)
+
+
+@pytest.mark.parametrize("big", [2**30 - 1, 2**30, 2**31 - 1, 2**31, -2**31, -2**31 - 1, 2**32 - 1, 2**32, 2**62, -2**63])
+def test_delta_sums_around_31_bits(bw, torch_cuda, oracle_mod, big):
+    """A block's sums are held in 32 bits only while its applied |delta| sum stays below 2^31."""
+    rng = np.random.default_rng(abs(big) % 1000)
+    S, C, E, Q = 700, 300, 9000, 300
+    parent = evgen.make_tree(S, "fork", rng)
+    ev, qs = evgen.make_events(S, C, E, rng), evgen.make_queries(S, C, Q, rng)
+    ev["delta"] = 0
+    ev["delta"][[E // 3, E // 2]] = [big, 1]
+    want = oracle_mod.ev_sweep(parent, C, ev, qs)
+    p, e, q = evgen.to_device(torch_cuda, parent, ev, qs)
+    for blocks in (1, 4):
+        r = bw.Replay(p, C, E, Q, blocks=blocks)
+        out = torch_cuda.empty(Q, dtype=torch_cuda.int64, device=p.device)
+        r.launch(p, e, q, out)
+        assert r.status() == 0
+        np.testing.assert_array_equal(out.cpu().numpy(), want)
