@@ -132,7 +132,7 @@ __device__ __forceinline__ void block_exclusive_scan_u64(unsigned long long* a, 
 // non-coherent path (__ldg, const __restrict__), whose loads may move ahead of the wait.
 // Saves 1.5 to 2 us a launch (building the tours of 46 trees, 24 kernels: 111 -> 67 us).
 // Long kernels (`early` false) are launched the ordinary way: successors that wait for them
-// take places on the SMs unevenly (14,000 trees, 27M states: 1.33 -> 1.46 ms).
+// take places on the SMs unevenly (4,096 trees, 27M states: 1.33 -> 1.46 ms).
 __device__ __forceinline__ void chain_wait() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");

@@ -724,8 +724,8 @@ struct PrepParams {
 // enter, flagged by `twice` since the sweep applies them twice); mode 1 (net
 // deltas) also skips enters of nodes that exit in the block, since the two cancel.
 // Each warp takes 32 consecutive steps at a time (lane l decodes step l), flattens
-// their kept events with a warp scan, and lanes take consecutive flattened events,
-// so steps with few events still fill the warp.  Loop bounds are warp-uniform and f
+// their kept events with a warp scan, moves the steps that have some to the first lanes,
+// and lanes take consecutive flattened events, so steps with few events still fill the warp.  Loop bounds are warp-uniform and f
 // is called by all 32 lanes (valid marks real events), so f may use warp-collective
 // operations.
 //
@@ -752,7 +752,7 @@ __device__ __forceinline__ void for_block_events(const PrepParams& p, int32_t t0
       npt = p.partner[t];
     }
   };
-  int32_t incl;          // inclusive sum of the events that the lanes' steps contribute
+  int32_t start;         // events of the steps before this lane's
   uint32_t base;         // this lane's first event less the events before it (modulo 2^32)
   unsigned negated, doubled;   // lanes whose events are taken off; are applied twice
   auto decode = [&](int32_t t, const StepDesc& d, int32_t pt) -> int32_t {   // pt: the node's other step
@@ -769,19 +769,33 @@ __device__ __forceinline__ void for_block_events(const PrepParams& p, int32_t t0
     }
     negated = __ballot_sync(0xffffffffu, neg);
     doubled = __ballot_sync(0xffffffffu, twice);
-    incl = cnt;
+    int32_t incl = cnt;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
       const int32_t y = __shfl_up_sync(0xffffffffu, incl, o);
       if (lane >= o) incl += y;
     }
-    base = e0 - (uint32_t)(incl - cnt);
-    return __shfl_sync(0xffffffffu, incl, 31);
+    // lane j takes over the j-th step that has events
+    const int32_t total = __shfl_sync(0xffffffffu, incl, 31);
+    const unsigned some = __ballot_sync(0xffffffffu, cnt > 0);
+    int32_t src = 0;   // the lane of the j-th set bit
+#pragma unroll
+    for (int step = 16; step; step >>= 1)
+      if (__popc(some & ((1u << (src + step)) - 1u)) <= lane) src += step;
+    const bool have = lane < __popc(some);
+    start = __shfl_sync(0xffffffffu, incl - cnt, src);
+    base = __shfl_sync(0xffffffffu, e0, src) - (uint32_t)start;
+    if (!have) start = 0x7fffffff;
+    negated = __ballot_sync(0xffffffffu, have && ((negated >> src) & 1u));
+    doubled = __ballot_sync(0xffffffffu, have && ((doubled >> src) & 1u));
+    return total;
   };
   // kPrepBatch flattened events a lane at a time: their reads are in flight together
-  // (one at a time left a memory latency per 32 events of a warp).  Bound by issue (61 %): one
-  // word a lane finds an event, the flags are warp masks, sums and signs are in 32 bits where
-  // they fit (14,000 trees: both passes 850 -> 776 us; 40M events, 300,000 states 286 -> 253)
+  // (one at a time left a memory latency per 32 events of a warp).  Bound by issue (61 %): an
+  // event's step is found by counting the starts before it, its place from one word of that
+  // step's lane, the flags are warp masks, sums and signs are in 32 bits where they fit (4,096
+  // trees: both passes 850 -> 741 us, of which the count in place of a bisection by shuffles
+  // 35; 40M events over 300,000 states 286 -> 243)
   auto batches = [&](int32_t first, int32_t total, int32_t stride) {
     for (uint32_t g0 = (uint32_t)first; g0 < (uint32_t)total; g0 += (uint32_t)stride) {
       uint4 e[kPrepBatch];
@@ -789,15 +803,12 @@ __device__ __forceinline__ void for_block_events(const PrepParams& p, int32_t t0
 #pragma unroll
       for (int u = 0; u < kPrepBatch; ++u) {
         const uint32_t g = g0 + 32 * u + lane;
-        int32_t lo = 0, hi = 31;   // first lane whose inclusive count exceeds g
-#pragma unroll
-        for (int it = 0; it < 5; ++it) {
-          const int32_t mid = (lo + hi) >> 1;
-          const int32_t v = __shfl_sync(0xffffffffu, incl, mid);
-          if ((uint32_t)v > g) hi = mid; else lo = mid + 1;
-        }
-        own[u] = lo;
-        const uint32_t at = __shfl_sync(0xffffffffu, base, lo) + g;
+        // the lane whose step the event is of: the starts among these 32 events, and those before
+        const uint32_t rel = (uint32_t)start - (g0 + 32 * u);
+        const unsigned here = __reduce_or_sync(0xffffffffu, rel < 32u ? 1u << rel : 0u);
+        const int32_t before = __popc(__ballot_sync(0xffffffffu, (int32_t)rel < 0));
+        own[u] = before + __popc(here & (0xffffffffu >> (31 - lane))) - 1;
+        const uint32_t at = __shfl_sync(0xffffffffu, base, own[u]) + g;
         e[u] = make_uint4(0, 0, 0, 0);
         if (g < (uint32_t)total) e[u] = __ldg(reinterpret_cast<const uint4*>(p.ev) + at);
       }
@@ -808,7 +819,7 @@ __device__ __forceinline__ void for_block_events(const PrepParams& p, int32_t t0
       }
     }
   };
-  // (with six groups a warp the warps finish together as it is: 14,000 trees 870 us of
+  // (with six groups a warp the warps finish together as it is: 4,096 trees 870 us of
   // prepare at 1,024 events a group, 820 at 2,048)
   const int32_t heavy = t1 - t0 >= 192 * nw ? 4 * kHeavySteps : kHeavySteps;
   fetch(t0 + 32 * warp + lane);
