@@ -35,7 +35,7 @@ record as the line (``--scale`` multiplies the sizes).
   copies parent/events/queries host->device and the answers device->host.
 * roofline: the dominant kernel -- the chain sweep (k_chain_sweep) on chains, the
   Euler-tile tree sweep (k_esweep) on forests, the query-step sweep (k_qsweep) or the
-  tree sweep (k_sweep) on single trees, the key-block sweep (k_kb_sweep) on versioned
+  Euler-tile sweep on single trees, the key-block sweep (k_kb_sweep) on versioned
   keys -- with its algorithmic bytes (16 per event
   record, 12 per query record, 8 per answer) over its mean launch time (CUDA
   events on the launch stream), against the measured HBM copy bandwidth.
@@ -428,8 +428,8 @@ def plain_record(args, bw, dev, name: str, scale: float, steps: int, warmup: int
         e2e = {"value": ws * Q / (ems / 1e3), "unit": "answers/s", "h2d_bytes_per_step": in_bytes,
                "d2h_bytes_per_step": 8 * Q, "ms_per_step": ems}
     peak, peak_kind = measured_peaks()
-    # single trees: the query-step sweep where a state is asked 24 queries and more
-    kernel = "k_chain_sweep" if chain_path else "k_qsweep" if Q >= 24 * S else "k_sweep"
+    # single trees: the query-step sweep where a state is asked 18 queries and more
+    kernel = "k_chain_sweep" if chain_path else "k_qsweep" if Q >= 18 * S else "k_esweep"
     sweep_bytes = 16 * E + 20 * Q
     sweep_ms = stage_mean["sweep"]
     achieved = sweep_bytes / (sweep_ms / 1e3) / 1e9

@@ -2403,12 +2403,11 @@ static inline size_t align_up(size_t x) { return (x + 255) & ~size_t(255); }
 
 static size_t sweep_budget(int ctas_per_sm) { return (size_t)(kSmemPerSM / ctas_per_sm) - 3072; }
 
-// Default sweep: the Euler-tile sweep for forests (measured fastest on batched
-// uneven trees), else by the query/event ratio.
+// Default sweep: the Euler-tile sweep, or the query-step sweep for single trees that are
+// asked much.
 static void finish_spec(PipeSpec& s, const Tuning& tune, bool forest) {
   s.tile = tune.tile >= kTileNarrowId && tune.tile <= kTileMaxId ? tune.tile
-           : forest ? kTileEulerId
-           : s.Q >= kQueryDense * (int64_t)s.S ? kTileQueryId : (s.Q * 8 >= s.E ? kTileNarrowId : kTileEulerId);
+           : !forest && query_steps(s.S, s.E, s.Q) ? kTileQueryId : kTileEulerId;
   s.contract = s.E < ((int64_t)1 << 31) &&   // (a node's events are counted in 32 bits)
                (tune.contract >= 0 ? tune.contract != 0 : s.Q * kContract <= (int64_t)s.S);
   if (s.tile == kTileQueryId) s.ctas_per_sm = 2;

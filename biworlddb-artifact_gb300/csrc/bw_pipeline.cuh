@@ -36,10 +36,19 @@ constexpr int64_t kQueryCost = 2;             // a query is two prefix probes
 constexpr int64_t kMinWork = 16384, kMinWorkCoarse = 65536;
 // A tour is contracted when at most one state in kContract has a query (see k_ct_nodes).
 constexpr int64_t kContract = 2;
-// Queries per state from which a tree is swept a step at a time by bw_qsweep.cu: measured
-// against k_sweep's narrow tile, 15 a state 1.02 and 1.18 ms, 18 a state 0.60 and 0.63 ms,
-// 167 a state 0.33 and 0.49 ms (4M events) and 2.3 and 4.6 ms (40M), 2 a state 0.94 and 0.44 ms.
-constexpr int64_t kQueryDense = 24;
+// Single trees take the query-step sweep where a state is asked kQueryDense queries and more
+// and, below kQueryStates states (whose blocks' chains of steps leave the GPU part empty),
+// where a step has work besides; else the Euler-tile sweep.  Query steps / Euler tiles, us a
+// replay: 100,000 states, 5M events, 2M queries 745 / 905, 100,000 states, 4M events, 1.7M queries
+// 710 / 684; 44,000 states, 1.7M events, 490,000 queries 502 / 395; 5,000 states, 60,000 events,
+// 250,000 queries 365 / 274, 500,000 queries 217 / 311; 10,000 states, 2.5M events, 180,000
+// queries 212 / 248.  (k_sweep, which trees with a query for every eight events took before,
+// needs 829, 779 and 302 us where the Euler tiles need 684, 395 and 182.)
+constexpr int64_t kQueryDense = 18;
+constexpr int64_t kQueryStates = 20'000;
+inline bool query_steps(int64_t S, int64_t E, int64_t Q) {
+  return Q >= kQueryDense * S && (S >= kQueryStates || E / 4 + Q >= 60 * S);
+}
 
 // Estimated sweep work of a tree (or a whole forest) from its sizes: every event is
 // applied on enter and on exit, every state is entered and left, and at most

@@ -33,10 +33,12 @@ def test_scan_of_many_tiles(bw, torch_cuda, S):
 
 
 @pytest.mark.parametrize("kind", ["fork", "chain", "star", "bushy"])
-@pytest.mark.parametrize("S,C,E,Q", [(1, 1, 40, 24), (50, 1, 500, 1200), (300, 70_000, 9000, 8000), (200, 300, 0, 5000),
-                                     (64, 20_000, 50_000, 1537), (3000, 4097, 100_000, 72_001)])
+@pytest.mark.parametrize("S,C,E,Q", [(1, 1, 40, 64), (50, 1, 500, 3100), (300, 70_000, 9000, 18_500), (200, 300, 0, 12_500),
+                                     (64, 20_000, 50_000, 1537), (3000, 4097, 600_000, 54_001),
+                                     (20_000, 4097, 50_000, 360_001), (19_999, 500, 40_000, 360_001)])
 def test_query_step_sweep(bw, torch_cuda, oracle_mod, S, C, E, Q, kind):
-    """Single trees whose states are asked 24 queries and more take the query-step sweep."""
+    """Single trees whose states are asked 18 queries and more take the query-step sweep (the
+    last case, just below 20,000 states, the Euler-tile sweep)."""
     rng = np.random.default_rng(S + C)
     parent = evgen.make_tree(S, kind, rng)
     ev, qs = evgen.make_events(S, C, E, rng, zipf=1.2, big=S == 300), evgen.make_queries(S, C, Q, rng)
