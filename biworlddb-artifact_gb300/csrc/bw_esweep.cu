@@ -768,7 +768,7 @@ __global__ void __launch_bounds__(kEsThreads, 1) k_esweep(EsParams p) {
     ps.t0 = bt.t0; ps.t1 = bt.t1;
     ps.dense = C <= (w64 ? p.cap64 : p.cap32);
     ps.crow = bt.carry_in >= 0 ? p.carry + bt.carry_in : nullptr;
-    const Slice* bsl = p.slices + (size_t)b * kMaxSlices;
+    const Slice* bsl = p.slices + (size_t)b * p.max_slices;
     const int32_t nsl = ps.dense ? 1 : p.nslices[b];
     // slices without keys change no answer: skipped, except that one pass (the first
     // slice with keys, else slice 0) writes every answer

@@ -710,7 +710,8 @@ struct PrepParams {
   uint32_t cap32, cap64;   // slice rank capacity with int32 / int64 sweep nodes
   uint64_t* bits;
   uint32_t* rlut;
-  Slice* slices;
+  Slice* slices;           // max_slices a block
+  int32_t max_slices;
   int32_t* nslices;
   int64_t* carry;
   int32_t* status;
@@ -871,7 +872,7 @@ __device__ void prepare_block_a(const PrepParams& p, int32_t b, unsigned char* s
   const int32_t t0 = bt.t0, t1 = bt.t1;
   uint64_t* gbits = p.bits + bt.bits_off;
   uint32_t* grl = p.rlut + bt.bits_off + b;
-  Slice* gsl = p.slices + (size_t)b * kMaxSlices;
+  Slice* gsl = p.slices + (size_t)b * p.max_slices;
   if (threadIdx.x == 0) s_nsl = 0;
   uint32_t rank_base = 0;
   uint32_t mass = 0, over = 0;  // per-thread partial of the block's applied |delta| sum
@@ -919,7 +920,7 @@ __device__ void prepare_block_a(const PrepParams& p, int32_t b, unsigned char* s
           const int32_t mid = (hi + top + 1) >> 1;
           if (srl[mid] - srl[lo] <= cap) hi = mid; else top = mid - 1;
         }
-        if (ns < kMaxSlices) {
+        if (ns < p.max_slices) {
           Slice s;
           s.word_lo = w0 + lo; s.word_hi = w0 + hi;
           s.rank_lo = rank_base + srl[lo]; s.n = srl[hi] - srl[lo];
@@ -935,8 +936,8 @@ __device__ void prepare_block_a(const PrepParams& p, int32_t b, unsigned char* s
   }
   if (threadIdx.x == 0) {
     grl[nwords] = rank_base;
-    if (s_nsl > kMaxSlices) set_status(p.status, BW_STATUS_TOO_MANY_SLICES);
-    p.nslices[b] = min(s_nsl, kMaxSlices);
+    if (s_nsl > p.max_slices) set_status(p.status, BW_STATUS_TOO_MANY_SLICES);
+    p.nslices[b] = min(s_nsl, p.max_slices);
     p.bmode[b] = s_mode;
   }
   __syncthreads();
@@ -975,7 +976,7 @@ __device__ void prepare_block_b(const PrepParams& p, int32_t b, unsigned char* s
   const int32_t t0 = bt.t0, t1 = bt.t1;
   const uint64_t* gbits = p.bits + bt.bits_off;
   const uint32_t* grl = p.rlut + bt.bits_off + b;
-  const Slice* gsl = p.slices + (size_t)b * kMaxSlices;
+  const Slice* gsl = p.slices + (size_t)b * p.max_slices;
   const int32_t nsl = p.nslices[b];
   int64_t* row = p.carry + bt.carry_out;
   const bool h32 = p.bmode[b] != 0;
@@ -1123,6 +1124,7 @@ struct SweepParams {
   const uint64_t* bits;
   const uint32_t* rlut;
   const Slice* slices;
+  int32_t max_slices;
   const int32_t* nslices;
   const int64_t* carry;
   int64_t* answers;
@@ -1303,7 +1305,7 @@ __device__ __forceinline__ void sweep_block(const SweepParams& p, const SweepLay
 
   // Slices without keys change no answer: they are skipped, except that one pass
   // (the first slice with keys, else slice 0) writes every answer.
-  const Slice* bsl = p.slices + (size_t)b * kMaxSlices;
+  const Slice* bsl = p.slices + (size_t)b * p.max_slices;
   int32_t first_si = 0;
   while (first_si < nsl && bsl[first_si].n == 0) ++first_si;
   if (first_si == nsl) first_si = 0;
@@ -2439,6 +2441,15 @@ static void finish_spec(PipeSpec& s, const Tuning& tune, bool forest) {
     if (s.SL.cap32 > cap) s.SL.cap32 = cap;
     if (s.SL.cap64 > cap) s.SL.cap64 = cap;
   }
+  // A single tree's block may touch every key, and the windows of these two sweeps hold fewer
+  // ranks than k_sweep's at one CTA an SM (4,095 int64 ranks and 13,824 against 16,384 over 2^18
+  // keys and more), so their slices are counted out: a slice that does not end its window
+  // holds more than cap - 64 ranks.
+  s.max_slices = kMaxSlices;
+  if (!forest && s.tile >= kTileEulerId) {
+    const int64_t keys = std::min<int64_t>(s.Cmax, s.E), windows = (nw + kWinWords - 1) / kWinWords;
+    s.max_slices = (int32_t)std::max<int64_t>(kMaxSlices, windows + keys / (s.SL.cap64 - 63) + 1);
+  }
 }
 
 int pipe_spec_one(int32_t S, uint32_t C, int64_t E, int64_t Q, int32_t blocks, bool chain, const Tuning& tune,
@@ -2606,7 +2617,7 @@ void pipe_layout(const PipeSpec& s, Layout& L) {
   take(W_BMODE, B * 4);
   take(W_BITS, (size_t)s.bits_words * 8);
   take(W_RLUT, ((size_t)s.bits_words + B) * 4);
-  take(W_SLICES, B * kMaxSlices * sizeof(Slice));
+  take(W_SLICES, B * (size_t)s.max_slices * sizeof(Slice));
   take(W_NSLICES, B * 4);
   take(W_CARRY, (size_t)s.carry_words * 8);
   take(W_GSUM, (size_t)s.gsum_words * 8);
@@ -2871,7 +2882,7 @@ int pipe_enqueue(const PipeSpec& s, void* workspace, const int32_t* parent, cons
   pp.ev = events; pp.desc = desc; pp.partner = partner; pp.blocks = blocks;
   pp.order = order; pp.B = B; pp.ww = SL.ww; pp.cap32 = SL.cap32; pp.cap64 = SL.cap64;
   pp.bits = reinterpret_cast<uint64_t*>(at(W_BITS)); pp.rlut = reinterpret_cast<uint32_t*>(at(W_RLUT));
-  pp.slices = reinterpret_cast<Slice*>(at(W_SLICES)); pp.nslices = reinterpret_cast<int32_t*>(at(W_NSLICES));
+  pp.slices = reinterpret_cast<Slice*>(at(W_SLICES)); pp.max_slices = s.max_slices; pp.nslices = reinterpret_cast<int32_t*>(at(W_NSLICES));
   pp.carry = reinterpret_cast<int64_t*>(at(W_CARRY)); pp.status = status; pp.bmode = bmode;
   pp.ticket = misc + M_PREP_TICKET;
   int occ_a = 0;
@@ -2905,14 +2916,14 @@ int pipe_enqueue(const PipeSpec& s, void* workspace, const int32_t* parent, cons
   if (s.Q > 0) {
     SweepParams sp;
     sp.ev = events; sp.qs = queries; sp.desc = desc; sp.blocks = blocks; sp.order = order; sp.B = B;
-    sp.bits = pp.bits; sp.rlut = pp.rlut; sp.slices = pp.slices; sp.nslices = pp.nslices; sp.carry = pp.carry;
+    sp.bits = pp.bits; sp.rlut = pp.rlut; sp.slices = pp.slices; sp.max_slices = s.max_slices; sp.nslices = pp.nslices; sp.carry = pp.carry;
     sp.answers = answers; sp.status = status; sp.bmode = bmode; sp.ticket = misc + M_SWEEP_TICKET;
     const int sgrid = std::min(B, s.ctas_per_sm * s.sms);
     if (s.tile == kTileEulerId || s.tile == kTileQueryId) {
       EsParams ep;
       ep.ev = reinterpret_cast<const uint4*>(events); ep.qs = queries; ep.desc = desc; ep.blocks = blocks;
       ep.order = order; ep.B = B; ep.cap32 = SL.cap32; ep.cap64 = SL.cap64;
-      ep.bits = pp.bits; ep.rlut = pp.rlut; ep.slices = pp.slices; ep.nslices = pp.nslices; ep.carry = pp.carry;
+      ep.bits = pp.bits; ep.rlut = pp.rlut; ep.slices = pp.slices; ep.max_slices = s.max_slices; ep.nslices = pp.nslices; ep.carry = pp.carry;
       ep.answers = answers; ep.status = status; ep.bmode = bmode; ep.ticket = misc + M_SWEEP_TICKET;
       if (s.tile == kTileEulerId) rc = report((cudaError_t)esweep_launch(ep, std::min(B, s.sms), st), "k_esweep");
       else rc = report((cudaError_t)qsweep_launch(ep, s.QL, std::min(B, 2 * s.sms), st), "k_qsweep");

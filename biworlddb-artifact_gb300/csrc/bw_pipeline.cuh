@@ -21,7 +21,7 @@ namespace bw {
 constexpr int kPrepThreads = 512;             // CTA width of the prepare kernel (two per SM)
 constexpr int kWinBits = 18;                  // rank window: 2^18 keys per smem bitmap
 constexpr int kWinWords = 1 << (kWinBits - 6);
-constexpr int kMaxSlices = 256;               // key slices per block
+constexpr int kMaxSlices = 256;               // key slices per block (single trees: see finish_spec)
 constexpr int kSmemLimit = 232448;            // 227 KiB dynamic smem per CTA on sm_100/103
 constexpr int kSmemPerSM = 233472;            // 228 KiB shared memory per SM
 constexpr int kCarryGroup = 16;               // rows per group of the carry scan
@@ -240,6 +240,7 @@ struct PipeSpec {
   int32_t sms = 0;
   SweepLayout SL{};
   QsLayout QL{};                // tile 7
+  int32_t max_slices = kMaxSlices;   // slices a block may have
   bool chain_hint = false;
   bool contract = false;        // the tour runs over contracted nodes, without those no query needs
   // one-tree scalars (T == 1): tables are written by a kernel at each launch
@@ -322,7 +323,8 @@ struct EsParams {
   uint32_t cap32, cap64;
   const uint64_t* bits;
   const uint32_t* rlut;
-  const Slice* slices;
+  const Slice* slices;    // max_slices a block
+  int32_t max_slices;
   const int32_t* nslices;
   const int64_t* carry;
   int64_t* answers;

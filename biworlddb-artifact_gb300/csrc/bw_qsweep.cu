@@ -124,7 +124,7 @@ __device__ __forceinline__ void qs_block(const EsParams& p, int32_t ww, uint32_t
   constexpr int kDepth = sizeof(Node) == 4 ? 3 : 2;   // steps copied ahead
   constexpr int kWords = sizeof(Node) == 4 ? 2 : 3;   // key and delta words; the bounds follow
   const int32_t nsl = p.nslices[b];
-  const Slice* bsl = p.slices + (size_t)b * kMaxSlices;
+  const Slice* bsl = p.slices + (size_t)b * p.max_slices;
   for (int32_t si = 0; si < nsl; ++si) {
     const Slice s = bsl[si];
     if (s.n == 0) continue;   // no keys: no part of any answer

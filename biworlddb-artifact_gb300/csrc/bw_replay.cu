@@ -58,20 +58,22 @@ int spec_of(const BwReplayArgs* a, PipeSpec& s, Layout& L) {
     return r;
   };
   if ((rc = plan(kMinWork)) || L.total <= small) return rc;
-  // does the plainest plan fit?
+  // does the plainest plan fit?  (k_sweep: its slice tables do not grow with the domain)
+  const int32_t plain = a->n_queries * 8 >= a->n_events ? kTileNarrowId : kTileWideId;
   tune.contract = 0;
+  tune.tile = plain;
   if ((rc = plan(kMinWorkCoarse))) return rc;
   const bool fits = L.total <= small;
-  tune.contract = -1;
-  if (!fits || a->blocks > 0) {
-    if ((rc = plan(kMinWork)) || !fits || L.total <= small) return rc;
-    tune.contract = 0;
-    return plan(kMinWork);
-  }
-  for (int64_t w = kMinWork; w < kMinWorkCoarse; w += w / 4) {
-    if ((rc = plan(w)) || L.total <= small) return rc;
+  tune = Tuning();
+  if (!fits) return plan(kMinWork);
+  if (a->blocks <= 0) {
+    for (int64_t w = kMinWork; w < kMinWorkCoarse; w += w / 4) {
+      if ((rc = plan(w)) || L.total <= small) return rc;
+    }
   }
   tune.contract = 0;
+  if ((rc = plan(kMinWorkCoarse)) || L.total <= small) return rc;
+  tune.tile = plain;
   return plan(kMinWorkCoarse);
 }
 
