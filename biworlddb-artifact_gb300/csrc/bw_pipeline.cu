@@ -2584,7 +2584,8 @@ void pipe_layout(const PipeSpec& s, Layout& L) {
   const size_t S = (size_t)s.S, S2 = 2 * S, T = (size_t)s.T, B = (size_t)s.B;
   size_t o = 0;
   auto take = [&](int i, size_t bytes) { L.off[i] = o; o = align_up(o + bytes); };
-  take(W_TSOFF, (T + 1) * 4);
+  take(W_TSOFF, 2 * (T + 1) * 4);
+  L.off[W_TTOFF] = L.off[W_TSOFF] + (T + 1) * 4;   // (a slot of its own would cost one tree 256 bytes)
   take(W_TEOFF, (T + 1) * 8);
   take(W_TQOFF, (T + 1) * 8);
   take(W_TC, T * 4);
@@ -2622,7 +2623,6 @@ void pipe_layout(const PipeSpec& s, Layout& L) {
   take(W_CARRY, (size_t)s.carry_words * 8);
   take(W_GSUM, (size_t)s.gsum_words * 8);
   take(W_TNOFF, s.contract ? (T + 1) * 4 : 0);
-  take(W_TTOFF, (T + 1) * 4);
   take(W_NEOFF, s.contract ? (S + 1) * 8 : 0);
   take(W_NQOFF, s.contract ? (S + 1) * 8 : 0);
   take(W_NPAR, s.contract ? S * 4 : 0);
