@@ -277,16 +277,17 @@ __device__ __forceinline__ void qs_block(const EsParams& p, int32_t ww, uint32_t
   }
 }
 
-// The carried part of every query's answer (0 where the block starts its tree).  CTA
-// (part, block): a warp takes eight consecutive steps at a time and their queries,
+// The carried part of every query's answer (0 where the block starts its tree).  A CTA
+// per part of a block: a warp takes eight consecutive steps at a time and their queries,
 // flattened.  The parts of a block run side by side, so that some eighty carry rows are
-// read at a time and stay in the L2.
+// read at a time and stay in the L2.  (One grid dimension for both: a caller may ask for
+// more blocks than the second one takes.)
 constexpr int kQcParts = 16, kQcSteps = 8;
 __global__ void __launch_bounds__(256) k_qcarry(EsParams p) {
   if (*p.status) return;
-  const BlockTab bt = p.blocks[blockIdx.y];
+  const BlockTab bt = p.blocks[blockIdx.x / kQcParts];
   const int64_t* crow = bt.carry_in >= 0 ? p.carry + bt.carry_in : nullptr;
-  const int lane = threadIdx.x & 31, warp = blockIdx.x * 8 + (threadIdx.x >> 5);
+  const int lane = threadIdx.x & 31, warp = (blockIdx.x % kQcParts) * 8 + (threadIdx.x >> 5);
   for (int32_t c = bt.t0 + kQcSteps * warp; c < bt.t1; c += kQcSteps * 8 * kQcParts) {
     const uint4 d = lane < kQcSteps && c + lane < bt.t1 ? __ldg(reinterpret_cast<const uint4*>(p.desc) + c + lane)
                                                         : make_uint4(0, 0, 0, 0);
@@ -355,7 +356,9 @@ int qsweep_attrs() {
 }
 
 int qsweep_launch(const EsParams& p, const QsLayout& q, int grid, cudaStream_t st) {
-  k_qcarry<<<dim3(kQcParts, (unsigned)p.B), 256, 0, st>>>(p);
+  k_qcarry<<<(unsigned)(p.B * kQcParts), 256, 0, st>>>(p);
+  const cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) return (int)e;   // (the sweep adds to what k_qcarry writes)
   k_qsweep<<<grid, kQsThreads, q.bytes, st>>>(p, q.ww, q.supers);
   return (int)cudaGetLastError();
 }
