@@ -41,6 +41,7 @@
 #include "bw_common.cuh"
 #include "bw_pipeline.cuh"
 #include "bw_keyblock.cuh"
+#include "bw_search.cuh"
 
 namespace bw {
 namespace {
@@ -146,11 +147,7 @@ __global__ void k_kb_key_hist(KbParams p) {
 
 // First step in [lo, hi] with ep[step] > j (there is one).
 __device__ __forceinline__ int32_t kb_find_step(const int64_t* ep, int32_t lo, int32_t hi, int64_t j) {
-  while (lo < hi) {
-    const int32_t mid = (lo + hi) >> 1;
-    if (ep[mid] > j) hi = mid; else lo = mid + 1;
-  }
-  return lo;
+  return first_after(lo, hi, [&](int32_t t) { return ep[t] > j; });
 }
 // Last column in [lo, hi] with coltime <= j.
 __device__ __forceinline__ int32_t kb_find_col(const uint32_t* coltime, int32_t lo, int32_t hi, uint32_t j) {
