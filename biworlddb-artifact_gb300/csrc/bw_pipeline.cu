@@ -2928,7 +2928,7 @@ int pipe_enqueue(const PipeSpec& s, void* workspace, const int32_t* parent, cons
       if (s.tile == kTileEulerId) rc = report((cudaError_t)esweep_launch(ep, std::min(B, s.sms), st), "k_esweep");
       else rc = report((cudaError_t)qsweep_launch(ep, s.QL, std::min(B, 2 * s.sms), st), "k_qsweep");
       if (rc) return rc;
-      ++kernels;
+      kernels += s.tile == kTileQueryId ? 2 : 1;   // (k_qcarry, k_qsweep)
       if ((rc = mark(6))) return rc;
       if (kernels_out) *kernels_out = kernels;
       return 0;
