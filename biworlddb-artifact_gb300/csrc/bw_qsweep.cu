@@ -35,6 +35,7 @@ constexpr int kQsThreads = 512, kQsWarps = kQsThreads / 32;
 constexpr uint32_t kQsGroup = 16, kQsRunGroups = 128, kQsSuper = kQsGroup * kQsRunGroups;   // ranks of a total, of a run
 constexpr uint32_t kQsMaxRuns = 16;                  // one warp each
 constexpr int kQsRing = 128;                         // step descriptors
+constexpr int kQsMore = 4;                           // queries a thread pair reads at a time past its first
 constexpr int kQsSlots = 9;                          // slot arrays of a word per thread
 constexpr uint32_t kFull = 0xffffffffu;
 static_assert(kQsRunGroups == 4 * 32, "a warp scans the totals of one run, four a lane");
@@ -260,10 +261,18 @@ __device__ __forceinline__ void qs_block(const EsParams& p, int32_t ww, uint32_t
           }
           spre -= own;
           answer(mine, d.y + (tid >> 1), x0, r0, spre);
-          for (int32_t q0 = kQsThreads / 2; q0 + warp * 16 < nq; q0 += kQsThreads / 2) {   // more than 256 queries
-            const int32_t q = q0 + (tid >> 1);
-            const uint32_t x = q < nq ? bound_at(d.y + q) : 0u;
-            answer(q < nq, d.y + q, x, q < nq ? key_rank(x) : 0u, spre);
+          for (int32_t q0 = kQsThreads / 2; q0 + warp * 16 < nq; q0 += kQsMore * kQsThreads / 2) {   // more than 256 queries
+            uint32_t x[kQsMore];   // (read together: a memory latency for every 256 queries else)
+#pragma unroll
+            for (int u = 0; u < kQsMore; ++u) {
+              const int32_t q = q0 + u * (kQsThreads / 2) + (tid >> 1);
+              x[u] = q < nq ? bound_at(d.y + q) : 0u;
+            }
+#pragma unroll
+            for (int u = 0; u < kQsMore; ++u) {
+              const int32_t q = q0 + u * (kQsThreads / 2) + (tid >> 1);
+              if (q - (tid >> 1) + warp * 16 < nq) answer(q < nq, d.y + q, x[u], q < nq ? key_rank(x[u]) : 0u, spre);
+            }
           }
         }
         __syncthreads();                       // probes done before the next updates
@@ -282,40 +291,87 @@ __device__ __forceinline__ void qs_block(const EsParams& p, int32_t ww, uint32_t
 // flattened.  The parts of a block run side by side, so that some eighty carry rows are
 // read at a time and stay in the L2.  (One grid dimension for both: a caller may ask for
 // more blocks than the second one takes.)
-constexpr int kQcParts = 16, kQcSteps = 8;
-__global__ void __launch_bounds__(256) k_qcarry(EsParams p) {
+// A group of steps with more than kQcHeavy queries is left for the end, when the CTA's
+// warps share it: a state asked much more than the others kept a single warp busy (a replay of
+// 30,000 states and 1M queries, half of them on one state, 13.0 -> 1.8 ms; one state, 2.8M queries
+// 70 -> 7.9; queries spread evenly unchanged).  Lists in device memory would let all parts share
+// a group, but the sweep, which takes such a step with one CTA, needs as long as one CTA here.
+constexpr int kQcParts = 16, kQcSteps = 8, kQcWarps = 8;
+constexpr int kQcBatch = 4;                 // queries a lane reads at a time
+constexpr uint32_t kQcHeavy = 1024;
+constexpr int kQcList = 32;                 // groups left for the end; further ones are done where they occur
+__global__ void __launch_bounds__(32 * kQcWarps) k_qcarry(EsParams p) {
   if (*p.status) return;
+  __shared__ int32_t s_heavy[kQcList], s_nheavy;
   const BlockTab bt = p.blocks[blockIdx.x / kQcParts];
   const int64_t* crow = bt.carry_in >= 0 ? p.carry + bt.carry_in : nullptr;
-  const int lane = threadIdx.x & 31, warp = (blockIdx.x % kQcParts) * 8 + (threadIdx.x >> 5);
-  for (int32_t c = bt.t0 + kQcSteps * warp; c < bt.t1; c += kQcSteps * 8 * kQcParts) {
+  const int lane = threadIdx.x & 31, own = threadIdx.x >> 5, warp = (blockIdx.x % kQcParts) * kQcWarps + own;
+  if (threadIdx.x == 0) s_nheavy = 0;
+  __syncthreads();
+  uint32_t n, incl, first;   // of this lane's step: queries, those up to it, the first one
+  auto decode = [&](int32_t c) -> uint32_t {
     const uint4 d = lane < kQcSteps && c + lane < bt.t1 ? __ldg(reinterpret_cast<const uint4*>(p.desc) + c + lane)
                                                         : make_uint4(0, 0, 0, 0);
-    const uint32_t n = (int32_t)d.w > 0 ? d.w : 0u;
-    uint32_t incl = n;
+    n = (int32_t)d.w > 0 ? d.w : 0u;
+    first = d.y;
+    incl = n;
 #pragma unroll
     for (int o = 1; o < kQcSteps; o <<= 1) {
       const uint32_t y = __shfl_up_sync(kFull, incl, o);
       if (lane >= o) incl += y;
     }
-    const uint32_t total = __shfl_sync(kFull, incl, kQcSteps - 1);
-#pragma unroll 2
-    for (uint32_t g0 = 0; g0 < total; g0 += 32) {
-      const uint32_t g = g0 + lane;
-      int lo = 0, hi = kQcSteps - 1;   // first step whose inclusive count exceeds g
+    return __shfl_sync(kFull, incl, kQcSteps - 1);
+  };
+  auto answer = [&](uint32_t from, uint32_t total, uint32_t stride) {
+    for (uint64_t g0 = from; g0 < total; g0 += stride) {
+      uint32_t q[kQcBatch], a[kQcBatch], z[kQcBatch];
 #pragma unroll
-      for (int it = 0; it < 3; ++it) {
-        const int mid = (lo + hi) >> 1;
-        if (__shfl_sync(kFull, incl, mid) > g) hi = mid; else lo = mid + 1;
+      for (int u = 0; u < kQcBatch; ++u) {
+        const uint32_t g = (uint32_t)g0 + 32 * u + lane;
+        int lo = 0, hi = kQcSteps - 1;   // first step whose inclusive count exceeds g
+#pragma unroll
+        for (int it = 0; it < 3; ++it) {
+          const int mid = (lo + hi) >> 1;
+          if (__shfl_sync(kFull, incl, mid) > g) hi = mid; else lo = mid + 1;
+        }
+        const uint32_t before = __shfl_sync(kFull, incl - n, lo), q0 = __shfl_sync(kFull, first, lo);
+        q[u] = q0 + (g - before);
+        a[u] = z[u] = 0;
+        if (g < total && crow) {
+          a[u] = __ldg(&p.qs[q[u]].lo);
+          z[u] = __ldg(&p.qs[q[u]].hi);
+        }
       }
-      const uint32_t before = __shfl_sync(kFull, incl - n, lo), q0 = __shfl_sync(kFull, d.y, lo);
-      if (g < total) {
-        const uint32_t q = q0 + (g - before);
-        const uint32_t a = __ldg(&p.qs[q].lo), z = __ldg(&p.qs[q].hi);
-        p.answers[q] = crow && a < z ? (int64_t)((uint64_t)__ldg(crow + z) - (uint64_t)__ldg(crow + a)) : 0;
+      int64_t ra[kQcBatch], rz[kQcBatch];
+#pragma unroll
+      for (int u = 0; u < kQcBatch; ++u) {
+        ra[u] = rz[u] = 0;
+        if (a[u] < z[u]) {
+          ra[u] = __ldg(crow + a[u]);
+          rz[u] = __ldg(crow + z[u]);
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < kQcBatch; ++u)
+        if ((uint32_t)g0 + 32 * u + lane < total) p.answers[q[u]] = (int64_t)((uint64_t)rz[u] - (uint64_t)ra[u]);
+    }
+  };
+  for (int32_t c = bt.t0 + kQcSteps * warp; c < bt.t1; c += kQcSteps * kQcWarps * kQcParts) {
+    const uint32_t total = decode(c);
+    if (total > kQcHeavy) {
+      int32_t i = 0;
+      if (lane == 0) i = atomicAdd(&s_nheavy, 1);
+      i = __shfl_sync(kFull, i, 0);
+      if (i < kQcList) {
+        if (lane == 0) s_heavy[i] = c;
+        continue;
       }
     }
+    answer(0, total, 32 * kQcBatch);
   }
+  __syncthreads();
+  const int32_t nh = min(s_nheavy, kQcList);
+  for (int32_t h = 0; h < nh; ++h) answer(own * 32 * kQcBatch, decode(s_heavy[h]), kQcWarps * 32 * kQcBatch);
 }
 
 __global__ void __launch_bounds__(kQsThreads, 2) k_qsweep(EsParams p, int32_t ww, uint32_t supers) {

@@ -1,4 +1,5 @@
-"""GPU parity of the query-step sweep at its own edges: many blocks, kernels enqueued."""
+"""GPU parity of the query-step sweep at its own edges: many blocks, kernels enqueued, states
+asked or edited much more than the others."""
 from __future__ import annotations
 
 import ctypes
@@ -47,3 +48,39 @@ def test_kernels_enqueued(bw, torch_cuda):
         assert rt.cudaGraphNodeGetType(ctypes.c_void_p(x), ctypes.byref(kind)) == 0
         kernels += kind.value == 0   # cudaGraphNodeTypeKernel
     assert plan.info()[0] == kernels
+
+
+@pytest.mark.parametrize("big", [False, True])   # int32 and int64 windows, several of each
+@pytest.mark.parametrize("blocks", [0, 1, 7])
+def test_hot_states(bw, torch_cuda, oracle_mod, blocks, big):
+    """Steps around 256 queries (a thread pair's first), 1,024 (a carry group's share), and
+    around 512 events, among ordinary ones."""
+    S, C, E, Q = 700, 90_000, 90_000, 60_000
+    rng = np.random.default_rng(blocks)
+    parent = evgen.make_tree(S, "fork", rng)
+    ev, qs = evgen.make_events(S, C, E, rng, big=big), evgen.make_queries(S, C, Q, rng)
+    counts = [255, 256, 257, 511, 512, 513, 1023, 1024, 1025, 1280, 1281, 4097, 9000]
+    hot = rng.choice(S, len(counts), replace=False)
+    for arr, n in ((qs, Q), (ev, E)):
+        state = rng.choice(np.setdiff1d(np.arange(S), hot), n)
+        state[: sum(counts)] = np.repeat(hot, counts)
+        arr["state"] = np.sort(state)
+    p, e, q = evgen.to_device(torch_cuda, parent, ev, qs)
+    got = bw.replay(p, C, e, q, blocks=blocks).cpu().numpy()
+    np.testing.assert_array_equal(got, oracle_mod.ev_sweep(parent, C, ev, qs))
+
+
+@pytest.mark.parametrize("hot", [0, 1500, 2599, None])
+def test_all_queries_heavy(bw, torch_cuda, oracle_mod, hot):
+    """More heavy groups than a carry CTA's list holds (every state asked some 300 queries, one
+    block), and every query on one state."""
+    S, C, E, Q = 2600, 3000, 20_000, 780_000
+    rng = np.random.default_rng(3)
+    parent = evgen.make_tree(S, "fork", rng)
+    ev, qs = evgen.make_events(S, C, E, rng), evgen.make_queries(S, C, Q, rng)
+    if hot is not None:
+        qs["state"] = hot
+    p, e, q = evgen.to_device(torch_cuda, parent, ev, qs)
+    want = oracle_mod.ev_sweep(parent, C, ev, qs)
+    for blocks in (0, 1, 2):
+        np.testing.assert_array_equal(bw.replay(p, C, e, q, blocks=blocks).cpu().numpy(), want)
