@@ -32,6 +32,7 @@
 // All arithmetic is int64 with two's-complement wrap (done in uint64), so any
 // summation order gives the reference's bits.
 #include <cuda_runtime.h>
+#include <cmath>
 #include <algorithm>
 #include <cstdint>
 #include <cstdio>
@@ -2467,6 +2468,9 @@ int pipe_spec_one(int32_t S, uint32_t C, int64_t E, int64_t Q, int32_t blocks, b
     B = 2 * (int64_t)sms;                            // two sweep CTAs per SM hide each other's latency
     if (tune.block_work > 0) B = (work + tune.block_work - 1) / tune.block_work;
     if (work / min_work < B) B = work / min_work;
+    // (rows of the domain's width against work: see kRowWork)
+    const int64_t balanced = (int64_t)std::sqrt((double)kRowWork * (double)work / ((double)C + 1.0));
+    B = std::min(B, std::max({balanced, work / kMinWorkCoarse, 2 * E / min_work}));
     const double carry_budget = 4.0e9;               // bytes of dense carry rows
     const int64_t by_mem = (int64_t)(carry_budget / (8.0 * ((double)C + 1.0)));
     if (by_mem < B) B = by_mem;

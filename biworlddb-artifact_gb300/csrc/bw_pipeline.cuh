@@ -34,6 +34,15 @@ constexpr int64_t kQueryCost = 2;             // a query is two prefix probes
 // took 752 us, at 25,000 (64 blocks) 269 us; 50,000 states and 1M events 702 and 288 us.  The larger value stays for callers whose scratch the
 // smaller blocks would outgrow.
 constexpr int64_t kMinWork = 16384, kMinWorkCoarse = 65536;
+// Above the coarse count and two events per unit of the block work, the blocks of one tree are
+// at most sqrt(kRowWork work / (C + 1)): a block more shortens the longest one by work / B^2
+// and adds a carry row of C + 1 words to write, scan and read.  300 states, 1,000 events, 1M
+// queries: over 262,144 keys 30 / 68 / 123 blocks 322 / 376 / 774 us, over 16,000 keys 123 blocks
+// 161 (30: 294 with the sweep of before); 300,000 states, 1,000 events, 5,000 queries over 262,144
+// keys 41 / 79 / 166 blocks 327 / 379 / 544.  With events the longest block weighs more: 228
+// states, 2.8M events, 51,613 queries over 259,872 keys 87 blocks 2,204, 304 blocks 794.  (With 300 in the
+// place of 600: 51,240 states, 1,623 events, 1.6M queries, 51,174 keys 444, else 420.)
+constexpr int64_t kRowWork = 600;
 // A tour is contracted when at most one state in kContract has a query (see k_ct_nodes).
 constexpr int64_t kContract = 2;
 // Single trees take the query-step sweep where a state is asked kQueryDense queries and more
