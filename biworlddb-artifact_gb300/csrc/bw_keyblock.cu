@@ -21,7 +21,7 @@
 //   points    k_kb_point_count / scan / k_kb_point_scatter   signed points grouped by
 //             key block, in tour order (a stable partition of up to 4,096 digits).
 //   rows      k_kb_seg, k_kb_segscan, k_kb_rows   R, in two passes over the tour cut in
-//             equal segments (net sum per segment and block, then the running vector
+//             segments of equal work (net sum per segment and block, then the running vector
 //             in shared memory, written out scanned over the blocks at every column).
 //   probes    k_kb_probe_count / scan / k_kb_probe_scatter   both bounds of every query
 //             grouped by key block, in tour order; the whole-block part goes to acc.
@@ -49,6 +49,11 @@ namespace {
 constexpr uint32_t kAll = 0xffffffffu;
 constexpr uint32_t kNone = 0xffffffffu;
 
+struct KbCut {
+  int64_t j;            // points
+  int64_t c;            // and columns before the segment
+};
+
 struct KbParams {
   const BwEvent* ev;
   const BwQuery* qs;
@@ -69,6 +74,7 @@ struct KbParams {
   uint32_t *pthist, *ptoff;   // tiles x B digit counts (then starts), B + 1 block starts
   uint4* pts;           // the swept points by key block, {time, slot, delta}
   uint64_t* seg;        // segs x B
+  KbCut* cut;           // segs + 1
   int64_t* rows;        // columns x Bs
   uint32_t *prhist, *proff;
   uint2* prs;           // {query in tour order, slot | lower bound << 31}
@@ -344,17 +350,44 @@ __device__ __forceinline__ void kb_add_points(const KbParams& p, unsigned long l
     shared_add_u64(vec + (x.y & ~kRowsOnly) / p.m, ((uint64_t)x.w << 32) | x.z);
   }
 }
-__device__ __forceinline__ int64_t kb_seg_start(const KbParams& p, int32_t g) {
-  return (int64_t)(((__int128)kb_points(p) * g) / p.segs);
+// Segment g of the tour: an equal share of points and columns, a column counted as
+// kColPoints points (each column of a segment is written out in turn, some 0.6 us and more; cut by
+// points alone, the columns of 74,000 states with 12 events met in a dozen CTAs and the
+// rows took 11 ms).  The walk takes a column once all points up to its enter step are
+// taken.  Whole warp.
+constexpr int64_t kColPoints = 256;
+__device__ __forceinline__ KbCut kb_cut(const KbParams& p, int32_t g, int lane) {
+  const int32_t nc = kb_columns(p);
+  const int64_t np = kb_points(p), total = np + kColPoints * nc;
+  const int64_t d = total / p.segs * g + total % p.segs * g / p.segs;
+  int32_t lo = 0, hi = nc;   // the columns wholly before the cut, 32 probes a round
+  while (lo < hi) {
+    const int32_t step = (hi - lo + 31) / 32, c = lo + lane * step;   // (columns stay below 2^30)
+    const int n = __popc(__ballot_sync(kAll, c < hi && p.ep[p.colstep[c]] + kColPoints * ((int64_t)c + 1) <= d));
+    if (!n) break;
+    const int32_t last = lo + (n - 1) * step;
+    hi = n < 32 && last + step < hi ? last + step : hi;
+    lo = last + 1;
+  }
+  return KbCut{min(d - kColPoints * lo, lo < nc ? p.ep[p.colstep[lo]] : np), lo};
 }
 
-// Net delta of every tour segment in every key block.
+// The cuts, and the net delta of every segment in every key block.
 __global__ void __launch_bounds__(512) k_kb_seg(KbParams p) {
   if (*p.status) return;
   extern __shared__ __align__(16) unsigned long long vec[];
+  __shared__ int64_t s_j[2];
   for (int32_t i = threadIdx.x; i < p.B; i += blockDim.x) vec[i] = 0;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (warp < 2) {
+    const KbCut x = kb_cut(p, blockIdx.x + warp, lane);
+    if (lane == 0) {
+      s_j[warp] = x.j;
+      if (warp == 0 || blockIdx.x + 1 == (unsigned)p.segs) p.cut[blockIdx.x + warp] = x;
+    }
+  }
   __syncthreads();
-  kb_add_points(p, vec, kb_seg_start(p, blockIdx.x), kb_seg_start(p, blockIdx.x + 1));
+  kb_add_points(p, vec, s_j[0], s_j[1]);
   __syncthreads();
   for (int32_t i = threadIdx.x; i < p.B; i += blockDim.x) p.seg[(size_t)blockIdx.x * p.B + i] = vec[i];
 }
@@ -381,16 +414,6 @@ __global__ void __launch_bounds__(1024) k_kb_segscan(KbParams p) {
     }
 }
 
-// First column whose points (all up to its enter step) number more than j.
-__device__ __forceinline__ int32_t kb_col_after(const KbParams& p, int32_t nc, int64_t j) {
-  int32_t lo = 0, hi = nc;
-  while (lo < hi) {
-    const int32_t mid = (lo + hi) >> 1;
-    if (p.ep[p.colstep[mid]] > j) hi = mid; else lo = mid + 1;
-  }
-  return lo;
-}
-
 // A segment's columns: the running vector over the key blocks (shared memory) takes
 // the points up to the column and is written out scanned, four entries a thread and
 // pass.  Two barriers a column: the vector is complete; the warps' sums are written
@@ -399,20 +422,12 @@ constexpr int kRowThreads = 512;
 __global__ void __launch_bounds__(kRowThreads, 3) k_kb_rows(KbParams p) {
   if (*p.status) return;
   extern __shared__ __align__(16) unsigned long long vec[];   // Bs
-  __shared__ int32_t s_c[2];
   __shared__ uint64_t s_sum[2][2][kRowThreads / 32];          // by column parity and pass
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int64_t j0 = kb_seg_start(p, blockIdx.x), j1 = kb_seg_start(p, blockIdx.x + 1);
-  if (threadIdx.x < 2) {
-    const bool last = blockIdx.x + 1 == (unsigned)p.segs;
-    const int32_t nc = kb_columns(p);
-    // columns of the segment: point counts in (j0, j1], and those without points in the first one
-    s_c[threadIdx.x] = threadIdx.x ? (last ? nc : kb_col_after(p, nc, j1)) : (blockIdx.x ? kb_col_after(p, nc, j0) : 0);
-  }
   for (int32_t i = threadIdx.x; i < p.Bs; i += kRowThreads) vec[i] = i < p.B ? p.seg[(size_t)blockIdx.x * p.B + i] : 0;
   __syncthreads();
-  int64_t j = j0;
-  const int32_t c0 = s_c[0], c1 = s_c[1];
+  int64_t j = p.cut[blockIdx.x].j;
+  const int32_t c0 = (int32_t)p.cut[blockIdx.x].c, c1 = (int32_t)p.cut[blockIdx.x + 1].c;
   for (int32_t c = c0; c < c1; ++c) {
     const int64_t je = p.ep[p.colstep[c]];
     kb_add_points(p, vec, j, je);
@@ -723,6 +738,7 @@ void kb_layout(const PipeSpec& s, KbSpec& k) {
   take(KB_PTOFF, (B + 1) * 4);
   take(KB_PTS, 2 * (size_t)s.E * 16);
   take(KB_SEG, (size_t)k.segs * B * 8);
+  take(KB_CUT, ((size_t)k.segs + 1) * sizeof(KbCut));
   take(KB_ROWS, cols * ((B + 3) & ~(size_t)3) * 8);
   take(KB_PRHIST, B * (size_t)k.pr_tiles * 4);
   take(KB_PROFF, (B + 1) * 4);
@@ -804,7 +820,7 @@ int kb_enqueue(const KbSpec& k, const PipeSpec& spec, const BwReplayArgs* a, Eve
   p.colstate = (int32_t*)at(KB_COLSTATE); p.coltime = (uint32_t*)at(KB_COLTIME); p.colstep = (int32_t*)at(KB_COLSTEP);
   p.pos = (uint32_t*)at(KB_POS); p.pthist = (uint32_t*)at(KB_PTHIST); p.pts = (uint4*)at(KB_PTS);
   p.tour = (uint4*)at(KB_TOUR); p.ptoff = (uint32_t*)at(KB_PTOFF); p.proff = (uint32_t*)at(KB_PROFF);
-  p.seg = (uint64_t*)at(KB_SEG); p.rows = (int64_t*)at(KB_ROWS); p.prhist = (uint32_t*)at(KB_PRHIST);
+  p.seg = (uint64_t*)at(KB_SEG); p.cut = (KbCut*)at(KB_CUT); p.rows = (int64_t*)at(KB_ROWS); p.prhist = (uint32_t*)at(KB_PRHIST);
   p.prs = (uint2*)at(KB_PRS); p.acc = (unsigned long long*)at(KB_ACC);
   p.status = ta.misc + M_STATUS; p.ticket = ta.misc + M_SWEEP_TICKET;
   p.E = k.E; p.Q = k.Q; p.pt_tiles = k.pt_tiles; p.pr_tiles = k.pr_tiles;
