@@ -773,9 +773,27 @@ int kb_attrs() {
 bool kb_select(const BwReplayArgs* a, const PipeSpec& s, size_t general_bytes, KbSpec& k) {
   if (s.T != 1 || s.Cmax <= kKbMinKeys || a->blocks > 0 || (a->flags & BW_REPLAY_GENERAL)) return false;
   if (s.E < 1 || s.Q < 1 || s.Q >= ((int64_t)1 << 30)) return false;
+  // Work for one or two state blocks and a domain of few windows: the state-block path has
+  // fewer kernels and no pass over the domain; its time goes by the query steps and events of every
+  // window (300 states, 1,000 events, 100 queries, us a replay, state blocks / key blocks:
+  // 262,145 keys 113 / 229, 1M 156 / 245, 2M 215 / 246, 4M 337 / 235; 71 states, 25 events, 2,558
+  // queries, 880,418 keys 480 / 226).
+  const int64_t windows = ((int64_t)s.Cmax + kKbMinKeys - 1) / kKbMinKeys;
+  if (est_work(s.S, s.E, s.Q) < 2 * kMinWork &&
+      windows * (600 + 4 * std::min<int64_t>(s.Q, 100 * (int64_t)s.S) + s.E / 2) < 9000)
+    return false;
   k = KbSpec();
   k.S = s.S; k.C = s.Cmax; k.E = s.E; k.Q = s.Q;
-  // about four blocks per sweep CTA, larger ones where the rows would
+  // At last few events with many queries: one CTA works off the probes of a key block, some
+  // 2 ns each (less where the block's points are one tile), and the state-block path's time goes
+  // by its domain, its carry rows and the queries of one state.  1,000 events (two key blocks), state
+  // blocks / key blocks, us: 300 states, 262,145 keys, 50,000 queries 226 / 394, 200,000 305 / 681, 3M
+  // 1,082 / 6,193; 600,000 keys 401 / 380, 637 / 682, 1,925 / 6,409; 4M keys 3,212 / 398, 2,001 / 680,
+  // 6,062 / 6,183; one state, 305 events, 393,917 queries, 1.4M keys 3,910 / 1,712; 43,129 states, 426
+  // events, 1.1M queries, 3.9M keys 6,092 / 4,600.  (With 30,000 events, 59 blocks, key blocks take
+  // 279 to 564 us where 1,000 are given, state blocks 217 to 6,148.)  The factors are the ones that
+  // took the slower path for none of 300 random shapes of 1 to 100,000 events.
+  // Before that, about four blocks per sweep CTA, larger ones where the rows would
   // not fit.  Never more scratch than twice the state-block pipeline's or 32 MiB, and nothing
   // that fits the allocation-free entry's 32 MiB there may outgrow them here.
   const size_t small = (size_t)32 << 20;
@@ -785,7 +803,9 @@ bool kb_select(const BwReplayArgs* a, const PipeSpec& s, size_t general_bytes, K
     k.m = (int32_t)steps * kKbSlotStep;
     if (s.E / k.m + 1 > kKbMaxBlocks) continue;
     kb_layout(s, k);
-    if (k.total <= limit) return true;
+    if (k.total <= limit)
+      return 2 * s.Q / k.B * std::min<int64_t>(s.E, 8) / 8 <=
+             s.Cmax / 3 + s.carry_words / 320 + windows * (s.Q / s.S);
   }
   return false;
 }

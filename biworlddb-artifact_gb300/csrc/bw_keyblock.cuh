@@ -14,7 +14,12 @@ constexpr int kKbMaxSlots = 16 * kKbSlotStep; // ... and at most 8,192 (64 KB of
 constexpr int kSwCtas = 3;                    // sweep CTAs per SM
 constexpr int kKbPtTile = 4096;               // points per partition tile
 constexpr int kKbPrTile = 4096;               // queries per partition tile (two probes each)
-constexpr uint32_t kKbMinKeys = 1u << kWinBits;   // smaller domains stay with the state-block pipeline
+// Domains up to kKbMinKeys (one window of the state-block path) stay with the state-block
+// pipeline.  Around the line the two
+// paths are close where there is work for both: 30,000 states, state blocks / key blocks, us, 262,145
+// keys: 1M events, 1M queries 939 / 952, 10M events, 10,000 queries 1,492 / 2,832; 600,000 keys 1,984 /
+// 956 and 2,518 / 2,840; 300 states, 262,145 keys 880 / 585 and 3,350 / 2,796.
+constexpr uint32_t kKbMinKeys = 1u << kWinBits;
 
 enum {
   KB_SOFF, KB_TEOFF, KB_TQOFF, KB_TC, KB_TBOFF, KB_TBITS, KB_TCARRY, KB_TGSUM, KB_LASTQ, KB_TTOFF, KB_MISC, KB_EOFF, KB_QOFF,
