@@ -77,13 +77,14 @@ struct KbParams {
   KbCut* cut;           // segs + 1
   int64_t* rows;        // columns x Bs
   uint32_t *prhist, *proff;
+  uint32_t* more;       // B + 1: parts of the key blocks before this one, beyond one each
   uint2* prs;           // {query in tour order, slot | lower bound << 31}
   unsigned long long* acc;   // per query in tour order
   const int32_t* status;
   int32_t* ticket;
   int64_t E, Q, pt_tiles, pr_tiles;
   int32_t S, B, Bs, segs;   // Bs: B rounded up to whole 32-byte sectors of a row
-  uint32_t C, m;
+  uint32_t C, m, part;  // part: probes that a CTA of the sweep takes at a time (whole pages)
 };
 
 // Tour steps of state v's enter and exit (one tree: the tour ends at step 2S).
@@ -196,10 +197,11 @@ __global__ void __launch_bounds__(128) k_kb_start_sum(const uint32_t* __restrict
   for (int64_t t = t0; t < t1; ++t) s += hist[t * B + d];
   part[(int64_t)blockIdx.y * B + d] = s;
 }
-__global__ void __launch_bounds__(1024) k_kb_start_scan(uint32_t* part, int32_t B, uint32_t* off,
-                                                        const int32_t* status) {
+// `more` (probes): the parts of `per` items that each digit takes beyond its first, as starts.
+__global__ void __launch_bounds__(1024) k_kb_start_scan(uint32_t* part, int32_t B, uint32_t* off, uint32_t* more,
+                                                        uint32_t per, const int32_t* status) {
   if (*status) return;
-  uint32_t carry = 0;
+  uint32_t carry = 0, parts = 0;
   for (int32_t d0 = 0; d0 < B; d0 += 1024) {
     const int32_t d = d0 + threadIdx.x;
     uint32_t n = 0, total = 0;
@@ -218,8 +220,16 @@ __global__ void __launch_bounds__(1024) k_kb_start_scan(uint32_t* part, int32_t 
       }
     }
     carry += total;
+    if (more) {
+      const uint32_t before = block_exclusive_scan<uint32_t>(n ? (n - 1) / per : 0, &total);
+      if (d < B) more[d] = parts + before;
+      parts += total;
+    }
   }
-  if (threadIdx.x == 0) off[B] = carry;
+  if (threadIdx.x == 0) {
+    off[B] = carry;
+    if (more) more[B] = parts;
+  }
 }
 __global__ void __launch_bounds__(128) k_kb_start_apply(uint32_t* __restrict__ hist, int32_t B, int64_t tiles,
                                                         const uint32_t* __restrict__ part, const int32_t* status) {
@@ -558,7 +568,16 @@ __global__ void __launch_bounds__(kPrThreads) k_kb_probe_scatter(KbParams p) {
 }
 
 // ------------------------------------------------------------------ sweep
-// One key block at a time per CTA: its points (signed deltas at slots) and probes
+// One key block at a time per CTA, or a part of its probes where it has many more than an
+// equal share (a key that most queries name, intervals over the whole domain, few key blocks): every part replays
+// the block's points from the first on, which costs it the tiles' barriers, so a part is
+// 32 probes a slot and more (half the time of its probes).  30,000 states, 1M events over 300,000
+// keys, 5M queries: all on one key 21.6 -> 0.84 ms a replay, all over the whole domain 10.2 ->
+// 0.80, uniform 1.18 -> 1.12; 100,000 states, 20M events over 10M keys, 50M Zipf point queries 56 ->
+// 11.3, uniform 11.9; 300 states, 1,000 events (two key blocks) over 262,145 keys, 3M queries 6.2 -> 0.39.
+// (Parts of half an equal share whatever the slots: 10M events, 5M queries, Zipf keys 4.76 -> 5.04.)
+//
+// The block's points (signed deltas at slots) and probes
 // (prefixes over the slots), both in tour order.  The points before the current tile
 // of 32 are held as a prefix structure over the slots: T0[s] = sum of the slots below s
 // in s's group of 32, T1 = sum of the groups below.  A probe reads one of each and adds
@@ -580,6 +599,7 @@ struct KbSweepSmem {
   uint4 pt[kSwRing][32];                     // by tile mod kSwRing: {time, slot, delta}
   unsigned long long T1[kKbMaxSlots / 32];
   int32_t block;
+  uint32_t part;
 };
 __device__ __forceinline__ void kb_copy16(void* dst, const void* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
@@ -613,12 +633,27 @@ __global__ void __launch_bounds__(kSwThreads, kSwCtas) k_kb_sweep(KbParams p) {
   const uint32_t g = p.m / kKbSlotStep, span = g * 32, first = warp * span;   // groups, slots, first slot of a warp
   for (;;) {
     __syncthreads();
-    if (tid == 0) sm.block = atomicAdd(p.ticket, 1);
+    if (tid == 0) {
+      // the blocks' first parts, then the others
+      int32_t b = atomicAdd(p.ticket, 1);
+      uint32_t part = 0;
+      if (b >= p.B) {
+        const uint32_t e = (uint32_t)(b - p.B);
+        b = p.B;
+        if (e < p.more[p.B]) {
+          b = first_after(0, p.B, [&](int32_t x) { return p.more[x + 1] > e; });
+          part = 1 + e - p.more[b];
+        }
+      }
+      sm.block = b;
+      sm.part = part;
+    }
     __syncthreads();
     const int32_t b = sm.block;
     if (b >= p.B) break;
-    const uint32_t p0 = p.ptoff[b], p1 = p.ptoff[b + 1], q1 = p.proff[b + 1];
-    uint32_t page = p.proff[b];
+    const uint32_t p0 = p.ptoff[b], p1 = p.ptoff[b + 1];
+    uint32_t page = p.proff[b] + sm.part * p.part;
+    const uint32_t q1 = min(p.proff[b + 1], page + p.part);   // (probes stay below 2^31, parts below 2^30)
     if (p0 == p1 || page == q1) continue;
     const uint32_t nt = (p1 - p0 + 31) / 32;
     for (uint32_t i = tid; i < p.m / 2; i += kSwThreads) reinterpret_cast<uint4*>(T0)[i] = make_uint4(0, 0, 0, 0);
@@ -742,6 +777,7 @@ void kb_layout(const PipeSpec& s, KbSpec& k) {
   take(KB_ROWS, cols * ((B + 3) & ~(size_t)3) * 8);
   take(KB_PRHIST, B * (size_t)k.pr_tiles * 4);
   take(KB_PROFF, (B + 1) * 4);
+  take(KB_MORE, (B + 1) * 4);
   take(KB_PART, kStartChunks * B * 4);
   take(KB_PRS, 2 * (size_t)s.Q * 8);
   take(KB_ACC, (size_t)s.Q * 8);
@@ -784,16 +820,7 @@ bool kb_select(const BwReplayArgs* a, const PipeSpec& s, size_t general_bytes, K
     return false;
   k = KbSpec();
   k.S = s.S; k.C = s.Cmax; k.E = s.E; k.Q = s.Q;
-  // At last few events with many queries: one CTA works off the probes of a key block, some
-  // 2 ns each (less where the block's points are one tile), and the state-block path's time goes
-  // by its domain, its carry rows and the queries of one state.  1,000 events (two key blocks), state
-  // blocks / key blocks, us: 300 states, 262,145 keys, 50,000 queries 226 / 394, 200,000 305 / 681, 3M
-  // 1,082 / 6,193; 600,000 keys 401 / 380, 637 / 682, 1,925 / 6,409; 4M keys 3,212 / 398, 2,001 / 680,
-  // 6,062 / 6,183; one state, 305 events, 393,917 queries, 1.4M keys 3,910 / 1,712; 43,129 states, 426
-  // events, 1.1M queries, 3.9M keys 6,092 / 4,600.  (With 30,000 events, 59 blocks, key blocks take
-  // 279 to 564 us where 1,000 are given, state blocks 217 to 6,148.)  The factors are the ones that
-  // took the slower path for none of 300 random shapes of 1 to 100,000 events.
-  // Before that, about four blocks per sweep CTA, larger ones where the rows would
+  // About four blocks per sweep CTA, larger ones where the rows would
   // not fit.  Never more scratch than twice the state-block pipeline's or 32 MiB, and nothing
   // that fits the allocation-free entry's 32 MiB there may outgrow them here.
   const size_t small = (size_t)32 << 20;
@@ -803,9 +830,7 @@ bool kb_select(const BwReplayArgs* a, const PipeSpec& s, size_t general_bytes, K
     k.m = (int32_t)steps * kKbSlotStep;
     if (s.E / k.m + 1 > kKbMaxBlocks) continue;
     kb_layout(s, k);
-    if (k.total <= limit)
-      return 2 * s.Q / k.B * std::min<int64_t>(s.E, 8) / 8 <=
-             s.Cmax / 3 + s.carry_words / 320 + windows * (s.Q / s.S);
+    if (k.total <= limit) return true;
   }
   return false;
 }
@@ -840,11 +865,14 @@ int kb_enqueue(const KbSpec& k, const PipeSpec& spec, const BwReplayArgs* a, Eve
   p.colstate = (int32_t*)at(KB_COLSTATE); p.coltime = (uint32_t*)at(KB_COLTIME); p.colstep = (int32_t*)at(KB_COLSTEP);
   p.pos = (uint32_t*)at(KB_POS); p.pthist = (uint32_t*)at(KB_PTHIST); p.pts = (uint4*)at(KB_PTS);
   p.tour = (uint4*)at(KB_TOUR); p.ptoff = (uint32_t*)at(KB_PTOFF); p.proff = (uint32_t*)at(KB_PROFF);
+  p.more = (uint32_t*)at(KB_MORE);
   p.seg = (uint64_t*)at(KB_SEG); p.cut = (KbCut*)at(KB_CUT); p.rows = (int64_t*)at(KB_ROWS); p.prhist = (uint32_t*)at(KB_PRHIST);
   p.prs = (uint2*)at(KB_PRS); p.acc = (unsigned long long*)at(KB_ACC);
   p.status = ta.misc + M_STATUS; p.ticket = ta.misc + M_SWEEP_TICKET;
   p.E = k.E; p.Q = k.Q; p.pt_tiles = k.pt_tiles; p.pr_tiles = k.pr_tiles;
   p.S = k.S; p.B = k.B; p.Bs = (k.B + 3) & ~3; p.segs = k.segs; p.C = k.C; p.m = (uint32_t)k.m;
+  const int64_t ctas = (int64_t)kSwCtas * s.sms;
+  p.part = (uint32_t)(std::max<int64_t>(32 * k.m, k.Q / ctas) / kSwThreads + 1) * kSwThreads;
 
   int rc = kb_attrs();
   if (rc) return rc;
@@ -869,11 +897,11 @@ int kb_enqueue(const KbSpec& k, const PipeSpec& spec, const BwReplayArgs* a, Eve
     return report((cudaError_t)rc, "scan");
   if ((rc = mark(3))) return rc;
   uint32_t* part = (uint32_t*)at(KB_PART);
-  auto starts = [&](uint32_t* hist, int64_t tiles, uint32_t* off) -> int {
+  auto starts = [&](uint32_t* hist, int64_t tiles, uint32_t* off, uint32_t* more) -> int {
     const dim3 g((unsigned)((k.B + 127) / 128), kStartChunks);
     k_kb_start_sum<<<g, 128, 0, st>>>(hist, k.B, tiles, part, p.status);
     if ((rc = chk("k_kb_start_sum"))) return rc;
-    k_kb_start_scan<<<1, 1024, 0, st>>>(part, k.B, off, p.status);
+    k_kb_start_scan<<<1, 1024, 0, st>>>(part, k.B, off, more, p.part, p.status);
     if ((rc = chk("k_kb_start_scan"))) return rc;
     k_kb_start_apply<<<g, 128, 0, st>>>(hist, k.B, tiles, part, p.status);
     return chk("k_kb_start_apply");
@@ -882,7 +910,7 @@ int kb_enqueue(const KbSpec& k, const PipeSpec& spec, const BwReplayArgs* a, Eve
   while ((1 << bits) < k.B) ++bits;
   k_kb_points<<<(unsigned)k.pt_tiles, 256, (size_t)k.B * 4, st>>>(p);
   if ((rc = chk("k_kb_points"))) return rc;
-  if ((rc = starts(p.pthist, k.pt_tiles, p.ptoff))) return rc;
+  if ((rc = starts(p.pthist, k.pt_tiles, p.ptoff, nullptr))) return rc;
   k_kb_point_scatter<<<(unsigned)k.pt_tiles, kPtWarps * 32, kb_scatter_smem(k.B), st>>>(p, bits);
   if ((rc = chk("k_kb_point_scatter"))) return rc;
   if ((rc = mark(4))) return rc;
@@ -895,11 +923,11 @@ int kb_enqueue(const KbSpec& k, const PipeSpec& spec, const BwReplayArgs* a, Eve
   if ((rc = mark(5))) return rc;
   k_kb_probe_count<<<(unsigned)k.pr_tiles, 512, (size_t)k.B * 4, st>>>(p);
   if ((rc = chk("k_kb_probe_count"))) return rc;
-  if ((rc = starts(p.prhist, k.pr_tiles, p.proff))) return rc;
+  if ((rc = starts(p.prhist, k.pr_tiles, p.proff, p.more))) return rc;
   static_assert((size_t)kKbMaxBlocks * 4 <= kPrSmem, "probe scatter shared memory");
   k_kb_probe_scatter<<<(unsigned)k.pr_tiles, kPrThreads, kPrSmem, st>>>(p);
   if ((rc = chk("k_kb_probe_scatter"))) return rc;
-  k_kb_sweep<<<std::min(k.B, kSwCtas * s.sms), kSwThreads, (size_t)k.m * 8, st>>>(p);
+  k_kb_sweep<<<(unsigned)std::min<int64_t>(k.B + 2 * k.Q / p.part, ctas), kSwThreads, (size_t)k.m * 8, st>>>(p);
   if ((rc = chk("k_kb_sweep"))) return rc;
   k_kb_answers<<<(unsigned)k.pr_tiles, 256, 0, st>>>(p);
   if ((rc = chk("k_kb_answers"))) return rc;

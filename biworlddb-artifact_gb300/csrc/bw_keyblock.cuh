@@ -25,7 +25,7 @@ enum {
   KB_SOFF, KB_TEOFF, KB_TQOFF, KB_TC, KB_TBOFF, KB_TBITS, KB_TCARRY, KB_TGSUM, KB_LASTQ, KB_TTOFF, KB_MISC, KB_EOFF, KB_QOFF,
   KB_FORK, KB_NEXT, KB_CNT, KB_EHEAD, KB_XHEAD, KB_RANK, KB_SCAN, KB_STEP, KB_W, KB_EP, KB_TIME, KB_COLSTATE,
   KB_COLTIME, KB_COLSTEP, KB_POS, KB_TOUR, KB_PTHIST, KB_PTOFF, KB_PTS, KB_SEG, KB_CUT, KB_ROWS, KB_PRHIST,
-  KB_PROFF, KB_PART, KB_PRS, KB_ACC, KB_COUNT
+  KB_PROFF, KB_MORE, KB_PART, KB_PRS, KB_ACC, KB_COUNT
 };
 
 struct KbSpec {

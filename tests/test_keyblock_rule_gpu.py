@@ -1,5 +1,5 @@
-"""Which path a single tree over a wide key domain takes, and that both agree there: few
-events with many queries and little work at all stay with the state blocks."""
+"""Which path a single tree over a wide key domain takes, and that both agree there: little
+work over few windows of the domain stays with the state blocks."""
 from __future__ import annotations
 
 import numpy as np
@@ -11,15 +11,13 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("S,C,E,Q,key_blocks", [
-    (300, 262_145, 1000, 1_000_000, False),     # two key blocks of a million probes
-    (127, 279_218, 148, 2_398_098, False),
-    (6518, 471_466, 4822, 3_655_433, False),
-    (300, 262_145, 30_000, 1_000_000, True),
-    (300, 4_000_000, 1000, 200_000, True),      # the domain outweighs the probes
+    (300, 262_145, 1000, 1_000_000, True),      # two key blocks of a million probes
+    (127, 279_218, 148, 2_398_098, True),
+    (6518, 471_466, 4822, 3_655_433, True),
     (300, 262_145, 1000, 100, False),           # one state block
     (1, 609_353, 23, 229, False),
-    (1, 4_000_000, 2, 3, True),
-    (1, 387_896, 3, 628_384, True),             # one state asked everything
+    (1, 4_000_000, 2, 3, True),                 # sixteen windows
+    (1, 387_896, 3, 628_384, True),
     (40_000, 300_000, 1, 2000, True),
 ])
 def test_route(bw, torch_cuda, oracle_mod, S, C, E, Q, key_blocks):
