@@ -260,28 +260,50 @@ __device__ __forceinline__ int64_t csr_rank(const BwCsr& x, int64_t m, uint64_t 
   return lo;
 }
 
-// Lookup inputs and outputs are streamed (evict first): they are read or written once,
-// and the L2 is left to the index.
-__device__ __forceinline__ ulonglong2 stream_ld(const ulonglong2* p) { return __ldcs(p); }
+// Lookup inputs and outputs are streamed (evict first, `Once`): they are read or written once,
+// and the L2 is left to the index.  Only where they and the LUT are more than kOnceBytes: smaller
+// ones come from and go to kernels beside this one through the L2 (3M points, 64 KiB LUT, streamed / not,
+// us: 3 keys 19.2 / 17.5, 15,000 keys 22.6 / 21.4, 10M keys 93.3 / 93.1; 64 MiB, 10M keys 39.7 / 41.5).
+constexpr int64_t kOnceBytes = (int64_t)64 << 20;
+template <bool Once, typename T>
+__device__ __forceinline__ T lookup_ld(const T* p) {
+  if constexpr (Once) return __ldcs(p);
+  else return *p;
+}
+template <bool Once, typename T>
+__device__ __forceinline__ void lookup_st(T* p, const T& v) {
+  if constexpr (Once) __stcs(p, v);
+  else *p = v;
+}
 
-template <bool V4>
-__global__ void k_csr_point(BwCsr x, const uint64_t* __restrict__ keys, int64_t n, int64_t* __restrict__ out) {
-  const int64_t m = *x.count;
+template <bool V4, bool Once>
+__device__ __forceinline__ void csr_points(const BwCsr& x, int64_t m, const uint64_t* __restrict__ keys, int64_t n,
+                                           int64_t* __restrict__ out) {
   const int64_t npairs = n >> 1;
   const ulonglong2* kv = reinterpret_cast<const ulonglong2*>(keys);
   longlong2* ov = reinterpret_cast<longlong2*>(out);
   for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < npairs; p += (int64_t)gridDim.x * blockDim.x) {
-    const ulonglong2 k = stream_ld(kv + p);
+    const ulonglong2 k = lookup_ld<Once>(kv + p);
     bool pa, pb;
     const int64_t ra = csr_rank<V4>(x, m, k.x, pa);
     const int64_t rb = csr_rank<V4>(x, m, k.y, pb);
-    __stcs(ov + p, make_longlong2(pa ? ra : -ra - 1, pb ? rb : -rb - 1));
+    lookup_st<Once>(ov + p, make_longlong2(pa ? ra : -ra - 1, pb ? rb : -rb - 1));
   }
   if ((n & 1) && blockIdx.x == 0 && threadIdx.x == 0) {
     bool pr;
     const int64_t r = csr_rank<V4>(x, m, keys[n - 1], pr);
     out[n - 1] = pr ? r : -r - 1;
   }
+}
+// The fours gain 3 to 8 % from some thousand keys on; below, and where a small LUT stays in the L1,
+// the selects cost more than the reads save (7M points, singly / in fours, us: 3 keys, 64 KiB LUT
+// 30.2 / 35.7, 4 MiB 33.4 / 37.8; 15,000 keys, 64 KiB 40.7 / 43.9, 4 MiB 57.2 / 51.9; 200,000 keys, 64 KiB
+// 85.2 / 79.1).  The count is known on the device only.
+template <bool V4, bool Once>
+__global__ void k_csr_point(BwCsr x, const uint64_t* __restrict__ keys, int64_t n, int64_t* __restrict__ out) {
+  const int64_t m = *x.count;
+  if (V4 && m >= (x.n_buckets >= (1 << 18) ? 1 << 12 : 1 << 16)) csr_points<V4, Once>(x, m, keys, n, out);
+  else csr_points<false, Once>(x, m, keys, n, out);
 }
 
 // Range lookups.  LUT, low bits and prefix sums together (164 MB for 10M keys and a
@@ -293,7 +315,13 @@ __global__ void k_csr_point(BwCsr x, const uint64_t* __restrict__ keys, int64_t 
 // misses (20M ranges, one pass / two, us: 60,000 keys 403 / 436, 1.5M 427 / 483, 3M 513 /
 // 494, 6M 803 / 524).  The LUT's entries are read one by one here: groups of four (above)
 // cost the large index 5% and gain 2% on the smallest.
-constexpr int kRangeCtas = 6;                       // CTAs of 256 threads an SM holds
+//
+// Calls of up to kRangeMany ranges are launched with the eight CTAs an SM holds, larger ones with six,
+// which leave more of the L1 and the L2 to each other (us, eight / six: 300,000 ranges, 10M keys, 64 MiB
+// LUT 20.9 / 23.2, 3M keys, 4 MiB 13.8 / 14.7; 7M ranges, 10M keys, 4 MiB 330 / 315, 1M keys, 64 KiB 286 /
+// 261; on indexes of a few keys eight stay faster, 46.8 / 50.4, but the count is known on the device only).
+constexpr int kRangeCtas = 8, kRangeFew = 6;        // CTAs of 256 threads, an SM
+constexpr int64_t kRangeMany = 1'000'000;
 constexpr int64_t kSplitKeys = (int64_t)7 << 19;    // 28 MB of prefix sums
 __device__ __forceinline__ longlong2 range_answer(const BwCsr& x, int64_t a, int64_t b) {
   uint64_t sum = 0;
@@ -304,6 +332,7 @@ __device__ __forceinline__ longlong2 range_answer(const BwCsr& x, int64_t a, int
   }
   return make_longlong2(b - a, (int64_t)sum);
 }
+template <bool Once>
 __global__ void __launch_bounds__(256, kRangeCtas) k_csr_range(BwCsr x, const uint64_t* __restrict__ bounds, int64_t n,
                                                               int64_t* out) {
   const int64_t m = *x.count;
@@ -312,16 +341,16 @@ __global__ void __launch_bounds__(256, kRangeCtas) k_csr_range(BwCsr x, const ui
   longlong2* ov = reinterpret_cast<longlong2*>(out);
   const int64_t i0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, step = (int64_t)gridDim.x * blockDim.x;
   for (int64_t i = i0; i < n; i += step) {
-    const ulonglong2 q = stream_ld(bv + i);
+    const ulonglong2 q = lookup_ld<Once>(bv + i);
     bool pr;
     const int64_t a = csr_rank<false>(x, m, q.x, pr);
     const int64_t b = csr_rank<false>(x, m, q.y, pr);
-    __stcs(ov + i, split ? make_longlong2(a, b) : range_answer(x, a, b));
+    lookup_st<Once>(ov + i, split ? make_longlong2(a, b) : range_answer(x, a, b));
   }
   if (!split) return;
   for (int64_t i = i0; i < n; i += step) {
-    const longlong2 r = __ldcs(ov + i);
-    __stcs(ov + i, range_answer(x, r.x, r.y));
+    const longlong2 r = lookup_ld<Once>(ov + i);
+    lookup_st<Once>(ov + i, range_answer(x, r.x, r.y));
   }
 }
 
@@ -524,8 +553,10 @@ extern "C" int bw_csr_point(const BwCsr* idx, const uint64_t* keys, int64_t n, i
   if (check_index(idx) || n < 0 || (n > 0 && (!keys || !out))) return BW_EINVAL;
   if (n == 0) return 0;
   if ((reinterpret_cast<uintptr_t>(keys) & 15) || (reinterpret_cast<uintptr_t>(out) & 15)) return BW_EINVAL;
-  (lut4(idx) ? k_csr_point<true> : k_csr_point<false>)<<<grid_for((n + 1) / 2, 256), 256, 0,
-                                                         static_cast<cudaStream_t>(stream)>>>(*idx, keys, n, out);
+  const bool once = n * 16 + idx->n_buckets * 4 > kOnceBytes;
+  (lut4(idx) ? once ? k_csr_point<true, true> : k_csr_point<true, false>
+             : once ? k_csr_point<false, true> : k_csr_point<false, false>)<<<
+      grid_for((n + 1) / 2, 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(*idx, keys, n, out);
   return report(cudaGetLastError(), "k_csr_point");
 }
 
@@ -534,8 +565,10 @@ extern "C" int bw_csr_range(const BwCsr* idx, const uint64_t* bounds, int64_t n,
   if (n == 0) return 0;
   if ((reinterpret_cast<uintptr_t>(bounds) & 15) || (reinterpret_cast<uintptr_t>(out) & 15)) return BW_EINVAL;
   const cudaStream_t st = static_cast<cudaStream_t>(stream);
+  const bool once = n * 32 + idx->n_buckets * 4 > kOnceBytes;
   // no more CTAs than are resident at once
-  k_csr_range<<<std::min(grid_for(n, 256), sm_count() * kRangeCtas), 256, 0, st>>>(*idx, bounds, n, out);
+  (once ? k_csr_range<true> : k_csr_range<false>)<<<
+      std::min(grid_for(n, 256), sm_count() * (n <= kRangeMany ? kRangeCtas : kRangeFew)), 256, 0, st>>>(*idx, bounds, n, out);
   return report(cudaGetLastError(), "k_csr_range");
 }
 
