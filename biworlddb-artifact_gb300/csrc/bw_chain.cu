@@ -903,10 +903,15 @@ int chain_spec(const BwReplayArgs* a, int sms, ChainSpec& s) {
   int64_t B = (s.E + kChainMinBlockEvents - 1) / kChainMinBlockEvents;
   int64_t floor = B;
   // few events: one block per SM when every block still gets 512 events or more (25,000
-  // events: 12 blocks 25 us a replay, 48 blocks 21 us)
+  // events: 12 blocks 25 us a replay, 48 blocks 21 us); but a single block, without carry and
+  // fix-up, up to some 4,000 events, a query counted as 16 and sixteen keys of a row as one (1 / 4
+  // blocks, us: 2,200 events, 1 query, 100 keys 11.8 / 13.9, 32,000 keys 31.4 / 45.3; 45 queries, 10,000
+  // keys 23.1 / 27.0; 2,200 queries, 100 keys 198 / 60; 4,400 events, 1 query, 100 keys 13.9 / 14.3, 32,000
+  // keys 33.4 / 45.8; 8,800 events, 32,000 keys 73 / 47)
   if (few && B < sms) {
     floor = std::min<int64_t>(sms, std::max<int64_t>(B, s.E / 2048));
     B = std::min<int64_t>(sms, std::max<int64_t>(B, s.E / 512));
+    if (s.E + 16 * s.Q < 4096 + (int64_t)s.C / 16) B = 1;
   } else if (pair) {
     floor = std::min<int64_t>(B, sms);
   }
@@ -955,7 +960,7 @@ int chain_enqueue(const ChainSpec& s, const BwReplayArgs* a, EventSet* evs, int*
   p.C = s.C;
   p.B = s.B;
   p.nch = s.nch;
-  p.qweight = s.Q * kQueryWeight > s.E ? kQueryWeight : 0;
+  p.qweight = s.B > 1 && s.Q * kQueryWeight > s.E ? kQueryWeight : 0;   // (one block has nothing to cut)
   p.rows = reinterpret_cast<int64_t*>(ws + s.off_rows);
   p.wide = reinterpret_cast<int64_t*>(ws + s.off_wide);
   p.btab = reinterpret_cast<int64_t*>(ws + s.off_btab);
