@@ -252,13 +252,20 @@ __device__ int64_t first_query_at_or_after(const BwQuery* qs, int64_t Q, uint32_
 // CTA, one probe of each per thread and round; ascending in b for sorted input, inside
 // [0, E] for any (so every event is in some block even then).
 __device__ void weighted_cut(const ChainParams& p, int64_t b, int64_t (&e)[2]) {
-  const int64_t K = p.qweight, work = p.E + K * p.Q, nt = blockDim.x;
+  const int64_t K = p.qweight, nt = blockDim.x;
+  // queries after the last event belong to the last block whatever the cut, and cost it little: they are
+  // left out where they are many (1M events, 441,437 queries all on the last state, 17 blocks: 1.14 ms, 3.75
+  // with them counted, as the events then went into two blocks)
+  int64_t Q = p.Q;
+  const uint32_t end = p.ev[p.E - 1].x;
+  if (p.qs[Q - 1 - Q / 16].state >= end) Q = first_query_at_or_after(p.qs, Q, end);
+  const int64_t work = p.E + K * Q;
   int64_t target[2], hi[2];
   bool done[2];
 #pragma unroll
   for (int i = 0; i < 2; ++i) {
     target[i] = work / p.B * (b + i) + work % p.B * (b + i) / p.B;
-    e[i] = max((int64_t)0, target[i] - K * p.Q);
+    e[i] = max((int64_t)0, target[i] - K * Q);
     hi[i] = min(target[i], p.E);
     done[i] = false;
   }
@@ -270,7 +277,7 @@ __device__ void weighted_cut(const ChainParams& p, int64_t b, int64_t (&e)[2]) {
       before[i] = false;
       if (pos < hi[i]) {
         const int64_t q = (target[i] - pos) / K;
-        before[i] = q >= p.Q || p.ev[pos].x <= p.qs[q].state;
+        before[i] = q >= Q || p.ev[pos].x <= p.qs[q].state;
       }
     }
 #pragma unroll
