@@ -110,9 +110,26 @@ __device__ __forceinline__ void warp_range(int64_t n, int64_t& lo, int64_t& hi) 
   lo = imin64(n, w * per);
   hi = imin64(n, lo + per);
 }
+// Last tree from t on that starts at or before x (off[t] <= x): tree by tree where every tree has
+// states and x is 32 states on; by doubling steps and bisection (tree_seek) where the next item's
+// tree may be far (1,931 trees, 294 queries: ingest 131 -> 21 us).
 template <typename Off>
 __device__ __forceinline__ int32_t tree_forward(const Off* off, int32_t T, int32_t t, int64_t x) {
   while (t + 1 < T && (int64_t)off[t + 1] <= x) ++t;
+  return t;
+}
+template <typename Off>
+__device__ __forceinline__ int32_t tree_seek(const Off* off, int32_t T, int32_t t, int64_t x) {
+  int32_t step = 1;
+  while (step < T - t && (int64_t)off[t + step] <= x) {
+    t += step;
+    step = min(2 * step, T);
+  }
+  int32_t hi = min(t + step, T);
+  while (t + 1 < hi) {
+    const int32_t mid = (t + hi) >> 1;   // (trees stay below 2^30)
+    if ((int64_t)off[mid] <= x) t = mid; else hi = mid;
+  }
   return t;
 }
 
@@ -158,9 +175,10 @@ __global__ void __launch_bounds__(256) k_offsets(const void* items, int64_t n, T
   const BwQuery* qs = static_cast<const BwQuery*>(items);
   const int lane = threadIdx.x & 31;
   // items a warp takes at a time: few, so that long runs of states without items do not
-  // meet in one warp, but enough for the tree search at their start
+  // meet in one warp, but enough for the tree search at their start (few items: 32, so that groups
+  // across many trees are not worked off one after the other)
   const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
-  const int64_t chunk = kEvents ? imin64(2048, (n / (4 * warps) + 128) & ~(int64_t)127) : 128;
+  const int64_t chunk = n <= 32 * warps ? 32 : kEvents ? imin64(2048, (n / (4 * warps) + 128) & ~(int64_t)127) : 128;
   struct Rec { uint32_t s, a; };   // state; key, or the larger bound
   auto load = [&](int64_t i) -> Rec {
     Rec r;
@@ -179,7 +197,7 @@ __global__ void __launch_bounds__(256) k_offsets(const void* items, int64_t n, T
   int32_t s0 = 0, ns = 0;
   uint32_t amax = 0;   // largest key, or bound
   auto enter = [&](int64_t i) {
-    if (T > 1) t = tree_forward(toff, T, t, i);
+    if (T > 1) t = tree_seek(toff, T, t, i);
     tend = toff[t + 1];
     s0 = tt.soff[t];
     ns = tt.soff[t + 1] - s0;
@@ -222,7 +240,7 @@ __global__ void __launch_bounds__(256) k_offsets(const void* items, int64_t n, T
         const bool valid = i < hi;
         int32_t g = -2;
         if (valid) {
-          const int32_t tr = T > 1 ? tree_forward(toff, T, t, i) : 0;
+          const int32_t tr = T > 1 ? tree_seek(toff, T, t, i) : 0;
           const Rec x = load(i);
           if (x.a > tt.C[tr] - (kEvents ? 1u : 0u))
             set_status(status, kEvents ? BW_STATUS_EVENT_KEY_RANGE : BW_STATUS_QUERY_RANGE);
