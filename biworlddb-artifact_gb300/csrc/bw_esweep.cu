@@ -67,13 +67,21 @@ constexpr int kEsQW = kEsQB / kEsNWC;      // queries per consumer warp per tile
 // 4.66 ms with one level above 4,096 entries, 4.35 ms so.
 constexpr uint32_t kEsFlat = 256;
 constexpr uint32_t kEsDeep = 4096;
+// Blocks with a step of kHotQueries and more (found by the prepare pass) are left to a second kernel
+// (`Hot`), in which a step's queries past its first tile, where they are kEsMore or more, are one
+// tile of their own, answered a thread per query (es_more).  As tiles of 60 queries they took 2.3 us
+// each: 30,000 states, 1M events, 360,000 queries, half of them on one state 7.36 -> 0.99 ms a replay (256
+// threads and Fenwick nodes, 1.18), 300,000 states, 3.6M queries 63.1 -> 5.1 (8.9).  A kernel of its own, as the
+// code for it cost the other tiles 3 to 8 % through their registers (1 % so, for the launch).
+constexpr int kEsMore = kHotQueries - 60;
 constexpr int kEsRing = 256;               // planner's descriptor ring (steps)
 constexpr uint32_t kEsWaitLimit = 1u << 22;
 constexpr uint32_t kFull = 0xffffffffu;
 
 struct EsMeta {
   int32_t nf, nb, nq, last;   // front (enter) events, back (exit) events, queries, last tile of the pass
-};
+};                            // (last & kLastMore: a tile of queries only, nb of them from nf on)
+constexpr int32_t kLastMore = 2;
 struct EsCtl {
   int32_t ticket, abort, pad0, pad1;
 };
@@ -198,10 +206,10 @@ __device__ __forceinline__ void pbar_sync(int id) { asm volatile("bar.sync %0, 6
 
 struct EsPlanMeta {
   uint32_t nq;     // queries of the tile before the batch | after it << 16
-  uint32_t flags;  // 1: the batch ends its tile, 2: it ends the pass
-  uint32_t nf, nb; // the tile's front and back events after the batch
+  uint32_t flags;  // 1: the batch ends its tile, 2: it ends the pass, 4: a tile of queries only
+  uint32_t nf, nb; // the tile's front and back events after the batch (4: first query, queries)
 };
-constexpr uint32_t kPlanTileEnd = 1, kPlanPassEnd = 2;
+constexpr uint32_t kPlanTileEnd = 1, kPlanPassEnd = 2, kPlanMore = 4;
 
 // The planner's cursor: step ct with its first coe events and coq queries already
 // taken; the descriptors of steps below wb have been requested into the ring (slot
@@ -241,6 +249,7 @@ __device__ __forceinline__ uint4 es_rec(uint32_t src, uint32_t q0, int32_t te, b
 
 // Planner: every batch of the pass, tiles cut at kEsTile events or kEsQB queries.
 // On an abort it ends the pass with an empty plan so that the issuer stops too.
+template <bool Hot>
 __device__ void es_plan(const EsParams& p, const EsPass& ps, uint4* ring, uint4* plan, EsPlanMeta* pmeta,
                         const EsCtl* ctl, int lane) {
   EsCursor c;
@@ -248,12 +257,20 @@ __device__ void es_plan(const EsParams& p, const EsPass& ps, uint4* ring, uint4*
   const int32_t t1 = ps.t1;
   int32_t nf = 0, nb = 0, nq = 0;   // the tile so far: front (enter) events, back (exit) events, queries
   uint32_t pb = 0;                  // batches planned in this pass
+  uint32_t left = 0, left_q0 = 0;   // (Hot) queries left of step ct, from left_q0 on, where they are a tile of their own
   for (;;) {
     const bool stop = *reinterpret_cast<const volatile int32_t*>(&ctl->abort) != 0;
     uint4 rec0 = make_uint4(0, 0, 0, 0), rec1 = rec0;
     uint32_t flags = 0, nq0 = (uint32_t)nq;
+    uint32_t more = 0;
     if (stop) {
       flags = kPlanTileEnd | kPlanPassEnd;
+    } else if (Hot && left) {   // the cut step's other queries (its tile ended with kEsQB of them)
+      more = left;
+      left = 0;
+      ++c.ct;
+      c.coe = c.coq = 0;
+      flags = kPlanTileEnd | kPlanMore | (c.ct >= t1 ? kPlanPassEnd : 0u);
     } else {
       es_ring_request(p, ring, c, t1, lane);
       es_ring_ready(c, ps.t0);
@@ -328,6 +345,12 @@ __device__ void es_plan(const EsParams& p, const EsPass& ps, uint4* ring, uint4*
         c.coe = (K == 0 ? c.coe : 0) + (int32_t)(kt & 0xffffu);
         c.coq = (K == 0 ? c.coq : 0) + (int32_t)(kt >> 16);
         c.ct += K;
+        if constexpr (Hot) {
+          const int32_t rest = (K & 1) ? (te1 == ne1 ? qn1 - tq1 : 0) : (te0 == ne0 ? qn0 - tq0 : 0);
+          left = (uint32_t)max(__shfl_sync(kFull, rest, K >> 1), 0);
+          left_q0 = __shfl_sync(kFull, (K & 1) ? d1.y + (uint32_t)tq1 : qa0 + (uint32_t)tq0, K >> 1);
+          if (left < kEsMore) left = 0;
+        }
       }
       if (c.ct >= t1) flags = kPlanTileEnd | kPlanPassEnd;
       else if (nf + nb >= kEsTile || nq >= kEsQB) flags = kPlanTileEnd;
@@ -339,6 +362,7 @@ __device__ void es_plan(const EsParams& p, const EsPass& ps, uint4* ring, uint4*
     if (lane == 0) {
       EsPlanMeta m;
       m.nq = nq0 | ((uint32_t)nq << 16); m.flags = flags; m.nf = (uint32_t)nf; m.nb = (uint32_t)nb;
+      if (Hot && more) { m.nf = left_q0; m.nb = more; }
       pmeta[b] = m;
     }
     pbar_arrive(kBarPlanFull + b);
@@ -363,6 +387,7 @@ __device__ __forceinline__ int es_next_break(uint32_t b0, uint32_t b1, int lane,
 // Issuer: turns the plans of a pass into stage copies, query records and stage
 // metadata, one tile per stage.  `cnt` counts tiles (the consumers' sequence).
 // Returns false when a wait for a free stage was lost (it still reads every plan).
+template <bool Hot>
 __device__ bool es_issue(const EsParams& p, unsigned char* sm, const uint4* plan, const EsPlanMeta* pmeta,
                          uint32_t& cnt, int lane) {
   constexpr EsSmem L = es_smem();
@@ -452,7 +477,7 @@ __device__ bool es_issue(const EsParams& p, unsigned char* sm, const uint4* plan
           mt->nf = (int32_t)m.nf;
           mt->nb = (int32_t)m.nb;
           mt->nq = (int32_t)(m.nq >> 16);
-          mt->last = (m.flags & kPlanPassEnd) ? 1 : 0;
+          mt->last = ((m.flags & kPlanPassEnd) ? 1 : 0) | (Hot && (m.flags & kPlanMore) ? kLastMore : 0);
         }
         // the stage completes when this lane's query copies have landed (the arrive
         // adds one pending arrival now and removes it when the copies complete)
@@ -540,9 +565,107 @@ __device__ __forceinline__ int32_t es_scan_packed(const uint2* pk, uint32_t j0, 
   return s;
 }
 
-// One pass of the consumers over the tiles of a pass.  Returns false on a lost wait.
+// The n queries from q0 on, all asked at the window as it stands: its entries become their
+// exclusive prefix in place (a warp per 32 entries, over prefixes of their totals in the packed tile's
+// place) and are taken apart again afterwards; between, a thread per query, two in flight, reads
+// two of them.
 template <typename HT>
-__device__ bool es_consume(const EsParams& p, const EsPass& ps, unsigned char* sm, uint32_t& cnt, uint32_t& bad) {
+__device__ void es_more(const EsParams& p, const EsPass& ps, unsigned char* sm, uint32_t q0, uint32_t n) {
+  constexpr EsSmem L = es_smem();
+  const uint64_t* bits = reinterpret_cast<const uint64_t*>(sm + L.bits);
+  const uint16_t* rl = reinterpret_cast<const uint16_t*>(sm + L.rl);
+  auto rank_of = [&](uint32_t k) -> uint32_t {   // window entry of a bound inside [klo, khi]
+    if (ps.dense) return k;
+    return k >= ps.khi ? ps.nr : es_rank(bits, rl, k - ps.klo);
+  };
+  HT* H = reinterpret_cast<HT*>(sm + L.H);
+  const HT* T = reinterpret_cast<const HT*>(sm + L.T);
+  HT* P = reinterpret_cast<HT*>(sm + L.pack);   // chunks + 1, then the warps' sums
+  constexpr int kChunks = kEsCap32 * 4 / sizeof(HT) / 32;
+  static_assert((kChunks + 1 + kEsNWC) * sizeof(HT) <= kEsTile * 8 && kChunks < kEsNC, "prefixes of the window");
+  HT* W = P + kChunks + 1;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int nch = (int)((ps.nr + 31) >> 5);
+  HT v = 0;
+  if (tid < nch) {
+    if (ps.nch) {
+      v = T[tid];
+    } else {
+      for (uint32_t k = 32u * tid; k < min(32u * tid + 32u, ps.nr); ++k) v += H[k];
+    }
+  }
+  auto scan = [&](HT x) -> HT {   // inclusive, over the warp
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const HT y = __shfl_up_sync(kFull, x, o);
+      if (lane >= o) x += y;
+    }
+    return x;
+  };
+  const HT incl = scan(v);
+  if (lane == 31) W[warp] = incl;
+  cons_sync();
+  HT before = 0;
+  for (int w = 0; w < warp; ++w) before += W[w];
+  if (tid <= nch) P[tid] = before + incl - v;
+  cons_sync();
+  for (int c = warp; c < nch; c += kEsNWC) {
+    const uint32_t k = 32u * c + lane;
+    const HT x = k < ps.nr ? H[k] : 0;
+    const HT y = P[c] + scan(x) - x;
+    if (k < ps.nr) H[k] = y;
+  }
+  cons_sync();
+  auto prefix = [&](uint32_t r) -> HT { return r < ps.nr ? H[r] : P[nch]; };   // window entries below r
+  constexpr int kU = 2;
+  for (uint32_t i0 = tid; i0 < n; i0 += kU * kEsNC) {
+    uint32_t lo[kU], hi[kU];
+    uint64_t c[kU];
+#pragma unroll
+    for (int u = 0; u < kU; ++u) {
+      const uint32_t i = i0 + u * kEsNC;
+      lo[u] = hi[u] = 0;
+      if (i < n) {
+        const uint32_t* q = reinterpret_cast<const uint32_t*>(p.qs + (q0 + i));
+        lo[u] = __ldg(q + 1);
+        hi[u] = __ldg(q + 2);
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < kU; ++u) {
+      c[u] = 0;
+      if (lo[u] < hi[u]) {
+        if (!ps.first) c[u] = (uint64_t)p.answers[q0 + i0 + u * kEsNC];
+        else if (ps.crow) c[u] = (uint64_t)__ldcg(ps.crow + hi[u]) - (uint64_t)__ldcg(ps.crow + lo[u]);
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < kU; ++u) {
+      const uint32_t i = i0 + u * kEsNC;
+      if (i >= n) break;
+      const uint32_t a = max(lo[u], ps.klo), z = min(hi[u], ps.khi);
+      if (a < z) {
+        const HT x = prefix(rank_of(z)) - prefix(rank_of(a));
+        c[u] += sizeof(HT) == 4 ? (uint64_t)(int64_t)(int32_t)x : (uint64_t)x;
+      }
+      if (ps.first || a < z) p.answers[q0 + i] = (int64_t)c[u];
+    }
+  }
+  cons_sync();
+  for (int c = warp; c < nch; c += kEsNWC) {
+    const uint32_t k = 32u * c + lane;
+    const HT x = k < ps.nr ? H[k] : 0;
+    const HT up = __shfl_down_sync(kFull, x, 1);
+    const HT next = lane == 31 || k + 1 >= ps.nr ? P[c + 1] : up;
+    if (k < ps.nr) H[k] = next - x;
+  }
+}
+
+// One pass of the consumers over the tiles of a pass, or (Hot) up to a tile of queries only: kMore, with
+// the tile still to be released and counted.
+enum { kLost = 0, kDone = 1, kMore = 2 };
+template <bool Hot, typename HT>
+__device__ int es_consume(const EsParams& p, const EsPass& ps, unsigned char* sm, uint32_t& cnt, uint32_t& bad) {
   constexpr EsSmem L = es_smem();
   HT* H = reinterpret_cast<HT*>(sm + L.H);
   HT* T = reinterpret_cast<HT*>(sm + L.T);
@@ -573,10 +696,11 @@ __device__ bool es_consume(const EsParams& p, const EsPass& ps, unsigned char* s
         es_status(p.status, BW_STATUS_TIMEOUT);
         ctl->abort = 1;
       }
-      return false;
+      return kLost;
     }
     if (warp != 0) mbar_wait(&full[s], ph);   // complete: this thread's acquire of the stage
     const EsMeta m = metas[s];
+    if (Hot && (m.last & kLastMore)) return kMore;
     const uint4* tile = stages + (size_t)s * kEsTile;
     const int32_t back = kEsTile - m.nb;      // first exit slot
     uint4 it[kEsEPT];
@@ -696,7 +820,7 @@ __device__ bool es_consume(const EsParams& p, const EsPass& ps, unsigned char* s
       }
     }
     ++cnt;
-    if (m.last) return true;
+    if (m.last) return kDone;
   }
 }
 
@@ -730,7 +854,14 @@ __device__ void es_setup(const EsParams& p, const EsPass& ps, const BlockTab& bt
   cons_sync();
 }
 
+template <bool Hot>
 __global__ void __launch_bounds__(kEsThreads, 1) k_esweep(EsParams p) {
+  if constexpr (Hot) {
+    chain_wait();
+    if (!*p.hot) return;
+  } else if (p.hot) {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // (its CTAs wait for this kernel's end)
+  }
   extern __shared__ __align__(128) unsigned char sm[];
   constexpr EsSmem L = es_smem();
   uint64_t* full = reinterpret_cast<uint64_t*>(sm + L.bar);
@@ -755,14 +886,16 @@ __global__ void __launch_bounds__(kEsThreads, 1) k_esweep(EsParams p) {
   for (;;) {
     __syncthreads();
     if (tid == 0) ctl->ticket = (*reinterpret_cast<volatile int32_t*>(p.status) || ctl->abort) ? p.B
-                                                                                                : atomicAdd(p.ticket, 1);
+                                                                                                : atomicAdd(Hot ? p.hot + 1 : p.ticket, 1);
     __syncthreads();
     const int32_t i = ctl->ticket;
     if (i >= p.B) break;
     const int32_t b = p.order ? p.order[i] : i;
     const BlockTab bt = p.blocks[b];
     if (bt.t0 >= bt.t1) continue;
-    const bool w64 = p.bmode[b] == 0;
+    const int32_t mode = p.bmode[b];
+    if (p.hot && ((mode & kModeHot) != 0) != Hot) continue;
+    const bool w64 = (mode & kMode32) == 0;
     const uint32_t C = bt.C;
     EsPass ps;
     ps.t0 = bt.t0; ps.t1 = bt.t1;
@@ -792,19 +925,31 @@ __global__ void __launch_bounds__(kEsThreads, 1) k_esweep(EsParams p) {
       ps.nsup = ps.nr > kEsDeep ? (int32_t)((ps.nr + 1023) >> 10) : 0;
       ps.first = si == first_si;
       if (warp == kEsNWC) {
-        es_plan(p, ps, ring, plan, pmeta, ctl, lane);
+        es_plan<Hot>(p, ps, ring, plan, pmeta, ctl, lane);
       } else if (producer) {
-        if (!es_issue(p, sm, plan, pmeta, cnt, lane)) aborted = true;
+        if (!es_issue<Hot>(p, sm, plan, pmeta, cnt, lane)) aborted = true;
       } else {
-        bool ok;
+        int r;
         if (w64) {
           es_setup<uint64_t>(p, ps, bt, s, b, sm);
-          ok = es_consume<uint64_t>(p, ps, sm, cnt, bad);
+          r = es_consume<Hot, uint64_t>(p, ps, sm, cnt, bad);
         } else {
           es_setup<int32_t>(p, ps, bt, s, b, sm);
-          ok = es_consume<int32_t>(p, ps, sm, cnt, bad);
+          r = es_consume<Hot, int32_t>(p, ps, sm, cnt, bad);
         }
-        if (!ok) aborted = true;
+        if constexpr (Hot) {
+          while (r == kMore) {
+            const EsMeta mt = reinterpret_cast<const EsMeta*>(sm + L.meta)[cnt % kEsStages];
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&empty[cnt % kEsStages]);
+            if (w64) es_more<uint64_t>(p, ps, sm, (uint32_t)mt.nf, (uint32_t)mt.nb);
+            else es_more<int32_t>(p, ps, sm, (uint32_t)mt.nf, (uint32_t)mt.nb);
+            ++cnt;
+            if (mt.last & 1) r = kDone;
+            else r = w64 ? es_consume<Hot, uint64_t>(p, ps, sm, cnt, bad) : es_consume<Hot, int32_t>(p, ps, sm, cnt, bad);
+          }
+        }
+        if (r == kLost) aborted = true;
       }
       __syncthreads();   // the pass is over in both roles (the window is reset next)
       if (ctl->abort) aborted = true;
@@ -828,12 +973,18 @@ __global__ void __launch_bounds__(kEsThreads, 1) k_esweep(EsParams p) {
 }  // namespace
 
 int esweep_attrs() {
-  return (int)cudaFuncSetAttribute(k_esweep, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)es_smem().bytes);
+  const cudaError_t e = cudaFuncSetAttribute(k_esweep<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)es_smem().bytes);
+  return e != cudaSuccess ? (int)e
+                          : (int)cudaFuncSetAttribute(k_esweep<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                      (int)es_smem().bytes);
 }
 
+// Where p.hot is given: the blocks without a hot step, then those with one.
 int esweep_launch(const EsParams& p, int grid, cudaStream_t st) {
-  k_esweep<<<grid, kEsThreads, es_smem().bytes, st>>>(p);
-  return (int)cudaGetLastError();
+  k_esweep<false><<<grid, kEsThreads, es_smem().bytes, st>>>(p);
+  const cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess || !p.hot) return (int)e;
+  return (int)launch_chained(true, k_esweep<true>, grid, kEsThreads, es_smem().bytes, st, p);
 }
 
 }  // namespace bw

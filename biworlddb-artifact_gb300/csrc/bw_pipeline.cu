@@ -736,6 +736,7 @@ struct PrepParams {
   int32_t* status;
   int32_t* bmode;
   int32_t* ticket;
+  int32_t* hot;            // set where a block has a step of kHotQueries
 };
 
 // Visit the events of the block's steps that matter (f takes the event, whether there is
@@ -757,7 +758,8 @@ constexpr int kPrepBatch = 4;
 constexpr int kHeavySteps = 512;    // (four batches of a warp)
 constexpr int kHeavyList = 96;      // groups left for the end; further ones are done where they occur
 template <typename F>
-__device__ __forceinline__ void for_block_events(const PrepParams& p, int32_t t0, int32_t t1, int mode, F&& f) {
+__device__ __forceinline__ void for_block_events(const PrepParams& p, int32_t t0, int32_t t1, int mode, int32_t& qmax,
+                                                 F&& f) {
   __shared__ int32_t s_heavy[kHeavyList], s_nheavy;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
   // (the callers' barriers separate this from an earlier pass's last read)
@@ -781,6 +783,7 @@ __device__ __forceinline__ void for_block_events(const PrepParams& p, int32_t t0
     bool neg = false, twice = false;
     if (t < t1) {
       neg = d.nq < 0;
+      qmax = max(qmax, d.nq);
       twice = !neg && pt < t1;
       bool keep = true;
       if (neg) keep = pt < t0;                   // entered in this block: keys known, deltas cancel
@@ -886,13 +889,14 @@ __device__ void prepare_block_a(const PrepParams& p, int32_t b, unsigned char* s
   uint64_t* sbits = reinterpret_cast<uint64_t*>(smem);                    // ww words
   uint32_t* srl = reinterpret_cast<uint32_t*>(sbits + p.ww);              // ww + 2
   __shared__ int32_t s_nsl;
-  __shared__ int32_t s_mode;
+  __shared__ int32_t s_mode, s_hot;
 
   const int32_t t0 = bt.t0, t1 = bt.t1;
   uint64_t* gbits = p.bits + bt.bits_off;
   uint32_t* grl = p.rlut + bt.bits_off + b;
   Slice* gsl = p.slices + (size_t)b * p.max_slices;
-  if (threadIdx.x == 0) s_nsl = 0;
+  if (threadIdx.x == 0) s_nsl = s_hot = 0;
+  int32_t qmax = 0;   // queries of the largest step this thread has seen
   uint32_t rank_base = 0;
   uint32_t mass = 0, over = 0;  // per-thread partial of the block's applied |delta| sum
 
@@ -903,7 +907,7 @@ __device__ void prepare_block_a(const PrepParams& p, int32_t b, unsigned char* s
     __syncthreads();
     const uint32_t klo = (uint32_t)w0 << 6;
     const uint32_t khi = (uint32_t)imin64((int64_t)(w0 + ww) << 6, (int64_t)C);
-    for_block_events(p, t0, t1, 0, [&](const uint4& e, bool valid, bool, bool twice) {
+    for_block_events(p, t0, t1, 0, qmax, [&](const uint4& e, bool valid, bool, bool twice) {
       if (valid && e.y - klo < khi - klo) shared_set_bit(sbits, e.y - klo);
       if (w0 == 0) {   // (a missing event's delta is 0)
         // |delta| summed over every application the sweep makes, in 31 bits; bit 31 of
@@ -916,6 +920,7 @@ __device__ void prepare_block_a(const PrepParams& p, int32_t b, unsigned char* s
       }
     });
     if (w0 == 0) {
+      if (qmax >= kHotQueries) s_hot = 1;
       uint64_t tot = 0;
       block_exclusive_scan<uint64_t>((over >> 31) ? 1ull << 31 : (uint64_t)mass, &tot);   // block total
       if (threadIdx.x == 0) s_mode = tot < (1ull << 31) ? 1 : 0;
@@ -957,7 +962,8 @@ __device__ void prepare_block_a(const PrepParams& p, int32_t b, unsigned char* s
     grl[nwords] = rank_base;
     if (s_nsl > p.max_slices) set_status(p.status, BW_STATUS_TOO_MANY_SLICES);
     p.nslices[b] = min(s_nsl, p.max_slices);
-    p.bmode[b] = s_mode;
+    p.bmode[b] = (s_mode ? kMode32 : 0) | (s_hot ? kModeHot : 0);
+    if (s_hot) *p.hot = 1;
   }
   __syncthreads();
 }
@@ -998,7 +1004,7 @@ __device__ void prepare_block_b(const PrepParams& p, int32_t b, unsigned char* s
   const Slice* gsl = p.slices + (size_t)b * p.max_slices;
   const int32_t nsl = p.nslices[b];
   int64_t* row = p.carry + bt.carry_out;
-  const bool h32 = p.bmode[b] != 0;
+  const bool h32 = (p.bmode[b] & kMode32) != 0;
   unsigned* hist32 = reinterpret_cast<unsigned*>(hist_raw);
   unsigned long long* hist64 = reinterpret_cast<unsigned long long*>(hist_raw);
   uint64_t base = 0;  // key prefix at the start of the slice (same in every thread)
@@ -1016,7 +1022,8 @@ __device__ void prepare_block_b(const PrepParams& p, int32_t b, unsigned char* s
     const uint32_t klo = (uint32_t)s.word_lo << 6;
     const uint32_t khi = (uint32_t)imin64((int64_t)s.word_hi << 6, (int64_t)C);
     if (s.n) {
-      for_block_events(p, t0, t1, 1, [&](const uint4& e, bool valid, bool neg, bool) {
+      int32_t qmax = 0;
+      for_block_events(p, t0, t1, 1, qmax, [&](const uint4& e, bool valid, bool neg, bool) {
         if (valid && e.y - klo < khi - klo) {
           const uint32_t r = local_rank(sbits, srl, e.y - klo);
           const uint64_t d = ((uint64_t)e.w << 32) | e.z;
@@ -1148,7 +1155,7 @@ struct SweepParams {
   const int64_t* carry;
   int64_t* answers;
   const int32_t* status;
-  const int32_t* bmode;   // per block: 1 = int32 Fenwick nodes are exact, 0 = int64
+  const int32_t* bmode;   // per block: kMode32 = int32 Fenwick nodes are exact, else int64; kModeHot
   int32_t* ticket;
 };
 
@@ -2414,7 +2421,7 @@ __global__ void __launch_bounds__(Cfg::kThreads, Cfg::kMinBlocks) k_sweep(SweepP
     const int32_t i = s_ticket;
     if (i >= p.B) break;
     const int32_t b = p.order ? p.order[i] : i;
-    if (p.bmode[b]) sweep_block<unsigned, Cfg>(p, L, smem, b);
+    if (p.bmode[b] & kMode32) sweep_block<unsigned, Cfg>(p, L, smem, b);
     else sweep_block<unsigned long long, Cfg>(p, L, smem, b);
   }
 }
@@ -2906,7 +2913,7 @@ int pipe_enqueue(const PipeSpec& s, void* workspace, const int32_t* parent, cons
   pp.bits = reinterpret_cast<uint64_t*>(at(W_BITS)); pp.rlut = reinterpret_cast<uint32_t*>(at(W_RLUT));
   pp.slices = reinterpret_cast<Slice*>(at(W_SLICES)); pp.max_slices = s.max_slices; pp.nslices = reinterpret_cast<int32_t*>(at(W_NSLICES));
   pp.carry = reinterpret_cast<int64_t*>(at(W_CARRY)); pp.status = status; pp.bmode = bmode;
-  pp.ticket = misc + M_PREP_TICKET;
+  pp.ticket = misc + M_PREP_TICKET; pp.hot = misc + M_HOT;
   int occ_a = 0;
   if ((rc = report(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_a, k_prepare<0>, kPrepThreads, asmem),
                    "occupancy")))
@@ -2947,10 +2954,11 @@ int pipe_enqueue(const PipeSpec& s, void* workspace, const int32_t* parent, cons
       ep.order = order; ep.B = B; ep.cap32 = SL.cap32; ep.cap64 = SL.cap64;
       ep.bits = pp.bits; ep.rlut = pp.rlut; ep.slices = pp.slices; ep.max_slices = s.max_slices; ep.nslices = pp.nslices; ep.carry = pp.carry;
       ep.answers = answers; ep.status = status; ep.bmode = bmode; ep.ticket = misc + M_SWEEP_TICKET;
+      ep.hot = s.tile == kTileEulerId && s.Q >= kHotMin ? misc + M_HOT : nullptr;
       if (s.tile == kTileEulerId) rc = report((cudaError_t)esweep_launch(ep, std::min(B, s.sms), st), "k_esweep");
       else rc = report((cudaError_t)qsweep_launch(ep, s.QL, std::min(B, 2 * s.sms), st), "k_qsweep");
       if (rc) return rc;
-      kernels += s.tile == kTileQueryId ? 2 : 1;   // (k_qcarry, k_qsweep)
+      kernels += s.tile == kTileQueryId || ep.hot ? 2 : 1;   // (k_qcarry, k_qsweep; k_esweep, hot blocks)
       if ((rc = mark(6))) return rc;
       if (kernels_out) *kernels_out = kernels;
       return 0;

@@ -121,6 +121,12 @@ constexpr int kTileMaxId = kTileEulerId;   // largest that a forest's tuning may
 constexpr uint32_t kEsCap32 = 27904;
 constexpr uint32_t kEsCap64 = 13952;
 
+// A step asked kHotQueries and more makes its block hot: the Euler-tile sweep leaves such blocks to a
+// second kernel, launched where a forest or tree has kHotMin queries and more.
+constexpr int kHotQueries = 316;
+constexpr int64_t kHotMin = 2048;
+enum { kMode32 = 1, kModeHot = 2 };   // of a block: int32 sums are exact; for the second kernel
+
 // ------------------------------------------------------------------ records
 struct StepDesc {        // one Euler step, 16 bytes
   uint32_t e0;           // first event of the node (global index)
@@ -276,6 +282,7 @@ enum {
 
 // misc words
 enum { M_STATUS = 0, M_PREP_TICKET = 1, M_SWEEP_TICKET = 2, M_CHAIN = 3, M_PREPB_TICKET = 4, M_NODES = 5, M_STEPS = 6,
+       M_HOT = 7, M_HOT_TICKET = 8,
        M_ROUNDS = 32 };  // 64 words
 
 // Stage timing events of one launch: stage i runs from ev[i] to ev[i + 1]; a chain
@@ -338,8 +345,9 @@ struct EsParams {
   const int64_t* carry;
   int64_t* answers;
   int32_t* status;
-  const int32_t* bmode;
+  const int32_t* bmode;   // kMode32 | kModeHot
   int32_t* ticket;
+  int32_t* hot;           // Euler tiles: whether there is a second kernel's work, and its ticket (NULL: all in one)
 };
 int esweep_attrs();   // one-time shared-memory opt-in (cudaError_t as int)
 int esweep_launch(const EsParams& p, int grid, cudaStream_t st);

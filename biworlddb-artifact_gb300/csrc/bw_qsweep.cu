@@ -385,7 +385,7 @@ __global__ void __launch_bounds__(kQsThreads, 2) k_qsweep(EsParams p, int32_t ww
     const int32_t i = s_ticket;
     if (i >= p.B) break;
     const int32_t b = p.order ? p.order[i] : i;
-    if (p.bmode[b]) qs_block<uint32_t>(p, ww, supers, sm, b);
+    if (p.bmode[b] & kMode32) qs_block<uint32_t>(p, ww, supers, sm, b);
     else qs_block<unsigned long long>(p, ww, supers, sm, b);
   }
 }
