@@ -428,8 +428,10 @@ def plain_record(args, bw, dev, name: str, scale: float, steps: int, warmup: int
         e2e = {"value": ws * Q / (ems / 1e3), "unit": "answers/s", "h2d_bytes_per_step": in_bytes,
                "d2h_bytes_per_step": 8 * Q, "ms_per_step": ems}
     peak, peak_kind = measured_peaks()
-    # single trees: the query-step sweep where a state is asked 18 queries and more
-    kernel = "k_chain_sweep" if chain_path else "k_qsweep" if Q >= 18 * S else "k_esweep"
+    # single trees: the query-step sweep where a state is asked 18 queries and more and, below
+    # 20,000 states, a step has work besides (query_steps of bw_pipeline.cuh)
+    query_steps = Q >= 18 * S and (S >= 20_000 or E // 4 + Q >= 60 * S)
+    kernel = "k_chain_sweep" if chain_path else "k_qsweep" if query_steps else "k_esweep"
     sweep_bytes = 16 * E + 20 * Q
     sweep_ms = stage_mean["sweep"]
     achieved = sweep_bytes / (sweep_ms / 1e3) / 1e9

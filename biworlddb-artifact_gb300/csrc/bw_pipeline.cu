@@ -1,7 +1,7 @@
 // bw_pipeline.cu -- GB300 (sm_103a) version-forest replay pipeline.
 //
-// Stages, all enqueued on one stream with no host round trip (kernels and one
-// memset only, so the whole pipeline can be captured in a CUDA graph):
+// Stages, all enqueued on one stream with no host round trip (kernels and memsets
+// only, so the whole pipeline can be captured in a CUDA graph):
 //
 //   1. ingest    k_offsets       per-state [begin,end) ranges of the state-grouped
 //                                event and query arrays, with input validation
@@ -24,10 +24,14 @@
 //   5. carry     k_carry_*       inclusive column scan of each tree's rows: the
 //                                key prefix at every block start
 //                                (batch_engine_v7.hpp:936-945, on the device)
-//   6. sweep     k_sweep         persistent CTAs take blocks from a queue and
-//                                replay each from a zero local prefix structure in
-//                                shared memory; answer = carry(hi) - carry(lo) +
-//                                local(hi) - local(lo) (batch_engine_v7.hpp:849-961)
+//   6. sweep     k_esweep        (bw_esweep.cu; forests and most trees), k_qcarry and
+//                                k_qsweep (bw_qsweep.cu; trees asked many queries a
+//                                state) or, by a forest's tuning and where scratch is
+//                                short, k_sweep below: persistent CTAs take blocks from
+//                                a queue and replay each from a zero local prefix
+//                                structure in shared memory; answer = carry(hi) -
+//                                carry(lo) + local(hi) - local(lo)
+//                                (batch_engine_v7.hpp:849-961)
 //
 // All arithmetic is int64 with two's-complement wrap (done in uint64), so any
 // summation order gives the reference's bits.

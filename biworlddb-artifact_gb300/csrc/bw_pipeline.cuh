@@ -217,7 +217,7 @@ __host__ __device__ inline SweepLayout sweep_layout(int32_t nwords, size_t budge
   return L;
 }
 
-// Window of the query-step sweep (bw_qsweep.cu): runs of 512 ranks that fit beside a
+// Window of the query-step sweep (bw_qsweep.cu): runs of 2,048 int32 ranks that fit beside a
 // rank table of `ww` words, and the rank capacities the prepare pass cuts slices with.
 struct QsLayout {
   int32_t ww = 0;
@@ -233,7 +233,7 @@ struct Tuning {
   int32_t ctas_per_sm = 0;  // persistent sweep CTAs per SM (1 or 2); 0 = auto
   int32_t slice_ranks = 0;  // cap on the ranks of one LUT slice (0 = all that fit shared memory)
   int32_t contract = -1;    // 1 / 0: contracted tour or not (-1: by the queries per state)
-  int32_t tile = 0;         // sweep tile geometry: kTileNarrowId, kTileWideId, 0 = by query/event ratio
+  int32_t tile = 0;         // sweep tile geometry: kTileNarrowId .. kTileEulerId, 0 = the default (finish_spec)
 };
 
 // Everything the enqueue needs that does not depend on the data.  Built on the

@@ -3,19 +3,19 @@
 //
 // A block's Euler steps are replayed one at a time by all 512 threads: thread i applies
 // event i of the step; at a step with queries threads 2i and 2i + 1 take the lower and
-// upper bound of query i.  The window over the block's key ranks (shared memory) holds
-// plain values, totals of 16 ranks (both by no-return atomics) and, rebuilt by sixteen
-// warp scans before a query step that follows updates, the prefixes of the totals inside
-// every 512 ranks; a warp scans the totals of the 512s itself.  A probe is one prefix,
-// one shuffle and at most four 128-bit reads of values -- per thread, so a step's queries
-// cost a few hundred cycles together, however many they are up to 256.
+// upper bound of query i (further ones, past 256, four at a time).  The window over the block's
+// key ranks (shared memory) holds Fenwick nodes inside groups of 16 ranks and the groups' totals
+// (an update is up to five no-return atomics) and, rebuilt by a warp a run before a query step that
+// follows updates, the prefixes of the totals inside every run of 2,048 ranks; a warp scans the
+// totals of the runs itself.  A probe is one prefix, one shuffle and up to four nodes -- per
+// thread, so a step's queries cost a few hundred cycles together, however many they are up to 256.
 //
 // The carried part of every answer is written beforehand by k_qcarry, a block's queries
 // side by side over its carry row (random reads of one 512 KB row at a time stay in the
 // L2; inside the sweep 304 rows were read at once); the sweep adds the window's part with
 // a no-return atomic.  A thread's event and bound of a step are copied into shared-memory
-// slots of its own three steps ahead (cp.async: register loads four steps ahead shared
-// their scoreboards with the step's own shared-memory reads and cost a memory latency a
+// slots of its own three steps ahead, two with int64 windows (cp.async: register loads four steps
+// ahead shared their scoreboards with the step's own shared-memory reads and cost a memory latency a
 // step), the step descriptors through a ring.
 //
 // Bound by the latency of the three barriers of a query step, two CTAs an SM to overlap

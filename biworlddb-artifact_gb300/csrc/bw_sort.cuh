@@ -90,7 +90,7 @@ __global__ void __launch_bounds__(kRsThreads) k_rs_hist(IO io, int64_t n, int sh
 
 // Counts -> starts: base[chunk][d] = items of smaller digits + those of earlier chunks,
 // hist[tile][d] = those of the chunk's earlier tiles.  Every chunk's CTA sums all chunks,
-// four groups of threads a quarter each (one group took 27 us for 256 chunks), and the
+// four groups of threads a quarter each (one group took 27 us for twice as many chunks), and the
 // groups take a quarter of the chunk's tiles each (one group took 21 us for 38 tiles a chunk,
 // four 9.5, and 12.5 for 76).
 __global__ void __launch_bounds__(4 * kRsDigits) k_rs_start(uint32_t* hist, const uint32_t* part, int64_t tiles,
