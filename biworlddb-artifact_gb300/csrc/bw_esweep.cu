@@ -72,7 +72,7 @@ constexpr uint32_t kEsDeep = 4096;
 // tile of their own, answered a thread per query (es_more).  As tiles of 60 queries they took 2.3 us
 // each: 30,000 states, 1M events, 360,000 queries, half of them on one state 7.36 -> 0.99 ms a replay (256
 // threads and Fenwick nodes, 1.18), 300,000 states, 3.6M queries 63.1 -> 5.1 (8.9).  A kernel of its own, as the
-// code for it cost the other tiles 3 to 8 % through their registers (1 % so, for the launch).
+// code for it cost the other tiles 3 to 8 % through their registers (some 2.5 us so, for the launch).
 constexpr int kEsMore = kHotQueries - 60;
 constexpr int kEsRing = 256;               // planner's descriptor ring (steps)
 constexpr uint32_t kEsWaitLimit = 1u << 22;

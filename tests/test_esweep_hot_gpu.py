@@ -1,6 +1,6 @@
 """GPU parity of the Euler-tile sweep where a state is asked much more than the others: steps of
 60 queries and some (a tile's), 256 and some past it (a tile of their own), with events before,
-behind and without, one block and many, dense windows, rank slices, forests."""
+behind and without, one block and many, dense windows, rank slices, forests, captured launches."""
 from __future__ import annotations
 
 import numpy as np
@@ -60,3 +60,22 @@ def test_forest_of_hot_states(bw, torch_cuda, oracle_mod, big):
     p, e, q = evgen.to_device(torch_cuda, *(np.concatenate(x) for x in zip(*parts)))
     got = bw.forest_replay(so, eo, qo, keys, p, e, q).cpu().numpy()
     np.testing.assert_array_equal(got, np.concatenate(want))
+
+
+def test_captured_launch(bw, torch_cuda, oracle_mod):
+    """A captured launch replays on new inputs: first without a state asked much, then with."""
+    torch = torch_cuda
+    S, C, E, Q = 4000, 3000, 60_000, 30_000
+    plain, hot = _case(S, C, E, Q, "fork", None, False, 1), _case(S, C, E, Q, "fork", "several", False, 1)
+    p, e, q = evgen.to_device(torch, *plain)
+    f, s = bw.Forest([0, S], [0, E], [0, Q], [C]), torch.cuda.Stream()
+    out = torch.empty(Q, dtype=torch.int64, device="cuda")
+    f.capture(p, e, q, out, s)
+    for parent, ev, qs in (plain, hot, plain):
+        for dst, src in zip((p, e, q), evgen.to_device(torch, parent, ev, qs)):
+            dst.copy_(src)
+        out.fill_(-1)
+        torch.cuda.synchronize()
+        f.replay(s)
+        assert f.status(s) == 0
+        np.testing.assert_array_equal(out.cpu().numpy(), oracle_mod.ev_sweep(parent, C, ev, qs))
